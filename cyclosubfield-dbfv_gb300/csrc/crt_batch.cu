@@ -1,0 +1,68 @@
+// Launches of the batched-transform kernel, and its form for slabs of any shape.
+#include <algorithm>
+
+#include "crt_batch.cuh"
+
+namespace hc {
+
+CrtBatchKernel crt_batch_f36864(int ctas_per_sm);
+CrtBatchKernel crt_batch_f49152(int ctas_per_sm);
+CrtBatchKernel crt_batch_mixed(int ctas_per_sm);
+
+/// Shared-memory words a slab of the batched transform needs: a padded 3072-residue line, one padded
+/// 4096-residue block of a 12288-residue line (line12288_seq), or the generic tile (the whole line,
+/// or deg_L' x 2^logv dimension-2 columns); the specialised column passes use none.
+size_t crt_slab_tile_words(int32_t shapes, int32_t dl, int32_t dk, int logv) {
+    const int s3 = shapes & 0xff, s2 = (shapes >> 8) & 0xff;
+    const bool f3 = (shapes >> 16) & 1, f2 = (shapes >> 17) & 1;
+    const size_t w3 = !f3 ? (size_t)dk
+                          : s3 == HC_SHAPE_L3072 ? (size_t)line_tile_words(HC_SHAPE_L3072)
+                          : s3 == HC_SHAPE_L12288 ? (size_t)(4096 + 4096 / 8) : (size_t)dk;
+    const size_t w2 = f2 && (s2 == HC_SHAPE_C12 || s2 == HC_SHAPE_C4) ? 0 : ((size_t)dl << logv);
+    const size_t w = std::max(w3, w2);
+    return (w + 1) & ~(size_t)1;
+}
+
+/// Whether a slab runs entirely on the specialised line and column code (crt_batch_kernel<false>).
+bool crt_slab_specialised(int32_t shapes) {
+    const int s3 = shapes & 0xff, s2 = (shapes >> 8) & 0xff;
+    return ((shapes >> 16) & 1) && (s3 == HC_SHAPE_L3072 || s3 == HC_SHAPE_L12288) && ((shapes >> 17) & 1) &&
+           (s2 == HC_SHAPE_C12 || s2 == HC_SHAPE_C4);
+}
+
+/// Shape class of specialised slab shapes (crt_batch_kernel's CLS): 1 field_36864, 2 field_49152
+/// (CLS 0: a launch over both).
+int crt_slab_kernel_class(int32_t shapes) { return (shapes & 0xff) == HC_SHAPE_L3072 ? 1 : 2; }
+
+/// Launches the persistent batched-transform kernel over `nslabs` device slab descriptors.
+/// `tile_words`: largest tile (deg_K, or deg_L' x 2^logv); `tw_words`: largest pair of twiddle
+/// tables (dimension-2 + dimension-3 plan) of a slab. `counter` is reset on the stream first.
+hc_status launch_crt_batch(hc_context ctx, const CrtSlab* slabs, int nslabs, int* counter, size_t tile_words,
+                           size_t tw_words, const CrtLaunch& L, bool generic, int cls) {
+    if (nslabs <= 0) return HC_OK;
+    CrtBatchKernel kern = generic    ? crt_batch_kernel<true, 0, 256, 2>
+                          : cls == 1 ? crt_batch_f36864(L.ctas_per_sm)
+                          : cls == 2 ? crt_batch_f49152(L.ctas_per_sm)
+                                     : crt_batch_mixed(L.ctas_per_sm);
+    if (L.threads < 32 || L.threads > 256 || L.threads % 32) return fail(HC_ERR_ARG, "batched transform: threads per CTA");
+    if (L.logv < 0 || L.logv > 6) return fail(HC_ERR_ARG, "batched transform: dimension-2 tile width");
+    const size_t smem = (tile_words + (generic ? tw_words : 0)) * 8;
+    if (smem > max_smem_optin(ctx)) return fail(HC_ERR_UNSUPPORTED, "batched transform: slab tiles exceed shared memory");
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_check(e, "batched transform smem attribute");
+    int occ = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, L.threads, smem);
+    if (e != cudaSuccess) return cuda_check(e, "batched transform occupancy");
+    if (occ < 1) return fail(HC_ERR_UNSUPPORTED, "batched transform: launch shape does not fit an SM");
+    int per = L.ctas_per_sm < 1 ? 1 : (L.ctas_per_sm < occ ? L.ctas_per_sm : occ);
+    int64_t grid = (int64_t)num_sms(ctx) * per;
+    if (grid > nslabs) grid = nslabs;
+    hc_status st = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), stream_of(ctx)), "batched transform counter");
+    if (st) return st;
+    kern<<<(unsigned)grid, (unsigned)L.threads, smem, stream_of(ctx)>>>(slabs, nslabs, counter, L.logv,
+                                                                      (int)tile_words);
+    count_launch(ctx);
+    return cuda_check(cudaGetLastError(), "batched transform launch");
+}
+
+}  // namespace hc

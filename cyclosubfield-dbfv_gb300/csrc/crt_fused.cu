@@ -56,8 +56,8 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 /// src/hal/ntt.rs:338-349, :465-476). Two warps share a column, one per h, so that each keeps
 /// six of the twelve values of a [4, 3] column (or of three [4] columns) in registers; the
 /// duplicated work is the four-point factor's one Barrett product per column.
-template <bool INV>
-__device__ __forceinline__ void four_half(const fast::Ctx& c, const fast::SF& f0, const fast::SF& f1, int h,
+template <bool INV, class CTX>
+__device__ __forceinline__ void four_half(const CTX& c, const fast::SF& f0, const fast::SF& f1, int h,
                                           int64_t x0, int64_t x1, int64_t x2, int64_t x3, int64_t& o0, int64_t& o1) {
     if (f0.red) {
         x0 = fast::red1(c, x0), x1 = fast::red1(c, x1), x2 = fast::red1(c, x2), x3 = fast::red1(c, x3);
@@ -66,68 +66,52 @@ __device__ __forceinline__ void four_half(const fast::Ctx& c, const fast::SF& f0
         // stage 0 (length 4, block 0): pairs (0, 2), (1, 3)
         int64_t t02 = x2, t13 = x3;
         if (!f0.skip_ok) {
-            int64_t z, u;
-            fast::twl(c, f0.tw_off, z, u);
-            t02 = bmul(z, u, x2, c.n), t13 = bmul(z, u, x3, c.n);
+            const auto w = c.get(f0.tw_off);
+            t02 = c.mul(w, x2), t13 = c.mul(w, x3);
         }
         int64_t p = h ? wsub(x0, t02) : wadd(x0, t02), q = h ? wsub(x1, t13) : wadd(x1, t13);
         if (f1.red) p = fast::red1(c, p), q = fast::red1(c, q);
         // stage 1 (length 2): block 0 = rows (0, 1), block 1 = rows (2, 3)
         int64_t t = q;
         if (h) {
-            int64_t z, u;
-            fast::twl(c, f1.tw_off + 1, z, u);
-            t = bmul(z, u, q, c.n);
+            t = c.mul(c.get(f1.tw_off + 1), q);
         } else if (!f1.skip_ok) {
-            int64_t z, u;
-            fast::twl(c, f1.tw_off, z, u);
-            t = bmul(z, u, q, c.n);
+            t = c.mul(c.get(f1.tw_off), q);
         }
         o0 = wadd(p, t), o1 = wsub(p, t);
     } else {
         // stage 0 (length 2): block 0 = (0, 1), block 1 = (2, 3)
         int64_t y0 = wadd(x0, x1), y1 = wsub(x0, x1), y2 = wadd(x2, x3), y3 = wsub(x2, x3);
         if (f0.last) {
-            y0 = bmul(c.il_z, c.il_u, y0, c.n), y1 = bmul(c.il_z, c.il_u, y1, c.n);
-            y2 = bmul(c.il_z, c.il_u, y2, c.n), y3 = bmul(c.il_z, c.il_u, y3, c.n);
+            y0 = c.scale(y0), y1 = c.scale(y1);
+            y2 = c.scale(y2), y3 = c.scale(y3);
         } else {
-            int64_t z, u;
-            fast::twl(c, f0.tw_off + 1, z, u);
-            if (z != 1) y3 = bmul(z, u, y3, c.n);
+            y3 = c.mul(c.get(f0.tw_off + 1), y3);  // block 1's twiddle, never 1
         }
         if (f1.red) {
             y0 = fast::red1(c, y0), y1 = fast::red1(c, y1), y2 = fast::red1(c, y2), y3 = fast::red1(c, y3);
         }
         // stage 1 (length 4): pairs (0, 2), (1, 3)
         o0 = h ? wsub(y0, y2) : wadd(y0, y2), o1 = h ? wsub(y1, y3) : wadd(y1, y3);
-        if (f1.last) o0 = bmul(c.il_z, c.il_u, o0, c.n), o1 = bmul(c.il_z, c.il_u, o1, c.n);
+        if (f1.last) o0 = c.scale(o0), o1 = c.scale(o1);
     }
 }
 
-/// Fused pass of a field_49152 slab: CTA 3k + b of the cluster owns block b of row k.
-template <int DIR, bool POST>
-__global__ void __launch_bounds__(THREADS, 6)
-    crt_slab12288_kernel(KView t, KView src, PlanPtrs p2, PlanPtrs p3, KView m2, KView m3, KMods mods, int reverse) {
-    extern __shared__ int64_t smem[];
-    cg::cluster_group cluster = cg::this_cluster();
+/// Both phases of one half for the schedules of primes just below 2^LG; the CTA's block is left in its
+/// shared memory. The caller has arrived at the cluster barrier (cluster_arrive_relaxed).
+template <int DIR, int LG>
+__device__ __forceinline__ void slab12288_half(int64_t* smem, cg::cluster_group& cluster, const KView& t, const KView& src,
+                                               const DevPlanHeader* P2, const DevPlanHeader* P3, const KView& m2,
+                                               const fast::MontL& mont, int64_t i, int64_t j) {
     const int rank = (int)cluster.block_rank();
-    const int row = rank / 3, blk = rank - 3 * (rank / 3);
-    // reverse: the last slab first, so that the clusters scheduled first read what the producer
-    // of the input (or the other half of the transform) wrote last, still in L2
-    const int64_t slab = reverse ? gridDim.x / CLUSTER - 1 - blockIdx.x / CLUSTER : blockIdx.x / CLUSTER;
-    const int64_t j = slab % t.n1, i = slab / t.n1;
-    const DevPlanHeader* P2 = p2.p[j];
-    const DevPlanHeader* P3 = p3.p[j];
-    const int64_t n = mods.n[j], ninv = mods.ninv[j];
     constexpr bool inv = DIR == 1;
-    const fast::Ctx c3 = make_ctx(P3, reinterpret_cast<const int64_t*>(P3 + 1));
-    const FixedSched<HC_SHAPE_L12288, inv> sch3{inv ? P3->inv : P3->fwd};
-    cluster_arrive_relaxed();
+    const fast::CtxL c3 = make_ctx<fast::CtxL>(P3);
+    const FixedSched<HC_SHAPE_L12288, LG, inv> sch3{inv ? P3->inv : P3->fwd};
     // ---- phase 1: positions p, p + 4096, p + 8192 of the four rows, over the cluster's threads;
     // warp w keeps rows 2h, 2h + 1 (h = w & 1) of 64 positions per CTA and step
     {
-        const fast::Ctx c2 = make_ctx(P2, reinterpret_cast<const int64_t*>(P2 + 1));
-        const FixedSched<HC_SHAPE_C4, inv> sch2{inv ? P2->inv : P2->fwd};
+        const fast::CtxL c2 = make_ctx<fast::CtxL>(P2);
+        const FixedSched<HC_SHAPE_C4, LG, inv> sch2{inv ? P2->inv : P2->fwd};
         const fast::SF f0 = fast::sflags(sch2, 0), f1 = fast::sflags(sch2, 1);
         const fast::SF f30 = fast::sflags(sch3, 0);
         const int warp = threadIdx.x >> 5, h = warp & 1;
@@ -143,7 +127,7 @@ __global__ void __launch_bounds__(THREADS, 6)
             for (int b = 0; b < 3; b++) {
                 const int64_t* col = gs + 4096 * b + p;
                 four_half<inv>(c2, f0, f1, h, col[0], col[src.s2], col[2 * src.s2], col[3 * src.s2], y[0][b], y[1][b]);
-                if (DIR == 0) y[0][b] = mul_mont(y[0][b], m2a, n, ninv), y[1][b] = mul_mont(y[1][b], m2b, n, ninv);
+                if (DIR == 0) y[0][b] = mont.mul(y[0][b], m2a), y[1][b] = mont.mul(y[1][b], m2b);
             }
 #pragma unroll
             for (int a = 0; a < 2; a++) {
@@ -180,6 +164,26 @@ __global__ void __launch_bounds__(THREADS, 6)
         __syncthreads();
         fast::r2_pass<true, 3, 3, 6, 0>(c3, smem, 512, sch3, 10, false);   // factor 64 (b): 8, 16, 32
     }
+}
+
+/// Fused pass of a field_49152 slab: CTA 3k + b of the cluster owns block b of row k.
+template <int DIR, bool POST>
+__global__ void __launch_bounds__(THREADS, 6)
+    crt_slab12288_kernel(KView t, KView src, PlanPtrs p2, PlanPtrs p3, KView m2, KView m3, KMods mods, int reverse) {
+    extern __shared__ int64_t smem[];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int row = rank / 3, blk = rank - 3 * (rank / 3);
+    // reverse: the last slab first, so that the clusters scheduled first read what the producer
+    // of the input (or the other half of the transform) wrote last, still in L2
+    const int64_t slab = reverse ? gridDim.x / CLUSTER - 1 - blockIdx.x / CLUSTER : blockIdx.x / CLUSTER;
+    const int64_t j = slab % t.n1, i = slab / t.n1;
+    const DevPlanHeader* P2 = p2.p[j];
+    const DevPlanHeader* P3 = p3.p[j];
+    const fast::MontL mont = fast::make_mont<fast::CtxL>(mods.n[j], mods.ninv[j]);
+    cluster_arrive_relaxed();
+    if (P3->cls == 57) slab12288_half<DIR, 57>(smem, cluster, t, src, P2, P3, m2, mont, i, j);
+    else slab12288_half<DIR, 56>(smem, cluster, t, src, P2, P3, m2, mont, i, j);
     __syncthreads();
     int64_t* g = reinterpret_cast<int64_t*>(t.p) + i * t.s0 + j * t.s1 + row * t.s2 + 4096 * blk;
     const int64_t* mulp = nullptr;
@@ -188,7 +192,7 @@ __global__ void __launch_bounds__(THREADS, 6)
         me = m3.b3 ? 0 : 1;
         mulp = kat<int64_t>(m3, i, j, row, 0) + (me ? 4096 * blk : 0);
     }
-    fast::line_store(smem, g, 4096, DIR == 0 || POST, mulp, me, n, ninv);
+    fast::line_store(smem, g, 4096, DIR == 0 || POST, mulp, me, mont);
 }
 
 template <class K>

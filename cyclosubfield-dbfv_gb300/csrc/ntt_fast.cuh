@@ -26,15 +26,33 @@ __device__ __forceinline__ int pad8(int i) { return i + (i >> 3); }
 /// group geometries used here: span a multiple of 8, or span < 8 with the base's low bits < span).
 __host__ __device__ constexpr int goff(int m, int span) { return m * span + ((m * span) >> 3); }
 
+/// Products of a plan with any schedule and modulus: (z, u) pairs.
 struct Ctx {
-    int64_t n, one_z, one_u, il_z, il_u;
-    const int64_t* tw;  // staged twiddle pairs
+    static constexpr bool LIMBS = false;
+    int64_t n, one_u, il_z, il_u;
+    const int64_t* tw;  // twiddle pairs
+    typedef longlong2 Tw;
+    __device__ __forceinline__ Tw get(int idx) const { return reinterpret_cast<const longlong2*>(tw)[idx]; }
+    __device__ __forceinline__ int64_t mul(const Tw& w, int64_t x) const { return bmul(w.x, w.y, x, n); }
+    __device__ __forceinline__ int64_t scale(int64_t x) const { return bmul(il_z, il_u, x, n); }
+    __device__ __forceinline__ int64_t red(int64_t x) const { return bmul1(one_u, x, n); }
 };
 
-__device__ __forceinline__ void twl(const Ctx& c, int idx, int64_t& z, int64_t& u) {
-    const longlong2 w = reinterpret_cast<const longlong2*>(c.tw)[idx];
-    z = w.x, u = w.y;
-}
+/// The same products in limbs (barrett_mul), for the plans with the compiled-in schedules.
+struct CtxL {
+    static constexpr bool LIMBS = true;
+    BarrettMod m;
+    BarrettLimbs il;
+    const int4* tw;  // twiddles (BarrettLimbs)
+    typedef BarrettLimbs Tw;
+    __device__ __forceinline__ Tw get(int idx) const {
+        const int4 a = __ldg(tw + idx);
+        return BarrettLimbs{a.x, a.y, a.z, a.w};
+    }
+    __device__ __forceinline__ int64_t mul(const Tw& w, int64_t x) const { return barrett_mul(w, x, m); }
+    __device__ __forceinline__ int64_t scale(int64_t x) const { return barrett_mul(il, x, m); }
+    __device__ __forceinline__ int64_t red(int64_t x) const { return barrett_red(x, m); }
+};
 
 /// Stage flags of the program, read once per pass (uniform).
 struct SF {
@@ -67,27 +85,24 @@ __device__ __forceinline__ SF sflags(const SCH& sch, int s) {
     return f;
 }
 
-__device__ __forceinline__ int64_t red1(const Ctx& c, int64_t x) { return bmul1(c.one_u, x, c.n); }
+template <class CTX>
+__device__ __forceinline__ int64_t red1(const CTX& c, int64_t x) { return c.red(x); }
 
 // ---------------------------------------------------------------- butterflies
 
 /// Forward radix-2 butterfly of block `tb` (src/hal/ntt.rs:338-349). UNIFORM0: the block is 0
 /// for the whole warp, so a permitted skip avoids the product.
-template <bool UNIFORM0>
-__device__ __forceinline__ void fwd2(const Ctx& c, const SF& f, bool fuse, int tb, int64_t& x, int64_t& y) {
+template <bool UNIFORM0, class CTX>
+__device__ __forceinline__ void fwd2(const CTX& c, const SF& f, bool fuse, int tb, int64_t& x, int64_t& y) {
     int64_t t;
     if (UNIFORM0) {
         if (f.skip_ok) {
             t = y;
         } else {
-            int64_t z, u;
-            twl(c, f.tw_off, z, u);
-            t = bmul(z, u, y, c.n);
+            t = c.mul(c.get(f.tw_off), y);
         }
     } else {
-        int64_t z, u;
-        twl(c, f.tw_off + tb, z, u);
-        t = bmul(z, u, y, c.n);
+        t = c.mul(c.get(f.tw_off + tb), y);
         if (f.skip_ok && tb == 0) t = y;
     }
     int64_t o0 = wadd(x, t), o1 = wsub(x, t);
@@ -100,31 +115,20 @@ __device__ __forceinline__ void fwd2(const Ctx& c, const SF& f, bool fuse, int t
 }
 
 /// Forward radix-3 butterfly of block `blk` (src/hal/ntt.rs:386-406).
-template <bool UNIFORM0>
-__device__ __forceinline__ void fwd3(const Ctx& c, const SF& f, bool fuse, int blk, int64_t& a, int64_t& b,
+template <bool UNIFORM0, class CTX>
+__device__ __forceinline__ void fwd3(const CTX& c, const SF& f, bool fuse, int blk, int64_t& a, int64_t& b,
                                      int64_t& d) {
     const int base = f.tw_off + 6 * blk;
-    int64_t w0z, w0u, w1z, w1u, w2z, w2u, w3z, w3u, w4z, w4u, w5z, w5u;
-    twl(c, base + 1, w1z, w1u);
-    twl(c, base + 2, w2z, w2u);
-    twl(c, base + 4, w4z, w4u);
-    twl(c, base + 5, w5z, w5u);
     int64_t t_b, t_c;
-    if (UNIFORM0 && f.skip_ok) {
+    if (f.skip_ok && blk == 0) {  // block 0's twiddle is 1
         t_b = b;
         t_c = d;
     } else {
-        twl(c, base, w0z, w0u);
-        twl(c, base + 3, w3z, w3u);
-        t_b = bmul(w0z, w0u, b, c.n);
-        t_c = bmul(w3z, w3u, d, c.n);
-        if (!UNIFORM0 && f.skip_ok && w0z == 1) {
-            t_b = b;
-            t_c = d;
-        }
+        t_b = c.mul(c.get(base), b);
+        t_c = c.mul(c.get(base + 3), d);
     }
-    const int64_t t_bz = bmul(w1z, w1u, b, c.n), t_bzz = bmul(w2z, w2u, b, c.n);
-    const int64_t t_cz = bmul(w4z, w4u, d, c.n), t_czz = bmul(w5z, w5u, d, c.n);
+    const int64_t t_bz = c.mul(c.get(base + 1), b), t_bzz = c.mul(c.get(base + 2), b);
+    const int64_t t_cz = c.mul(c.get(base + 4), d), t_czz = c.mul(c.get(base + 5), d);
     int64_t o0 = wadd(wadd(a, t_b), t_c), o1 = wadd(wadd(a, t_bz), t_czz), o2 = wadd(wadd(a, t_bzz), t_cz);
     if (fuse) {
         o0 = red1(c, o0);
@@ -140,18 +144,16 @@ __device__ __forceinline__ void fwd3(const Ctx& c, const SF& f, bool fuse, int b
 /// of the specialised shapes is the single stage of a factor of length 3: it has one block, whose
 /// twiddles are v^0 = 1, so the reference's twiddle-1 skip always applies and the outputs take
 /// no block-twiddle product (only the fused len^-1 scaling when the stage is the last one).
-__device__ __forceinline__ void inv3(const Ctx& c, const SF& f, int64_t& a, int64_t& b, int64_t& d) {
-    int64_t zz0, zu0, zz1, zu1;
-    twl(c, f.zeta_off, zz0, zu0);
-    twl(c, f.zeta_off + 1, zz1, zu1);
-    const int64_t y1z = bmul(zz0, zu0, b, c.n), y1zz = bmul(zz1, zu1, b, c.n);
-    const int64_t y2z = bmul(zz0, zu0, d, c.n), y2zz = bmul(zz1, zu1, d, c.n);
+template <class CTX>
+__device__ __forceinline__ void inv3(const CTX& c, const SF& f, int64_t& a, int64_t& b, int64_t& d) {
+    const auto w1 = c.get(f.zeta_off), w2 = c.get(f.zeta_off + 1);
+    const int64_t y1z = c.mul(w1, b), y1zz = c.mul(w2, b), y2z = c.mul(w1, d), y2zz = c.mul(w2, d);
     const int64_t s0 = wadd(wadd(a, b), d);
     const int64_t sy = wadd(wadd(a, y1zz), y2z), sz = wadd(wadd(a, y1z), y2zz);
     if (f.last) {
-        a = bmul(c.il_z, c.il_u, s0, c.n);
-        b = bmul(c.il_z, c.il_u, sy, c.n);
-        d = bmul(c.il_z, c.il_u, sz, c.n);
+        a = c.scale(s0);
+        b = c.scale(sy);
+        d = c.scale(sz);
         return;
     }
     a = s0;
@@ -163,8 +165,8 @@ __device__ __forceinline__ void inv3(const Ctx& c, const SF& f, int64_t& a, int6
 
 /// K forward radix-2 stages on the group x[0..2^K) (element m at distance m * span). block0:
 /// the group's twiddle block at the first stage (0 for the whole warp when NB0 == 1).
-template <int K, bool NB1>
-__device__ __forceinline__ void fwd_group(const Ctx& c, const SF* f, const bool* fuse, int block0, int64_t* x) {
+template <int K, bool NB1, class CTX>
+__device__ __forceinline__ void fwd_group(const CTX& c, const SF* f, const bool* fuse, int block0, int64_t* x) {
     constexpr int M = 1 << K;
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -185,8 +187,8 @@ __device__ __forceinline__ void fwd_group(const Ctx& c, const SF* f, const bool*
 
 /// K inverse radix-2 stages (distances growing) on the group x[0..2^K); blockK: the group's block
 /// at the pass's last stage (NBK1: 0 for the whole warp).
-template <int K, bool NBK1>
-__device__ __forceinline__ void inv_group(const Ctx& c, const SF* f, int blockK, int64_t* x) {
+template <int K, bool NBK1, class CTX>
+__device__ __forceinline__ void inv_group(const CTX& c, const SF* f, int blockK, int64_t* x) {
     constexpr int M = 1 << K;
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -201,18 +203,16 @@ __device__ __forceinline__ void inv_group(const Ctx& c, const SF* f, int blockK,
             const int tbc = m1 >> (q + 1);
             const int64_t sum = wadd(x[m1], x[m2]), dif = wsub(x[m1], x[m2]);
             if (f[q].last) {
-                x[m1] = bmul(c.il_z, c.il_u, sum, c.n);
-                x[m2] = bmul(c.il_z, c.il_u, dif, c.n);
+                x[m1] = c.scale(sum);
+                x[m2] = c.scale(dif);
             } else if (NBK1 && tbc == 0) {
                 // block 0 for the whole warp: twiddle 1, product skipped
                 x[m1] = sum;
                 x[m2] = dif;
             } else {
                 const int tb = (blockK << (K - 1 - q)) + tbc;
-                int64_t z, u;
-                twl(c, f[q].tw_off + tb, z, u);
-                int64_t t = bmul(z, u, dif, c.n);
-                if (z == 1) t = dif;
+                int64_t t = c.mul(c.get(f[q].tw_off + tb), dif);
+                if (tbc == 0 && tb == 0) t = dif;  // block 0's twiddle is 1, no other block's is
                 x[m1] = sum;
                 x[m2] = t;
             }
@@ -223,8 +223,8 @@ __device__ __forceinline__ void inv_group(const Ctx& c, const SF* f, int blockK,
 /// One pass of K radix-2 stages of a factor over a padded shared-memory tile: groups of 2^K
 /// elements at distance SPAN (= 2^LOG_SPAN) inside blocks of 2^LOG_GLEN elements, 2^LOG_NB twiddle
 /// blocks per factor at the pass's reference stage (first stage forward, last stage inverse).
-template <bool INV, int K, int LOG_SPAN, int LOG_GLEN, int LOG_NB, class SCH>
-__device__ __forceinline__ void r2_pass(const Ctx& c, int64_t* s, int ngroups, const SCH& sch, int s0,
+template <bool INV, int K, int LOG_SPAN, int LOG_GLEN, int LOG_NB, class SCH, class CTX>
+__device__ __forceinline__ void r2_pass(const CTX& c, int64_t* s, int ngroups, const SCH& sch, int s0,
                                         bool reduce_output) {
     constexpr int M = 1 << K, SPAN = 1 << LOG_SPAN;
     SF f[K];
@@ -251,21 +251,38 @@ __device__ __forceinline__ void r2_pass(const Ctx& c, int64_t* s, int ngroups, c
 
 // ---------------------------------------------------------------- lines
 
+/// The Montgomery product of modes 2 and 3: mul_mont for any modulus, its limb form beside the limb
+/// Barrett products.
+struct Mont {
+    int64_t n, ninv;
+    __device__ __forceinline__ int64_t mul(int64_t a, int64_t b) const { return mul_mont(a, b, n, ninv); }
+};
+struct MontL {
+    MontLimbs m;
+    __device__ __forceinline__ int64_t mul(int64_t a, int64_t b) const { return mont_mul(a, b, m); }
+};
+template <class CTX>
+__device__ __forceinline__ auto make_mont(int64_t n, int64_t ninv) {
+    if constexpr (CTX::LIMBS) return MontL{mont_limbs(n, ninv)};
+    else return Mont{n, ninv};
+}
+
 /// Copies a padded tile of `len` elements to global memory, multiplying (mode 2/3) by
 /// mulp[e * me] in Montgomery form.
+template <class MONT>
 __device__ __forceinline__ void line_store(const int64_t* s, int64_t* g, int len, bool mul, const int64_t* mulp,
-                                           int64_t me, int64_t mn, int64_t mi) {
+                                           int64_t me, const MONT& mont) {
     for (int e = threadIdx.x; e < len; e += blockDim.x) {
         int64_t v = s[pad8(e)];
-        if (mul) v = mul_mont(v, mulp[e * me], mn, mi);
+        if (mul) v = mont.mul(v, mulp[e * me]);
         g[e] = v;
     }
 }
 
 /// Reduces every element of a register group when the stage asks for it (src/hal/ntt.rs: the
 /// reduction pass before a stage whose growth could overflow).
-template <int N>
-__device__ __forceinline__ void red_all(const Ctx& c, bool red, int64_t* x) {
+template <int N, class CTX>
+__device__ __forceinline__ void red_all(const CTX& c, bool red, int64_t* x) {
     if (red) {
 #pragma unroll
         for (int m = 0; m < N; m++) x[m] = red1(c, x[m]);
@@ -276,8 +293,8 @@ __device__ __forceinline__ void red_all(const Ctx& c, bool red, int64_t* x) {
 /// tile kernel (0 forward, 1 inverse, 2 forward + product, 3 inverse + product); the schedule
 /// SCH is that of the programme of MODE's direction. Stages: 0 = factor 2, 1 = factor 3,
 /// 2..4 = factor 8, 5..10 = factor 64.
-template <int MODE, class SCH>
-__device__ __forceinline__ void line3072(const SCH& sch, const Ctx& c, int64_t* s, int64_t* g, const int64_t* mulp,
+template <int MODE, class SCH, class CTX>
+__device__ __forceinline__ void line3072(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
                                          int64_t me, int64_t mn, int64_t mi) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     // pass 1: factors 2 (distance 1536) and 3 (distance 512), straight from global memory
@@ -303,8 +320,8 @@ __device__ __forceinline__ void line3072(const SCH& sch, const Ctx& c, int64_t* 
                     // factor 2: one block, twiddle 1 unless fused
                     const int64_t sum = wadd(x[0][a], x[1][a]), dif = wsub(x[0][a], x[1][a]);
                     if (f0.last) {
-                        x[0][a] = bmul(c.il_z, c.il_u, sum, c.n);
-                        x[1][a] = bmul(c.il_z, c.il_u, dif, c.n);
+                        x[0][a] = c.scale(sum);
+                        x[1][a] = c.scale(dif);
                     } else {
                         x[0][a] = sum;
                         x[1][a] = dif;
@@ -335,13 +352,13 @@ __device__ __forceinline__ void line3072(const SCH& sch, const Ctx& c, int64_t* 
         r2_pass<true, 3, 3, 6, 0>(c, s, 384, sch, 8, false);  // factor 64: 8, 16, 32
     }
     __syncthreads();
-    line_store(s, g, 3072, MODE & 2, mulp, me, mn, mi);
+    line_store(s, g, 3072, MODE & 2, mulp, me, make_mont<CTX>(mn, mi));
 }
 
 /// [3, 64, 64] line (12288 residues): stages 0 = factor 3 (distance 4096), 1..6 = first factor
 /// 64 (distances 2048 .. 64), 7..12 = second factor 64 (32 .. 1).
-template <int MODE, class SCH>
-__device__ __forceinline__ void line12288(const SCH& sch, const Ctx& c, int64_t* s, int64_t* g, const int64_t* mulp,
+template <int MODE, class SCH, class CTX>
+__device__ __forceinline__ void line12288(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
                                           int64_t me, int64_t mn, int64_t mi) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     // pass 1: factor 3 and three stages of the first factor 64, straight from global memory
@@ -396,7 +413,7 @@ __device__ __forceinline__ void line12288(const SCH& sch, const Ctx& c, int64_t*
         r2_pass<true, 3, 3, 6, 0>(c, s, 1536, sch, 10, false);  // factor 64 (b): 8, 16, 32
     }
     __syncthreads();
-    line_store(s, g, 12288, MODE & 2, mulp, me, mn, mi);
+    line_store(s, g, 12288, MODE & 2, mulp, me, make_mont<CTX>(mn, mi));
 }
 
 /// One of the three 4096-residue blocks of a [3, 64, 64] line, computed by one CTA of a 3-CTA
@@ -405,8 +422,8 @@ __device__ __forceinline__ void line12288(const SCH& sch, const Ctx& c, int64_t*
 /// positions and computes just its output; the remaining 12 stages act within the block. The
 /// line is transformed in place, so no CTA may store before all three have read their inputs:
 /// `cluster_sync` (a cluster-wide barrier) separates the first pass from the stores.
-template <int MODE, class SCH, class SYNC>
-__device__ __forceinline__ void line12288_block(const SCH& sch, const Ctx& c, int64_t* s, int64_t* g, int blk,
+template <int MODE, class SCH, class CTX, class SYNC>
+__device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, int blk,
                                                 const int64_t* mulp, int64_t me, int64_t mn, int64_t mi,
                                                 SYNC cluster_sync) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
@@ -420,15 +437,9 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const Ctx& c, in
         }
         // twiddles of the factor-3 stage (one block, whose block twiddles are 1: the inverse
         // outputs take no block-twiddle product, as inv3 explains)
-        int64_t wz0, wu0, wz1, wu1;  // forward: the two products of output blk; inverse: zeta, zeta^2
-        if (!inv) {
-            const int i0 = blk == 0 ? 0 : (blk == 1 ? 1 : 2), i1 = blk == 0 ? 3 : (blk == 1 ? 5 : 4);
-            twl(c, f[0].tw_off + i0, wz0, wu0);
-            twl(c, f[0].tw_off + i1, wz1, wu1);
-        } else {
-            twl(c, f[0].zeta_off, wz0, wu0);
-            twl(c, f[0].zeta_off + 1, wz1, wu1);
-        }
+        // forward: the two products of output blk; inverse: zeta, zeta^2
+        const int i0 = blk == 0 ? 0 : (blk == 1 ? 1 : 2), i1 = blk == 0 ? 3 : (blk == 1 ? 5 : 4);
+        const auto w0 = c.get(inv ? f[0].zeta_off : f[0].tw_off + i0), w1 = c.get(inv ? f[0].zeta_off + 1 : f[0].tw_off + i1);
         constexpr int span = inv ? 64 : 512;
         for (int gg = threadIdx.x; gg < 512; gg += blockDim.x) {
             const int base = inv ? ((gg >> 6) << 9) + (gg & 63) : gg;
@@ -450,8 +461,8 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const Ctx& c, in
                         tb = b;
                         tc = d;
                     } else {
-                        tb = bmul(wz0, wu0, b, c.n);
-                        tc = bmul(wz1, wu1, d, c.n);
+                        tb = c.mul(w0, b);
+                        tc = c.mul(w1, d);
                     }
                     o = wadd(wadd(a, tb), tc);
                     if (fz[0]) o = red1(c, o);
@@ -460,11 +471,11 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const Ctx& c, in
                     if (blk == 0) {
                         o = wadd(wadd(a, b), d);
                     } else if (blk == 1) {
-                        o = wadd(wadd(a, bmul(wz1, wu1, b, c.n)), bmul(wz0, wu0, d, c.n));
+                        o = wadd(wadd(a, c.mul(w1, b)), c.mul(w0, d));
                     } else {
-                        o = wadd(wadd(a, bmul(wz0, wu0, b, c.n)), bmul(wz1, wu1, d, c.n));
+                        o = wadd(wadd(a, c.mul(w0, b)), c.mul(w1, d));
                     }
-                    if (f[0].last) o = bmul(c.il_z, c.il_u, o, c.n);
+                    if (f[0].last) o = c.scale(o);
                 }
                 x[m] = o;
             }
@@ -489,7 +500,8 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const Ctx& c, in
         r2_pass<true, 3, 3, 6, 0>(c, s, 512, sch, 10, false);  // factor 64 (b): 8, 16, 32
     }
     __syncthreads();
-    line_store(s, g + 4096 * blk, 4096, MODE & 2, mulp + (me ? 4096 * blk : 0), me, mn, mi);
+    line_store(s, g + 4096 * blk, 4096, MODE & 2, mulp + (me ? 4096 * blk : 0), me,
+                   make_mont<CTX>(mn, mi));
 }
 
 /// A [3, 64, 64] line with a tile of one 4096-residue block (for kernels that cannot give a CTA the
@@ -498,8 +510,8 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const Ctx& c, in
 /// first pass); stages 1..12, which act within a block, then run block by block exactly as
 /// line12288_block runs them. The first pass's global writes are the CTA's own, visible to its
 /// threads after the barrier.
-template <int MODE, class SCH>
-__device__ __forceinline__ void line12288_seq(const SCH& sch, const Ctx& c, int64_t* s, int64_t* g,
+template <int MODE, class SCH, class CTX>
+__device__ __forceinline__ void line12288_seq(const SCH& sch, const CTX& c, int64_t* s, int64_t* g,
                                               const int64_t* mulp, int64_t me, int64_t mn, int64_t mi) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     SF f[4];
@@ -549,7 +561,8 @@ __device__ __forceinline__ void line12288_seq(const SCH& sch, const Ctx& c, int6
             r2_pass<true, 3, 3, 6, 0>(c, s, 512, sch, 10, false);  // factor 64 (b): 8, 16, 32
         }
         __syncthreads();
-        line_store(s, gb, 4096, MODE & 2, mulp + (me ? 4096 * blk : 0), me, mn, mi);
+        line_store(s, gb, 4096, MODE & 2, mulp + (me ? 4096 * blk : 0), me,
+                   make_mont<CTX>(mn, mi));
         __syncthreads();  // the tile is refilled by the next block
     }
 }
@@ -559,7 +572,8 @@ __device__ __forceinline__ void line12288_seq(const SCH& sch, const Ctx& c, int6
 /// [4, 3] column (12 residues at element stride ge): factor 4 (distance 3) then factor 3
 /// (distance 1). Forward stages: 0 = factor 4 length 4, 1 = factor 4 length 2, 2 = factor 3;
 /// inverse stages: 0 = factor 4 length 2, 1 = factor 4 length 4, 2 = factor 3.
-__device__ __forceinline__ void col12(const Ctx& c, const SF* f, bool inv, bool reduce_output, int64_t (&x)[4][3]) {
+template <class CTX>
+__device__ __forceinline__ void col12(const CTX& c, const SF* f, bool inv, bool reduce_output, int64_t (&x)[4][3]) {
     if (!inv) {
         if (f[0].red)
 #pragma unroll
@@ -580,9 +594,7 @@ __device__ __forceinline__ void col12(const Ctx& c, const SF* f, bool inv, bool 
         for (int b = 0; b < 3; b++) {
             fwd2<true>(c, f[1], z1, 0, x[0][b], x[1][b]);
             // block 1: an ordinary twiddle (not 1), product always taken
-            int64_t z, u;
-            twl(c, f[1].tw_off + 1, z, u);
-            const int64_t t = bmul(z, u, x[3][b], c.n);
+            const int64_t t = c.mul(c.get(f[1].tw_off + 1), x[3][b]);
             int64_t o0 = wadd(x[2][b], t), o1 = wsub(x[2][b], t);
             if (z1) {
                 o0 = red1(c, o0);
@@ -611,18 +623,14 @@ __device__ __forceinline__ void col12(const Ctx& c, const SF* f, bool inv, bool 
             for (int h = 0; h < 2; h++) {
                 const int64_t sum = wadd(x[2 * h][b], x[2 * h + 1][b]), dif = wsub(x[2 * h][b], x[2 * h + 1][b]);
                 if (f[0].last) {
-                    x[2 * h][b] = bmul(c.il_z, c.il_u, sum, c.n);
-                    x[2 * h + 1][b] = bmul(c.il_z, c.il_u, dif, c.n);
+                    x[2 * h][b] = c.scale(sum);
+                    x[2 * h + 1][b] = c.scale(dif);
                 } else if (h == 0) {
                     x[0][b] = sum;
                     x[1][b] = dif;
                 } else {
-                    int64_t z, u;
-                    twl(c, f[0].tw_off + 1, z, u);
-                    int64_t t = bmul(z, u, dif, c.n);
-                    if (z == 1) t = dif;
                     x[2][b] = sum;
-                    x[3][b] = t;
+                    x[3][b] = c.mul(c.get(f[0].tw_off + 1), dif);  // block 1's twiddle, never 1
                 }
             }
         }
@@ -637,8 +645,8 @@ __device__ __forceinline__ void col12(const Ctx& c, const SF* f, bool inv, bool 
             for (int b = 0; b < 3; b++) {
                 const int64_t sum = wadd(x[a][b], x[a + 2][b]), dif = wsub(x[a][b], x[a + 2][b]);
                 if (f[1].last) {
-                    x[a][b] = bmul(c.il_z, c.il_u, sum, c.n);
-                    x[a + 2][b] = bmul(c.il_z, c.il_u, dif, c.n);
+                    x[a][b] = c.scale(sum);
+                    x[a + 2][b] = c.scale(dif);
                 } else {
                     x[a][b] = sum;
                     x[a + 2][b] = dif;
@@ -655,7 +663,8 @@ __device__ __forceinline__ void col12(const Ctx& c, const SF* f, bool inv, bool 
 }
 
 /// [4] column (4 residues): forward stages 0 = length 4, 1 = length 2; inverse the reverse.
-__device__ __forceinline__ void col4(const Ctx& c, const SF* f, bool inv, bool reduce_output, int64_t (&x)[4]) {
+template <class CTX>
+__device__ __forceinline__ void col4(const CTX& c, const SF* f, bool inv, bool reduce_output, int64_t (&x)[4]) {
     if (!inv) {
         if (f[0].red)
 #pragma unroll
@@ -667,9 +676,7 @@ __device__ __forceinline__ void col4(const Ctx& c, const SF* f, bool inv, bool r
 #pragma unroll
             for (int a = 0; a < 4; a++) x[a] = red1(c, x[a]);
         fwd2<true>(c, f[1], z1, 0, x[0], x[1]);
-        int64_t z, u;
-        twl(c, f[1].tw_off + 1, z, u);
-        const int64_t t = bmul(z, u, x[3], c.n);
+        const int64_t t = c.mul(c.get(f[1].tw_off + 1), x[3]);
         int64_t o0 = wadd(x[2], t), o1 = wsub(x[2], t);
         if (z1) {
             o0 = red1(c, o0);
@@ -685,18 +692,14 @@ __device__ __forceinline__ void col4(const Ctx& c, const SF* f, bool inv, bool r
         for (int h = 0; h < 2; h++) {
             const int64_t sum = wadd(x[2 * h], x[2 * h + 1]), dif = wsub(x[2 * h], x[2 * h + 1]);
             if (f[0].last) {
-                x[2 * h] = bmul(c.il_z, c.il_u, sum, c.n);
-                x[2 * h + 1] = bmul(c.il_z, c.il_u, dif, c.n);
+                x[2 * h] = c.scale(sum);
+                x[2 * h + 1] = c.scale(dif);
             } else if (h == 0) {
                 x[0] = sum;
                 x[1] = dif;
             } else {
-                int64_t z, u;
-                twl(c, f[0].tw_off + 1, z, u);
-                int64_t t = bmul(z, u, dif, c.n);
-                if (z == 1) t = dif;
                 x[2] = sum;
-                x[3] = t;
+                x[3] = c.mul(c.get(f[0].tw_off + 1), dif);
             }
         }
         if (f[1].red)
@@ -706,8 +709,8 @@ __device__ __forceinline__ void col4(const Ctx& c, const SF* f, bool inv, bool r
         for (int a = 0; a < 2; a++) {
             const int64_t sum = wadd(x[a], x[a + 2]), dif = wsub(x[a], x[a + 2]);
             if (f[1].last) {
-                x[a] = bmul(c.il_z, c.il_u, sum, c.n);
-                x[a + 2] = bmul(c.il_z, c.il_u, dif, c.n);
+                x[a] = c.scale(sum);
+                x[a + 2] = c.scale(dif);
             } else {
                 x[a] = sum;
                 x[a + 2] = dif;

@@ -1,0 +1,64 @@
+// Dimension-3 lines of field_49152 ([3, 64, 64], 12288 residues): one line per 3-CTA cluster.
+#include <cooperative_groups.h>
+
+#include "ntt_run.cuh"
+
+namespace {
+
+/// [3, 64, 64] lines along dimension 3 as 3-CTA clusters: CTA `blk` of a cluster computes block
+/// blk (4096 residues) of one line.
+template <int MODE, bool FIX>
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(128, 6)
+    ntt_line3_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
+    extern __shared__ int64_t smem[];
+    const int64_t tile = blockIdx.x / 3;
+    const int blk = (int)(blockIdx.x % 3);
+    const int64_t k = tile % t.n2, r = tile / t.n2;
+    const int64_t j = r % t.n1, i = r / t.n1;
+    const DevPlanHeader* P = plans.p[j];
+    int64_t* g = reinterpret_cast<int64_t*>(t.p) + i * t.s0 + j * t.s1 + k * t.s2;
+    const int64_t* mulp = nullptr;
+    int64_t me = 0, mn = 0, mi = 0;
+    if (MODE & 2) {
+        mulp = kat<int64_t>(mul, i, j, k, 0);
+        me = mul.b3 ? 0 : 1;
+        mn = mods.n[j], mi = mods.ninv[j];
+    }
+    auto csync = [] { cooperative_groups::this_cluster().sync(); };
+    // twiddles are read from the plan in global memory (L1-cached): the CTA's shared memory holds
+    // only its 4096-residue block, so that six CTAs fit on an SM
+    const auto c = make_ctx<PassCtx<FIX>>(P);
+    with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, FIX>(
+        P, [&](const auto& sch) { fast::line12288_block<MODE>(sch, c, smem, g, blk, mulp, me, mn, mi, csync); });
+}
+
+template <int MODE, bool FIX>
+hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    // one 3-CTA cluster per line: a padded 4096-residue block per CTA
+    constexpr size_t smem = 4608 * 8;
+    auto kern = ntt_line3_kernel<MODE, FIX>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
+    if (tiles * 3 > 0x7fffffff) return hc::fail(HC_ERR_UNSUPPORTED, "too many NTT lines in one call");
+    kern<<<(unsigned)(tiles * 3), 128, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
+    hc::count_launch(ctx);
+    return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
+}
+
+template <bool FIX>
+hc_status launch_mode(hc_context ctx, int mode, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    if (mode == 0) return launch<0, FIX>(ctx, t, pp, mul, mods, tiles);
+    if (mode == 1) return launch<1, FIX>(ctx, t, pp, mul, mods, tiles);
+    if (mode == 2) return launch<2, FIX>(ctx, t, pp, mul, mods, tiles);
+    return launch<3, FIX>(ctx, t, pp, mul, mods, tiles);
+}
+
+}  // namespace
+
+namespace hc {
+
+hc_status launch_ntt_line12288(hc_context ctx, int mode, bool fix, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    return fix ? launch_mode<true>(ctx, mode, t, pp, mul, mods, tiles) : launch_mode<false>(ctx, mode, t, pp, mul, mods, tiles);
+}
+
+}  // namespace hc

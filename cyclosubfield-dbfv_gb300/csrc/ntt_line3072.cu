@@ -1,0 +1,56 @@
+// Dimension-3 lines of field_36864 ([2, 3, 8, 64], 3072 residues): one line per CTA.
+#include "ntt_run.cuh"
+
+namespace {
+
+#ifndef HC_L3072_MIN_BLOCKS
+#define HC_L3072_MIN_BLOCKS 8  // resident CTAs per SM the 3072-residue line kernel's registers must allow (8 fit its shared memory)
+#endif
+
+/// Specialised dimension-3 NTT: one line (i, j, k) per CTA.
+template <int SHAPE, int MODE, bool FIX, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
+    extern __shared__ int64_t smem[];
+    const int64_t tile = blockIdx.x;
+    const int64_t k = tile % t.n2, r = tile / t.n2;
+    const int64_t j = r % t.n1, i = r / t.n1;
+    const DevPlanHeader* P = plans.p[j];
+    int64_t* g = reinterpret_cast<int64_t*>(t.p) + i * t.s0 + j * t.s1 + k * t.s2;
+    const int64_t* mulp = nullptr;
+    int64_t me = 0, mn = 0, mi = 0;
+    if (MODE & 2) {
+        mulp = kat<int64_t>(mul, i, j, k, 0);
+        me = mul.b3 ? 0 : 1;
+        mn = mods.n[j], mi = mods.ninv[j];
+    }
+    run_line<SHAPE, MODE, FIX>(P, smem, g, mulp, me, mn, mi);
+}
+
+template <int MODE, bool FIX>
+hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    constexpr size_t smem = (size_t)line_tile_words(HC_SHAPE_L3072) * 8;
+    auto kern = ntt_line_kernel<HC_SHAPE_L3072, MODE, FIX, 128, HC_L3072_MIN_BLOCKS>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
+    kern<<<(unsigned)tiles, 128, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
+    hc::count_launch(ctx);
+    return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
+}
+
+template <bool FIX>
+hc_status launch_mode(hc_context ctx, int mode, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    if (mode == 0) return launch<0, FIX>(ctx, t, pp, mul, mods, tiles);
+    if (mode == 1) return launch<1, FIX>(ctx, t, pp, mul, mods, tiles);
+    if (mode == 2) return launch<2, FIX>(ctx, t, pp, mul, mods, tiles);
+    return launch<3, FIX>(ctx, t, pp, mul, mods, tiles);
+}
+
+}  // namespace
+
+namespace hc {
+
+hc_status launch_ntt_line3072(hc_context ctx, int mode, bool fix, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    return fix ? launch_mode<true>(ctx, mode, t, pp, mul, mods, tiles) : launch_mode<false>(ctx, mode, t, pp, mul, mods, tiles);
+}
+
+}  // namespace hc

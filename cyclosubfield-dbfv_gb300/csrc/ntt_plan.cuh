@@ -3,9 +3,9 @@
 // shapes of the two large field descriptors with their compiled-in schedules, and the register /
 // shared-memory building blocks of ntt_fast.cuh.
 #pragma once
-#include "common.cuh"
+#include <type_traits>
 
-namespace {
+#include "common.cuh"
 
 /// Division by an invariant divisor d (1 <= d < 2^32) with a multiply-high and shifts
 /// (Granlund & Montgomery, "Division by invariant integers using multiplication", 1994, fig. 4.1).
@@ -28,7 +28,7 @@ struct DevStage {
     FastDiv div_nblocks;  // group -> twiddle block (group mod flen / stage_len)
 };
 
-FastDiv make_fastdiv(uint32_t d) {
+inline FastDiv make_fastdiv(uint32_t d) {
     FastDiv f;
     f.d = d;
     uint32_t l = 0;
@@ -62,19 +62,22 @@ struct DevPlanHeader {
     int32_t ntw;
     int32_t nfpass;
     int32_t nipass;
+    int32_t cls;  // fixed plans: 56 or 57 (the schedule's fixed_masks), else 0
+    int32_t pad;
     int64_t one_z, one_u, invlen_z, invlen_u;
+    BarrettMod mod;  // limb forms, used by the plans whose products fit them (hc_ntt_plan_s::fixed)
+    BarrettLimbs invlen;
     DevStage fwd[HC_MAX_STAGES];
     DevStage inv[HC_MAX_STAGES];
     DevPass fpass[HC_MAX_STAGES];
     DevPass ipass[HC_MAX_STAGES];
-    // followed by the twiddle table: ntw pairs (z, u)
+    // followed by the twiddle table as ntw pairs (z, u), then as ntw BarrettLimbs
 };
 
 struct PlanPtrs {
     const DevPlanHeader* p[HC_MAX_MODS];
 };
-
-}  // namespace
+static_assert(sizeof(DevPlanHeader) % 16 == 0, "plan twiddle tables must be 16-byte aligned");
 
 namespace {
 #include "ntt_fast.cuh"
@@ -86,31 +89,67 @@ namespace {
 #define HC_SHAPE_C4 4      // dimension-2 column [4]
 
 __host__ __device__ constexpr int line_len(int shape) { return shape == HC_SHAPE_L3072 ? 3072 : 12288; }
+#define HC_COL_THREADS 256  // of the column kernel
+
 __host__ __device__ constexpr int line_tile_words(int shape) { return line_len(shape) + line_len(shape) / 8; }
 
-__device__ __forceinline__ fast::Ctx make_ctx(const DevPlanHeader* P, const int64_t* tw) {
-    fast::Ctx c;
-    c.n = P->n, c.one_z = P->one_z, c.one_u = P->one_u, c.il_z = P->invlen_z, c.il_u = P->invlen_u;
-    c.tw = tw;
+/// Contexts of a plan: its twiddles are read from global memory (L1-cached).
+template <class CTX>
+__device__ __forceinline__ CTX make_ctx(const DevPlanHeader* P) {
+    CTX c;
+    const int64_t* tw = reinterpret_cast<const int64_t*>(P + 1);
+    if constexpr (CTX::LIMBS) {
+        c.m = P->mod, c.il = P->invlen;
+        c.tw = reinterpret_cast<const int4*>(tw + 2 * P->ntw);
+    } else {
+        c.n = P->n, c.one_u = P->one_u, c.il_z = P->invlen_z, c.il_u = P->invlen_u;
+        c.tw = tw;
+    }
     return c;
 }
 
-/// The reduction / skip / fused-final schedule that the plans of the rings' primes have, per shape
-/// and direction (bit s = the flag of stage s): field_36864 samples primes just below 2^57,
-/// field_49152 primes just below 2^56.
+/// The reduction / skip / fused-final schedule (bit s = the flag of stage s) of a specialised shape's
+/// plan for a prime just below 2^lg, by the bound tracking of build_plan in units of the prime (k
+/// primes fit a signed word exactly when k <= 2^(63 - lg)). The rings sample their primes below 2^57
+/// and 2^56, often both in one base, so a kernel carries these two schedules and each CTA takes its
+/// row's (`cls` of the plan): compiled in, the flags fold into straight-line code (intt along dimension
+/// 3 of a [24, 20, 12, 3072] tensor 111 us, 146 us with the flags read from the plan). A plan
+/// counts as fixed when it has one of the two and its products fit the limb forms (BarrettLimbs).
 struct SchedMasks {
     uint32_t fred, fskip, flast, ired, ilast;
 };
-__host__ __device__ constexpr SchedMasks fixed_masks(int shape) {
-    return shape == HC_SHAPE_L3072    ? SchedMasks{0u, 0xFu, 1u << 10, 0x410u, 1u << 10}
-           : shape == HC_SHAPE_L12288 ? SchedMasks{0u, 0x1Fu, 1u << 12, 0x1020u, 1u << 12}
-           : shape == HC_SHAPE_C12    ? SchedMasks{0u, 0x7u, 1u << 2, 0u, 1u << 2}
-           : shape == HC_SHAPE_C4     ? SchedMasks{0u, 0x3u, 1u << 1, 0u, 1u << 1}
-                                      : SchedMasks{0u, 0u, 0u, 0u, 0u};
+__host__ __device__ constexpr SchedMasks fixed_masks(int shape, int lg) {
+    // radices of the stages, forward and inverse (a factor's stages are alike in both directions)
+    const int nst = shape == HC_SHAPE_L3072 ? 11 : shape == HC_SHAPE_L12288 ? 13 : shape == HC_SHAPE_C12 ? 3 : shape == HC_SHAPE_C4 ? 2 : 0;
+    const int r3 = shape == HC_SHAPE_L3072 ? 1 : shape == HC_SHAPE_L12288 ? 0 : shape == HC_SHAPE_C12 ? 2 : -1;
+    const int64_t max = (int64_t)1 << (63 - lg);
+    SchedMasks m{0u, 0u, 0u, 0u, 0u};
+    int64_t f = 2, v = 2;
+    for (int s = 0; s < nst; s++) {
+        const int64_t radix = s == r3 ? 3 : 2;
+        if (f + radix - 1 > max) m.fred |= 1u << s, f = 1;
+        if (radix * f <= max) m.fskip |= 1u << s, f *= radix;
+        else f += radix - 1;
+        if (radix * v > max) m.ired |= 1u << s, v = 1;
+        v *= radix;
+    }
+    if (nst) m.flast = m.ilast = 1u << (nst - 1);
+    return m;
 }
-template <int SHAPE, bool INV>
-using FixedSched = fast::FixSched<INV ? fixed_masks(SHAPE).ired : fixed_masks(SHAPE).fred,
-                                  INV ? 0u : fixed_masks(SHAPE).fskip,
-                                  INV ? fixed_masks(SHAPE).ilast : fixed_masks(SHAPE).flast>;
+template <int SHAPE, int LG, bool INV>
+using FixedSched = fast::FixSched<INV ? fixed_masks(SHAPE, LG).ired : fixed_masks(SHAPE, LG).fred,
+                                  INV ? 0u : fixed_masks(SHAPE, LG).fskip,
+                                  INV ? fixed_masks(SHAPE, LG).ilast : fixed_masks(SHAPE, LG).flast>;
+
+/// Calls f with the compiled-in schedule of a fixed plan (SHAPE, direction INV), or with the
+/// schedule read from any plan (FIX = false). Uniform over a CTA that works for one plan.
+template <int SHAPE, bool INV, bool FIX, class F>
+__device__ __forceinline__ void with_sched(const DevPlanHeader* P, F f) {
+    const DevStage* st = INV ? P->inv : P->fwd;
+    if constexpr (!FIX) f(fast::DynSched{st});
+    else if (std::is_same_v<FixedSched<SHAPE, 56, INV>, FixedSched<SHAPE, 57, INV>> || P->cls == 57)
+        f(FixedSched<SHAPE, 57, INV>{st});
+    else f(FixedSched<SHAPE, 56, INV>{st});
+}
 
 }  // namespace
