@@ -40,15 +40,16 @@ __device__ __forceinline__ T* kat(const KView& v, int64_t i, int64_t j, int64_t 
     return reinterpret_cast<T*>(v.p) + i * v.s0 + j * v.s1 + k * v.s2 + (v.b3 ? 0 : l);
 }
 
+struct BarrettLimbs;
+
 /// Device tables of one base conversion (built by the ring layer; bconv_fused_kernel reads them).
 struct BconvConsts {
-    const int64_t* qinv;   // [r] plain lifts of (Q_b / p_u)^-1 mod p_u, Montgomery factors
-    const int64_t* qinvp;  // [r] qinv[u] * (-p_u^-1) mod 2^64
+    const BarrettLimbs* qinv;  // [r] Montgomery factors of the plain lifts of (Q_b / p_u)^-1 mod p_u
     const int64_t* mat;    // [nb][rd + 1][r] conversion matrix; row rd of each block: correction row
     const int4* mat3;      // [nb][rd][r] rows 0..rd-1 as limbs (m mod 2^29, m >> 29, their sum, 0)
     const int64_t* qmodp;  // [nb][rd]
     const int64_t* qtab;   // [nb][rd][2 qhalf + 1] mul_mont(q, qmodp) for |q| <= qhalf
-    const int64_t* r2p;    // [rd] (R^2 mod p_j) * (-p_j^-1) mod 2^64
+    const BarrettLimbs* r2;  // [rd] Montgomery factors R^2 mod p_j
     const int32_t* ucol;   // [nb][2] source column range of output block b
     int qhalf;
     int corr_limb;         // the correction row fits the limb products
@@ -141,22 +142,6 @@ __device__ __forceinline__ int64_t to_mont64(int64_t x, int64_t n, int64_t ninv,
 }
 __device__ __forceinline__ int64_t to_mont128(i128 x, int64_t n, int64_t ninv, int64_t r3) {
     return mul_mont(red128(x, n, ninv), r3, n, ninv);
-}
-
-/// mul_mont(a, b) for a constant b with bp = b * ninv mod 2^64: the Montgomery quotient
-/// m = lo(a b) ninv equals a bp mod 2^64, and lo(a b) != 0 exactly when m != 0 (ninv is odd), so
-/// the low word of a b is never formed. The same integers as mul_mont(a, b, n, ninv).
-__device__ __forceinline__ int64_t mul_mont_c(int64_t a, int64_t b, int64_t bp, int64_t n) {
-    const int64_t m = (int64_t)((uint64_t)a * (uint64_t)bp);
-    return (int64_t)((uint64_t)__mul64hi(a, b) + (uint64_t)__mul64hi(m, n) + (uint64_t)(m != 0));
-}
-
-/// double_red128 of the 128-bit value hi:lo: the first reduction's carry out of the low word is
-/// (lo != 0) (the low words of x and m n cancel), so the low word of m n is never formed.
-__device__ __forceinline__ int64_t double_red_words(uint64_t lo, int64_t hi, int64_t n, int64_t ninv) {
-    const int64_t m = (int64_t)(lo * (uint64_t)ninv);
-    const i128 r1 = (i128)hi + (i128)__mul64hi(m, n) + (i128)(lo != 0);
-    return red128((uint64_t)r1, (int64_t)(r1 >> 64), n, ninv);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -303,6 +288,57 @@ __device__ __forceinline__ int64_t mont_mul(int64_t a, int64_t b, const MontLimb
     int64_t c = mad_wide(q1, m.n0, mad_wide(a0, b1, mad_wide(a1, b0, m.k)));
     c = (int64_t)mad_wide_u(q0, (uint32_t)m.n1, (uint64_t)c);
     return mad_wide(q1, m.n1, mad_wide(a1, b1, c >> 32));
+}
+
+/// The Montgomery reduction (hi 2^64 + lo + m n) / 2^64 = red128(lo, hi, n, ninv), the same integer, for
+/// n < 2^57 and |hi| <= 2^62: as in mont_mul only the middle limbs of m n are formed, here with the
+/// upper word of lo beside them; what is left out lies in [0, 2^31 + 1) 2^32 for n0 >= 0 and (-2^31, 1) 2^32
+/// for n0 < 0. Six products (21 cycles) instead of eight and their sign corrections.
+__device__ __forceinline__ int64_t mont_red(uint64_t lo, int64_t hi, const MontLimbs& m) {
+    const uint32_t l0 = lo32((int64_t)lo), l1 = hi32((int64_t)lo);
+    const uint64_t q = (uint64_t)l0 * m.i0;
+    const uint32_t q0 = lo32((int64_t)q);
+    const int32_t q1 = (int32_t)(hi32((int64_t)q) + l1 * m.i0 + l0 * m.i1);
+    const int64_t k = m.n0 >= 0 ? 0x80000001ll : 1;
+    int64_t c = mad_wide(q1, m.n0, (int64_t)((uint64_t)l1 + (uint64_t)k));
+    c = (int64_t)mad_wide_u(q0, (uint32_t)m.n1, (uint64_t)c);
+    return mad_wide(q1, m.n1, wadd(c >> 32, hi));
+}
+/// double_red128 of hi 2^64 + lo (|hi| <= 2^62), the same integer: the first reduction fits one word, the
+/// second has its sign as the upper word (floor division keeps the middle limbs' carry exact).
+__device__ __forceinline__ int64_t mont_red_double(uint64_t lo, int64_t hi, const MontLimbs& m) {
+    const int64_t r = mont_red(lo, hi, m);
+    return mont_red((uint64_t)r, r >> 63, m);
+}
+
+/// mul_mont(a, b, n, ninv) for a constant b in the limbs of a Barrett product, for n < 2^57 and |a| <= 0.9 x
+/// 2^63: with b' = b 2^-64 mod n and s = (b' 2^64 - b) / n the Montgomery product is b' a - q n, q =
+/// round(s a / 2^64) (|a b / 2^64 - b' a + q n| <= n / 2, ties as the signed quotient of the reduction
+/// takes them), which is barrett_mul modulo -n. 8 products instead of 12 of mont_mul.
+__host__ __device__ __forceinline__ BarrettMod mont_const_mod(int64_t n) {
+    BarrettMod m;
+    m.n0 = (int32_t)(0u - lo32(n)), m.nn0 = (int32_t)lo32(n), m.nn1 = bal_hi(n);
+    m.red_add = m.red_shift = 0;
+    return m;
+}
+inline BarrettLimbs mont_const_limbs(int64_t b, int64_t n) {
+    uint64_t inv = 1;  // n^-1 mod 2^64
+    for (int i = 0; i < 6; i++) inv *= 2 - (uint64_t)n * inv;
+    // b' 2^64 = b + n s with s = -b n^-1 mod 2^64; signed s keeps b' centred
+    const i128 s = (int64_t)(0 - (uint64_t)b * inv);
+    const i128 z = ((i128)b + s * n) >> 64;
+    i128 u = s, zz = z;
+    if (u >= ((i128)1 << 63) - ((i128)1 << 31)) u -= (i128)1 << 64, zz -= n;
+    BarrettLimbs w;
+    w.u0 = (int32_t)(uint32_t)u;
+    w.u1 = (int32_t)((u - w.u0) >> 32);
+    w.z0 = (int32_t)(uint32_t)zz;
+    w.e1 = bal_hi(b);
+    return w;
+}
+__device__ __forceinline__ BarrettLimbs load_limbs(const BarrettLimbs* p) {
+    const int4 a = __ldg(reinterpret_cast<const int4*>(p));
+    return BarrettLimbs{a.x, a.y, a.z, a.w};
 }
 
 __device__ __forceinline__ i128 ld128(const void* p) {

@@ -25,7 +25,7 @@
 
 namespace hc {
 hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst, const BconvConsts& c, int r, int rd,
-                             int nb, const KMods& sm, const KMods& dm, int64_t ns, const int64_t* sub_mul);
+                             int nb, const KMods& sm, const KMods& dm, int64_t ns, const BarrettLimbs* sub_mul);
 hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const uint32_t* p2, const uint32_t* p3);
 hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys, int nterms, const KView* add0,
                            const KView* add1, int full0, int full1, const KView& dst, const KMods& m,
@@ -466,14 +466,13 @@ int64_t mul_mont_host(int64_t a, int64_t b, int64_t n, int64_t ninv) {
 ///  - mat3: the matrix rows 0..rd-1 as 29-bit limbs (m mod 2^29, m >> 29, their sum), for the
 ///    kernel's exact int64 multiply-accumulate; it needs |m| < 2^56 and lifts |x| < 2^57, i.e.
 ///    source primes below 2^57 (the ring's RNS factor size rule; checked here all the same);
-///  - qinvp, r2p: the Montgomery factors qinv[u] and R^2 mod p_j times -p^-1 mod 2^64, so that the
-///    kernel's products with them skip one 64-bit multiplication (mul_mont_c);
+///  - qinv, r2: the Montgomery factors as Barrett limbs (mont_const_limbs);
 ///  - qtab: mul_mont(q, qmodp) for every correction q in [-qhalf, qhalf] (|q| is at most the
 ///    block's source count, because 2^shift exceeds 4 r max(p)); larger q would be computed;
 ///  - corr_limb: whether the correction row (round(2^shift / p_u)) is small enough for the limb
 ///    products too.
 struct BconvTables {
-    DBuf qinv, qinvp, mat, mat3, qmodp, qtab, r2p, ucol;
+    DBuf qinv, mat, mat3, qmodp, qtab, r2, ucol;
     BconvConsts c{};
 };
 
@@ -488,7 +487,8 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
     size_t maxlen = 0;
     for (size_t b = 0; b < nb; b++) maxlen = std::max(maxlen, (size_t)(uc[2 * b + 1] - uc[2 * b]));
     std::vector<int32_t> m3(nb * rd * r * 4, 0);
-    std::vector<int64_t> qinvp(r), r2p(rd), qtab;
+    std::vector<BarrettLimbs> qinvl(r), r2l(rd);
+    std::vector<int64_t> qtab;
     int64_t maxmq = 0;
     for (size_t b = 0; b < nb; b++) {
         for (size_t j = 0; j < rd; j++)
@@ -503,25 +503,24 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
             }
         for (size_t u = 0; u < r; u++) maxmq = std::max(maxmq, std::abs(mat[(b * (rd + 1) + rd) * r + u]));
     }
-    for (size_t u = 0; u < r; u++) qinvp[u] = (int64_t)((uint64_t)qinv[u] * (uint64_t)sm[u].neg_inv_n);
-    for (size_t j = 0; j < rd; j++) r2p[j] = (int64_t)((uint64_t)dm[j].r2_mod_n * (uint64_t)dm[j].neg_inv_n);
+    for (size_t u = 0; u < r; u++) qinvl[u] = mont_const_limbs(qinv[u], sm[u].n);
+    for (size_t j = 0; j < rd; j++) r2l[j] = mont_const_limbs(dm[j].r2_mod_n, dm[j].n);
     const int qhalf = (int)maxlen;
     for (size_t b = 0; b < nb; b++)
         for (size_t j = 0; j < rd; j++)
             for (int q = -qhalf; q <= qhalf; q++)
                 qtab.push_back(mul_mont_host(q, qm[b * rd + j], dm[j].n, dm[j].neg_inv_n));
-    t.qinv = DBuf(ctx, qinv.data(), r * 8);
-    t.qinvp = DBuf(ctx, qinvp.data(), r * 8);
+    t.qinv = DBuf(ctx, qinvl.data(), r * sizeof(BarrettLimbs));
     t.mat = DBuf(ctx, mat.data(), mat.size() * 8);
     t.mat3 = DBuf(ctx, m3.data(), m3.size() * 4);
     t.qmodp = DBuf(ctx, qm.data(), qm.size() * 8);
     t.qtab = DBuf(ctx, qtab.data(), qtab.size() * 8);
-    t.r2p = DBuf(ctx, r2p.data(), rd * 8);
+    t.r2 = DBuf(ctx, r2l.data(), rd * sizeof(BarrettLimbs));
     t.ucol = DBuf(ctx, uc.data(), uc.size() * 4);
     BconvConsts& c = t.c;
-    c.qinv = t.qinv.as<int64_t>(), c.qinvp = t.qinvp.as<int64_t>(), c.mat = t.mat.as<int64_t>();
+    c.qinv = t.qinv.as<BarrettLimbs>(), c.mat = t.mat.as<int64_t>();
     c.mat3 = t.mat3.as<int4>(), c.qmodp = t.qmodp.as<int64_t>(), c.qtab = t.qtab.as<int64_t>();
-    c.r2p = t.r2p.as<int64_t>(), c.ucol = t.ucol.as<int32_t>();
+    c.r2 = t.r2.as<BarrettLimbs>(), c.ucol = t.ucol.as<int32_t>();
     c.qhalf = qhalf, c.shift = shift, c.chunk = chunk;
     // the correction row's limb products x0 mq, x1 mq summed over a block stay below 2^63
     c.corr_limb = maxmq < ((int64_t)1 << 30) && (i128)maxmq * ((i128)1 << 29) * (i128)maxlen < ((i128)1 << 63);
@@ -565,7 +564,7 @@ struct hc_ring_s {
     std::map<Base, std::unique_ptr<DBuf>> one_cache;
     std::map<std::pair<Base, i128>, std::unique_ptr<Tensor>> scalar_cache;
     std::map<std::pair<Base, Base>, std::unique_ptr<Tensor>> qinv_cache;
-    std::map<std::pair<Base, Base>, std::unique_ptr<DBuf>> qinv_pair_cache;
+    std::map<std::pair<Base, Base>, std::unique_ptr<DBuf>> qinv_limb_cache;
     // dBFV reduction tables (dbfv_tables) by (log2 b, log2 t, base), type-erased: their type is
     // defined with the dBFV code below
     std::map<std::tuple<size_t, size_t, Base>, std::shared_ptr<void>> dbfv_cache;
@@ -881,11 +880,10 @@ struct hc_ring_s {
         return *bcache.back();
     }
 
-    /// `sub_mul` (optional, [2][rd]: one Montgomery factor b per destination prime, then b times
-    /// -p^-1 mod 2^64): instead of writing the conversion v, dst <- mul_mont(dst - v, b) (the
-    /// caller's hal_sub_i64 and hal_mul_mont64, fused into the store)
+    /// `sub_mul` (optional, [rd]: one Montgomery factor b per destination prime, mont_const_limbs):
+    /// instead of writing the conversion v, dst <- mul_mont(dst - v, b) (the caller's hal_sub_i64 and hal_mul_mont64, fused into the store)
     void bconv(const hc_view& dst, const Base& db, const hc_view& src, const Base& sb,
-               const int64_t* sub_mul = nullptr) {
+               const BarrettLimbs* sub_mul = nullptr) {
         check_view(src, src.shape[0], (int64_t)sb.size(), src.shape[2], src.shape[3], "bconv src");
         check_view(dst, src.shape[0], (int64_t)db.size(), src.shape[2], src.shape[3], "bconv dst");
         BconvCache& c = bconv_cache(sb, db);
@@ -1030,21 +1028,20 @@ struct hc_ring_s {
         qinv_cache[key] = std::move(t);
         return ref;
     }
-    /// The factors of inv_modulus_tensor(of, div) as the base conversion's `sub_mul` pairs:
-    /// [2][|of|] = (b_j, b_j * (-p_j^-1) mod 2^64), cached
-    const DBuf& inv_modulus_pairs(const Base& of, const Base& div) {
+    /// The factors of inv_modulus_tensor(of, div) as the base conversion's `sub_mul` (mont_const_limbs),
+    /// cached
+    const DBuf& inv_modulus_limbs(const Base& of, const Base& div) {
         auto key = std::make_pair(of, div);
-        auto it = qinv_pair_cache.find(key);
-        if (it != qinv_pair_cache.end()) return *it->second;
-        std::vector<int64_t> v(2 * of.size());
+        auto it = qinv_limb_cache.find(key);
+        if (it != qinv_limb_cache.end()) return *it->second;
+        std::vector<BarrettLimbs> v(of.size());
         for (size_t j = 0; j < of.size(); j++) {
             const int64_t p = prime(of[j]);
-            v[j] = mont_repr(centred(invm(q_mod(div, p), p), p), p);
-            v[of.size() + j] = (int64_t)((uint64_t)v[j] * (uint64_t)factors[of[j]].mod.neg_inv_n);
+            v[j] = mont_const_limbs(mont_repr(centred(invm(q_mod(div, p), p), p), p), p);
         }
-        auto t = std::make_unique<DBuf>(ctx, v.data(), v.size() * 8);
+        auto t = std::make_unique<DBuf>(ctx, v.data(), v.size() * sizeof(BarrettLimbs));
         auto& ref = *t;
-        qinv_pair_cache[key] = std::move(t);
+        qinv_limb_cache[key] = std::move(t);
         return ref;
     }
     /// [1, r, 1, 1] tensor holding mont(smallest_lift(residue(p))) (src/ring.rs:890-902)
@@ -1415,7 +1412,7 @@ Tensor rescale_to_base(hc_ring R, const hc_view& x, const Base& lifted, size_t b
     if (!pre_scaled) CK(hc_mul_mont64(R->ctx, x, R->scalar_tensor(lifted, t).view(), ml.data(), ml.size()));
     hc_view xlo = vbase(x, 0, (int64_t)base_len), xhi = vbase(x, (int64_t)base_len, (int64_t)lifted.size());
     // xhi <- (xhi - bconv(xlo)) * (Q_base^-1 mod p), the subtraction and product in the conversion's store
-    R->bconv(xhi, ext, xlo, base, R->inv_modulus_pairs(ext, base).as<int64_t>());
+    R->bconv(xhi, ext, xlo, base, R->inv_modulus_limbs(ext, base).as<BarrettLimbs>());
     Tensor out = temp(R->ctx, count, (int64_t)base_len, R->dl(), R->dk());
     R->bconv(out.view(), base, xhi, ext);
     return out;

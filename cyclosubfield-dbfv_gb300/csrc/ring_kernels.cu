@@ -29,7 +29,7 @@ struct BconvArgs {
     int r, rd, nb;
     int ochunk;  // outputs per CTA (even): blockIdx.z selects the outputs [z ochunk, (z + 1) ochunk)
     int64_t npos;
-    const int64_t* sub_mul;  // optional [2][rd]: store mul_mont(dst - v, b_j) instead of v (b_j, b_j ninv)
+    const BarrettLimbs* sub_mul;  // optional [rd]: store mul_mont(dst - v, b_j) instead of v
 };
 
 constexpr int LIMB_BITS = 29;
@@ -58,12 +58,12 @@ __device__ __forceinline__ void limb_terms(const int2* __restrict__ xp, const in
             const int2 x = xp[t * BCONV_THREADS];
             const int xs = x.x + x.y;
             const int4 p = __ldg(p0 + t), q = __ldg(p1 + t);
-            s[0] += (int64_t)x.x * p.x;
-            s[1] += (int64_t)x.y * p.y;
-            s[2] += (int64_t)xs * p.z;
-            s[3] += (int64_t)x.x * q.x;
-            s[4] += (int64_t)x.y * q.y;
-            s[5] += (int64_t)xs * q.z;
+            s[0] = mad_wide(x.x, p.x, s[0]);
+            s[1] = mad_wide(x.y, p.y, s[1]);
+            s[2] = mad_wide(xs, p.z, s[2]);
+            s[3] = mad_wide(x.x, q.x, s[3]);
+            s[4] = mad_wide(x.y, q.y, s[4]);
+            s[5] = mad_wide(xs, q.z, s[5]);
         }
     }
 }
@@ -96,9 +96,10 @@ __device__ __forceinline__ void bconv_store(const BconvArgs& a, const KMods& dm,
     const int64_t* qt = a.c.qtab + (b * a.rd + j) * (2 * a.c.qhalf + 1) + a.c.qhalf;
     const int64_t qm = (q >= -a.c.qhalf && q <= a.c.qhalf) ? __ldg(qt + q)
                                                             : mul_mont(q, a.c.qmodp[b * a.rd + j], n, ninv);
-    const int64_t y = mul_mont_c(wadd(v, qm), dm.r2[j], __ldg(a.c.r2p + j), n);  // to_mont64
+    const BarrettMod mm = mont_const_mod(n);
+    const int64_t y = barrett_mul(load_limbs(a.c.r2 + j), wadd(v, qm), mm);  // to_mont64
     if constexpr (SUB)
-        *p = mul_mont_c(wsub(old, y), __ldg(a.sub_mul + j), __ldg(a.sub_mul + a.rd + j), n);
+        *p = barrett_mul(load_limbs(a.sub_mul + j), wsub(old, y), mm);
     else
         *p = y;
 }
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a,
     // the source is multiplied by (Q/p)^-1 in Montgomery form, giving plain lifts in (-p, p)
     for (int u = u0; u < u1; u++) {
         int64_t x = srcp[u * a.src.s1];
-        x = mul_mont_c(x, __ldg(a.c.qinv + u), __ldg(a.c.qinvp + u), sm.n[u]);
+        x = barrett_mul(load_limbs(a.c.qinv + u), x, mont_const_mod(sm.n[u]));
         xs[u * BCONV_THREADS + threadIdx.x] = make_int2((int)(x & ((1 << LIMB_BITS) - 1)), (int)(x >> LIMB_BITS));
     }
     const i128 half = (i128)1 << (a.c.shift - 1);
@@ -139,8 +140,8 @@ __global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a,
         for (int u = u0; u < u1; u++) {
             const int2 x = xcol[u * BCONV_THREADS];
             const int m = (int)__ldg(mq + u);
-            c0 += (int64_t)x.x * m;
-            c1 += (int64_t)x.y * m;
+            c0 = mad_wide(x.x, m, c0);
+            c1 = mad_wide(x.y, m, c1);
         }
         corr = (i128)c0 + (i128)((u128)(i128)c1 << LIMB_BITS);
     } else {
@@ -172,8 +173,8 @@ __global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a,
             uint64_t l0 = 0, l1 = 0;
             int64_t h0 = 0, h1 = 0;
             limb_mac2(xcol, m0, m1, u0, u1, l0, h0, l1, h1);
-            v0 = double_red_words(l0, h0, dm.n[j], dm.ninv[j]);
-            v1 = double_red_words(l1, h1, dm.n[j + two], dm.ninv[j + two]);
+            v0 = mont_red_double(l0, h0, mont_limbs(dm.n[j], dm.ninv[j]));
+            v1 = mont_red_double(l1, h1, mont_limbs(dm.n[j + two], dm.ninv[j + two]));
         } else {
             bool first = true;
             for (int c0 = 0; c0 < a.r; c0 += a.c.chunk) {
@@ -181,10 +182,10 @@ __global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a,
                 uint64_t l0 = 0, l1 = 0;
                 int64_t h0 = 0, h1 = 0;
                 limb_mac2(xcol, m0, m1, lo, hi, l0, h0, l1, h1);
-                const int64_t r0 = double_red_words(l0, h0, dm.n[j], dm.ninv[j]);
+                const int64_t r0 = mont_red_double(l0, h0, mont_limbs(dm.n[j], dm.ninv[j]));
                 v0 = first ? r0 : wadd(v0, r0);
                 if (two) {
-                    const int64_t r1 = double_red_words(l1, h1, dm.n[j + 1], dm.ninv[j + 1]);
+                    const int64_t r1 = mont_red_double(l1, h1, mont_limbs(dm.n[j + 1], dm.ninv[j + 1]));
                     v1 = first ? r1 : wadd(v1, r1);
                 }
                 first = false;
@@ -537,7 +538,7 @@ void grid_lines(hc_context ctx, int64_t n3, int64_t lines, int* chunks, unsigned
 namespace hc {
 
 hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst, const BconvConsts& c, int r, int rd,
-                             int nb, const KMods& sm, const KMods& dm, int64_t ns, const int64_t* sub_mul) {
+                             int nb, const KMods& sm, const KMods& dm, int64_t ns, const BarrettLimbs* sub_mul) {
     BconvArgs a;
     a.src = src;
     a.dst = dst;
