@@ -21,9 +21,9 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
             int64_t* g = S.data + k * S.s2;
             const int64_t* mulp = mode == 3 ? S.op + k * S.op_s2 : mulrow;
             if (CLS != 2 && (CLS == 1 || shape == HC_SHAPE_L3072)) {
-                if (mode == 2) run_line<HC_SHAPE_L3072, 2, true>(P, s, g, mulp, 1, S.n, S.ninv);
-                else if (mode == 3) run_line<HC_SHAPE_L3072, 3, true>(P, s, g, mulp, 1, S.n, S.ninv);
-                else run_line<HC_SHAPE_L3072, 1, true>(P, s, g, mulp, 1, S.n, S.ninv);
+                if (mode == 2) run_line3072<2, true>(P, s, g, mulp, 1, S.n, S.ninv);
+                else if (mode == 3) run_line3072<3, true>(P, s, g, mulp, 1, S.n, S.ninv);
+                else run_line3072<1, true>(P, s, g, mulp, 1, S.n, S.ninv);
             } else if (CLS != 1) {
                 // one 4096-residue block in shared memory at a time (crt_slab_tile_words)
                 const auto c = make_ctx<fast::CtxL>(P);

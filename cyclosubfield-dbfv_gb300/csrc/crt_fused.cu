@@ -39,7 +39,6 @@ int32_t plan_shape(hc_ntt_plan p);
 namespace {
 
 constexpr int CLUSTER = 12;  // CTAs per slab
-constexpr int THREADS = 128;
 constexpr size_t SMEM12288 = 4608 * 8;  // one padded 4096-residue block
 
 /// Split cluster barrier: every CTA arrives when it starts and waits before its first store into
@@ -97,18 +96,18 @@ __device__ __forceinline__ void four_half(const CTX& c, const fast::SF& f0, cons
     }
 }
 
-/// Both phases of one half for the schedules of primes just below 2^LG; the CTA's block is left in its
-/// shared memory. The caller has arrived at the cluster barrier (cluster_arrive_relaxed).
-template <int DIR, int LG>
+/// Both phases of one half for the schedules of primes just below 2^LG. The caller has arrived at the cluster barrier (cluster_arrive_relaxed).
+template <int DIR, bool POST, int LG, int THREADS>
 __device__ __forceinline__ void slab12288_half(int64_t* smem, cg::cluster_group& cluster, const KView& t, const KView& src,
                                                const DevPlanHeader* P2, const DevPlanHeader* P3, const KView& m2,
-                                               const fast::MontL& mont, int64_t i, int64_t j) {
+                                               const KView& m3, const fast::MontL& mont, int64_t i, int64_t j) {
     const int rank = (int)cluster.block_rank();
+    const int row = rank / 3, blk = rank - 3 * (rank / 3);
     constexpr bool inv = DIR == 1;
     const fast::CtxL c3 = make_ctx<fast::CtxL>(P3);
     const FixedSched<HC_SHAPE_L12288, LG, inv> sch3{inv ? P3->inv : P3->fwd};
     // ---- phase 1: positions p, p + 4096, p + 8192 of the four rows, over the cluster's threads;
-    // warp w keeps rows 2h, 2h + 1 (h = w & 1) of 64 positions per CTA and step
+    // warp w keeps rows 2h, 2h + 1 (h = w & 1) of THREADS / 2 positions per CTA and step
     {
         const fast::CtxL c2 = make_ctx<fast::CtxL>(P2);
         const FixedSched<HC_SHAPE_C4, LG, inv> sch2{inv ? P2->inv : P2->fwd};
@@ -120,8 +119,8 @@ __device__ __forceinline__ void slab12288_half(int64_t* smem, cg::cluster_group&
         const int64_t* gs = reinterpret_cast<const int64_t*>(src.p) + i * src.s0 + j * src.s1;
 #pragma unroll 1
         for (int q = 0;; q++) {
-            const int p = 768 * q + 64 * rank + 32 * (warp >> 1) + (threadIdx.x & 31);
-            if (p >= 4096) break;  // warp-uniform (4096 and 768 are multiples of 32)
+            const int p = THREADS / 2 * (CLUSTER * q + rank) + 32 * (warp >> 1) + (threadIdx.x & 31);
+            if (p >= 4096) break;  // warp-uniform: p / 32 is the same for the warp
             int64_t y[2][3];  // rows 2h, 2h + 1 by block b
 #pragma unroll
             for (int b = 0; b < 3; b++) {
@@ -138,7 +137,7 @@ __device__ __forceinline__ void slab12288_half(int64_t* smem, cg::cluster_group&
                 if (inv) fast::inv3(c3, f30, y[a][0], y[a][1], y[a][2]);
                 else fast::fwd3<true>(c3, f30, false, 0, y[a][0], y[a][1], y[a][2]);
             }
-            if (q == 0) cluster_wait();  // every thread runs q = 0 (p < 768)
+            if (q == 0) cluster_wait();  // every thread runs q = 0 (p < 6 THREADS <= 4096)
 #pragma unroll
             for (int a = 0; a < 2; a++)
 #pragma unroll
@@ -151,39 +150,11 @@ __device__ __forceinline__ void slab12288_half(int64_t* smem, cg::cluster_group&
         fast::r2_pass<false, 3, 9, 12, 0>(c3, smem, 512, sch3, 1, false);  // factor 64 (a): 2048, 1024, 512
         __syncthreads();
         fast::r2_pass<false, 3, 6, 9, 3>(c3, smem, 512, sch3, 4, false);   // factor 64 (a): 256, 128, 64
-        __syncthreads();
-        fast::r2_pass<false, 3, 3, 6, 0>(c3, smem, 512, sch3, 7, false);   // factor 64 (b): 32, 16, 8
-        __syncthreads();
-        fast::r2_pass<false, 3, 0, 3, 3>(c3, smem, 512, sch3, 10, false);  // factor 64 (b): 4, 2, 1
     } else {
         fast::r2_pass<true, 3, 6, 9, 3>(c3, smem, 512, sch3, 1, false);    // factor 64 (a): 64, 128, 256
         __syncthreads();
         fast::r2_pass<true, 3, 9, 12, 0>(c3, smem, 512, sch3, 4, false);   // factor 64 (a): 512, 1024, 2048
-        __syncthreads();
-        fast::r2_pass<true, 3, 0, 3, 3>(c3, smem, 512, sch3, 7, false);    // factor 64 (b): 1, 2, 4
-        __syncthreads();
-        fast::r2_pass<true, 3, 3, 6, 0>(c3, smem, 512, sch3, 10, false);   // factor 64 (b): 8, 16, 32
     }
-}
-
-/// Fused pass of a field_49152 slab: CTA 3k + b of the cluster owns block b of row k.
-template <int DIR, bool POST>
-__global__ void __launch_bounds__(THREADS, 6)
-    crt_slab12288_kernel(KView t, KView src, PlanPtrs p2, PlanPtrs p3, KView m2, KView m3, KMods mods, int reverse) {
-    extern __shared__ int64_t smem[];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int row = rank / 3, blk = rank - 3 * (rank / 3);
-    // reverse: the last slab first, so that the clusters scheduled first read what the producer
-    // of the input (or the other half of the transform) wrote last, still in L2
-    const int64_t slab = reverse ? gridDim.x / CLUSTER - 1 - blockIdx.x / CLUSTER : blockIdx.x / CLUSTER;
-    const int64_t j = slab % t.n1, i = slab / t.n1;
-    const DevPlanHeader* P2 = p2.p[j];
-    const DevPlanHeader* P3 = p3.p[j];
-    const fast::MontL mont = fast::make_mont<fast::CtxL>(mods.n[j], mods.ninv[j]);
-    cluster_arrive_relaxed();
-    if (P3->cls == 57) slab12288_half<DIR, 57>(smem, cluster, t, src, P2, P3, m2, mont, i, j);
-    else slab12288_half<DIR, 56>(smem, cluster, t, src, P2, P3, m2, mont, i, j);
     __syncthreads();
     int64_t* g = reinterpret_cast<int64_t*>(t.p) + i * t.s0 + j * t.s1 + row * t.s2 + 4096 * blk;
     const int64_t* mulp = nullptr;
@@ -192,16 +163,34 @@ __global__ void __launch_bounds__(THREADS, 6)
         me = m3.b3 ? 0 : 1;
         mulp = kat<int64_t>(m3, i, j, row, 0) + (me ? 4096 * blk : 0);
     }
-    fast::line_store(smem, g, 4096, DIR == 0 || POST, mulp, me, mont);
+    fast::tail64<DIR == 0 ? 2 : POST ? 3 : 1>(c3, smem, 4096, sch3, 7, false, g, mulp, me, mont);  // factor 64 (b)
+}
+
+/// Fused pass of a field_49152 slab: CTA 3k + b of the cluster owns block b of row k.
+template <int DIR, bool POST, int THREADS>
+__global__ void __launch_bounds__(THREADS, 768 / THREADS)
+    crt_slab12288_kernel(KView t, KView src, PlanPtrs p2, PlanPtrs p3, KView m2, KView m3, KMods mods, int reverse) {
+    extern __shared__ int64_t smem[];
+    cg::cluster_group cluster = cg::this_cluster();
+    // reverse: the last slab first, so that the clusters scheduled first read what the producer
+    // of the input (or the other half of the transform) wrote last, still in L2
+    const int64_t slab = reverse ? gridDim.x / CLUSTER - 1 - blockIdx.x / CLUSTER : blockIdx.x / CLUSTER;
+    const int64_t j = slab % t.n1, i = slab / t.n1;
+    const DevPlanHeader* P2 = p2.p[j];
+    const DevPlanHeader* P3 = p3.p[j];
+    const fast::MontL mont = fast::make_mont<fast::CtxL>(mods.n[j], mods.ninv[j]);
+    cluster_arrive_relaxed();
+    if (P3->cls == 57) slab12288_half<DIR, POST, 57, THREADS>(smem, cluster, t, src, P2, P3, m2, m3, mont, i, j);
+    else slab12288_half<DIR, POST, 56, THREADS>(smem, cluster, t, src, P2, P3, m2, m3, mont, i, j);
 }
 
 template <class K>
-hc_status cluster_launch(hc_context ctx, K kern, int64_t slabs, size_t smem, const KView& t, const KView& src,
+hc_status cluster_launch(hc_context ctx, K kern, int threads, int64_t slabs, size_t smem, const KView& t, const KView& src,
                          const PlanPtrs& p2, const PlanPtrs& p3, const KView& m2, const KView& m3, const KMods& mods,
                          int reverse) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(slabs * CLUSTER), 1, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = hc::stream_of(ctx);
     cudaLaunchAttribute attr[1];
@@ -216,24 +205,25 @@ hc_status cluster_launch(hc_context ctx, K kern, int64_t slabs, size_t smem, con
     return st;
 }
 
-/// Sets the kernel's attributes (shared memory, a 12-CTA cluster) and tells whether at least one
-/// such cluster fits the device; done once per kernel and device.
+/// Sets the kernel's attributes (shared memory, a 12-CTA cluster) and tells how many such clusters the
+/// device holds at a time; done once per kernel and device.
 template <class K>
-bool cluster_ready(K kern, size_t smem) {
+int resident_clusters(K kern, int threads, size_t smem) {
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, bool> done;
+    static std::map<std::pair<const void*, int>, int> done;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     std::lock_guard<std::mutex> lock(mu);
     auto key = std::make_pair((const void*)kern, dev);
     auto it = done.find(key);
     if (it != done.end()) return it->second;
+    int clusters = 0;
     bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
               cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     if (ok) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(CLUSTER, 1, 1);
-        cfg.blockDim = dim3(THREADS, 1, 1);
+        cfg.blockDim = dim3((unsigned)threads, 1, 1);
         cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -242,18 +232,25 @@ bool cluster_ready(K kern, size_t smem) {
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        int clusters = 0;
-        ok = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) clusters = 0;
     }
     cudaGetLastError();  // a refused attribute leaves no sticky error behind
-    done[key] = ok;
-    return ok;
+    done[key] = clusters;
+    return clusters;
 }
 
+/// Threads per CTA: 128 (six CTAs per SM, the finest granularity of the last wave) unless all slabs fit
+/// the device at once with 256 each, where a slab's own latency is the launch's: 23 slabs 53.7 -> 45.4
+/// us per transform, 8 slabs 45.2 -> 33.5 us, while 46 slabs, more than one such wave, take 84 instead
+/// of 72 us.
 template <int DIR, bool POST>
 hc_status launch_fused(hc_context ctx, int64_t slabs, const KView& t, const KView& src, const PlanPtrs& p2,
                        const PlanPtrs& p3, const KView& m2, const KView& m3, const KMods& mods, int reverse) {
-    return cluster_launch(ctx, crt_slab12288_kernel<DIR, POST>, slabs, SMEM12288, t, src, p2, p3, m2, m3, mods, reverse);
+    if (slabs <= resident_clusters(crt_slab12288_kernel<DIR, POST, 256>, 256, SMEM12288))
+        return cluster_launch(ctx, crt_slab12288_kernel<DIR, POST, 256>, 256, slabs, SMEM12288, t, src, p2, p3, m2, m3, mods,
+                              reverse);
+    return cluster_launch(ctx, crt_slab12288_kernel<DIR, POST, 128>, 128, slabs, SMEM12288, t, src, p2, p3, m2, m3, mods,
+                          reverse);
 }
 
 /// Whether a transform's plans are field_49152's shapes ([4] along dimension 2, [3, 64, 64] along
@@ -278,9 +275,9 @@ namespace hc {
 /// and the device runs the 12-CTA clusters of all three kernels of that shape.
 bool crt_pass_ready(hc_context ctx, const hc_ntt_plan* plans2, const hc_ntt_plan* plans3, size_t r, const KView& t) {
     (void)ctx;
-    return fused_shape(plans2, plans3, r, t) && cluster_ready(crt_slab12288_kernel<0, false>, SMEM12288) &&
-           cluster_ready(crt_slab12288_kernel<1, false>, SMEM12288) &&
-           cluster_ready(crt_slab12288_kernel<1, true>, SMEM12288);
+    return fused_shape(plans2, plans3, r, t) && resident_clusters(crt_slab12288_kernel<0, false, 128>, 128, SMEM12288) &&
+           resident_clusters(crt_slab12288_kernel<1, false, 128>, 128, SMEM12288) &&
+           resident_clusters(crt_slab12288_kernel<1, true, 128>, 128, SMEM12288);
 }
 
 /// One fused half of a CRT transform over t [count, r, deg_L', deg_K] (dimension 3 contiguous):

@@ -267,15 +267,73 @@ __device__ __forceinline__ auto make_mont(int64_t n, int64_t ninv) {
     else return Mont{n, ninv};
 }
 
-/// Copies a padded tile of `len` elements to global memory, multiplying (mode 2/3) by
-/// mulp[e * me] in Montgomery form.
-template <class MONT>
-__device__ __forceinline__ void line_store(const int64_t* s, int64_t* g, int len, bool mul, const int64_t* mulp,
-                                           int64_t me, const MONT& mont) {
-    for (int e = threadIdx.x; e < len; e += blockDim.x) {
-        int64_t v = s[pad8(e)];
-        if (mul) v = mont.mul(v, mulp[e * me]);
-        g[e] = v;
+/// The last six stages of a line (a factor 64: distances 32 .. 1 forward, 1 .. 32 inverse; first stage s0)
+/// and its way to global memory, multiplying (modes 2 and 3) by mulp[e * me] in Montgomery form.
+/// They act within 64 consecutive elements, so each warp takes 256 of them (32 register groups of
+/// eight per pass) through both passes and the store with warp barriers only: no block barrier, and
+/// no warp waits for another's loads of the multiplier, which are all in flight before the warp turns
+/// the forward pass's eight neighbours per lane into coalesced rows through its part of the tile
+/// (the inverse pass's lanes hold runs of eight already and store from registers). Against block
+/// barriers around each pass and a store loop that loaded its multipliers as it went: pb_to_crt of
+/// [24, 23, 4, 12288] 611 -> 561 us, of [24, 34, 12, 3072] 574 -> 557 us.
+template <int MODE, class SCH, class CTX, class MONT>
+__device__ __forceinline__ void tail64(const CTX& c, int64_t* s, int len, const SCH& sch, int s0, bool reduce_output,
+                                       int64_t* g, const int64_t* mulp, int64_t me, const MONT& mont) {
+    constexpr bool inv = MODE & 1, mul = MODE & 2;
+    SF f[6];
+    bool fuse[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        f[q] = sflags(sch, s0 + q);
+        fuse[q] = f[q].last && reduce_output;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int e0 = (threadIdx.x >> 5) << 8; e0 < len; e0 += blockDim.x << 3) {
+        // groups of eight at distance 8 (lane = 8 block + offset), and of eight neighbours
+        const int ea = e0 + ((lane >> 3) << 6) + (lane & 7), eb = e0 + (lane << 3);
+        int64_t* pa = s + pad8(ea);
+        int64_t* pb = s + pad8(eb);
+        int64_t x[8];
+        if (!inv) {
+#pragma unroll
+            for (int m = 0; m < 8; m++) x[m] = pa[goff(m, 8)];
+            fwd_group<3, true>(c, f, fuse, 0, x);
+#pragma unroll
+            for (int m = 0; m < 8; m++) pa[goff(m, 8)] = x[m];
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 8; m++) x[m] = pb[m];
+            fwd_group<3, false>(c, f + 3, fuse + 3, lane & 7, x);
+            int64_t w[8];
+            if (mul) {
+#pragma unroll
+                for (int m = 0; m < 8; m++) w[m] = mulp[(e0 + 32 * m + lane) * me];
+            }
+#pragma unroll
+            for (int m = 0; m < 8; m++) pb[m] = x[m];
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                int64_t v = s[pad8(e0 + 32 * m + lane)];
+                if (mul) v = mont.mul(v, w[m]);
+                g[e0 + 32 * m + lane] = v;
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < 8; m++) x[m] = pb[m];
+            inv_group<3, false>(c, f, lane & 7, x);
+#pragma unroll
+            for (int m = 0; m < 8; m++) pb[m] = x[m];
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 8; m++) x[m] = pa[goff(m, 8)];
+            inv_group<3, true>(c, f + 3, 0, x);
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                if (mul) x[m] = mont.mul(x[m], mulp[(ea + 8 * m) * me]);
+                g[ea + 8 * m] = x[m];
+            }
+        }
     }
 }
 
@@ -340,80 +398,11 @@ __device__ __forceinline__ void line3072(const SCH& sch, const CTX& c, int64_t* 
     __syncthreads();
     if (!inv) {
         r2_pass<false, 3, 6, 9, 0>(c, s, 384, sch, 2, reduce_output);  // factor 8: distances 256, 128, 64
-        __syncthreads();
-        r2_pass<false, 3, 3, 6, 0>(c, s, 384, sch, 5, reduce_output);  // factor 64: 32, 16, 8
-        __syncthreads();
-        r2_pass<false, 3, 0, 3, 3>(c, s, 384, sch, 8, reduce_output);  // factor 64: 4, 2, 1
     } else {
         r2_pass<true, 3, 6, 9, 0>(c, s, 384, sch, 2, false);  // factor 8: distances 64, 128, 256
-        __syncthreads();
-        r2_pass<true, 3, 0, 3, 3>(c, s, 384, sch, 5, false);  // factor 64: 1, 2, 4
-        __syncthreads();
-        r2_pass<true, 3, 3, 6, 0>(c, s, 384, sch, 8, false);  // factor 64: 8, 16, 32
     }
     __syncthreads();
-    line_store(s, g, 3072, MODE & 2, mulp, me, make_mont<CTX>(mn, mi));
-}
-
-/// [3, 64, 64] line (12288 residues): stages 0 = factor 3 (distance 4096), 1..6 = first factor
-/// 64 (distances 2048 .. 64), 7..12 = second factor 64 (32 .. 1).
-template <int MODE, class SCH, class CTX>
-__device__ __forceinline__ void line12288(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
-                                          int64_t me, int64_t mn, int64_t mi) {
-    constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
-    // pass 1: factor 3 and three stages of the first factor 64, straight from global memory
-    {
-        SF f[4];
-        bool fz[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            f[q] = sflags(sch, q);
-            fz[q] = f[q].last && reduce_output;
-        }
-        // forward: elements o + 512 m + 4096 a (o < 512); inverse: base + 64 m + 4096 a with
-        // base = (gg >> 6) * 512 + (gg & 63)
-        constexpr int span = inv ? 64 : 512;
-        for (int gg = threadIdx.x; gg < 512; gg += blockDim.x) {
-            const int base = inv ? ((gg >> 6) << 9) + (gg & 63) : gg;
-            int64_t x[3][8];
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int m = 0; m < 8; m++) x[a][m] = g[base + span * m + 4096 * a];
-            red_all<24>(c, f[0].red, &x[0][0]);
-            if (!inv) {
-#pragma unroll
-                for (int m = 0; m < 8; m++) fwd3<true>(c, f[0], fz[0], 0, x[0][m], x[1][m], x[2][m]);
-#pragma unroll
-                for (int a = 0; a < 3; a++) fwd_group<3, true>(c, f + 1, fz + 1, 0, x[a]);
-            } else {
-#pragma unroll
-                for (int m = 0; m < 8; m++) inv3(c, f[0], x[0][m], x[1][m], x[2][m]);
-#pragma unroll
-                for (int a = 0; a < 3; a++) inv_group<3, false>(c, f + 1, gg >> 6, x[a]);
-            }
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int m = 0; m < 8; m++) s[pad8(base + span * m + 4096 * a)] = x[a][m];
-        }
-    }
-    __syncthreads();
-    if (!inv) {
-        r2_pass<false, 3, 6, 9, 3>(c, s, 1536, sch, 4, reduce_output);   // factor 64 (a): 256, 128, 64
-        __syncthreads();
-        r2_pass<false, 3, 3, 6, 0>(c, s, 1536, sch, 7, reduce_output);   // factor 64 (b): 32, 16, 8
-        __syncthreads();
-        r2_pass<false, 3, 0, 3, 3>(c, s, 1536, sch, 10, reduce_output);  // factor 64 (b): 4, 2, 1
-    } else {
-        r2_pass<true, 3, 9, 12, 0>(c, s, 1536, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
-        __syncthreads();
-        r2_pass<true, 3, 0, 3, 3>(c, s, 1536, sch, 7, false);   // factor 64 (b): 1, 2, 4
-        __syncthreads();
-        r2_pass<true, 3, 3, 6, 0>(c, s, 1536, sch, 10, false);  // factor 64 (b): 8, 16, 32
-    }
-    __syncthreads();
-    line_store(s, g, 12288, MODE & 2, mulp, me, make_mont<CTX>(mn, mi));
+    tail64<MODE>(c, s, 3072, sch, 5, reduce_output, g, mulp, me, make_mont<CTX>(mn, mi));  // factor 64
 }
 
 /// One of the three 4096-residue blocks of a [3, 64, 64] line, computed by one CTA of a 3-CTA
@@ -487,21 +476,13 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, in
     }
     cluster_sync();  // also a barrier of this CTA
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);   // factor 64 (a): 256, 128, 64
-        __syncthreads();
-        r2_pass<false, 3, 3, 6, 0>(c, s, 512, sch, 7, reduce_output);   // factor 64 (b): 32, 16, 8
-        __syncthreads();
-        r2_pass<false, 3, 0, 3, 3>(c, s, 512, sch, 10, reduce_output);  // factor 64 (b): 4, 2, 1
+        r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
     } else {
         r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
-        __syncthreads();
-        r2_pass<true, 3, 0, 3, 3>(c, s, 512, sch, 7, false);   // factor 64 (b): 1, 2, 4
-        __syncthreads();
-        r2_pass<true, 3, 3, 6, 0>(c, s, 512, sch, 10, false);  // factor 64 (b): 8, 16, 32
     }
     __syncthreads();
-    line_store(s, g + 4096 * blk, 4096, MODE & 2, mulp + (me ? 4096 * blk : 0), me,
-                   make_mont<CTX>(mn, mi));
+    tail64<MODE>(c, s, 4096, sch, 7, reduce_output, g + 4096 * blk, mulp + (me ? 4096 * blk : 0), me,
+                 make_mont<CTX>(mn, mi));  // factor 64 (b)
 }
 
 /// A [3, 64, 64] line with a tile of one 4096-residue block (for kernels that cannot give a CTA the
@@ -548,21 +529,13 @@ __device__ __forceinline__ void line12288_seq(const SCH& sch, const CTX& c, int6
         }
         __syncthreads();
         if (!inv) {
-            r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);   // factor 64 (a): 256, 128, 64
-            __syncthreads();
-            r2_pass<false, 3, 3, 6, 0>(c, s, 512, sch, 7, reduce_output);   // factor 64 (b): 32, 16, 8
-            __syncthreads();
-            r2_pass<false, 3, 0, 3, 3>(c, s, 512, sch, 10, reduce_output);  // factor 64 (b): 4, 2, 1
+            r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
         } else {
             r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
-            __syncthreads();
-            r2_pass<true, 3, 0, 3, 3>(c, s, 512, sch, 7, false);   // factor 64 (b): 1, 2, 4
-            __syncthreads();
-            r2_pass<true, 3, 3, 6, 0>(c, s, 512, sch, 10, false);  // factor 64 (b): 8, 16, 32
         }
         __syncthreads();
-        line_store(s, gb, 4096, MODE & 2, mulp + (me ? 4096 * blk : 0), me,
-                   make_mont<CTX>(mn, mi));
+        tail64<MODE>(c, s, 4096, sch, 7, reduce_output, gb, mulp + (me ? 4096 * blk : 0), me,
+                     make_mont<CTX>(mn, mi));  // factor 64 (b)
         __syncthreads();  // the tile is refilled by the next block
     }
 }

@@ -7,8 +7,8 @@ namespace {
 
 /// [3, 64, 64] lines along dimension 3 as 3-CTA clusters: CTA `blk` of a cluster computes block
 /// blk (4096 residues) of one line.
-template <int MODE, bool FIX>
-__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(128, 6)
+template <int MODE, bool FIX, int THREADS>
+__global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(THREADS, 768 / THREADS)
     ntt_line3_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
     extern __shared__ int64_t smem[];
     const int64_t tile = blockIdx.x / 3;
@@ -32,17 +32,24 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(128, 6)
         P, [&](const auto& sch) { fast::line12288_block<MODE>(sch, c, smem, g, blk, mulp, me, mn, mi, csync); });
 }
 
-template <int MODE, bool FIX>
-hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+template <int MODE, bool FIX, int THREADS>
+hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
     // one 3-CTA cluster per line: a padded 4096-residue block per CTA
     constexpr size_t smem = 4608 * 8;
-    auto kern = ntt_line3_kernel<MODE, FIX>;
+    auto kern = ntt_line3_kernel<MODE, FIX, THREADS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
     if (tiles * 3 > 0x7fffffff) return hc::fail(HC_ERR_UNSUPPORTED, "too many NTT lines in one call");
-    kern<<<(unsigned)(tiles * 3), 128, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
+    kern<<<(unsigned)(tiles * 3), THREADS, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
+}
+/// 128 threads per CTA, or 256 for lines that all fit the device at once (three CTAs per SM, one line
+/// per SM), where a line's own latency is the launch's.
+template <int MODE, bool FIX>
+hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    if (tiles <= hc::num_sms(ctx)) return launch_as<MODE, FIX, 256>(ctx, t, pp, mul, mods, tiles);
+    return launch_as<MODE, FIX, 128>(ctx, t, pp, mul, mods, tiles);
 }
 
 template <bool FIX>

@@ -8,7 +8,7 @@ namespace {
 #endif
 
 /// Specialised dimension-3 NTT: one line (i, j, k) per CTA.
-template <int SHAPE, int MODE, bool FIX, int THREADS, int MINB>
+template <int MODE, bool FIX, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
     extern __shared__ int64_t smem[];
     const int64_t tile = blockIdx.x;
@@ -23,18 +23,27 @@ __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPt
         me = mul.b3 ? 0 : 1;
         mn = mods.n[j], mi = mods.ninv[j];
     }
-    run_line<SHAPE, MODE, FIX>(P, smem, g, mulp, me, mn, mi);
+    run_line3072<MODE, FIX>(P, smem, g, mulp, me, mn, mi);
 }
 
-template <int MODE, bool FIX>
-hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+template <int MODE, bool FIX, int THREADS, int MINB>
+hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
     constexpr size_t smem = (size_t)line_tile_words(HC_SHAPE_L3072) * 8;
-    auto kern = ntt_line_kernel<HC_SHAPE_L3072, MODE, FIX, 128, HC_L3072_MIN_BLOCKS>;
+    auto kern = ntt_line_kernel<MODE, FIX, THREADS, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
-    kern<<<(unsigned)tiles, 128, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
+    kern<<<(unsigned)tiles, THREADS, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
+}
+/// 128 threads per line, eight lines per SM: the fewest idle slots in the last wave, and 8 independent
+/// CTAs to cover each other's barriers. Up to two lines per SM (one element of 24 factors is 288
+/// lines) a line's own latency is the launch's, and 384 threads shorten it: one element at r = 16 41.5
+/// -> 36.7 us per transform; at 384 lines the two are level.
+template <int MODE, bool FIX>
+hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
+    if (tiles <= 2 * (int64_t)hc::num_sms(ctx)) return launch_as<MODE, FIX, 384, 2>(ctx, t, pp, mul, mods, tiles);
+    return launch_as<MODE, FIX, 128, HC_L3072_MIN_BLOCKS>(ctx, t, pp, mul, mods, tiles);
 }
 
 template <bool FIX>

@@ -10,16 +10,14 @@ namespace {
 template <bool FIX>
 using PassCtx = std::conditional_t<FIX, fast::CtxL, fast::Ctx>;
 
-/// One specialised line g of plan P through the CTA's shared-memory line buffer s; FIX: the plan
-/// has the fixed schedule.
-template <int SHAPE, int MODE, bool FIX>
-__device__ __forceinline__ void run_line(const DevPlanHeader* P, int64_t* s, int64_t* g, const int64_t* mulp,
-                                         int64_t me, int64_t mn, int64_t mi) {
+/// One [2, 3, 8, 64] line g of plan P through the CTA's shared-memory line buffer s; FIX: the plan is
+/// fixed.
+template <int MODE, bool FIX>
+__device__ __forceinline__ void run_line3072(const DevPlanHeader* P, int64_t* s, int64_t* g, const int64_t* mulp,
+                                             int64_t me, int64_t mn, int64_t mi) {
     const auto c = make_ctx<PassCtx<FIX>>(P);
-    with_sched<SHAPE, (MODE & 1) != 0, FIX>(P, [&](const auto& sch) {
-        if constexpr (SHAPE == HC_SHAPE_L3072) fast::line3072<MODE>(sch, c, s, g, mulp, me, mn, mi);
-        else fast::line12288<MODE>(sch, c, s, g, mulp, me, mn, mi);
-    });
+    with_sched<HC_SHAPE_L3072, (MODE & 1) != 0, FIX>(
+        P, [&](const auto& sch) { fast::line3072<MODE>(sch, c, s, g, mulp, me, mn, mi); });
 }
 
 /// One specialised column g[0], g[ge], ... of shape SHAPE transformed in registers; it is read
