@@ -46,7 +46,7 @@ struct BarrettLimbs;
 struct BconvConsts {
     const BarrettLimbs* qinv;  // [r] Montgomery factors of the plain lifts of (Q_b / p_u)^-1 mod p_u
     const int64_t* mat;    // [nb][rd + 1][r] conversion matrix; row rd of each block: correction row
-    const int4* mat3;      // [nb][rd][r] rows 0..rd-1 as limbs (m mod 2^29, m >> 29, their sum, 0)
+    const int2* mat2;      // [nb][rd][r] rows 0..rd-1 as limbs (m mod 2^29, m >> 29)
     const int64_t* qmodp;  // [nb][rd]
     const int64_t* qtab;   // [nb][rd][2 qhalf + 1] mul_mont(q, qmodp) for |q| <= qhalf
     const BarrettLimbs* r2;  // [rd] Montgomery factors R^2 mod p_j

@@ -463,7 +463,7 @@ int64_t mul_mont_host(int64_t a, int64_t b, int64_t n, int64_t ninv) {
 /// ucol[b]), as bconv_fused_kernel reads them (BconvConsts):
 ///  - qinv / mat / qmodp / ucol: the reference's factors (the conversion matrix [nb][rd + 1][r] with
 ///    the correction row last in each block);
-///  - mat3: the matrix rows 0..rd-1 as 29-bit limbs (m mod 2^29, m >> 29, their sum), for the
+///  - mat2: the matrix rows 0..rd-1 as 29-bit limbs (m mod 2^29, m >> 29), for the
 ///    kernel's exact int64 multiply-accumulate; it needs |m| < 2^56 and lifts |x| < 2^57, i.e.
 ///    source primes below 2^57 (the ring's RNS factor size rule; checked here all the same);
 ///  - qinv, r2: the Montgomery factors as Barrett limbs (mont_const_limbs);
@@ -472,7 +472,7 @@ int64_t mul_mont_host(int64_t a, int64_t b, int64_t n, int64_t ninv) {
 ///  - corr_limb: whether the correction row (round(2^shift / p_u)) is small enough for the limb
 ///    products too.
 struct BconvTables {
-    DBuf qinv, mat, mat3, qmodp, qtab, r2, ucol;
+    DBuf qinv, mat, mat2, qmodp, qtab, r2, ucol;
     BconvConsts c{};
 };
 
@@ -486,7 +486,7 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
     REQUIRE(maxsrc < ((int64_t)1 << 57), HC_ERR_UNSUPPORTED, "base conversion: source prime above 2^57");
     size_t maxlen = 0;
     for (size_t b = 0; b < nb; b++) maxlen = std::max(maxlen, (size_t)(uc[2 * b + 1] - uc[2 * b]));
-    std::vector<int32_t> m3(nb * rd * r * 4, 0);
+    std::vector<int32_t> m2(nb * rd * r * 2, 0);
     std::vector<BarrettLimbs> qinvl(r), r2l(rd);
     std::vector<int64_t> qtab;
     int64_t maxmq = 0;
@@ -496,10 +496,9 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
                 const int64_t m = mat[(b * (rd + 1) + j) * r + u];
                 REQUIRE(m < ((int64_t)1 << 56) && m > -((int64_t)1 << 56), HC_ERR_UNSUPPORTED,
                         "base conversion: matrix entry above 2^56");
-                const size_t o = ((b * rd + j) * r + u) * 4;
-                m3[o] = (int32_t)(m & ((1 << 29) - 1));
-                m3[o + 1] = (int32_t)(m >> 29);
-                m3[o + 2] = m3[o] + m3[o + 1];
+                const size_t o = ((b * rd + j) * r + u) * 2;
+                m2[o] = (int32_t)(m & ((1 << 29) - 1));
+                m2[o + 1] = (int32_t)(m >> 29);
             }
         for (size_t u = 0; u < r; u++) maxmq = std::max(maxmq, std::abs(mat[(b * (rd + 1) + rd) * r + u]));
     }
@@ -512,14 +511,14 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
                 qtab.push_back(mul_mont_host(q, qm[b * rd + j], dm[j].n, dm[j].neg_inv_n));
     t.qinv = DBuf(ctx, qinvl.data(), r * sizeof(BarrettLimbs));
     t.mat = DBuf(ctx, mat.data(), mat.size() * 8);
-    t.mat3 = DBuf(ctx, m3.data(), m3.size() * 4);
+    t.mat2 = DBuf(ctx, m2.data(), m2.size() * 4);
     t.qmodp = DBuf(ctx, qm.data(), qm.size() * 8);
     t.qtab = DBuf(ctx, qtab.data(), qtab.size() * 8);
     t.r2 = DBuf(ctx, r2l.data(), rd * sizeof(BarrettLimbs));
     t.ucol = DBuf(ctx, uc.data(), uc.size() * 4);
     BconvConsts& c = t.c;
     c.qinv = t.qinv.as<BarrettLimbs>(), c.mat = t.mat.as<int64_t>();
-    c.mat3 = t.mat3.as<int4>(), c.qmodp = t.qmodp.as<int64_t>(), c.qtab = t.qtab.as<int64_t>();
+    c.mat2 = t.mat2.as<int2>(), c.qmodp = t.qmodp.as<int64_t>(), c.qtab = t.qtab.as<int64_t>();
     c.r2 = t.r2.as<BarrettLimbs>(), c.ucol = t.ucol.as<int32_t>();
     c.qhalf = qhalf, c.shift = shift, c.chunk = chunk;
     // the correction row's limb products x0 mq, x1 mq summed over a block stay below 2^63

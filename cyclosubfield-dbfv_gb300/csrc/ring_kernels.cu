@@ -43,47 +43,48 @@ __device__ __forceinline__ void fold_limbs(uint64_t& lo, int64_t& hi, int64_t a0
                    (uint64_t)(s >> 64));
 }
 
-/// One output pair's multiply-accumulate over the lifts u in [lo, hi): the exact sums
-/// sum_u m_u x_u as 128-bit words. Operands are split as v = v1 2^29 + v0 with 0 <= v0 < 2^29;
-/// with |x| < 2^57 and |m| < 2^56 (so |x1| <= 2^28, |m1| <= 2^27) the products x0 m0 < 2^58,
-/// |x1 m1| <= 2^55 and |(x0 + x1)(m0 + m1)| < 2^58.91 add up over 16 terms in int64 without
-/// overflow; the middle column x0 m1 + x1 m0 is the Karatsuba difference of the three sums.
-/// Terms [u, u + n) of one group into the six int64 column sums (xp, p0, p1 at term u).
-template <int N>
-__device__ __forceinline__ void limb_terms(const int2* __restrict__ xp, const int4* __restrict__ p0,
-                                           const int4* __restrict__ p1, int n, int64_t (&s)[6]) {
+/// Multiply-accumulate of O output rows (r limb pairs each, consecutive from m) over the lifts u in
+/// [lo, hi): the exact sums sum_u m_u x_u as 128-bit words h:l. Operands are split as v = v1 2^29 + v0
+/// with 0 <= v0 < 2^29; with |x| < 2^57 and |m| < 2^56 (so |x1| <= 2^28, |m1| <= 2^27) the products
+/// x0 m0 < 2^58, |x1 m1| <= 2^55 and |(x0 + x1)(m0 + m1)| < 2^58.91 add up over 16 terms in int64
+/// without overflow; the middle column x0 m1 + x1 m0 is the Karatsuba difference of the three.
+/// N terms of one group (n of them valid) into the column sums.
+template <int O, int N>
+__device__ __forceinline__ void limb_terms(const int2* __restrict__ xp, const int2* __restrict__ m, int r, int n,
+                                           int64_t (&s)[O][3]) {
 #pragma unroll
     for (int t = 0; t < N; t++) {
         if (N == LIMB_GROUP || t < n) {
             const int2 x = xp[t * BCONV_THREADS];
             const int xs = x.x + x.y;
-            const int4 p = __ldg(p0 + t), q = __ldg(p1 + t);
-            s[0] = mad_wide(x.x, p.x, s[0]);
-            s[1] = mad_wide(x.y, p.y, s[1]);
-            s[2] = mad_wide(xs, p.z, s[2]);
-            s[3] = mad_wide(x.x, q.x, s[3]);
-            s[4] = mad_wide(x.y, q.y, s[4]);
-            s[5] = mad_wide(xs, q.z, s[5]);
+#pragma unroll
+            for (int o = 0; o < O; o++) {
+                const int2 w = __ldg(m + o * r + t);
+                s[o][0] = mad_wide(x.x, w.x, s[o][0]);
+                s[o][1] = mad_wide(x.y, w.y, s[o][1]);
+                s[o][2] = mad_wide(xs, w.x + w.y, s[o][2]);
+            }
         }
     }
 }
-
-__device__ __forceinline__ void limb_mac2(const int2* __restrict__ xcol, const int4* __restrict__ m0,
-                                          const int4* __restrict__ m1, int lo, int hi, uint64_t& l0, int64_t& h0,
-                                          uint64_t& l1, int64_t& h1) {
+template <int O>
+__device__ __forceinline__ void limb_mac(const int2* __restrict__ xcol, const int2* __restrict__ m, int r, int lo, int hi,
+                                         uint64_t (&l)[O], int64_t (&h)[O]) {
+#pragma unroll
+    for (int o = 0; o < O; o++) l[o] = 0, h[o] = 0;
     for (int g0 = lo; g0 < hi; g0 += LIMB_GROUP) {
         const int n = min(LIMB_GROUP, hi - g0);
-        int64_t s[6] = {0, 0, 0, 0, 0, 0};  // a00, a11, am, b00, b11, bm
+        int64_t s[O][3] = {};
         const int2* xp = xcol + g0 * BCONV_THREADS;
         // a full group fully unrolled (every address an immediate offset), a partial one in
         // steps of four
         if (n == LIMB_GROUP) {
-            limb_terms<LIMB_GROUP>(xp, m0 + g0, m1 + g0, n, s);
+            limb_terms<O, LIMB_GROUP>(xp, m + g0, r, n, s);
         } else {
-            for (int t = 0; t < n; t += 4) limb_terms<4>(xp + t * BCONV_THREADS, m0 + g0 + t, m1 + g0 + t, n - t, s);
+            for (int t = 0; t < n; t += 4) limb_terms<O, 4>(xp + t * BCONV_THREADS, m + g0 + t, r, n - t, s);
         }
-        fold_limbs(l0, h0, s[0], s[2] - s[0] - s[1], s[1]);
-        fold_limbs(l1, h1, s[3], s[5] - s[3] - s[4], s[4]);
+#pragma unroll
+        for (int o = 0; o < O; o++) fold_limbs(l[o], h[o], s[o][0], s[o][2] - s[o][0] - s[o][1], s[o][1]);
     }
 }
 
@@ -104,15 +105,53 @@ __device__ __forceinline__ void bconv_store(const BconvArgs& a, const KMods& dm,
         *p = y;
 }
 
-/// BEHZ base conversion of one position per thread (BConvCache::bconv, src/ring.rs:1660-1702,
-/// and the gadget form of :1800-1852). CTA (x, y, z): 128 positions of source row y / nb, output
-/// block y % nb (a gadget digit), outputs [z ochunk, (z + 1) ochunk) of the block; only the
-/// block's own source columns are lifted. The products with the conversion matrix use its limb
-/// form: the shared array holds each lift as its limb pair (x mod 2^29, x >> 29).
-/// ONE_CHUNK: the block's columns form one chunk of the reference's chunked matmul (always for
-/// 57-bit primes); SUB: rescale's subtract-and-multiply store (BconvArgs::sub_mul).
+/// Outputs j .. j + O - 1 of the conversion (dst row j at d + j * s1).
+template <bool ONE_CHUNK, bool SUB, int O>
+__device__ __forceinline__ void bconv_outputs(const BconvArgs& a, const KMods& dm, int b, int j, int u0, int u1,
+                                              const int2* xcol, int64_t q, int64_t* d) {
+    const int2* m = a.c.mat2 + ((int64_t)b * a.rd + j) * a.r;
+    // the subtract-and-multiply store's operands, loaded before the sums so that their latency hides
+    // behind the multiply-accumulate
+    int64_t old[O] = {}, v[O] = {};
+    if constexpr (SUB) {
+#pragma unroll
+        for (int o = 0; o < O; o++) old[o] = d[(j + o) * a.dst.s1];
+    }
+    // the reference's chunked matmul (src/ring.rs:1678-1691) splits the columns into chunks of `chunk` (one
+    // chunk whenever r <= chunk, which holds for all 57-bit bases up to 8192 factors) and
+    // double-reduces each chunk's sum
+    uint64_t l[O];
+    int64_t h[O];
+    bool first = true;
+    for (int c0 = 0; ONE_CHUNK ? first : c0 < a.r; c0 += a.c.chunk) {
+        const int lo = ONE_CHUNK ? u0 : max(c0, u0), hi = ONE_CHUNK ? u1 : min(min(c0 + a.c.chunk, a.r), u1);
+        limb_mac<O>(xcol, m, a.r, lo, hi, l, h);
+#pragma unroll
+        for (int o = 0; o < O; o++) {
+            const int64_t r = mont_red_double(l[o], h[o], mont_limbs(dm.n[j + o], dm.ninv[j + o]));
+            v[o] = first ? r : wadd(v[o], r);
+        }
+        first = false;
+    }
+#pragma unroll
+    for (int o = 0; o < O; o++) bconv_store<SUB>(a, dm, b, j + o, q, v[o], d + (j + o) * a.dst.s1, old[o]);
+}
+
+/// BEHZ base conversion of one position per thread (BConvCache::bconv, src/ring.rs:1660-1702, and the
+/// gadget form of :1800-1852). CTA (x, y, z): 128 positions of source row y / nb, output block y % nb
+/// (a gadget digit), outputs [z ochunk, (z + 1) ochunk) of the block; only the block's own source
+/// columns are lifted. The products with the conversion matrix use its limb form: the shared array
+/// holds each lift as its limb pair (x mod 2^29, x >> 29).
+/// What bounds it: the multiply pipe, 70 % busy; each lane's copy of a matrix entry takes the load path
+/// as long as a lift does, so a thread holds four output rows (one lift and four 8-byte entries for
+/// twelve wide products, the entries' limb sums formed, not read). With two rows and 16-byte entries
+/// the load path was 75 % busy beside 67 % of the multiply pipe: [2, 16 -> 18] of field_36864 32 -> 24
+/// us, [6, 23 -> 24] of field_49152 160 -> 130 us, [24, 16 -> 18] 209 -> 202 us. Two positions per
+/// thread on top take 128 registers and gain nothing.
+/// ONE_CHUNK: the block's columns form one chunk of the reference's chunked matmul (always for 57-bit
+/// primes); SUB: rescale's subtract-and-multiply store (BconvArgs::sub_mul).
 template <bool ONE_CHUNK, bool SUB>
-__global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a, KMods sm, KMods dm) {
+__global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs a, KMods sm, KMods dm) {
     extern __shared__ int2 xs[];  // [r][BCONV_THREADS]
     const int b = (int)(blockIdx.y % (unsigned)a.nb);
     const int64_t i = blockIdx.y / (unsigned)a.nb;
@@ -121,12 +160,11 @@ __global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a,
     const int64_t pos = (int64_t)blockIdx.x * BCONV_THREADS + threadIdx.x;
     if (pos >= a.npos) return;
     const int64_t k = pos / a.src.n3, l = pos - k * a.src.n3;
-    const int64_t* __restrict__ srcp = kat<int64_t>(a.src, i, 0, k, l);       // row u at u * src.s1
-    int64_t* __restrict__ dstp = kat<int64_t>(a.dst, i * a.nb + b, 0, k, l);  // row j at j * dst.s1
+    const int64_t* __restrict__ srcp = kat<int64_t>(a.src, i, 0, k, l);  // row u at u * src.s1
+    int64_t* dstp = kat<int64_t>(a.dst, i * a.nb + b, 0, k, l);          // row j at j * dst.s1
     // the source is multiplied by (Q/p)^-1 in Montgomery form, giving plain lifts in (-p, p)
     for (int u = u0; u < u1; u++) {
-        int64_t x = srcp[u * a.src.s1];
-        x = barrett_mul(load_limbs(a.c.qinv + u), x, mont_const_mod(sm.n[u]));
+        const int64_t x = barrett_mul(load_limbs(a.c.qinv + u), srcp[u * a.src.s1], mont_const_mod(sm.n[u]));
         xs[u * BCONV_THREADS + threadIdx.x] = make_int2((int)(x & ((1 << LIMB_BITS) - 1)), (int)(x >> LIMB_BITS));
     }
     const i128 half = (i128)1 << (a.c.shift - 1);
@@ -153,47 +191,10 @@ __global__ void __launch_bounds__(BCONV_THREADS) bconv_fused_kernel(BconvArgs a,
         }
     }
     const int64_t q = (int64_t)((i128)((u128)corr + (u128)half) >> a.c.shift);
-    // two output rows per pass over the lifts (each lift is read once for both); the
-    // reference's chunked matmul (src/ring.rs:1678-1691) splits the columns into chunks of
-    // `chunk` (one chunk whenever r <= chunk, which holds for all 57-bit bases up to 8192
-    // factors) and double-reduces each chunk's sum
-    for (int j = jbeg; j < jend; j += 2) {
-        const bool two = j + 1 < jend;
-        const int4* __restrict__ m0 = a.c.mat3 + ((int64_t)b * a.rd + j) * a.r;
-        const int4* __restrict__ m1 = two ? m0 + a.r : m0;
-        int64_t v0 = 0, v1 = 0;
-        // the subtract-and-multiply store's operands, loaded before the sums so that their
-        // latency hides behind the multiply-accumulate
-        int64_t old0 = 0, old1 = 0;
-        if constexpr (SUB) {
-            old0 = dstp[j * a.dst.s1];
-            if (two) old1 = dstp[(j + 1) * a.dst.s1];
-        }
-        if constexpr (ONE_CHUNK) {
-            uint64_t l0 = 0, l1 = 0;
-            int64_t h0 = 0, h1 = 0;
-            limb_mac2(xcol, m0, m1, u0, u1, l0, h0, l1, h1);
-            v0 = mont_red_double(l0, h0, mont_limbs(dm.n[j], dm.ninv[j]));
-            v1 = mont_red_double(l1, h1, mont_limbs(dm.n[j + two], dm.ninv[j + two]));
-        } else {
-            bool first = true;
-            for (int c0 = 0; c0 < a.r; c0 += a.c.chunk) {
-                const int lo = max(c0, u0), hi = min(min(c0 + a.c.chunk, a.r), u1);
-                uint64_t l0 = 0, l1 = 0;
-                int64_t h0 = 0, h1 = 0;
-                limb_mac2(xcol, m0, m1, lo, hi, l0, h0, l1, h1);
-                const int64_t r0 = mont_red_double(l0, h0, mont_limbs(dm.n[j], dm.ninv[j]));
-                v0 = first ? r0 : wadd(v0, r0);
-                if (two) {
-                    const int64_t r1 = mont_red_double(l1, h1, mont_limbs(dm.n[j + 1], dm.ninv[j + 1]));
-                    v1 = first ? r1 : wadd(v1, r1);
-                }
-                first = false;
-            }
-        }
-        bconv_store<SUB>(a, dm, b, j, q, v0, dstp + j * a.dst.s1, old0);
-        if (two) bconv_store<SUB>(a, dm, b, j + 1, q, v1, dstp + (j + 1) * a.dst.s1, old1);
-    }
+    int j = jbeg;
+    for (; j + 4 <= jend; j += 4) bconv_outputs<ONE_CHUNK, SUB, 4>(a, dm, b, j, u0, u1, xcol, q, dstp);
+    if (j + 2 <= jend) bconv_outputs<ONE_CHUNK, SUB, 2>(a, dm, b, j, u0, u1, xcol, q, dstp), j += 2;
+    if (j < jend) bconv_outputs<ONE_CHUNK, SUB, 1>(a, dm, b, j, u0, u1, xcol, q, dstp);
 }
 
 /// dst[i,j,k,l] = src[i,j,p2[k],p3[l]]
@@ -547,28 +548,30 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
     a.sub_mul = sub_mul;
     a.npos = src.n2 * src.n3;
     if (a.npos == 0 || ns == 0 || rd == 0) return HC_OK;
-    size_t smem = (size_t)r * BCONV_THREADS * 8;
-    if (smem > 49152) {
-        if (smem > max_smem_optin(ctx)) return fail(HC_ERR_UNSUPPORTED, "base conversion: too many source rows");
-        for (auto kern : {bconv_fused_kernel<true, false>, bconv_fused_kernel<true, true>,
-                          bconv_fused_kernel<false, false>, bconv_fused_kernel<false, true>}) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return cuda_check(e, "bconv smem attribute");
-        }
-    }
     if (ns * nb > 65535) return fail(HC_ERR_UNSUPPORTED, "base conversion: batch too large");
-    // split the outputs over CTAs while the grid is below about two waves of 8 CTAs per SM
-    // (each split recomputes the block's lifts and correction, a small part of the work)
-    const int64_t cols = (a.npos + BCONV_THREADS - 1) / BCONV_THREADS, base_ctas = cols * ns * nb;
-    const int64_t target = (int64_t)num_sms(ctx) * 16;
-    int splits = (int)std::min<int64_t>((target + base_ctas - 1) / base_ctas, (rd + 1) / 2);
-    splits = std::max(splits, 1);
-    a.ochunk = 2 * ((rd + 2 * splits - 1) / (2 * splits));
-    splits = (rd + a.ochunk - 1) / a.ochunk;
-    dim3 grid((unsigned)cols, (unsigned)(ns * nb), (unsigned)splits);
+    const size_t smem = (size_t)r * BCONV_THREADS * 8;
+    if (smem > max_smem_optin(ctx)) return fail(HC_ERR_UNSUPPORTED, "base conversion: too many source rows");
     const bool one_chunk = c.chunk >= r, sub = sub_mul != nullptr;
     auto kern = one_chunk ? (sub ? bconv_fused_kernel<true, true> : bconv_fused_kernel<true, false>)
                           : (sub ? bconv_fused_kernel<false, true> : bconv_fused_kernel<false, false>);
+    if (smem > 49152) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_check(e, "bconv smem attribute");
+    }
+    // the outputs of a position are split over CTAs while the grid leaves SMs short of work; each
+    // split lifts the block's columns again. An SM is busy with four CTAs, so chunks of `oc` outputs
+    // take about max(CTAs per SM, 4) times a CTA's cost, in wide products: 8 per lifted column, and per
+    // output 3 per column and 32 of reductions ([2, 16 -> 18] of field_36864: 24 us whole, 28 us in two)
+    const int64_t cols = (a.npos + BCONV_THREADS - 1) / BCONV_THREADS, base_ctas = cols * ns * nb;
+    const int64_t sms = num_sms(ctx);
+    const int lifted = (r + nb - 1) / nb;  // columns of a block
+    int64_t best = -1;
+    for (int oc = (rd + 1) / 2 * 2; oc >= 2; oc -= 2) {
+        const int64_t n = (base_ctas * ((rd + oc - 1) / oc) + sms - 1) / sms;
+        const int64_t cost = std::max<int64_t>(n, 4) * (8 * lifted + oc * (3 * lifted + 32));
+        if (best < 0 || cost < best) best = cost, a.ochunk = oc;
+    }
+    dim3 grid((unsigned)cols, (unsigned)(ns * nb), (unsigned)((rd + a.ochunk - 1) / a.ochunk));
     kern<<<grid, BCONV_THREADS, smem, stream_of(ctx)>>>(a, sm, dm);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "bconv kernel launch");
