@@ -32,10 +32,21 @@ struct BconvArgs {
     const BarrettLimbs* sub_mul;  // optional [rd]: store mul_mont(dst - v, b_j) instead of v
 };
 
+// Exact multiply-accumulate of 64-bit words in limbs: v = v1 2^29 + v0 with 0 <= v0 < 2^29, three wide
+// products per term (12.75 cycles of the multiply pipe; a 64 x 64 -> 128 product and its 128-bit
+// addition take 33). The middle column x0 y1 + x1 y0 is the Karatsuba difference of the column sums, which
+// may wrap: it is right modulo 2^64, so only x0 y0 (unsigned) and the middle column itself must stay
+// in range.
 constexpr int LIMB_BITS = 29;
-constexpr int LIMB_GROUP = 16;  // terms per int64 partial-sum group
+constexpr int LIMB_UNROLL = 16;  // terms unrolled together
+constexpr int LIMB_TERMS = 28;   // terms whose column sums fit, for |x| < 2^57, |y| < 2^57 (middle: 28 2^58 < 2^63)
+constexpr int LIMB_TERMS2 = 15;  // the same for |x|, |y| <= 2^58, twice a factor (middle: 15 2^59 < 2^63)
 
-/// hi:lo += a00 + a01 2^29 + a11 2^58 (a00 >= 0).
+__device__ __forceinline__ int2 limb_split(int64_t v) {
+    return make_int2((int)(v & ((1 << LIMB_BITS) - 1)), (int)(v >> LIMB_BITS));
+}
+
+/// hi:lo += a00 + a01 2^29 + a11 2^58 (a00 unsigned).
 __device__ __forceinline__ void fold_limbs(uint64_t& lo, int64_t& hi, int64_t a00, int64_t a01, int64_t a11) {
     const u128 s = (u128)lo + (uint64_t)a00 + ((uint64_t)a01 << LIMB_BITS) + ((uint64_t)a11 << (2 * LIMB_BITS));
     lo = (uint64_t)s;
@@ -43,26 +54,33 @@ __device__ __forceinline__ void fold_limbs(uint64_t& lo, int64_t& hi, int64_t a0
                    (uint64_t)(s >> 64));
 }
 
+/// Column sums x0 y0, x1 y1 and (x0 + x1) (y0 + y1) of up to LIMB_TERMS terms.
+struct LimbSum {
+    int64_t a, b, m;
+    __device__ __forceinline__ void zero() { a = b = m = 0; }
+    __device__ __forceinline__ void mac(int2 x, int xs, int2 y, int ys) {
+        a = mad_wide(x.x, y.x, a);
+        b = mad_wide(x.y, y.y, b);
+        m = mad_wide(xs, ys, m);
+    }
+    __device__ __forceinline__ void fold(uint64_t& lo, int64_t& hi) const { fold_limbs(lo, hi, a, wsub(wsub(m, a), b), b); }
+};
+
 /// Multiply-accumulate of O output rows (r limb pairs each, consecutive from m) over the lifts u in
-/// [lo, hi): the exact sums sum_u m_u x_u as 128-bit words h:l. Operands are split as v = v1 2^29 + v0
-/// with 0 <= v0 < 2^29; with |x| < 2^57 and |m| < 2^56 (so |x1| <= 2^28, |m1| <= 2^27) the products
-/// x0 m0 < 2^58, |x1 m1| <= 2^55 and |(x0 + x1)(m0 + m1)| < 2^58.91 add up over 16 terms in int64
-/// without overflow; the middle column x0 m1 + x1 m0 is the Karatsuba difference of the three.
-/// N terms of one group (n of them valid) into the column sums.
+/// [lo, hi): the exact sums sum_u m_u x_u (|x| < 2^57, |m| < 2^56) as 128-bit words h:l.
+/// N terms (n of them valid) into the column sums.
 template <int O, int N>
 __device__ __forceinline__ void limb_terms(const int2* __restrict__ xp, const int2* __restrict__ m, int r, int n,
-                                           int64_t (&s)[O][3]) {
+                                           LimbSum (&s)[O]) {
 #pragma unroll
     for (int t = 0; t < N; t++) {
-        if (N == LIMB_GROUP || t < n) {
+        if (N == LIMB_UNROLL || t < n) {
             const int2 x = xp[t * BCONV_THREADS];
             const int xs = x.x + x.y;
 #pragma unroll
             for (int o = 0; o < O; o++) {
                 const int2 w = __ldg(m + o * r + t);
-                s[o][0] = mad_wide(x.x, w.x, s[o][0]);
-                s[o][1] = mad_wide(x.y, w.y, s[o][1]);
-                s[o][2] = mad_wide(xs, w.x + w.y, s[o][2]);
+                s[o].mac(x, xs, w, w.x + w.y);
             }
         }
     }
@@ -72,19 +90,18 @@ __device__ __forceinline__ void limb_mac(const int2* __restrict__ xcol, const in
                                          uint64_t (&l)[O], int64_t (&h)[O]) {
 #pragma unroll
     for (int o = 0; o < O; o++) l[o] = 0, h[o] = 0;
-    for (int g0 = lo; g0 < hi; g0 += LIMB_GROUP) {
-        const int n = min(LIMB_GROUP, hi - g0);
-        int64_t s[O][3] = {};
-        const int2* xp = xcol + g0 * BCONV_THREADS;
-        // a full group fully unrolled (every address an immediate offset), a partial one in
-        // steps of four
-        if (n == LIMB_GROUP) {
-            limb_terms<O, LIMB_GROUP>(xp, m + g0, r, n, s);
-        } else {
-            for (int t = 0; t < n; t += 4) limb_terms<O, 4>(xp + t * BCONV_THREADS, m + g0 + t, r, n - t, s);
-        }
+    for (int g0 = lo; g0 < hi; g0 += LIMB_TERMS) {
+        const int n = min(LIMB_TERMS, hi - g0);
+        LimbSum s[O];
 #pragma unroll
-        for (int o = 0; o < O; o++) fold_limbs(l[o], h[o], s[o][0], s[o][2] - s[o][0] - s[o][1], s[o][1]);
+        for (int o = 0; o < O; o++) s[o].zero();
+        const int2* xp = xcol + g0 * BCONV_THREADS;
+        // sixteen terms fully unrolled (every address an immediate offset), the rest in steps of four
+        int t = 0;
+        if (n >= LIMB_UNROLL) limb_terms<O, LIMB_UNROLL>(xp, m + g0, r, n, s), t = LIMB_UNROLL;
+        for (; t < n; t += 4) limb_terms<O, 4>(xp + t * BCONV_THREADS, m + g0 + t, r, n - t, s);
+#pragma unroll
+        for (int o = 0; o < O; o++) s[o].fold(l[o], h[o]);
     }
 }
 
@@ -165,7 +182,7 @@ __global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs
     // the source is multiplied by (Q/p)^-1 in Montgomery form, giving plain lifts in (-p, p)
     for (int u = u0; u < u1; u++) {
         const int64_t x = barrett_mul(load_limbs(a.c.qinv + u), srcp[u * a.src.s1], mont_const_mod(sm.n[u]));
-        xs[u * BCONV_THREADS + threadIdx.x] = make_int2((int)(x & ((1 << LIMB_BITS) - 1)), (int)(x >> LIMB_BITS));
+        xs[u * BCONV_THREADS + threadIdx.x] = limb_split(x);
     }
     const i128 half = (i128)1 << (a.c.shift - 1);
     const int2* xcol = xs + threadIdx.x;  // this thread's lifts, stride BCONV_THREADS
@@ -245,10 +262,39 @@ struct KsArgs {
     int reverse;
 };
 
-__device__ __forceinline__ int64_t finish_wide(i128 acc, bool full, const KMods& m, int j) {
-    return full ? to_mont64(double_red128(acc, m.n[j], m.ninv[j]), m.n[j], m.ninv[j], m.r2[j])
-                : red128(acc, m.n[j], m.ninv[j]);
+/// A sum of at most HC_MAX_TERMS + 1 products of words within 2p: reduced once, or twice and back to
+/// Montgomery form.
+__device__ __forceinline__ int64_t finish_wide(uint64_t lo, int64_t hi, bool full, const MontLimbs& m, int64_t r2) {
+    return full ? mont_mul(mont_red_double(lo, hi, m), r2, m) : mont_red(lo, hi, m);
 }
+
+/// R accumulators of one position: one digit word times R key words per step.
+template <int R>
+struct KsAcc {
+    LimbSum s[R];
+    uint64_t lo[R];
+    int64_t hi[R];
+    __device__ __forceinline__ void start() {
+#pragma unroll
+        for (int q = 0; q < R; q++) s[q].zero(), lo[q] = 0, hi[q] = 0;
+    }
+    __device__ __forceinline__ void add(int64_t x, const int64_t (&y)[R]) {
+        const int2 v = limb_split(x);
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            const int2 w = limb_split(y[q]);
+            s[q].mac(v, v.x + v.y, w, w.x + w.y);
+        }
+    }
+    __device__ __forceinline__ void add1(int q, int64_t x, int64_t y) {
+        const int2 v = limb_split(x), w = limb_split(y);
+        s[q].mac(v, v.x + v.y, w, w.x + w.y);
+    }
+    __device__ __forceinline__ void fold() {
+#pragma unroll
+        for (int q = 0; q < R; q++) s[q].fold(lo[q], hi[q]), s[q].zero();
+    }
+};
 
 __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, const int64_t* one, int64_t lines,
                                                         int chunks) {
@@ -260,19 +306,21 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
         int64_t k = line % a.dst.n2, r = line / a.dst.n2;
         int64_t j = r % a.dst.n1, i = r / a.dst.n1;
         const int64_t sk = a.p2 ? (int64_t)a.p2[k] : k, sl = a.p3 ? (int64_t)a.p3[l] : l;
-        i128 acc0 = 0, acc1 = 0;
+        KsAcc<2> acc;
+        acc.start();
         for (int t = 0; t < a.nterms; t++) {
-            int64_t x = *kat<int64_t>(a.parts[t], i, j, sk, sl);
-            int64_t k0 = *kat<int64_t>(a.keys[t], 0, j, k, l);
-            int64_t k1 = *kat<int64_t>(a.keys[t], 1, j, k, l);
-            acc0 = (i128)((u128)acc0 + (u128)((i128)x * (i128)k0));
-            acc1 = (i128)((u128)acc1 + (u128)((i128)x * (i128)k1));
+            const int64_t x = *kat<int64_t>(a.parts[t], i, j, sk, sl);
+            const int64_t y[2] = {*kat<int64_t>(a.keys[t], 0, j, k, l), *kat<int64_t>(a.keys[t], 1, j, k, l)};
+            acc.add(x, y);
+            if ((t + 1) % (LIMB_TERMS2 - 1) == 0) acc.fold();
         }
         const int64_t o = one[j];
-        if (a.has_add0) acc0 = (i128)((u128)acc0 + (u128)((i128)*kat<int64_t>(a.add0, i, j, sk, sl) * (i128)o));
-        if (a.has_add1) acc1 = (i128)((u128)acc1 + (u128)((i128)*kat<int64_t>(a.add1, i, j, sk, sl) * (i128)o));
-        *kat<int64_t>(a.dst, 2 * i, j, k, l) = finish_wide(acc0, a.full0, m, (int)j);
-        *kat<int64_t>(a.dst, 2 * i + 1, j, k, l) = finish_wide(acc1, a.full1, m, (int)j);
+        if (a.has_add0) acc.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl), o);
+        if (a.has_add1) acc.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl), o);
+        acc.fold();
+        const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
+        *kat<int64_t>(a.dst, 2 * i, j, k, l) = finish_wide(acc.lo[0], acc.hi[0], a.full0, ml, m.r2[j]);
+        *kat<int64_t>(a.dst, 2 * i + 1, j, k, l) = finish_wide(acc.lo[1], acc.hi[1], a.full1, ml, m.r2[j]);
     }
 }
 
@@ -290,7 +338,8 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
 /// addresses are one addition each.
 constexpr int KS_STAGES = 3;
 
-template <bool COMMON>
+/// FOLD: more digits than the column sums hold (LIMB_TERMS2), folded into 128-bit sums on the way.
+template <bool COMMON, bool FOLD>
 __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods m, const int64_t* one,
                                                                  int64_t lines, int chunks) {
     __shared__ int64_t sx[KS_STAGES][2][256];
@@ -332,31 +381,34 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
         };
 #pragma unroll
         for (int t = 0; t < KS_STAGES - 1; t++) issue(t);
-        i128 acc00 = 0, acc01 = 0, acc10 = 0, acc11 = 0;  // acc<row><position>
+        KsAcc<2> acc0, acc1;  // rows 0, 1 of the two positions
+        acc0.start(), acc1.start();
         for (int t = 0; t < a.nterms; t++) {
             issue(t + KS_STAGES - 1);
             cp_async_wait<KS_STAGES - 1>();  // digit t's group has landed
             const int s = t % KS_STAGES;
-            const int64_t x0 = sx[s][0][tid], x1 = sx[s][1][tid];
             const longlong2 k0 = skey[s][0][tid], k1 = skey[s][1][tid];
-            acc00 = (i128)((u128)acc00 + (u128)((i128)x0 * (i128)k0.x));
-            acc01 = (i128)((u128)acc01 + (u128)((i128)x1 * (i128)k0.y));
-            acc10 = (i128)((u128)acc10 + (u128)((i128)x0 * (i128)k1.x));
-            acc11 = (i128)((u128)acc11 + (u128)((i128)x1 * (i128)k1.y));
+            const int64_t y0[2] = {k0.x, k1.x}, y1[2] = {k0.y, k1.y};
+            acc0.add(sx[s][0][tid], y0);
+            acc1.add(sx[s][1][tid], y1);
+            if (FOLD && (t + 1) % (LIMB_TERMS2 - 1) == 0) acc0.fold(), acc1.fold();
         }
         cp_async_wait<0>();
         const int64_t o = one[j];
         if (a.has_add0) {
-            acc00 = (i128)((u128)acc00 + (u128)((i128)*kat<int64_t>(a.add0, i, j, sk, sl0) * (i128)o));
-            acc01 = (i128)((u128)acc01 + (u128)((i128)*kat<int64_t>(a.add0, i, j, sk, sl1) * (i128)o));
+            acc0.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl0), o);
+            acc1.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl1), o);
         }
         if (a.has_add1) {
-            acc10 = (i128)((u128)acc10 + (u128)((i128)*kat<int64_t>(a.add1, i, j, sk, sl0) * (i128)o));
-            acc11 = (i128)((u128)acc11 + (u128)((i128)*kat<int64_t>(a.add1, i, j, sk, sl1) * (i128)o));
+            acc0.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl0), o);
+            acc1.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl1), o);
         }
+        acc0.fold(), acc1.fold();
+        const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
+        const int64_t r2 = m.r2[j];
         longlong2 w0, w1;
-        w0.x = finish_wide(acc00, a.full0, m, (int)j), w0.y = finish_wide(acc01, a.full0, m, (int)j);
-        w1.x = finish_wide(acc10, a.full1, m, (int)j), w1.y = finish_wide(acc11, a.full1, m, (int)j);
+        w0.x = finish_wide(acc0.lo[0], acc0.hi[0], a.full0, ml, r2), w0.y = finish_wide(acc1.lo[0], acc1.hi[0], a.full0, ml, r2);
+        w1.x = finish_wide(acc0.lo[1], acc0.hi[1], a.full1, ml, r2), w1.y = finish_wide(acc1.lo[1], acc1.hi[1], a.full1, ml, r2);
         *reinterpret_cast<longlong2*>(kat<int64_t>(a.dst, 2 * i, j, k, l)) = w0;
         *reinterpret_cast<longlong2*>(kat<int64_t>(a.dst, 2 * i + 1, j, k, l)) = w1;
     }
@@ -404,17 +456,28 @@ __global__ void __launch_bounds__(256) tensor_kernel(KView d, KView lhs_lo, KVie
         const int64_t* lp = lo ? kat<int64_t>(lhs_lo, 2 * i, js, k, l) : kat<int64_t>(lhs_hi, 2 * i, js, k, l);
         const int64_t* rp = lo ? kat<int64_t>(rhs_lo, 2 * i, js, k, l) : kat<int64_t>(rhs_hi, 2 * i, js, k, l);
         const int64_t ls = lo ? lhs_lo.s0 : lhs_hi.s0, rs = lo ? rhs_lo.s0 : rhs_hi.s0;
+        const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
+        const int64_t r2 = m.r2[j];
         int64_t l0[W], l1[W], r0[W], r1[W], o0[W], o1[W], o2[W];
         load_words<W>(lp, l0), load_words<W>(lp + ls, l1);
         load_words<W>(rp, r0), load_words<W>(rp + rs, r1);
 #pragma unroll
         for (int w = 0; w < W; w++) {
-            const i128 a0 = (i128)l0[w] * (i128)r0[w];
-            const i128 a1 = (i128)((u128)((i128)l0[w] * (i128)r1[w]) + (u128)((i128)l1[w] * (i128)r0[w]));
-            const i128 a2 = (i128)l1[w] * (i128)r1[w];
-            o0[w] = finish_wide(a0, full0, m, (int)j);
-            o1[w] = finish_wide(a1, full1, m, (int)j);
-            o2[w] = finish_wide(a2, full2, m, (int)j);
+            const int2 x0 = limb_split(l0[w]), x1 = limb_split(l1[w]), y0 = limb_split(r0[w]), y1 = limb_split(r1[w]);
+            const int xs0 = x0.x + x0.y, xs1 = x1.x + x1.y, ys0 = y0.x + y0.y, ys1 = y1.x + y1.y;
+            LimbSum s[3];
+            uint64_t lo[3] = {0, 0, 0};
+            int64_t hi[3] = {0, 0, 0};
+#pragma unroll
+            for (int q = 0; q < 3; q++) s[q].zero();
+            s[0].mac(x0, xs0, y0, ys0);
+            s[1].mac(x0, xs0, y1, ys1), s[1].mac(x1, xs1, y0, ys0);
+            s[2].mac(x1, xs1, y1, ys1);
+#pragma unroll
+            for (int q = 0; q < 3; q++) s[q].fold(lo[q], hi[q]);
+            o0[w] = finish_wide(lo[0], hi[0], full0, ml, r2);
+            o1[w] = finish_wide(lo[1], hi[1], full1, ml, r2);
+            o2[w] = finish_wide(lo[2], hi[2], full2, ml, r2);
         }
         const int64_t B = d.n0 / 3;
         store_words<W>(kat<int64_t>(d, 2 * i, j, k, l), o0);
@@ -463,10 +526,11 @@ struct GiantUnits {
     int n;
 };
 
-__global__ void __launch_bounds__(256) giant_kernel(GiantArgs a, GiantUnits un, KMods m, const int64_t* one,
-                                                    int64_t lines, int chunks) {
-    extern __shared__ int64_t gsm[];  // [GIANT_STAGES][2][256] staging, then the tile's lcoef
-    int64_t* slc = gsm + GIANT_STAGES * 2 * 256;
+template <int NOUT>
+__global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs a, GiantUnits un, KMods m, const int64_t* one,
+                                                             int64_t lines, int chunks) {
+    extern __shared__ int64_t gsm[];  // [GIANT_STAGES][2][256] staging, then the tile's lcoef as limb pairs
+    int2* slc = reinterpret_cast<int2*>(gsm + GIANT_STAGES * 2 * 256);
     const int64_t tiles = lines * chunks;
     const int nt = (int)a.lcoef.n0;
     const int tid = threadIdx.x;
@@ -475,7 +539,7 @@ __global__ void __launch_bounds__(256) giant_kernel(GiantArgs a, GiantUnits un, 
         const int64_t l = (tile - line * chunks) * blockDim.x + tid;
         const int64_t k = line % a.dst.n2, j = line / a.dst.n2;
         __syncthreads();  // the previous tile's readers of slc are done
-        for (int t = tid; t < nt; t += blockDim.x) slc[t] = *kat<int64_t>(a.lcoef, t, j, k, 0);
+        for (int t = tid; t < nt; t += blockDim.x) slc[t] = limb_split(*kat<int64_t>(a.lcoef, t, j, k, 0));
         __syncthreads();
         if (l >= a.dst.n3) continue;
         const int64_t rs = a.babies.s0;  // row stride of the baby-step tensor
@@ -491,38 +555,57 @@ __global__ void __launch_bounds__(256) giant_kernel(GiantArgs a, GiantUnits un, 
         };
 #pragma unroll
         for (int u = 0; u < GIANT_STAGES - 1; u++) issue(u);
-        i128 acc0[GIANT_OUT], acc1[GIANT_OUT];
+        LimbSum s0[NOUT], s1[NOUT];
+        uint64_t lo0[NOUT], lo1[NOUT];
+        int64_t hi0[NOUT], hi1[NOUT];
 #pragma unroll
-        for (int o = 0; o < GIANT_OUT; o++) acc0[o] = acc1[o] = 0;
+        for (int o = 0; o < NOUT; o++) s0[o].zero(), s1[o].zero(), lo0[o] = lo1[o] = 0, hi0[o] = hi1[o] = 0;
+        auto fold = [&] {
+#pragma unroll
+            for (int o = 0; o < NOUT; o++) {
+                s0[o].fold(lo0[o], hi0[o]), s1[o].fold(lo1[o], hi1[o]);
+                s0[o].zero(), s1[o].zero();
+            }
+        };
         for (int u = 0; u < un.n; u++) {
             issue(u + GIANT_STAGES - 1);
             cp_async_wait<GIANT_STAGES - 1>();  // unit u's words have landed
             const unsigned mask = un.w[u] >> 16;
             const int fb = un.fb[u];
             const int64_t* slot = gsm + (u % GIANT_STAGES) * 512;
-            const int64_t x0 = slot[tid], x1 = slot[256 + tid];
+            const int2 x0 = limb_split(slot[tid]), x1 = limb_split(slot[256 + tid]);
+            const int xs0 = x0.x + x0.y, xs1 = x1.x + x1.y;
 #pragma unroll
-            for (int o = 0; o < GIANT_OUT; o++) {
+            for (int o = 0; o < NOUT; o++) {
                 if ((mask >> o) & 1) {
-                    const int64_t f = slc[fb + o];
-                    acc0[o] = (i128)((u128)acc0[o] + (u128)((i128)x0 * (i128)f));
-                    acc1[o] = (i128)((u128)acc1[o] + (u128)((i128)x1 * (i128)f));
+                    const int2 f = slc[fb + o];
+                    s0[o].mac(x0, xs0, f, f.x + f.y);
+                    s1[o].mac(x1, xs1, f, f.x + f.y);
                 }
             }
+            if ((u + 1) % (LIMB_TERMS2 - 1) == 0) fold();
         }
         cp_async_wait<0>();
+        const int64_t on = one[j];
+        const int2 w = limb_split(on);
 #pragma unroll
-        for (int o = 0; o < GIANT_OUT; o++) {
-            if (o >= a.nout) break;
-            const int od = a.out0 + o;
-            if (od < a.nadd) {
-                const int64_t on = one[j];
-                acc0[o] = (i128)((u128)acc0[o] + (u128)((i128)*kat<int64_t>(a.add, 2 * od, j, k, l) * (i128)on));
-                acc1[o] = (i128)((u128)acc1[o] + (u128)((i128)*kat<int64_t>(a.add, 2 * od + 1, j, k, l) * (i128)on));
+        for (int o = 0; o < NOUT; o++) {
+            if (a.out0 + o < a.nadd) {
+                const int2 v0 = limb_split(*kat<int64_t>(a.add, 2 * (a.out0 + o), j, k, l));
+                const int2 v1 = limb_split(*kat<int64_t>(a.add, 2 * (a.out0 + o) + 1, j, k, l));
+                s0[o].mac(v0, v0.x + v0.y, w, w.x + w.y);
+                s1[o].mac(v1, v1.x + v1.y, w, w.x + w.y);
             }
+        }
+        fold();
+        const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
+        const int64_t r2 = m.r2[j];
+#pragma unroll
+        for (int o = 0; o < NOUT; o++) {
             const bool full = (a.full >> o) & 1;
-            *kat<int64_t>(a.dst, 2 * od, j, k, l) = finish_wide(acc0[o], full, m, (int)j);
-            *kat<int64_t>(a.dst, 2 * od + 1, j, k, l) = finish_wide(acc1[o], full, m, (int)j);
+            const int od = a.out0 + o;
+            *kat<int64_t>(a.dst, 2 * od, j, k, l) = finish_wide(lo0[o], hi0[o], full, ml, r2);
+            *kat<int64_t>(a.dst, 2 * od + 1, j, k, l) = finish_wide(lo1[o], hi1[o], full, ml, r2);
         }
     }
 }
@@ -627,8 +710,10 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
         common = common && p.s0 == p0.s0 && p.s1 == p0.s1 && p.s2 == p0.s2 && p.b3 == p0.b3 && k.s0 == k0.s0 &&
                  k.s1 == k0.s1 && k.s2 == k0.s2;
     }
-    if (common) keyswitch_async_kernel<true><<<blocks, 256, 0, stream_of(ctx)>>>(a, m, one_dev, lines, chunks);
-    else keyswitch_async_kernel<false><<<blocks, 256, 0, stream_of(ctx)>>>(a, m, one_dev, lines, chunks);
+    const bool fold = nterms >= LIMB_TERMS2;  // with the summand more than LIMB_TERMS2 terms
+    auto kern = common ? (fold ? keyswitch_async_kernel<true, true> : keyswitch_async_kernel<true, false>)
+                       : (fold ? keyswitch_async_kernel<false, true> : keyswitch_async_kernel<false, false>);
+    kern<<<blocks, 256, 0, stream_of(ctx)>>>(a, m, one_dev, lines, chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "keyswitch kernel launch");
 }
@@ -679,7 +764,11 @@ hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, 
                 un.w[un.n] = (unsigned)row | (mask << 16);
                 un.fb[un.n++] = (short)fb;
             }
-        giant_kernel<<<blocks, 256, smem, stream_of(ctx)>>>(a, un, m, one_dev, lines, chunks);
+        auto kern = a.nout == 1   ? giant_kernel<1>
+                    : a.nout == 2 ? giant_kernel<2>
+                    : a.nout == 3 ? giant_kernel<3>
+                                  : giant_kernel<4>;
+        kern<<<blocks, 256, smem, stream_of(ctx)>>>(a, un, m, one_dev, lines, chunks);
         count_launch(ctx);
         hc_status st = cuda_check(cudaGetLastError(), "giant-step kernel launch");
         if (st) return st;

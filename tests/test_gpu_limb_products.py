@@ -89,3 +89,28 @@ def test_quotients_at_the_rounding_boundary(be, po, p):
     d = be.tensor(data)
     be.hal_intt_mont64_dim(d, [be.hal_create_ntt_plan(be.hal_create_modulus(p), [4])], 2)
     assert (d.to_numpy() == exp).all()
+
+
+@pytest.fixture(scope="module")
+def small_ring(po, be):
+    import ringcuda
+
+    return po.Ring("field_192", 2300, 2340, 4), ringcuda.RingContext("field_192", 2300, 2340, 4, backend=be)
+
+
+@pytest.mark.parametrize("r,rd", [(1, 1), (1, 6), (2, 3), (3, 2), (15, 5), (16, 4), (17, 7), (28, 9), (29, 1), (31, 2), (33, 8)])
+def test_base_conversion_sizes(small_ring, r, rd):
+    """Base conversions around the kernel's edges: output remainders of 1, 2 and 3 rows behind groups of four, source
+    counts around its groups of columns, and positions that end inside a CTA; residues at +-(p - 1), 0 and random."""
+    o, d = small_ring
+    src, dst = list(range(r)), list(range(r, r + rd))
+    g = np.random.default_rng(r * 100 + rd)
+    x = np.empty(o.shape(3, r), dtype=np.int64)
+    for j, i in enumerate(src):
+        p = o.primes[i]
+        x[0, j] = g.choice(np.array([p - 1, 1 - p, 0, 1, -1]), size=x[0, j].shape)
+        x[1, j] = g.integers(1 - p, p, size=x[1, j].shape)
+        x[2, j] = p - 1
+    out = d.allocate(3, rd)
+    d.bconv(out, dst, d.tensor(x), src)
+    assert (out.to_numpy() == o.bconv(x, src, dst)).all()
