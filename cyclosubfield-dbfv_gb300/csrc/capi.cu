@@ -52,6 +52,7 @@ hc_status destroy_plan(hc_ntt_plan p);
 hc_status launch_ntt(hc_context ctx, const KView& t, const hc_ntt_plan* plans, size_t nplans, int dim, int mode,
                      const KView& mul, const KMods& mods, const KView* src = nullptr);
 bool ntt_column_path(const hc_ntt_plan* plans, size_t nplans, int dim);
+bool ntt_limb_path(const hc_ntt_plan* plans, size_t nplans, int dim);
 hc_status launch_pointwise(hc_context ctx, int op, const KView& d, const KView& a, const KView& b, const KMods& m);
 hc_status launch_matmul(hc_context ctx, const KView& d, const KView& lhs, const KView& rhs, int64_t U);
 hc_status launch_inner_product(hc_context ctx, const KView& d, const KView* l, const KView* r, int n);
@@ -426,37 +427,50 @@ hc_status intt_mul_mont64_dim(hc_context ctx, hc_view dst, const hc_ntt_plan* pl
     return ntt_call(ctx, dst, plans, nplans, dim, 3, &mul, mods, nmods);
 }
 
-/// hc_assign(dst, src) followed by hc_ntt_mul_mont64_dim on dst, with the copy folded into the
-/// transform's reads where the column kernel runs the call; used by the ring layer.
-hc_status ntt_mul_mont64_dim_from(hc_context ctx, hc_view dst, hc_view src, const hc_ntt_plan* plans, size_t nplans,
-                                  hc_data_dim dim, hc_view mul, const hc_modulus* mods, size_t nmods) {
+/// hc_assign(dst, src) (with `src`) followed by the forward transform of dst along `dim` times the ring's
+/// kernel: hc_ntt_mul_mont64_dim by `mul` ([1, r, deg_L', 1] or [1, r, 1, deg_K]), or by the same
+/// kernel as a table of limbs ([r][extent of dim], mont_const_limbs) where the specialised kernels run
+/// the call. The copy is folded into the transform's reads where the column kernel runs it.
+hc_status ntt_kernel_dim(hc_context ctx, hc_view dst, const hc_view* src, const hc_ntt_plan* plans, size_t nplans,
+                         hc_data_dim dim, hc_view mul, const BarrettLimbs* limbs, const hc_modulus* mods, size_t nmods) {
     hc_status st;
     if (!ctx) return fail(HC_ERR_ARG, "null context");
     if (nplans && !plans) return fail(HC_ERR_ARG, "null plans");
-    // the column kernel reads each column whole before writing it: an exact alias is an in-place
-    // call; any other overlap of the two views' address ranges takes the copy path
-    auto range = [](const hc_view& v, const char** lo, const char** hi) {
-        int64_t last = 0;
-        for (int d = 0; d < 4; d++) last += (v.shape[d] > 0 ? v.shape[d] - 1 : 0) * (d == 3 ? 1 : v.strides[d]);
-        *lo = (const char*)v.ptr;
-        *hi = (const char*)v.ptr + 8 * (last + 1);
-    };
-    const char *dl, *dh, *sl, *sh;
-    range(dst, &dl, &dh);
-    range(src, &sl, &sh);
-    const bool overlap = src.ptr != dst.ptr && sl < dh && dl < sh;
-    if (overlap || !ntt_column_path(plans, nplans, (int)dim)) {
-        if ((st = hc_assign(ctx, dst, src))) return st;
-        return ntt_call(ctx, dst, plans, nplans, dim, 2, &mul, mods, nmods);
+    if ((st = check_view(dst, "dst"))) return st;
+    KView s;
+    const KView* from = nullptr;
+    if (src) {
+        // the column kernel reads each column whole before writing it: an exact alias is an in-place
+        // call; any other overlap of the two views' address ranges takes the copy path
+        auto range = [](const hc_view& v, const char** lo, const char** hi) {
+            int64_t last = 0;
+            for (int d = 0; d < 4; d++) last += (v.shape[d] > 0 ? v.shape[d] - 1 : 0) * (d == 3 ? 1 : v.strides[d]);
+            *lo = (const char*)v.ptr;
+            *hi = (const char*)v.ptr + 8 * (last + 1);
+        };
+        const char *dl, *dh, *sl, *sh;
+        range(dst, &dl, &dh);
+        range(*src, &sl, &sh);
+        const bool overlap = src->ptr != dst.ptr && sl < dh && dl < sh;
+        if (overlap || !ntt_column_path(plans, nplans, (int)dim)) {
+            if ((st = hc_assign(ctx, dst, *src))) return st;
+        } else {
+            if ((st = check_view(*src, "src"))) return st;
+            for (int d = 0; d < 4; d++)
+                if (src->shape[d] != dst.shape[d]) return fail(HC_ERR_SHAPE, "source and destination shapes differ");
+            s = kview(*src);
+            from = &s;
+        }
     }
-    if ((st = check_view(dst, "dst")) || (st = check_view(src, "src"))) return st;
-    for (int d = 0; d < 4; d++)
-        if (src.shape[d] != dst.shape[d]) return fail(HC_ERR_SHAPE, "source and destination shapes differ");
-    KView t = kview(dst), s = kview(src), m = t;
+    KView t = kview(dst), m = t;
     KMods km;
     if ((st = bview(mul, dst.shape, "mul", &m))) return st;
     if ((st = kmods(mods, nmods, dst.shape[1], &km))) return st;
-    return launch_ntt(ctx, t, plans, nplans, (int)dim, 2, m, km, &s);
+    if (!limbs || !ntt_limb_path(plans, nplans, (int)dim))
+        return launch_ntt(ctx, t, plans, nplans, (int)dim, 2, m, km, from);
+    m.p = (char*)limbs;
+    m.s0 = 0, m.s1 = dst.shape[(int)dim], m.s2 = dim == HC_DIM2 ? 1 : 0, m.b3 = dim == HC_DIM2;
+    return launch_ntt(ctx, t, plans, nplans, (int)dim, 6, m, km, from);
 }
 }  // namespace hc
 

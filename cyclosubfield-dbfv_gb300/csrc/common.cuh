@@ -321,11 +321,9 @@ __host__ __device__ __forceinline__ BarrettMod mont_const_mod(int64_t n) {
     m.red_add = m.red_shift = 0;
     return m;
 }
-inline BarrettLimbs mont_const_limbs(int64_t b, int64_t n) {
-    uint64_t inv = 1;  // n^-1 mod 2^64
-    for (int i = 0; i < 6; i++) inv *= 2 - (uint64_t)n * inv;
+inline BarrettLimbs mont_const_limbs(int64_t b, int64_t n, int64_t ninv) {
     // b' 2^64 = b + n s with s = -b n^-1 mod 2^64; signed s keeps b' centred
-    const i128 s = (int64_t)(0 - (uint64_t)b * inv);
+    const i128 s = (int64_t)((uint64_t)b * (uint64_t)ninv);
     const i128 z = ((i128)b + s * n) >> 64;
     i128 u = s, zz = z;
     if (u >= ((i128)1 << 63) - ((i128)1 << 31)) u -= (i128)1 << 64, zz -= n;
@@ -362,8 +360,10 @@ struct CrtSlab {
     const void* plan3;     // NTT plan along dimension 3 (length deg_K)
     int64_t* data;         // row k at data + k * s2, contiguous
     const int64_t* op;     // operand slab (HC_CRT_MUL), row k at op + k * op_s2
-    const int64_t* kl;     // CRT kernel of this factor along dimension 2 (deg_L' entries)
-    const int64_t* kk;     // ... along dimension 3 (deg_K entries)
+    // CRT kernel of this factor along dimension 2 (deg_L' entries) and 3 (deg_K entries): Montgomery
+    // words, or BarrettLimbs where the dimension's shape is specialised and its plan fixed (`shapes`)
+    const int64_t* kl;
+    const int64_t* kk;
     const int64_t* ikl;    // inverse kernels
     const int64_t* ikk;
     int64_t s2, op_s2;
@@ -398,7 +398,7 @@ size_t max_smem_optin(hc_context ctx);
 int device_of(hc_context ctx);
 hc_status intt_mul_mont64_dim(hc_context ctx, hc_view dst, const hc_ntt_plan* plans, size_t nplans, hc_data_dim dim,
                               hc_view mul, const hc_modulus* mods, size_t nmods);
-hc_status ntt_mul_mont64_dim_from(hc_context ctx, hc_view dst, hc_view src, const hc_ntt_plan* plans, size_t nplans,
-                                  hc_data_dim dim, hc_view mul, const hc_modulus* mods, size_t nmods);
+hc_status ntt_kernel_dim(hc_context ctx, hc_view dst, const hc_view* src, const hc_ntt_plan* plans, size_t nplans,
+                         hc_data_dim dim, hc_view mul, const BarrettLimbs* limbs, const hc_modulus* mods, size_t nmods);
 
 }  // namespace hc

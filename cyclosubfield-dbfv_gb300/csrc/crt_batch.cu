@@ -23,12 +23,15 @@ size_t crt_slab_tile_words(int32_t shapes, int32_t dl, int32_t dk, int logv) {
     return (w + 1) & ~(size_t)1;
 }
 
-/// Whether a slab runs entirely on the specialised line and column code (crt_batch_kernel<false>).
-bool crt_slab_specialised(int32_t shapes) {
+/// Whether slab_pass runs the passes along `dim` on the specialised code, with the CRT kernels as limbs.
+bool crt_slab_limbs(int32_t shapes, int dim) {
     const int s3 = shapes & 0xff, s2 = (shapes >> 8) & 0xff;
-    return ((shapes >> 16) & 1) && (s3 == HC_SHAPE_L3072 || s3 == HC_SHAPE_L12288) && ((shapes >> 17) & 1) &&
-           (s2 == HC_SHAPE_C12 || s2 == HC_SHAPE_C4);
+    return dim == 3 ? ((shapes >> 16) & 1) && (s3 == HC_SHAPE_L3072 || s3 == HC_SHAPE_L12288)
+                    : ((shapes >> 17) & 1) && (s2 == HC_SHAPE_C12 || s2 == HC_SHAPE_C4);
 }
+
+/// Whether a slab runs entirely on the specialised line and column code (crt_batch_kernel<false>).
+bool crt_slab_specialised(int32_t shapes) { return crt_slab_limbs(shapes, 3) && crt_slab_limbs(shapes, 2); }
 
 /// Shape class of specialised slab shapes (crt_batch_kernel's CLS): 1 field_36864, 2 field_49152
 /// (CLS 0: a launch over both).

@@ -21,7 +21,7 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
             int64_t* g = S.data + k * S.s2;
             const int64_t* mulp = mode == 3 ? S.op + k * S.op_s2 : mulrow;
             if (CLS != 2 && (CLS == 1 || shape == HC_SHAPE_L3072)) {
-                if (mode == 2) run_line3072<2, true>(P, s, g, mulp, 1, S.n, S.ninv);
+                if (mode == 2) run_line3072<6, true>(P, s, g, mulp, 1, S.n, S.ninv);
                 else if (mode == 3) run_line3072<3, true>(P, s, g, mulp, 1, S.n, S.ninv);
                 else run_line3072<1, true>(P, s, g, mulp, 1, S.n, S.ninv);
             } else if (CLS != 1) {
@@ -34,7 +34,7 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
                     });
                 } else {  // mode 2: forward, then the kernel product
                     with_sched<HC_SHAPE_L12288, false, true>(
-                        P, [&](const auto& sch) { fast::line12288_seq<2>(sch, c, s, g, mulp, 1, S.n, S.ninv); });
+                        P, [&](const auto& sch) { fast::line12288_seq<6>(sch, c, s, g, mulp, 1, S.n, S.ninv); });
                 }
             }
             __syncthreads();
@@ -45,10 +45,10 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
         for (int l = threadIdx.x; l < S.dk; l += blockDim.x) {
             int64_t* g = S.data + l;
             if (CLS != 2 && (CLS == 1 || shape == HC_SHAPE_C12)) {
-                if (mode == 2) run_column<HC_SHAPE_C12, 2, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
+                if (mode == 2) run_column<HC_SHAPE_C12, 6, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
                 else run_column<HC_SHAPE_C12, 1, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
             } else if (CLS != 1) {
-                if (mode == 2) run_column<HC_SHAPE_C4, 2, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
+                if (mode == 2) run_column<HC_SHAPE_C4, 6, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
                 else run_column<HC_SHAPE_C4, 1, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
             }
         }

@@ -413,8 +413,21 @@ bool ntt_column_path(const hc_ntt_plan* plans, size_t nplans, int dim) {
     return shape == HC_SHAPE_C12 || shape == HC_SHAPE_C4;
 }
 
+/// Whether launch_ntt can run a call with its multipliers as a table of limbs (mode 6): the specialised
+/// kernels over fixed plans.
+bool ntt_limb_path(const hc_ntt_plan* plans, size_t nplans, int dim) {
+    if (nplans == 0 || !plans[0]) return false;
+    const int shape = plans[0]->shape;
+    for (size_t j = 0; j < nplans; j++)
+        if (!plans[j] || plans[j]->shape != shape || !plans[j]->fixed) return false;
+    return dim == 2 ? shape == HC_SHAPE_C12 || shape == HC_SHAPE_C4 : shape == HC_SHAPE_L3072 || shape == HC_SHAPE_L12288;
+}
+
+/// mode 6: the forward transform times the limb table mul.p (BarrettLimbs elements, strides in them);
+/// only where ntt_limb_path holds.
 hc_status launch_ntt(hc_context ctx, const KView& t, const hc_ntt_plan* plans, size_t nplans, int dim, int mode,
                      const KView& mul, const KMods& mods, const KView* src) {
+    if (mode == 6 && !ntt_limb_path(plans, nplans, dim)) return fail(HC_ERR_UNSUPPORTED, "limb multipliers of a general NTT");
     if (src && !ntt_column_path(plans, nplans, dim)) return fail(HC_ERR_UNSUPPORTED, "out-of-place NTT form");
     if ((int64_t)nplans != t.n1) return fail(HC_ERR_SHAPE, "one NTT plan per RNS row required");
     if (nplans > HC_MAX_MODS) return fail(HC_ERR_UNSUPPORTED, "too many RNS rows in one call");
@@ -445,7 +458,7 @@ hc_status launch_ntt(hc_context ctx, const KView& t, const hc_ntt_plan* plans, s
         if (tiles <= 0x7fffffff)
             return launch_ntt_col(ctx, shape, mode, fix, t, pp, mul, mods, tiles, (int)ncb, src ? *src : KView());
     }
-    if (src) return fail(HC_ERR_UNSUPPORTED, "out-of-place NTT form");
+    if (src || mode == 6) return fail(HC_ERR_UNSUPPORTED, "specialised NTT form");
     int V = 1, logv = 0;
     int64_t ntile2 = 1;
     if (dim == 2) {

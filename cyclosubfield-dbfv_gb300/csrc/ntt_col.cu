@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(HC_COL_THREADS, SHAPE == HC_SHAPE_C12 ? HC_COL
     const int64_t* mulp = nullptr;
     int64_t ms = 0, mn = 0, mi = 0;
     if (MODE & 2) {
-        mulp = kat<int64_t>(mul, i, j, 0, l);
+        mulp = multiplier<MODE>(mul, i, j, 0, l);
         ms = mul.s2;
         mn = mods.n[j], mi = mods.ninv[j];
     }
@@ -48,6 +48,7 @@ hc_status launch_mode(hc_context ctx, int mode, const KView& t, const PlanPtrs& 
     if (mode == 0) return launch<SHAPE, 0, FIX>(ctx, t, pp, mul, mods, tiles, ncb, src);
     if (mode == 1) return launch<SHAPE, 1, FIX>(ctx, t, pp, mul, mods, tiles, ncb, src);
     if (mode == 2) return launch<SHAPE, 2, FIX>(ctx, t, pp, mul, mods, tiles, ncb, src);
+    if (FIX && mode == 6) return launch<SHAPE, 6, true>(ctx, t, pp, mul, mods, tiles, ncb, src);
     return launch<SHAPE, 3, FIX>(ctx, t, pp, mul, mods, tiles, ncb, src);
 }
 

@@ -252,19 +252,39 @@ __device__ __forceinline__ void r2_pass(const CTX& c, int64_t* s, int ngroups, c
 // ---------------------------------------------------------------- lines
 
 /// The Montgomery product of modes 2 and 3: mul_mont for any modulus, its limb form beside the limb
-/// Barrett products.
+/// Barrett products, and for a mode with bit 2 (6: forward, multipliers in a table of limbs) the
+/// product by a constant (mont_const_limbs: 8 multiplications instead of 12).
 struct Mont {
     int64_t n, ninv;
-    __device__ __forceinline__ int64_t mul(int64_t a, int64_t b) const { return mul_mont(a, b, n, ninv); }
+    typedef int64_t W;
+    __device__ __forceinline__ W load(const int64_t* p, int64_t i) const { return p[i]; }
+    __device__ __forceinline__ int64_t mul(int64_t a, W b) const { return mul_mont(a, b, n, ninv); }
 };
 struct MontL {
     MontLimbs m;
-    __device__ __forceinline__ int64_t mul(int64_t a, int64_t b) const { return mont_mul(a, b, m); }
+    typedef int64_t W;
+    __device__ __forceinline__ W load(const int64_t* p, int64_t i) const { return p[i]; }
+    __device__ __forceinline__ int64_t mul(int64_t a, W b) const { return mont_mul(a, b, m); }
 };
-template <class CTX>
+struct MontC {
+    BarrettMod m;
+    typedef BarrettLimbs W;
+    __device__ __forceinline__ W load(const int64_t* p, int64_t i) const {
+        return load_limbs(reinterpret_cast<const BarrettLimbs*>(p) + i);
+    }
+    __device__ __forceinline__ int64_t mul(int64_t a, const W& b) const { return barrett_mul(b, a, m); }
+};
+template <class CTX, int MODE>
 __device__ __forceinline__ auto make_mont(int64_t n, int64_t ninv) {
-    if constexpr (CTX::LIMBS) return MontL{mont_limbs(n, ninv)};
+    if constexpr ((MODE & 4) != 0) return MontC{mont_const_mod(n)};
+    else if constexpr (CTX::LIMBS) return MontL{mont_limbs(n, ninv)};
     else return Mont{n, ninv};
+}
+
+/// The multipliers of 4096-residue block blk of a line (words, or limbs of 16 bytes; me = 0: one for all).
+template <int MODE>
+__device__ __forceinline__ const int64_t* block_multiplier(const int64_t* mulp, int64_t me, int blk) {
+    return mulp + me * 4096 * blk * ((MODE & 4) ? 2 : 1);
 }
 
 /// The last six stages of a line (a factor 64: distances 32 .. 1 forward, 1 .. 32 inverse; first stage s0)
@@ -304,10 +324,11 @@ __device__ __forceinline__ void tail64(const CTX& c, int64_t* s, int len, const 
 #pragma unroll
             for (int m = 0; m < 8; m++) x[m] = pb[m];
             fwd_group<3, false>(c, f + 3, fuse + 3, lane & 7, x);
-            int64_t w[8];
+            constexpr int AHEAD = sizeof(typename MONT::W) == 8 ? 8 : 2;  // multipliers in registers
+            typename MONT::W w[AHEAD];
             if (mul) {
 #pragma unroll
-                for (int m = 0; m < 8; m++) w[m] = mulp[(e0 + 32 * m + lane) * me];
+                for (int m = 0; m < AHEAD; m++) w[m] = mont.load(mulp, (e0 + 32 * m + lane) * me);
             }
 #pragma unroll
             for (int m = 0; m < 8; m++) pb[m] = x[m];
@@ -315,7 +336,10 @@ __device__ __forceinline__ void tail64(const CTX& c, int64_t* s, int len, const 
 #pragma unroll
             for (int m = 0; m < 8; m++) {
                 int64_t v = s[pad8(e0 + 32 * m + lane)];
-                if (mul) v = mont.mul(v, w[m]);
+                if (mul) {
+                    v = mont.mul(v, w[m % AHEAD]);
+                    if (m + AHEAD < 8) w[m % AHEAD] = mont.load(mulp, (e0 + 32 * (m + AHEAD) + lane) * me);
+                }
                 g[e0 + 32 * m + lane] = v;
             }
         } else {
@@ -330,7 +354,7 @@ __device__ __forceinline__ void tail64(const CTX& c, int64_t* s, int len, const 
             inv_group<3, true>(c, f + 3, 0, x);
 #pragma unroll
             for (int m = 0; m < 8; m++) {
-                if (mul) x[m] = mont.mul(x[m], mulp[(ea + 8 * m) * me]);
+                if (mul) x[m] = mont.mul(x[m], mont.load(mulp, (ea + 8 * m) * me));
                 g[ea + 8 * m] = x[m];
             }
         }
@@ -402,7 +426,7 @@ __device__ __forceinline__ void line3072(const SCH& sch, const CTX& c, int64_t* 
         r2_pass<true, 3, 6, 9, 0>(c, s, 384, sch, 2, false);  // factor 8: distances 64, 128, 256
     }
     __syncthreads();
-    tail64<MODE>(c, s, 3072, sch, 5, reduce_output, g, mulp, me, make_mont<CTX>(mn, mi));  // factor 64
+    tail64<MODE>(c, s, 3072, sch, 5, reduce_output, g, mulp, me, make_mont<CTX, MODE>(mn, mi));  // factor 64
 }
 
 /// One of the three 4096-residue blocks of a [3, 64, 64] line, computed by one CTA of a 3-CTA
@@ -481,61 +505,71 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, in
         r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
     }
     __syncthreads();
-    tail64<MODE>(c, s, 4096, sch, 7, reduce_output, g + 4096 * blk, mulp + (me ? 4096 * blk : 0), me,
-                 make_mont<CTX>(mn, mi));  // factor 64 (b)
+    tail64<MODE>(c, s, 4096, sch, 7, reduce_output, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me,
+                 make_mont<CTX, MODE>(mn, mi));  // factor 64 (b)
 }
 
-/// A [3, 64, 64] line with a tile of one 4096-residue block (for kernels that cannot give a CTA the
-/// whole 12288-residue line): stage 0, the factor-3 stage that couples the three blocks, runs in
-/// place in global memory, each thread owning whole position triples (the butterfly of line12288's
-/// first pass); stages 1..12, which act within a block, then run block by block exactly as
-/// line12288_block runs them. The first pass's global writes are the CTA's own, visible to its
-/// threads after the barrier.
-template <int MODE, class SCH, class CTX>
-__device__ __forceinline__ void line12288_seq(const SCH& sch, const CTX& c, int64_t* s, int64_t* g,
-                                              const int64_t* mulp, int64_t me, int64_t mn, int64_t mi) {
+/// Stages 1..12 of one 4096-residue block of a [3, 64, 64] line (the two factors 64, which act within the
+/// block): g -> g via the padded tile s; mulp: the block's multipliers.
+template <int MODE, class SCH, class CTX, class MONT>
+__device__ __forceinline__ void block4096(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
+                                          int64_t me, const MONT& mont) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
-    SF f[4];
-    bool fz[4];
+    {
+        SF f[3];
+        bool fz[3];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        f[q] = sflags(sch, q);
-        fz[q] = f[q].last && reduce_output;
-    }
-    for (int p = threadIdx.x; p < 4096; p += blockDim.x) {
-        int64_t a = g[p], b = g[p + 4096], d = g[p + 8192];
-        if (f[0].red) {
-            a = red1(c, a);
-            b = red1(c, b);
-            d = red1(c, d);
+        for (int q = 0; q < 3; q++) {
+            f[q] = sflags(sch, 1 + q);
+            fz[q] = f[q].last && reduce_output;
         }
-        if (!inv) fwd3<true>(c, f[0], fz[0], 0, a, b, d);
-        else inv3(c, f[0], a, b, d);
-        g[p] = a, g[p + 4096] = b, g[p + 8192] = d;
-    }
-    __syncthreads();
-    constexpr int span = inv ? 64 : 512;
-    for (int blk = 0; blk < 3; blk++) {
-        int64_t* gb = g + 4096 * blk;
+        // factor 64 (a): distances 2048, 1024, 512 forward, 64, 128, 256 inverse, straight from global memory
+        constexpr int span = inv ? 64 : 512;
         for (int gg = threadIdx.x; gg < 512; gg += blockDim.x) {
             const int base = inv ? ((gg >> 6) << 9) + (gg & 63) : gg;
             int64_t x[8];
 #pragma unroll
-            for (int m = 0; m < 8; m++) x[m] = gb[base + span * m];
-            if (!inv) fwd_group<3, true>(c, f + 1, fz + 1, 0, x);
-            else inv_group<3, false>(c, f + 1, gg >> 6, x);
+            for (int m = 0; m < 8; m++) x[m] = g[base + span * m];
+            if (!inv) fwd_group<3, true>(c, f, fz, 0, x);
+            else inv_group<3, false>(c, f, gg >> 6, x);
 #pragma unroll
             for (int m = 0; m < 8; m++) s[pad8(base + span * m)] = x[m];
         }
-        __syncthreads();
-        if (!inv) {
-            r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
-        } else {
-            r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
+    }
+    __syncthreads();
+    if (!inv) {
+        r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
+    } else {
+        r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
+    }
+    __syncthreads();
+    tail64<MODE>(c, s, 4096, sch, 7, reduce_output, g, mulp, me, mont);  // factor 64 (b)
+}
+
+/// A [3, 64, 64] line with a tile of one 4096-residue block (for kernels that cannot give a CTA the
+/// whole 12288-residue line): stage 0, the factor-3 stage that couples the three blocks, runs in
+/// place in global memory, each thread owning whole position triples (the butterfly of
+/// first pass); stages 1..12, which act within a block, then run block by block. The first pass's global writes are the CTA's own, visible to its
+/// threads after the barrier.
+template <int MODE, class SCH, class CTX>
+__device__ __forceinline__ void line12288_seq(const SCH& sch, const CTX& c, int64_t* s, int64_t* g,
+                                              const int64_t* mulp, int64_t me, int64_t mn, int64_t mi) {
+    constexpr bool inv = MODE & 1;
+    const SF f = sflags(sch, 0);
+    for (int p = threadIdx.x; p < 4096; p += blockDim.x) {
+        int64_t a = g[p], b = g[p + 4096], d = g[p + 8192];
+        if (f.red) {
+            a = red1(c, a);
+            b = red1(c, b);
+            d = red1(c, d);
         }
-        __syncthreads();
-        tail64<MODE>(c, s, 4096, sch, 7, reduce_output, gb, mulp + (me ? 4096 * blk : 0), me,
-                     make_mont<CTX>(mn, mi));  // factor 64 (b)
+        if (!inv) fwd3<true>(c, f, false, 0, a, b, d);
+        else inv3(c, f, a, b, d);
+        g[p] = a, g[p + 4096] = b, g[p + 8192] = d;
+    }
+    __syncthreads();
+    for (int blk = 0; blk < 3; blk++) {
+        block4096<MODE>(sch, c, s, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me, make_mont<CTX, MODE>(mn, mi));
         __syncthreads();  // the tile is refilled by the next block
     }
 }

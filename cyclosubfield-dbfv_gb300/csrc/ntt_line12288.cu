@@ -20,7 +20,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(THREADS, 768 / THREA
     const int64_t* mulp = nullptr;
     int64_t me = 0, mn = 0, mi = 0;
     if (MODE & 2) {
-        mulp = kat<int64_t>(mul, i, j, k, 0);
+        mulp = multiplier<MODE>(mul, i, j, k, 0);
         me = mul.b3 ? 0 : 1;
         mn = mods.n[j], mi = mods.ninv[j];
     }
@@ -57,6 +57,7 @@ hc_status launch_mode(hc_context ctx, int mode, const KView& t, const PlanPtrs& 
     if (mode == 0) return launch<0, FIX>(ctx, t, pp, mul, mods, tiles);
     if (mode == 1) return launch<1, FIX>(ctx, t, pp, mul, mods, tiles);
     if (mode == 2) return launch<2, FIX>(ctx, t, pp, mul, mods, tiles);
+    if (FIX && mode == 6) return launch<6, true>(ctx, t, pp, mul, mods, tiles);
     return launch<3, FIX>(ctx, t, pp, mul, mods, tiles);
 }
 

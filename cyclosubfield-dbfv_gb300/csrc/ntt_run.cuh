@@ -10,6 +10,13 @@ namespace {
 template <bool FIX>
 using PassCtx = std::conditional_t<FIX, fast::CtxL, fast::Ctx>;
 
+/// The multiplier of tile element (i, j, k, l): Montgomery words, or a table of limbs (mode bit 2).
+template <int MODE>
+__device__ __forceinline__ const int64_t* multiplier(const KView& mul, int64_t i, int64_t j, int64_t k, int64_t l) {
+    if constexpr ((MODE & 4) != 0) return reinterpret_cast<const int64_t*>(kat<BarrettLimbs>(mul, i, j, k, l));
+    else return kat<int64_t>(mul, i, j, k, l);
+}
+
 /// One [2, 3, 8, 64] line g of plan P through the CTA's shared-memory line buffer s; FIX: the plan is
 /// fixed.
 template <int MODE, bool FIX>
@@ -29,7 +36,7 @@ __device__ __forceinline__ void run_column(const DevPlanHeader* P, int64_t* g, i
     constexpr bool inv = MODE & 1;
     typedef PassCtx<FIX> CTX;
     const CTX c = make_ctx<CTX>(P);
-    const auto mont = fast::make_mont<CTX>(mn, mi);
+    const auto mont = fast::make_mont<CTX, MODE>(mn, mi);
     constexpr int NST = SHAPE == HC_SHAPE_C12 ? 3 : 2;
     with_sched<SHAPE, inv, FIX>(P, [&](const auto& sch) {
         fast::SF f[NST];
@@ -47,7 +54,7 @@ __device__ __forceinline__ void run_column(const DevPlanHeader* P, int64_t* g, i
 #pragma unroll
                 for (int b = 0; b < 3; b++) {
                     int64_t v = x[a][b];
-                    if (MODE & 2) v = mont.mul(v, mulp[(3 * a + b) * mstride]);
+                    if (MODE & 2) v = mont.mul(v, mont.load(mulp, (3 * a + b) * mstride));
                     g[(3 * a + b) * ge] = v;
                 }
         } else {
@@ -58,7 +65,7 @@ __device__ __forceinline__ void run_column(const DevPlanHeader* P, int64_t* g, i
 #pragma unroll
             for (int a = 0; a < 4; a++) {
                 int64_t v = x[a];
-                if (MODE & 2) v = mont.mul(v, mulp[a * mstride]);
+                if (MODE & 2) v = mont.mul(v, mont.load(mulp, a * mstride));
                 g[a * ge] = v;
             }
         }

@@ -35,12 +35,13 @@ hc_status launch_tensor(hc_context ctx, const KView& d, const KView& lhs_lo, con
                         int f1, int f2);
 bool crt_pass_ready(hc_context ctx, const hc_ntt_plan* plans2, const hc_ntt_plan* plans3, size_t r, const KView& t);
 hc_status launch_crt_pass(hc_context ctx, int dir, const KView& t, const KView* src, const hc_ntt_plan* plans2,
-                          const hc_ntt_plan* plans3, size_t r, const KView& m2, const KView& m3, bool post,
-                          const KMods& mods);
+                          const hc_ntt_plan* plans3, size_t r, const BarrettLimbs* m2, const BarrettLimbs* m3,
+                          const KView& pm, bool post, const KMods& mods);
 hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, int nbaby, int d, const int* lfirst,
                        const int* lcount, const KView* add, int nadd, const unsigned char* full, int used,
                        const KView& dst, const KMods& m, const int64_t* one_dev);
 size_t crt_slab_tile_words(int32_t shapes, int32_t dl, int32_t dk, int logv);
+bool crt_slab_limbs(int32_t shapes, int dim);
 }  // namespace hc
 
 using namespace hc;
@@ -448,6 +449,7 @@ struct TransformCache {
     std::vector<hc_modulus> mods;
     std::vector<hc_ntt_plan> plp, pk;
     Tensor kl, kk, ikl, ikk;
+    DBuf kll, kkl, ikll, ikkl;  // the same kernels as limbs (mont_const_limbs), [r][deg_L'] and [r][deg_K]
 };
 
 /// Host mirror of the device Montgomery product mul_mont (the same integers).
@@ -502,8 +504,8 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
             }
         for (size_t u = 0; u < r; u++) maxmq = std::max(maxmq, std::abs(mat[(b * (rd + 1) + rd) * r + u]));
     }
-    for (size_t u = 0; u < r; u++) qinvl[u] = mont_const_limbs(qinv[u], sm[u].n);
-    for (size_t j = 0; j < rd; j++) r2l[j] = mont_const_limbs(dm[j].r2_mod_n, dm[j].n);
+    for (size_t u = 0; u < r; u++) qinvl[u] = mont_const_limbs(qinv[u], sm[u].n, sm[u].neg_inv_n);
+    for (size_t j = 0; j < rd; j++) r2l[j] = mont_const_limbs(dm[j].r2_mod_n, dm[j].n, dm[j].neg_inv_n);
     const int qhalf = (int)maxlen;
     for (size_t b = 0; b < nb; b++)
         for (size_t j = 0; j < rd; j++)
@@ -752,6 +754,13 @@ struct hc_ring_s {
             t = Tensor(ctx, 1, r, lp ? dl() : 1, lp ? 1 : dk());
             CK(hc_import(ctx, t.view(), v.data(), v.size()));
         };
+        auto limbs = [&](DBuf& t, const std::vector<int64_t>& v) {
+            std::vector<BarrettLimbs> l(v.size());
+            const size_t len = v.size() / b.size();
+            for (size_t i = 0; i < v.size(); i++) l[i] = mont_const_limbs(v[i], c->mods[i / len].n, c->mods[i / len].neg_inv_n);
+            t = DBuf(ctx, l.data(), l.size() * sizeof(BarrettLimbs));
+        };
+        if (!b.empty()) limbs(c->kll, kl), limbs(c->kkl, kk), limbs(c->ikll, ikl), limbs(c->ikkl, ikk);
         up(c->kl, kl, true);
         up(c->kk, kk, false);
         up(c->ikl, ikl, true);
@@ -761,10 +770,9 @@ struct hc_ring_s {
     }
 
     // ---------------------------------------------------------------- transforms
-    /// The two fused launches of a transform (csrc/crt_fused.cu: both dimensions' NTTs of each
-    /// half in one cluster launch) where the plans are the fused shapes; false: nothing was
-    /// launched, the caller runs the per-dimension calls.
-    bool fused_transform(TransformCache& c, const hc_view& v, bool inverse, const hc_view* post_mul,
+    /// field_49152's transforms (csrc/crt_slab.cu: its lines' leading stage goes with the columns); false:
+    /// nothing was launched, the caller runs the per-dimension calls.
+    bool slab_transform(TransformCache& c, const hc_view& v, bool inverse, const hc_view* post_mul,
                          const hc_view* src) {
         const size_t r = c.base.size();
         if (v.strides[3] != 1 || (src && src->strides[3] != 1)) return false;
@@ -780,9 +788,7 @@ struct hc_ring_s {
             }
             return m.strides[3] == 1 || m.shape[3] == 1;
         };
-        KView m2{}, m3{}, pm{};
-        if (!bcast(inverse ? c.ikl.view() : c.kl.view(), &m2) || !bcast(inverse ? c.ikk.view() : c.kk.view(), &m3))
-            return false;
+        KView pm{};
         if (post_mul && !bcast(*post_mul, &pm)) return false;
         const KView t = kv(v);
         KView sv;
@@ -808,8 +814,9 @@ struct hc_ring_s {
         const KMods km = kmods(c.base);
         if (!crt_pass_ready(ctx, c.plp.data(), c.pk.data(), r, t)) return false;
         if (copy_first) CK(hc_assign(ctx, v, *src));
-        CK(launch_crt_pass(ctx, 0, t, sp, c.plp.data(), c.pk.data(), r, m2, m3, false, km));
-        CK(launch_crt_pass(ctx, 1, t, nullptr, c.plp.data(), c.pk.data(), r, KView(), pm, post_mul != nullptr, km));
+        CK(launch_crt_pass(ctx, 0, t, sp, c.plp.data(), c.pk.data(), r, (inverse ? c.ikll : c.kll).as<BarrettLimbs>(),
+                           (inverse ? c.ikkl : c.kkl).as<BarrettLimbs>(), pm, false, km));
+        CK(launch_crt_pass(ctx, 1, t, nullptr, c.plp.data(), c.pk.data(), r, nullptr, nullptr, pm, post_mul != nullptr, km));
         return true;
     }
 
@@ -822,15 +829,11 @@ struct hc_ring_s {
                 "transform: tensor shape does not match the ring and base");
         TransformCache& c = transform_cache(b);
         const size_t r = b.size();
-        if (fused_transform(c, v, inverse, post_mul, src)) return;
-        if (src)
-            CK(ntt_mul_mont64_dim_from(ctx, v, *src, c.plp.data(), r, HC_DIM2, inverse ? c.ikl.view() : c.kl.view(),
-                                       c.mods.data(), r));
-        else
-            CK(hc_ntt_mul_mont64_dim(ctx, v, c.plp.data(), r, HC_DIM2, inverse ? c.ikl.view() : c.kl.view(),
-                                     c.mods.data(), r));
-        CK(hc_ntt_mul_mont64_dim(ctx, v, c.pk.data(), r, HC_DIM3, inverse ? c.ikk.view() : c.kk.view(),
-                                 c.mods.data(), r));
+        if (slab_transform(c, v, inverse, post_mul, src)) return;
+        CK(ntt_kernel_dim(ctx, v, src, c.plp.data(), r, HC_DIM2, inverse ? c.ikl.view() : c.kl.view(),
+                          (inverse ? c.ikll : c.kll).as<BarrettLimbs>(), c.mods.data(), r));
+        CK(ntt_kernel_dim(ctx, v, nullptr, c.pk.data(), r, HC_DIM3, inverse ? c.ikk.view() : c.kk.view(),
+                          (inverse ? c.ikkl : c.kkl).as<BarrettLimbs>(), c.mods.data(), r));
         CK(hc_intt_mont64_dim(ctx, v, c.plp.data(), r, HC_DIM2));
         if (post_mul) CK(intt_mul_mont64_dim(ctx, v, c.pk.data(), r, HC_DIM3, *post_mul, c.mods.data(), r));
         else CK(hc_intt_mont64_dim(ctx, v, c.pk.data(), r, HC_DIM3));
@@ -1036,7 +1039,7 @@ struct hc_ring_s {
         std::vector<BarrettLimbs> v(of.size());
         for (size_t j = 0; j < of.size(); j++) {
             const int64_t p = prime(of[j]);
-            v[j] = mont_const_limbs(mont_repr(centred(invm(q_mod(div, p), p), p), p), p);
+            v[j] = mont_const_limbs(mont_repr(centred(invm(q_mod(div, p), p), p), p), p, factors[of[j]].mod.neg_inv_n);
         }
         auto t = std::make_unique<DBuf>(ctx, v.data(), v.size() * sizeof(BarrettLimbs));
         auto& ref = *t;
@@ -2104,10 +2107,6 @@ hc_status hc_crt_batch_create(hc_context ctx, const hc_crt_item* items, size_t n
                                j * I.op.strides[1];
                         s.op_s2 = I.op.strides[2];
                     }
-                    s.kl = (const int64_t*)tc.kl.view().ptr + j * R->dl();
-                    s.kk = (const int64_t*)tc.kk.view().ptr + j * R->dk();
-                    s.ikl = (const int64_t*)tc.ikl.view().ptr + j * R->dl();
-                    s.ikk = (const int64_t*)tc.ikk.view().ptr + j * R->dk();
                     s.n = tc.mods[j].n, s.ninv = tc.mods[j].neg_inv_n;
                     s.dl = (int32_t)R->dl(), s.dk = (int32_t)R->dk();
                     s.ops = ops;
@@ -2116,6 +2115,12 @@ hc_status hc_crt_batch_create(hc_context ctx, const hc_crt_item* items, size_t n
                         const int32_t s3 = plan_shape(tc.pk[j]), s2 = plan_shape(tc.plp[j]);
                         s.shapes = (s3 & 0xff) | ((s2 & 0xff) << 8) | (((s3 >> 8) & 1) << 16) | (((s2 >> 8) & 1) << 17);
                     }
+                    const bool l2 = crt_slab_limbs(s.shapes, 2), l3 = crt_slab_limbs(s.shapes, 3);
+                    auto row = [&](bool l, const DBuf& t, const Tensor& w, int64_t len) {
+                        return l ? (const int64_t*)(t.as<BarrettLimbs>() + j * len) : (const int64_t*)w.view().ptr + j * len;
+                    };
+                    s.kl = row(l2, tc.kll, tc.kl, R->dl()), s.kk = row(l3, tc.kkl, tc.kk, R->dk());
+                    s.ikl = row(l2, tc.ikll, tc.ikl, R->dl()), s.ikk = row(l3, tc.ikkl, tc.ikk, R->dk());
                     slabs.push_back(s);
                     tws.push_back(2 * (size_t)(plan_ntw(tc.plp[j]) + plan_ntw(tc.pk[j])));
                 }
