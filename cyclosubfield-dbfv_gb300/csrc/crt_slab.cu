@@ -37,8 +37,8 @@ __device__ __forceinline__ void lead12288(const KView& t, const KView& src, cons
                                           int p) {
     constexpr bool inv = DIR == 1;
     const fast::CtxL c2 = make_ctx<fast::CtxL>(P2), c3 = make_ctx<fast::CtxL>(P3);
-    const FixedSched<HC_SHAPE_C4, LG, inv> sch2{inv ? P2->inv : P2->fwd};
-    const FixedSched<HC_SHAPE_L12288, LG, inv> sch3{inv ? P3->inv : P3->fwd};
+    const FixedSched<HC_SHAPE_C4, LG, inv> sch2{};
+    const FixedSched<HC_SHAPE_L12288, LG, inv> sch3{};
     const fast::SF f2[2] = {fast::sflags(sch2, 0), fast::sflags(sch2, 1)};
     const fast::SF f3 = fast::sflags(sch3, 0);
     const int64_t* gs = reinterpret_cast<const int64_t*>(src.p) + i * src.s0 + j * src.s1 + p;

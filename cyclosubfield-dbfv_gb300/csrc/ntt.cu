@@ -77,6 +77,7 @@ struct hc_ntt_plan_s {
     int64_t n;
     int32_t len;
     int32_t ntw;      // twiddle pairs
+    int32_t counts[4];  // stages forward and inverse, passes forward and inverse
     int32_t shape;    // HC_SHAPE_*: factorisation with a specialised kernel
     bool fixed;       // the schedule is the shape's compiled-in one and the limb products are exact
     size_t bytes;
@@ -358,10 +359,18 @@ hc_status build_plan(hc_context ctx, const hc_modulus* m, const size_t* shape, s
             m.ired |= (uint32_t)(hp.h.inv[i].reduce_before != 0) << i;
             m.ilast |= (uint32_t)(hp.h.inv[i].last != 0) << i;
         }
+        bool laid = shape_id != HC_SHAPE_GENERIC;  // the table's offsets are the compiled-in ones
+        if (laid) {
+            const TableLayout t = table_layout(shape_id);
+            laid = t.words == hp.next_tw();
+            for (int i = 0; i < hp.h.nfwd; i++) laid = laid && hp.h.fwd[i].tw_off == t.fwd[i];
+            for (int i = 0; i < hp.h.ninv; i++)
+                laid = laid && hp.h.inv[i].tw_off == t.inv[i] && (hp.h.inv[i].radix == 2 || hp.h.inv[i].zeta_off == t.zeta[i]);
+        }
         for (int lg : {56, 57}) {
             const SchedMasks f = fixed_masks(shape_id, lg);
-            if (limbs && shape_id != HC_SHAPE_GENERIC && m.fred == f.fred && m.fskip == f.fskip && m.flast == f.flast &&
-                m.ired == f.ired && m.ilast == f.ilast)
+            if (limbs && laid && m.fred == f.fred && m.fskip == f.fskip && m.flast == f.flast && m.ired == f.ired &&
+                m.ilast == f.ilast)
                 hp.h.cls = lg;
         }
     }
@@ -385,6 +394,7 @@ hc_status build_plan(hc_context ctx, const hc_modulus* m, const size_t* shape, s
     plan->n = n;
     plan->len = (int32_t)len;
     plan->ntw = hp.h.ntw;
+    plan->counts[0] = hp.h.nfwd, plan->counts[1] = hp.h.ninv, plan->counts[2] = hp.h.nfpass, plan->counts[3] = hp.h.nipass;
     plan->bytes = bytes;
     *out = plan;
     return HC_OK;
@@ -401,6 +411,7 @@ int64_t plan_modulus(hc_ntt_plan p) { return p->n; }
 int32_t plan_len(hc_ntt_plan p) { return p->len; }
 const void* plan_device(hc_ntt_plan p) { return p->dev; }
 int32_t plan_ntw(hc_ntt_plan p) { return p->ntw; }
+void plan_counts(hc_ntt_plan p, int32_t counts[4]) { std::copy(p->counts, p->counts + 4, counts); }
 int32_t plan_shape(hc_ntt_plan p) { return p->shape | (p->fixed ? 0x100 : 0); }
 /// Launches the tile kernel for one HAL NTT call (mode 0 ntt, 1 intt, 2 ntt_mul).
 /// Whether launch_ntt runs a call on the specialised column kernel, the one form that can read a

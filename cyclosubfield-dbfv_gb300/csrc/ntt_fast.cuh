@@ -60,27 +60,32 @@ struct SF {
     bool red, skip_ok, last;
 };
 
-/// The plan's reduction / skip / fused-final schedule read at run time (any prime).
+/// The plan's reduction / skip / fused-final schedule and table offsets read at run time (any prime).
 struct DynSched {
     const DevStage* st;
     __device__ __forceinline__ bool red(int s) const { return st[s].reduce_before; }
     __device__ __forceinline__ bool skip(int s) const { return st[s].skip_ok; }
     __device__ __forceinline__ bool last(int s) const { return st[s].last; }
+    __device__ __forceinline__ int tw(int s) const { return st[s].tw_off; }
+    __device__ __forceinline__ int zeta(int s) const { return st[s].zeta_off; }
 };
-/// A schedule known at compile time (bit s = the flag of stage s), for primes whose plan has
-/// exactly this schedule; the flags then fold into straight-line code.
-template <uint32_t RED, uint32_t SKIP, uint32_t LAST>
+/// A schedule known at compile time (bit s = the flag of stage s) with the table offsets T of its
+/// shape and direction, for primes whose plan has exactly this schedule: flags fold into
+/// straight-line code and offsets into addresses, with no load of the stage program in front of the
+/// loads of its twiddles.
+template <uint32_t RED, uint32_t SKIP, uint32_t LAST, class T>
 struct FixSched {
-    const DevStage* st;
     __device__ __forceinline__ bool red(int s) const { return (RED >> s) & 1; }
     __device__ __forceinline__ bool skip(int s) const { return (SKIP >> s) & 1; }
     __device__ __forceinline__ bool last(int s) const { return (LAST >> s) & 1; }
+    __device__ __forceinline__ int tw(int s) const { return T::offset(s); }
+    __device__ __forceinline__ int zeta(int s) const { return T::zeta(s); }
 };
 
 template <class SCH>
 __device__ __forceinline__ SF sflags(const SCH& sch, int s) {
     SF f;
-    f.tw_off = sch.st[s].tw_off, f.zeta_off = sch.st[s].zeta_off;
+    f.tw_off = sch.tw(s), f.zeta_off = sch.zeta(s);
     f.red = sch.red(s), f.skip_ok = sch.skip(s), f.last = sch.last(s);
     return f;
 }

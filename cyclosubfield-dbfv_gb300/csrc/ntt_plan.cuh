@@ -136,20 +136,51 @@ __host__ __device__ constexpr SchedMasks fixed_masks(int shape, int lg) {
     if (nst) m.flast = m.ilast = 1u << (nst - 1);
     return m;
 }
+/// Offsets of a specialised shape's twiddle table as build_plan lays it out: per factor the two cube roots
+/// of a factor 3, then its forward stages (2^s or 6 3^s entries), then its inverse stages.
+struct TableLayout {
+    int fwd[16], inv[16], zeta[16];  // by stage; zeta: of the inverse stage's factor
+    int words;
+};
+__host__ __device__ constexpr TableLayout table_layout(int shape) {
+    TableLayout t{};
+    const int factors[4][4] = {{2, 3, 8, 64}, {3, 64, 64, 1}, {4, 3, 1, 1}, {4, 1, 1, 1}};
+    int at = 0, st = 0;
+    for (int i = 0; i < 4; i++) {
+        const int f = factors[shape - HC_SHAPE_L3072][i], radix = f == 3 ? 3 : 2;
+        int nst = 0, zeta = 0;
+        for (int l = 1; l < f; l *= radix) nst++;
+        if (f == 3) zeta = at, at += 2;
+        for (int q = 0, n = 1; q < nst; q++, n *= radix) t.fwd[st + q] = at, at += radix == 3 ? 6 * n : n;
+        for (int q = 0; q < nst; q++) {  // the inverse runs the stages in reverse order
+            int n = 1;
+            for (int e = 0; e < nst - 1 - q; e++) n *= radix;
+            t.inv[st + q] = at, t.zeta[st + q] = zeta, at += radix == 3 ? 2 * n : n;
+        }
+        st += nst;
+    }
+    t.words = at;
+    return t;
+}
+template <int SHAPE, bool INV>
+struct Table {
+    __host__ __device__ static constexpr int offset(int s) { return INV ? table_layout(SHAPE).inv[s] : table_layout(SHAPE).fwd[s]; }
+    __host__ __device__ static constexpr int zeta(int s) { return table_layout(SHAPE).zeta[s]; }
+};
+
 template <int SHAPE, int LG, bool INV>
 using FixedSched = fast::FixSched<INV ? fixed_masks(SHAPE, LG).ired : fixed_masks(SHAPE, LG).fred,
                                   INV ? 0u : fixed_masks(SHAPE, LG).fskip,
-                                  INV ? fixed_masks(SHAPE, LG).ilast : fixed_masks(SHAPE, LG).flast>;
+                                  INV ? fixed_masks(SHAPE, LG).ilast : fixed_masks(SHAPE, LG).flast, Table<SHAPE, INV>>;
 
 /// Calls f with the compiled-in schedule of a fixed plan (SHAPE, direction INV), or with the
 /// schedule read from any plan (FIX = false). Uniform over a CTA that works for one plan.
 template <int SHAPE, bool INV, bool FIX, class F>
 __device__ __forceinline__ void with_sched(const DevPlanHeader* P, F f) {
-    const DevStage* st = INV ? P->inv : P->fwd;
-    if constexpr (!FIX) f(fast::DynSched{st});
-    else if (std::is_same_v<FixedSched<SHAPE, 56, INV>, FixedSched<SHAPE, 57, INV>> || P->cls == 57)
-        f(FixedSched<SHAPE, 57, INV>{st});
-    else f(FixedSched<SHAPE, 56, INV>{st});
+    if constexpr (!FIX) f(fast::DynSched{INV ? P->inv : P->fwd});
+    else if constexpr (std::is_same_v<FixedSched<SHAPE, 56, INV>, FixedSched<SHAPE, 57, INV>>) f(FixedSched<SHAPE, 57, INV>{});
+    else if (P->cls == 57) f(FixedSched<SHAPE, 57, INV>{});
+    else f(FixedSched<SHAPE, 56, INV>{});
 }
 
 }  // namespace

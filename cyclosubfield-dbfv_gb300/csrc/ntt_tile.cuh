@@ -33,18 +33,39 @@ struct Tile {
     int len, logv;
     bool swz;
     __device__ __forceinline__ int64_t& at(int e, int v) const { return s[sw((e << logv) + v, swz)]; }
+    /// n items per vector: their number over all vectors, and item b's index and vector.
+    __device__ __forceinline__ int count(int n) const { return n << logv; }
+    __device__ __forceinline__ uint32_t split(int b, int& v) const {
+        v = b & ((1 << logv) - 1);
+        return (uint32_t)(b >> logv);
+    }
+};
+
+/// A whole slab of V vectors in shared memory: element e of vector v at e * se + v * sv.
+struct SlabTile {
+    int64_t* __restrict__ s;
+    int len, V, se, sv;
+    FastDiv div_v;
+    __device__ __forceinline__ int64_t& at(int e, int v) const { return s[e * se + v * sv]; }
+    __device__ __forceinline__ int count(int n) const { return n * V; }
+    __device__ __forceinline__ uint32_t split(int b, int& v) const {
+        const uint32_t q = fdiv((uint32_t)b, div_v);
+        v = b - (int)q * V;
+        return q;
+    }
 };
 
 /// One forward stage (radix 2 or 3) over the tile in shared memory.
-__device__ __forceinline__ void fwd_stage(const Tile& T, const DevStage st, const int64_t* __restrict__ tw,
+template <class TILE>
+__device__ __forceinline__ void fwd_stage(const TILE& T, const DevStage st, const int64_t* __restrict__ tw,
                                           int64_t n, int64_t one_z, int64_t one_u, bool reduce_output) {
     const int radix = st.radix;
     const bool fuse = st.last && reduce_output;
-    const int nbf = (T.len / radix) << T.logv;
-    const int vmask = (1 << T.logv) - 1;
+    const int nbf = T.count(T.len / radix);
     for (int b = threadIdx.x; b < nbf; b += blockDim.x) {
-        int block;
-        const int e = leg0((uint32_t)(b >> T.logv), st, &block), v = b & vmask;
+        int block, v;
+        const uint32_t bb = T.split(b, v);
+        const int e = leg0(bb, st, &block);
         int64_t& x = T.at(e, v);
         int64_t& y = T.at(e + st.span, v);
         if (radix == 2) {
@@ -93,15 +114,16 @@ __device__ __forceinline__ void fwd_stage(const Tile& T, const DevStage st, cons
 }
 
 /// One inverse stage (radix 2 or 3) over the tile in shared memory.
-__device__ __forceinline__ void inv_stage(const Tile& T, const DevStage st, const int64_t* __restrict__ tw,
+template <class TILE>
+__device__ __forceinline__ void inv_stage(const TILE& T, const DevStage st, const int64_t* __restrict__ tw,
                                           int64_t n, int64_t il_z, int64_t il_u, int64_t one_z, int64_t one_u) {
     const int radix = st.radix;
     const bool fused = st.last;
-    const int nbf = (T.len / radix) << T.logv;
-    const int vmask = (1 << T.logv) - 1;
+    const int nbf = T.count(T.len / radix);
     for (int b = threadIdx.x; b < nbf; b += blockDim.x) {
-        int block;
-        const int e = leg0((uint32_t)(b >> T.logv), st, &block), v = b & vmask;
+        int block, v;
+        const uint32_t bb = T.split(b, v);
+        const int e = leg0(bb, st, &block);
         int64_t& x = T.at(e, v);
         int64_t& y = T.at(e + st.span, v);
         if (radix == 2) {
@@ -154,8 +176,8 @@ __device__ __forceinline__ void inv_stage(const Tile& T, const DevStage st, cons
 /// K consecutive forward radix-2 stages of one factor in registers. Group element m lies at
 /// g * glen + o + m * span; at the q-th stage of the pass the butterflies pair m with
 /// m + 2^(K-1-q) and use the twiddle of block block0 * 2^q + (m >> (K-q)).
-template <int K>
-__device__ __forceinline__ void fwd_pass_r2(const Tile& T, const DevPass ps, const DevStage* sts,
+template <int K, class TILE>
+__device__ __forceinline__ void fwd_pass_r2(const TILE& T, const DevPass ps, const DevStage* sts,
                                             const int64_t* __restrict__ tw, int64_t n, int64_t one_z, int64_t one_u,
                                             bool reduce_output) {
     constexpr int M = 1 << K;
@@ -170,11 +192,10 @@ __device__ __forceinline__ void fwd_pass_r2(const Tile& T, const DevPass ps, con
         skip_ok[q] = st.skip_ok;
         fuse[q] = st.last && reduce_output;
     }
-    const int ng = (T.len >> K) << T.logv;
-    const int vmask = (1 << T.logv) - 1;
+    const int ng = T.count(T.len >> K);
     for (int gi = threadIdx.x; gi < ng; gi += blockDim.x) {
-        const int v = gi & vmask;
-        const uint32_t gg = (uint32_t)(gi >> T.logv);
+        int v;
+        const uint32_t gg = T.split(gi, v);
         const uint32_t g = fdiv(gg, ps.div_span);
         const int o = (int)(gg - g * (uint32_t)ps.span);
         const int block0 = (int)(g - fdiv(g, ps.div_nb) * (uint32_t)ps.nb);
@@ -214,8 +235,8 @@ __device__ __forceinline__ void fwd_pass_r2(const Tile& T, const DevPass ps, con
 /// K consecutive inverse radix-2 stages (stage lengths growing) in registers: at the q-th stage
 /// of the pass the butterflies pair m with m + 2^q and use the twiddle of block
 /// blockK * 2^(K-1-q) + (m >> (q+1)), blockK being the group's block at the pass's last stage.
-template <int K>
-__device__ __forceinline__ void inv_pass_r2(const Tile& T, const DevPass ps, const DevStage* sts,
+template <int K, class TILE>
+__device__ __forceinline__ void inv_pass_r2(const TILE& T, const DevPass ps, const DevStage* sts,
                                             const int64_t* __restrict__ tw, int64_t n, int64_t il_z, int64_t il_u,
                                             int64_t one_z, int64_t one_u) {
     constexpr int M = 1 << K;
@@ -228,11 +249,10 @@ __device__ __forceinline__ void inv_pass_r2(const Tile& T, const DevPass ps, con
         red[q] = st.reduce_before;
         fused[q] = st.last;
     }
-    const int ng = (T.len >> K) << T.logv;
-    const int vmask = (1 << T.logv) - 1;
+    const int ng = T.count(T.len >> K);
     for (int gi = threadIdx.x; gi < ng; gi += blockDim.x) {
-        const int v = gi & vmask;
-        const uint32_t gg = (uint32_t)(gi >> T.logv);
+        int v;
+        const uint32_t gg = T.split(gi, v);
         const uint32_t g = fdiv(gg, ps.div_span);
         const int o = (int)(gg - g * (uint32_t)ps.span);
         const int blockK = (int)(g - fdiv(g, ps.div_nb) * (uint32_t)ps.nb);
@@ -271,6 +291,53 @@ __device__ __forceinline__ void inv_pass_r2(const Tile& T, const DevPass ps, con
     }
 }
 
+/// A plan's stage programme and constants, in global or shared memory.
+struct Program {
+    const DevStage *fwd, *inv;
+    const DevPass *fpass, *ipass;
+    int nfpass, nipass;
+    int64_t n, one_z, one_u, il_z, il_u;
+    const int64_t* tw;
+};
+__device__ __forceinline__ Program program_of(const DevPlanHeader* P, const int64_t* tw) {
+    return Program{P->fwd, P->inv, P->fpass, P->ipass, P->nfpass, P->nipass, P->n, P->one_z, P->one_u, P->invlen_z, P->invlen_u, tw};
+}
+
+/// All passes of a programme over a tile in place (modes as tile_run, without the multiplication); a
+/// block barrier after each.
+template <class TILE>
+__device__ __forceinline__ void run_passes(const TILE& T, const Program& P, int mode) {
+    const bool inverse = mode & 1;
+    const int npass = inverse ? P.nipass : P.nfpass;
+    for (int pi = 0; pi < npass; pi++) {
+        const DevPass ps = inverse ? P.ipass[pi] : P.fpass[pi];
+        if (ps.kind == 0) {
+            if (inverse) inv_stage(T, P.inv[ps.first], P.tw, P.n, P.il_z, P.il_u, P.one_z, P.one_u);
+            else fwd_stage(T, P.fwd[ps.first], P.tw, P.n, P.one_z, P.one_u, mode == 0);
+        } else if (inverse) {
+            if (ps.k == 3) inv_pass_r2<3>(T, ps, P.inv, P.tw, P.n, P.il_z, P.il_u, P.one_z, P.one_u);
+            else if (ps.k == 2) inv_pass_r2<2>(T, ps, P.inv, P.tw, P.n, P.il_z, P.il_u, P.one_z, P.one_u);
+            else inv_pass_r2<1>(T, ps, P.inv, P.tw, P.n, P.il_z, P.il_u, P.one_z, P.one_u);
+        } else {
+            if (ps.k == 3) fwd_pass_r2<3>(T, ps, P.fwd, P.tw, P.n, P.one_z, P.one_u, mode == 0);
+            else if (ps.k == 2) fwd_pass_r2<2>(T, ps, P.fwd, P.tw, P.n, P.one_z, P.one_u, mode == 0);
+            else fwd_pass_r2<1>(T, ps, P.fwd, P.tw, P.n, P.one_z, P.one_u, mode == 0);
+        }
+        __syncthreads();
+    }
+    // plans without factors (length 1): the inverse scales by 1^-1, the reduced forward
+    // reduces; an unreduced forward leaves the data unchanged
+    if (npass == 0 && (mode == 0 || inverse)) {
+        const int64_t fz = inverse ? P.il_z : P.one_z, fu = inverse ? P.il_u : P.one_u;
+        for (int b = threadIdx.x; b < T.count(T.len); b += blockDim.x) {
+            int v;
+            const int e = (int)T.split(b, v);
+            T.at(e, v) = bmul(fz, fu, T.at(e, v), P.n);
+        }
+        __syncthreads();
+    }
+}
+
 /// Where one tile lives in global memory and where its Montgomery multiplier (modes 2 and 3)
 /// comes from: element (e, v) of the tile is g[e * ge + v] and is multiplied by
 /// mulp[e * me + v * mv] modulo (mn, mi).
@@ -292,7 +359,6 @@ __device__ __forceinline__ void tile_run(const DevPlanHeader* __restrict__ P, co
                                          int64_t* s, int len, int logv, bool use_smem, int mode,
                                          const TileIO& io) {
     const int V = 1 << logv, vmask = V - 1;
-    const int64_t n = P->n;
     const int total = len * V;
     Tile T{use_smem ? s : io.g, len, logv, use_smem && logv == 0 && (len & 15) == 0};
     if (use_smem) {
@@ -302,35 +368,7 @@ __device__ __forceinline__ void tile_run(const DevPlanHeader* __restrict__ P, co
         }
     }
     __syncthreads();
-    const bool inverse = mode & 1;
-    const int npass = inverse ? P->nipass : P->nfpass;
-    const int64_t one_z = P->one_z, one_u = P->one_u, il_z = P->invlen_z, il_u = P->invlen_u;
-    for (int pi = 0; pi < npass; pi++) {
-        const DevPass ps = inverse ? P->ipass[pi] : P->fpass[pi];
-        if (ps.kind == 0) {
-            if (inverse) inv_stage(T, P->inv[ps.first], tw, n, il_z, il_u, one_z, one_u);
-            else fwd_stage(T, P->fwd[ps.first], tw, n, one_z, one_u, mode == 0);
-        } else if (inverse) {
-            if (ps.k == 3) inv_pass_r2<3>(T, ps, P->inv, tw, n, il_z, il_u, one_z, one_u);
-            else if (ps.k == 2) inv_pass_r2<2>(T, ps, P->inv, tw, n, il_z, il_u, one_z, one_u);
-            else inv_pass_r2<1>(T, ps, P->inv, tw, n, il_z, il_u, one_z, one_u);
-        } else {
-            if (ps.k == 3) fwd_pass_r2<3>(T, ps, P->fwd, tw, n, one_z, one_u, mode == 0);
-            else if (ps.k == 2) fwd_pass_r2<2>(T, ps, P->fwd, tw, n, one_z, one_u, mode == 0);
-            else fwd_pass_r2<1>(T, ps, P->fwd, tw, n, one_z, one_u, mode == 0);
-        }
-        __syncthreads();
-    }
-    // plans without factors (length 1): the inverse scales by 1^-1, the reduced forward
-    // reduces; an unreduced forward leaves the data unchanged
-    if (npass == 0 && (mode == 0 || inverse)) {
-        int64_t fz = inverse ? P->invlen_z : P->one_z, fu = inverse ? P->invlen_u : P->one_u;
-        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-            int e = idx >> logv, v = idx & vmask;
-            T.at(e, v) = bmul(fz, fu, T.at(e, v), n);
-        }
-        __syncthreads();
-    }
+    run_passes(T, program_of(P, tw), mode);
     if (mode & 2) {
         for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
             int e = idx >> logv, v = idx & vmask;

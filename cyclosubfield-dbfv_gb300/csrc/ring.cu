@@ -33,6 +33,9 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
 hc_status launch_tensor(hc_context ctx, const KView& d, const KView& lhs_lo, const KView& lhs_hi, const KView& rhs_lo,
                         const KView& rhs_hi, int rsplit, const KMods& m, int f0,
                         int f1, int f2);
+hc_status launch_crt_small(hc_context ctx, const KView& t, const KView* src, const hc_ntt_plan* plans2,
+                           const hc_ntt_plan* plans3, size_t r, const int64_t* kl, const int64_t* kk, const KView* post,
+                           const KMods& mods, bool* done);
 bool crt_pass_ready(hc_context ctx, const hc_ntt_plan* plans2, const hc_ntt_plan* plans3, size_t r, const KView& t);
 hc_status launch_crt_pass(hc_context ctx, int dir, const KView& t, const KView* src, const hc_ntt_plan* plans2,
                           const hc_ntt_plan* plans3, size_t r, const BarrettLimbs* m2, const BarrettLimbs* m3,
@@ -770,8 +773,9 @@ struct hc_ring_s {
     }
 
     // ---------------------------------------------------------------- transforms
-    /// field_49152's transforms (csrc/crt_slab.cu: its lines' leading stage goes with the columns); false:
-    /// nothing was launched, the caller runs the per-dimension calls.
+    /// field_49152's transforms (csrc/crt_slab.cu: its lines' leading stage goes with the columns) and small
+    /// rings' (csrc/crt_small.cu: one launch); false: nothing was launched, the caller runs the
+    /// per-dimension calls.
     bool slab_transform(TransformCache& c, const hc_view& v, bool inverse, const hc_view* post_mul,
                          const hc_view* src) {
         const size_t r = c.base.size();
@@ -812,7 +816,14 @@ struct hc_ring_s {
             sp = copy_first ? nullptr : &sv;
         }
         const KMods km = kmods(c.base);
-        if (!crt_pass_ready(ctx, c.plp.data(), c.pk.data(), r, t)) return false;
+        if (!crt_pass_ready(ctx, c.plp.data(), c.pk.data(), r, t)) {
+            bool done = false;
+            if (!copy_first)
+                CK(launch_crt_small(ctx, t, sp, c.plp.data(), c.pk.data(), r,
+                                    (const int64_t*)(inverse ? c.ikl : c.kl).view().ptr,
+                                    (const int64_t*)(inverse ? c.ikk : c.kk).view().ptr, post_mul ? &pm : nullptr, km, &done));
+            return done;
+        }
         if (copy_first) CK(hc_assign(ctx, v, *src));
         CK(launch_crt_pass(ctx, 0, t, sp, c.plp.data(), c.pk.data(), r, (inverse ? c.ikll : c.kll).as<BarrettLimbs>(),
                            (inverse ? c.ikkl : c.kkl).as<BarrettLimbs>(), pm, false, km));
