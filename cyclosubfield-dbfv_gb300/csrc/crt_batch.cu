@@ -5,29 +5,29 @@
 
 namespace hc {
 
+bool crt_slab_limbs(int32_t shapes, int dim);
+
 CrtBatchKernel crt_batch_f36864(int ctas_per_sm);
 CrtBatchKernel crt_batch_f49152(int ctas_per_sm);
 CrtBatchKernel crt_batch_mixed(int ctas_per_sm);
 
-/// Shared-memory words a slab of the batched transform needs: a padded 3072-residue line, one padded
-/// 4096-residue block of a 12288-residue line (line12288_seq), or the generic tile (the whole line,
-/// or deg_L' x 2^logv dimension-2 columns); the specialised column passes use none.
+/// Shared-memory words a slab of the batched transform needs: two padded 3072-residue lines (one per team of
+/// 128 threads), one padded 4096-residue block of a 12288-residue line, or the generic tile (the whole
+/// line, or deg_L' x 2^logv dimension-2 columns); the specialised column passes use none.
 size_t crt_slab_tile_words(int32_t shapes, int32_t dl, int32_t dk, int logv) {
-    const int s3 = shapes & 0xff, s2 = (shapes >> 8) & 0xff;
-    const bool f3 = (shapes >> 16) & 1, f2 = (shapes >> 17) & 1;
-    const size_t w3 = !f3 ? (size_t)dk
-                          : s3 == HC_SHAPE_L3072 ? (size_t)line_tile_words(HC_SHAPE_L3072)
-                          : s3 == HC_SHAPE_L12288 ? (size_t)(4096 + 4096 / 8) : (size_t)dk;
-    const size_t w2 = f2 && (s2 == HC_SHAPE_C12 || s2 == HC_SHAPE_C4) ? 0 : ((size_t)dl << logv);
+    if (crt_slab_12288(shapes)) return 4096 + 4096 / 8;
+    const size_t w3 = crt_slab_limbs(shapes, 3) ? 2 * (size_t)line_tile_words(HC_SHAPE_L3072) : (size_t)dk;
+    const size_t w2 = crt_slab_limbs(shapes, 2) ? 0 : ((size_t)dl << logv);
     const size_t w = std::max(w3, w2);
     return (w + 1) & ~(size_t)1;
 }
 
-/// Whether slab_pass runs the passes along `dim` on the specialised code, with the CRT kernels as limbs.
+/// Whether the passes along `dim` run on the specialised code, with the CRT kernels as limbs:
+/// field_36864's columns and lines each on their own, field_49152's together.
 bool crt_slab_limbs(int32_t shapes, int dim) {
-    const int s3 = shapes & 0xff, s2 = (shapes >> 8) & 0xff;
-    return dim == 3 ? ((shapes >> 16) & 1) && (s3 == HC_SHAPE_L3072 || s3 == HC_SHAPE_L12288)
-                    : ((shapes >> 17) & 1) && (s2 == HC_SHAPE_C12 || s2 == HC_SHAPE_C4);
+    if (crt_slab_12288(shapes)) return true;
+    return dim == 3 ? ((shapes >> 16) & 1) && (shapes & 0xff) == HC_SHAPE_L3072
+                    : ((shapes >> 17) & 1) && ((shapes >> 8) & 0xff) == HC_SHAPE_C12;
 }
 
 /// Whether a slab runs entirely on the specialised line and column code (crt_batch_kernel<false>).

@@ -5,52 +5,76 @@
 
 namespace {
 
+/// Whether a slab has field_49152's shapes with fixed plans in both dimensions (slab12288_half).
+__host__ __device__ inline bool crt_slab_12288(int32_t shapes) {
+    return (shapes & 0x3ffff) == (HC_SHAPE_L12288 | HC_SHAPE_C4 << 8 | 3 << 16);
+}
+
+/// Half a transform of a field_49152 slab, as crt_slab.cu's two kernels run it: the lead pass over its
+/// positions, then its twelve blocks one after the other. MODE 6: forward, times the kernels kl [4] and
+/// kk [12288] (limbs); 1: inverse; 3: inverse, times the operand.
+template <int MODE>
+__device__ __forceinline__ void slab12288_half(const CrtSlab& S, const DevPlanHeader* P2, const DevPlanHeader* P3, int64_t* s,
+                                               const int64_t* kl, const int64_t* kk) {
+    const fast::CtxL c3 = make_ctx<fast::CtxL>(P3);
+    {
+        const fast::CtxL c2 = make_ctx<fast::CtxL>(P2);
+        const BarrettLimbs* m2 = reinterpret_cast<const BarrettLimbs*>(kl);
+        for (int p = threadIdx.x; p < 4096; p += blockDim.x) {
+            if (P3->cls == 57) lead12288<(MODE & 1), 57>(c2, c3, S.data + p, S.s2, S.data + p, S.s2, m2, S.n);
+            else lead12288<(MODE & 1), 56>(c2, c3, S.data + p, S.s2, S.data + p, S.s2, m2, S.n);
+        }
+    }
+    __syncthreads();
+    const auto mont = fast::make_mont<fast::CtxL, MODE>(S.n, S.ninv);
+    with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, true>(P3, [&](const auto& sch) {
+        for (int q = 0; q < 12; q++) {
+            const int k = q / 3, blk = q - 3 * (q / 3);
+            const int64_t* mulp = MODE == 6   ? fast::block_multiplier<MODE>(kk, 1, blk)
+                                  : MODE == 3 ? S.op + k * S.op_s2 + 4096 * blk
+                                              : nullptr;
+            fast::block4096<MODE>(fast::CtaTeam{}, sch, c3, s, S.data + k * S.s2 + 4096 * blk, mulp, 1, mont);
+            __syncthreads();  // the tile is refilled by the next block
+        }
+    });
+}
+
+/// The [2, 3, 8, 64] lines of a slab. 256 threads work as two teams of 128 with a tile each: a line's
+/// 384 register groups and 12 tail rows fill 128 threads exactly and 256 to three quarters.
+template <int MODE>
+__device__ __forceinline__ void slab_lines3072(const CrtSlab& S, const DevPlanHeader* P, int64_t* s, const int64_t* mulrow) {
+    const int teams = blockDim.x == 256 ? 2 : 1, t = (int)threadIdx.x / 128 % teams;
+    const fast::PartTeam tm{(int)threadIdx.x - 128 * t, (int)blockDim.x / teams, 1 + t};
+    int64_t* tile = s + t * line_tile_words(HC_SHAPE_L3072);
+    for (int k = t; k < S.dl; k += teams) {
+        run_line3072<MODE, true>(tm, P, tile, S.data + k * S.s2, MODE == 3 ? S.op + k * S.op_s2 : mulrow, 1, S.n, S.ninv);
+        tm.sync();
+    }
+    __syncthreads();
+}
+
 /// One pass of a batched transform over a whole slab: its deg_L' lines (dimension 3) or its
 /// column blocks of 2^logv columns (dimension 2). Modes as tile_run; `mulrow` is the CRT kernel
 /// row of the pass (modes 2 and 3 along dimension 2, mode 2 along dimension 3), while mode 3
 /// along dimension 3 multiplies by the slab's operand.
-template <bool GENERIC, int CLS>
+template <bool GENERIC>
 __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader* P, const int64_t* tw, int64_t* s,
                                           int dim, int mode, const int64_t* mulrow, int logv) {
-    // specialised kernels for slabs whose plans have the fixed schedule (bit 16: dimension-3
-    // plan, bit 17: dimension-2 plan), the generic tile programme otherwise
+    // specialised kernels for slabs whose plans are fixed (bit 16: dimension-3 plan, bit 17: dimension-2
+    // plan), the generic tile programme otherwise
     const int shape = dim == 3 ? (S.shapes & 0xff) : ((S.shapes >> 8) & 0xff);
     const bool fix = (S.shapes >> (dim == 3 ? 16 : 17)) & 1;
-    if (fix && dim == 3 && (shape == HC_SHAPE_L3072 || shape == HC_SHAPE_L12288)) {
-        for (int k = 0; k < S.dl; k++) {
-            int64_t* g = S.data + k * S.s2;
-            const int64_t* mulp = mode == 3 ? S.op + k * S.op_s2 : mulrow;
-            if (CLS != 2 && (CLS == 1 || shape == HC_SHAPE_L3072)) {
-                if (mode == 2) run_line3072<6, true>(P, s, g, mulp, 1, S.n, S.ninv);
-                else if (mode == 3) run_line3072<3, true>(P, s, g, mulp, 1, S.n, S.ninv);
-                else run_line3072<1, true>(P, s, g, mulp, 1, S.n, S.ninv);
-            } else if (CLS != 1) {
-                // one 4096-residue block in shared memory at a time (crt_slab_tile_words)
-                const auto c = make_ctx<fast::CtxL>(P);
-                if (mode & 1) {  // modes 1 (inverse) and 3 (inverse, then the operand product)
-                    with_sched<HC_SHAPE_L12288, true, true>(P, [&](const auto& sch) {
-                        if (mode == 3) fast::line12288_seq<3>(sch, c, s, g, mulp, 1, S.n, S.ninv);
-                        else fast::line12288_seq<1>(sch, c, s, g, mulp, 1, S.n, S.ninv);
-                    });
-                } else {  // mode 2: forward, then the kernel product
-                    with_sched<HC_SHAPE_L12288, false, true>(
-                        P, [&](const auto& sch) { fast::line12288_seq<6>(sch, c, s, g, mulp, 1, S.n, S.ninv); });
-                }
-            }
-            __syncthreads();
-        }
+    if (fix && dim == 3 && shape == HC_SHAPE_L3072) {
+        if (mode == 2) slab_lines3072<6>(S, P, s, mulrow);
+        else if (mode == 3) slab_lines3072<3>(S, P, s, mulrow);
+        else slab_lines3072<1>(S, P, s, mulrow);
         return;
     }
-    if (fix && dim == 2 && (shape == HC_SHAPE_C12 || shape == HC_SHAPE_C4)) {
+    if (fix && dim == 2 && shape == HC_SHAPE_C12) {
         for (int l = threadIdx.x; l < S.dk; l += blockDim.x) {
             int64_t* g = S.data + l;
-            if (CLS != 2 && (CLS == 1 || shape == HC_SHAPE_C12)) {
-                if (mode == 2) run_column<HC_SHAPE_C12, 6, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
-                else run_column<HC_SHAPE_C12, 1, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
-            } else if (CLS != 1) {
-                if (mode == 2) run_column<HC_SHAPE_C4, 6, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
-                else run_column<HC_SHAPE_C4, 1, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
-            }
+            if (mode == 2) run_column<HC_SHAPE_C12, 6, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
+            else run_column<HC_SHAPE_C12, 1, true>(P, g, S.s2, g, S.s2, mulrow, 1, S.n, S.ninv);
         }
         __syncthreads();
         return;
@@ -110,11 +134,21 @@ __global__ void __launch_bounds__(MAXT, MINB)
             stage_twiddles(P3, tw3);
             __syncthreads();
         }
+        // one half of a transform: dimension 2, then dimension 3 (modes as slab_pass)
+        const bool slab12288 = CLS == 2 || (CLS == 0 && crt_slab_12288(S.shapes));
+        auto half = [&](auto mode3, int mode2, const int64_t* kl, const int64_t* kk) {
+            constexpr int M = decltype(mode3)::value;
+            if (CLS != 1 && slab12288) {
+                slab12288_half<M == 2 ? 6 : M>(S, P2, P3, smem, kl, kk);
+            } else if constexpr (CLS != 2) {
+                slab_pass<GENERIC>(S, P2, tw2, smem, 2, mode2, kl, logv);
+                slab_pass<GENERIC>(S, P3, tw3, smem, 3, M, kk, logv);
+            }
+        };
         if (S.ops & HC_CRT_FORWARD) {
-            slab_pass<GENERIC, CLS>(S, P2, tw2, smem, 2, 2, S.kl, logv);
-            slab_pass<GENERIC, CLS>(S, P3, tw3, smem, 3, 2, S.kk, logv);
-            slab_pass<GENERIC, CLS>(S, P2, tw2, smem, 2, 1, nullptr, logv);
-            slab_pass<GENERIC, CLS>(S, P3, tw3, smem, 3, (S.ops & HC_CRT_MUL) ? 3 : 1, nullptr, logv);
+            half(std::integral_constant<int, 2>{}, 2, S.kl, S.kk);
+            if (S.ops & HC_CRT_MUL) half(std::integral_constant<int, 3>{}, 1, nullptr, nullptr);
+            else half(std::integral_constant<int, 1>{}, 1, nullptr, nullptr);
         } else if (S.ops & HC_CRT_MUL) {
             const int total = S.dl * S.dk;
             for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
@@ -125,10 +159,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
             __syncthreads();
         }
         if (S.ops & HC_CRT_INVERSE) {
-            slab_pass<GENERIC, CLS>(S, P2, tw2, smem, 2, 2, S.ikl, logv);
-            slab_pass<GENERIC, CLS>(S, P3, tw3, smem, 3, 2, S.ikk, logv);
-            slab_pass<GENERIC, CLS>(S, P2, tw2, smem, 2, 1, nullptr, logv);
-            slab_pass<GENERIC, CLS>(S, P3, tw3, smem, 3, 1, nullptr, logv);
+            half(std::integral_constant<int, 2>{}, 2, S.ikl, S.ikk);
+            half(std::integral_constant<int, 1>{}, 1, nullptr, nullptr);
         }
     }
 }

@@ -17,7 +17,7 @@
 // the two kernels saves half the traffic, but its CTAs wait for one another and for twelve free places
 // at once: pb_to_crt of [24, 23, 4, 12288] 563 us against 510 us, of [8, 23, 4, 12288] 202 against 186.
 #include "common.cuh"
-#include "ntt_plan.cuh"
+#include "ntt_run.cuh"
 
 namespace hc {
 const void* plan_device(hc_ntt_plan p);
@@ -31,43 +31,6 @@ constexpr size_t SMEM4096 = 4608 * 8;  // one padded 4096-residue block
 
 /// lead: CTAs over (slab, 256 positions). DIR 0: forward, times the dimension-2 kernel m2 [r][4] (limbs),
 /// reading src, writing t; DIR 1: inverse, in place (src = t).
-template <int DIR, int LG>
-__device__ __forceinline__ void lead12288(const KView& t, const KView& src, const DevPlanHeader* P2,
-                                          const DevPlanHeader* P3, const BarrettLimbs* m2, int64_t n, int64_t i, int64_t j,
-                                          int p) {
-    constexpr bool inv = DIR == 1;
-    const fast::CtxL c2 = make_ctx<fast::CtxL>(P2), c3 = make_ctx<fast::CtxL>(P3);
-    const FixedSched<HC_SHAPE_C4, LG, inv> sch2{};
-    const FixedSched<HC_SHAPE_L12288, LG, inv> sch3{};
-    const fast::SF f2[2] = {fast::sflags(sch2, 0), fast::sflags(sch2, 1)};
-    const fast::SF f3 = fast::sflags(sch3, 0);
-    const int64_t* gs = reinterpret_cast<const int64_t*>(src.p) + i * src.s0 + j * src.s1 + p;
-    int64_t* g = reinterpret_cast<int64_t*>(t.p) + i * t.s0 + j * t.s1 + p;
-    int64_t x[3][4];
-#pragma unroll
-    for (int b = 0; b < 3; b++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) x[b][k] = gs[k * src.s2 + 4096 * b];
-#pragma unroll
-    for (int b = 0; b < 3; b++) fast::col4(c2, f2, inv, false, x[b]);
-    const fast::MontC mont{mont_const_mod(n)};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        if (DIR == 0) {
-            const BarrettLimbs w = load_limbs(m2 + k);
-#pragma unroll
-            for (int b = 0; b < 3; b++) x[b][k] = mont.mul(x[b][k], w);
-        }
-        if (f3.red) {
-#pragma unroll
-            for (int b = 0; b < 3; b++) x[b][k] = fast::red1(c3, x[b][k]);
-        }
-        if (inv) fast::inv3(c3, f3, x[0][k], x[1][k], x[2][k]);
-        else fast::fwd3<true>(c3, f3, false, 0, x[0][k], x[1][k], x[2][k]);
-#pragma unroll
-        for (int b = 0; b < 3; b++) g[k * t.s2 + 4096 * b] = x[b][k];
-    }
-}
 template <int DIR>
 __global__ void __launch_bounds__(LEAD_THREADS, 4)
     lead12288_kernel(KView t, KView src, PlanPtrs p2, PlanPtrs p3, const BarrettLimbs* m2, KMods mods) {
@@ -75,10 +38,12 @@ __global__ void __launch_bounds__(LEAD_THREADS, 4)
     const int64_t tile = gridDim.x - 1 - blockIdx.x;
     const int64_t slab = tile / (4096 / LEAD_THREADS), j = slab % t.n1, i = slab / t.n1;
     const int p = (int)(tile % (4096 / LEAD_THREADS)) * LEAD_THREADS + threadIdx.x;
-    const DevPlanHeader* P2 = p2.p[j];
     const DevPlanHeader* P3 = p3.p[j];
-    if (P3->cls == 57) lead12288<DIR, 57>(t, src, P2, P3, m2 + 4 * j, mods.n[j], i, j, p);
-    else lead12288<DIR, 56>(t, src, P2, P3, m2 + 4 * j, mods.n[j], i, j, p);
+    const fast::CtxL c2 = make_ctx<fast::CtxL>(p2.p[j]), c3 = make_ctx<fast::CtxL>(P3);
+    const int64_t* gs = reinterpret_cast<const int64_t*>(src.p) + i * src.s0 + j * src.s1 + p;
+    int64_t* g = reinterpret_cast<int64_t*>(t.p) + i * t.s0 + j * t.s1 + p;
+    if (P3->cls == 57) lead12288<DIR, 57>(c2, c3, gs, src.s2, g, t.s2, m2 + 4 * j, mods.n[j]);
+    else lead12288<DIR, 56>(c2, c3, gs, src.s2, g, t.s2, m2 + 4 * j, mods.n[j]);
 }
 
 /// blocks: CTAs over (line, block). MODE 6: forward, times the dimension-3 kernel m3 [r][12288] (limbs); 1:
@@ -103,7 +68,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS)
         mulp = kat<int64_t>(pm, i, j, k, 0) + me * 4096 * blk;
     }
     with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, true>(P, [&](const auto& sch) {
-        fast::block4096<MODE>(sch, c, smem, g, mulp, me, fast::make_mont<fast::CtxL, MODE>(mods.n[j], mods.ninv[j]));
+        fast::block4096<MODE>(fast::CtaTeam{}, sch, c, smem, g, mulp, me, fast::make_mont<fast::CtxL, MODE>(mods.n[j], mods.ninv[j]));
     });
 }
 

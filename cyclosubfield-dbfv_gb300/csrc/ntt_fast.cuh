@@ -93,6 +93,20 @@ __device__ __forceinline__ SF sflags(const SCH& sch, int s) {
 template <class CTX>
 __device__ __forceinline__ int64_t red1(const CTX& c, int64_t x) { return c.red(x); }
 
+/// The threads that run one line or block together: a whole CTA, or a part of it with a barrier of its
+/// own (named barrier `bar`).
+struct CtaTeam {
+    __device__ __forceinline__ int tid() const { return threadIdx.x; }
+    __device__ __forceinline__ int size() const { return blockDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+struct PartTeam {
+    int rank, threads, bar;
+    __device__ __forceinline__ int tid() const { return rank; }
+    __device__ __forceinline__ int size() const { return threads; }
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory"); }
+};
+
 // ---------------------------------------------------------------- butterflies
 
 /// Forward radix-2 butterfly of block `tb` (src/hal/ntt.rs:338-349). UNIFORM0: the block is 0
@@ -228,8 +242,8 @@ __device__ __forceinline__ void inv_group(const CTX& c, const SF* f, int blockK,
 /// One pass of K radix-2 stages of a factor over a padded shared-memory tile: groups of 2^K
 /// elements at distance SPAN (= 2^LOG_SPAN) inside blocks of 2^LOG_GLEN elements, 2^LOG_NB twiddle
 /// blocks per factor at the pass's reference stage (first stage forward, last stage inverse).
-template <bool INV, int K, int LOG_SPAN, int LOG_GLEN, int LOG_NB, class SCH, class CTX>
-__device__ __forceinline__ void r2_pass(const CTX& c, int64_t* s, int ngroups, const SCH& sch, int s0,
+template <bool INV, int K, int LOG_SPAN, int LOG_GLEN, int LOG_NB, class SCH, class CTX, class TEAM>
+__device__ __forceinline__ void r2_pass(const TEAM& tm, const CTX& c, int64_t* s, int ngroups, const SCH& sch, int s0,
                                         bool reduce_output) {
     constexpr int M = 1 << K, SPAN = 1 << LOG_SPAN;
     SF f[K];
@@ -239,7 +253,7 @@ __device__ __forceinline__ void r2_pass(const CTX& c, int64_t* s, int ngroups, c
         f[q] = sflags(sch, s0 + q);
         fuse[q] = f[q].last && reduce_output;
     }
-    for (int gg = threadIdx.x; gg < ngroups; gg += blockDim.x) {
+    for (int gg = tm.tid(); gg < ngroups; gg += tm.size()) {
         const int g = gg >> LOG_SPAN, o = gg & (SPAN - 1);
         const int blk = g & ((1 << LOG_NB) - 1);
         const int base = (g << LOG_GLEN) + o;
@@ -301,8 +315,8 @@ __device__ __forceinline__ const int64_t* block_multiplier(const int64_t* mulp, 
 /// (the inverse pass's lanes hold runs of eight already and store from registers). Against block
 /// barriers around each pass and a store loop that loaded its multipliers as it went: pb_to_crt of
 /// [24, 23, 4, 12288] 611 -> 561 us, of [24, 34, 12, 3072] 574 -> 557 us.
-template <int MODE, class SCH, class CTX, class MONT>
-__device__ __forceinline__ void tail64(const CTX& c, int64_t* s, int len, const SCH& sch, int s0, bool reduce_output,
+template <int MODE, class SCH, class CTX, class MONT, class TEAM>
+__device__ __forceinline__ void tail64(const TEAM& tm, const CTX& c, int64_t* s, int len, const SCH& sch, int s0, bool reduce_output,
                                        int64_t* g, const int64_t* mulp, int64_t me, const MONT& mont) {
     constexpr bool inv = MODE & 1, mul = MODE & 2;
     SF f[6];
@@ -312,8 +326,8 @@ __device__ __forceinline__ void tail64(const CTX& c, int64_t* s, int len, const 
         f[q] = sflags(sch, s0 + q);
         fuse[q] = f[q].last && reduce_output;
     }
-    const int lane = threadIdx.x & 31;
-    for (int e0 = (threadIdx.x >> 5) << 8; e0 < len; e0 += blockDim.x << 3) {
+    const int lane = tm.tid() & 31;
+    for (int e0 = (tm.tid() >> 5) << 8; e0 < len; e0 += tm.size() << 3) {
         // groups of eight at distance 8 (lane = 8 block + offset), and of eight neighbours
         const int ea = e0 + ((lane >> 3) << 6) + (lane & 7), eb = e0 + (lane << 3);
         int64_t* pa = s + pad8(ea);
@@ -380,15 +394,15 @@ __device__ __forceinline__ void red_all(const CTX& c, bool red, int64_t* x) {
 /// tile kernel (0 forward, 1 inverse, 2 forward + product, 3 inverse + product); the schedule
 /// SCH is that of the programme of MODE's direction. Stages: 0 = factor 2, 1 = factor 3,
 /// 2..4 = factor 8, 5..10 = factor 64.
-template <int MODE, class SCH, class CTX>
-__device__ __forceinline__ void line3072(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
+template <int MODE, class SCH, class CTX, class TEAM>
+__device__ __forceinline__ void line3072(const TEAM& tm, const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
                                          int64_t me, int64_t mn, int64_t mi) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     // pass 1: factors 2 (distance 1536) and 3 (distance 512), straight from global memory
     {
         const SF f0 = sflags(sch, 0), f1 = sflags(sch, 1);
         const bool fz0 = f0.last && reduce_output, fz1 = f1.last && reduce_output;
-        for (int o = threadIdx.x; o < 512; o += blockDim.x) {
+        for (int o = tm.tid(); o < 512; o += tm.size()) {
             int64_t x[2][3];
 #pragma unroll
             for (int b = 0; b < 2; b++)
@@ -424,14 +438,14 @@ __device__ __forceinline__ void line3072(const SCH& sch, const CTX& c, int64_t* 
                 for (int a = 0; a < 3; a++) s[pad8(o + 512 * a + 1536 * b)] = x[b][a];
         }
     }
-    __syncthreads();
+    tm.sync();
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 0>(c, s, 384, sch, 2, reduce_output);  // factor 8: distances 256, 128, 64
+        r2_pass<false, 3, 6, 9, 0>(tm, c, s, 384, sch, 2, reduce_output);  // factor 8: distances 256, 128, 64
     } else {
-        r2_pass<true, 3, 6, 9, 0>(c, s, 384, sch, 2, false);  // factor 8: distances 64, 128, 256
+        r2_pass<true, 3, 6, 9, 0>(tm, c, s, 384, sch, 2, false);  // factor 8: distances 64, 128, 256
     }
-    __syncthreads();
-    tail64<MODE>(c, s, 3072, sch, 5, reduce_output, g, mulp, me, make_mont<CTX, MODE>(mn, mi));  // factor 64
+    tm.sync();
+    tail64<MODE>(tm, c, s, 3072, sch, 5, reduce_output, g, mulp, me, make_mont<CTX, MODE>(mn, mi));  // factor 64
 }
 
 /// One of the three 4096-residue blocks of a [3, 64, 64] line, computed by one CTA of a 3-CTA
@@ -505,19 +519,19 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, in
     }
     cluster_sync();  // also a barrier of this CTA
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
+        r2_pass<false, 3, 6, 9, 3>(CtaTeam{}, c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
     } else {
-        r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
+        r2_pass<true, 3, 9, 12, 0>(CtaTeam{}, c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
     }
     __syncthreads();
-    tail64<MODE>(c, s, 4096, sch, 7, reduce_output, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me,
+    tail64<MODE>(CtaTeam{}, c, s, 4096, sch, 7, reduce_output, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me,
                  make_mont<CTX, MODE>(mn, mi));  // factor 64 (b)
 }
 
 /// Stages 1..12 of one 4096-residue block of a [3, 64, 64] line (the two factors 64, which act within the
 /// block): g -> g via the padded tile s; mulp: the block's multipliers.
-template <int MODE, class SCH, class CTX, class MONT>
-__device__ __forceinline__ void block4096(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
+template <int MODE, class SCH, class CTX, class MONT, class TEAM>
+__device__ __forceinline__ void block4096(const TEAM& tm, const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
                                           int64_t me, const MONT& mont) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     {
@@ -530,7 +544,7 @@ __device__ __forceinline__ void block4096(const SCH& sch, const CTX& c, int64_t*
         }
         // factor 64 (a): distances 2048, 1024, 512 forward, 64, 128, 256 inverse, straight from global memory
         constexpr int span = inv ? 64 : 512;
-        for (int gg = threadIdx.x; gg < 512; gg += blockDim.x) {
+        for (int gg = tm.tid(); gg < 512; gg += tm.size()) {
             const int base = inv ? ((gg >> 6) << 9) + (gg & 63) : gg;
             int64_t x[8];
 #pragma unroll
@@ -541,42 +555,14 @@ __device__ __forceinline__ void block4096(const SCH& sch, const CTX& c, int64_t*
             for (int m = 0; m < 8; m++) s[pad8(base + span * m)] = x[m];
         }
     }
-    __syncthreads();
+    tm.sync();
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 3>(c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
+        r2_pass<false, 3, 6, 9, 3>(tm, c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
     } else {
-        r2_pass<true, 3, 9, 12, 0>(c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
+        r2_pass<true, 3, 9, 12, 0>(tm, c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
     }
-    __syncthreads();
-    tail64<MODE>(c, s, 4096, sch, 7, reduce_output, g, mulp, me, mont);  // factor 64 (b)
-}
-
-/// A [3, 64, 64] line with a tile of one 4096-residue block (for kernels that cannot give a CTA the
-/// whole 12288-residue line): stage 0, the factor-3 stage that couples the three blocks, runs in
-/// place in global memory, each thread owning whole position triples (the butterfly of
-/// first pass); stages 1..12, which act within a block, then run block by block. The first pass's global writes are the CTA's own, visible to its
-/// threads after the barrier.
-template <int MODE, class SCH, class CTX>
-__device__ __forceinline__ void line12288_seq(const SCH& sch, const CTX& c, int64_t* s, int64_t* g,
-                                              const int64_t* mulp, int64_t me, int64_t mn, int64_t mi) {
-    constexpr bool inv = MODE & 1;
-    const SF f = sflags(sch, 0);
-    for (int p = threadIdx.x; p < 4096; p += blockDim.x) {
-        int64_t a = g[p], b = g[p + 4096], d = g[p + 8192];
-        if (f.red) {
-            a = red1(c, a);
-            b = red1(c, b);
-            d = red1(c, d);
-        }
-        if (!inv) fwd3<true>(c, f, false, 0, a, b, d);
-        else inv3(c, f, a, b, d);
-        g[p] = a, g[p + 4096] = b, g[p + 8192] = d;
-    }
-    __syncthreads();
-    for (int blk = 0; blk < 3; blk++) {
-        block4096<MODE>(sch, c, s, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me, make_mont<CTX, MODE>(mn, mi));
-        __syncthreads();  // the tile is refilled by the next block
-    }
+    tm.sync();
+    tail64<MODE>(tm, c, s, 4096, sch, 7, reduce_output, g, mulp, me, mont);  // factor 64 (b)
 }
 
 // ---------------------------------------------------------------- columns

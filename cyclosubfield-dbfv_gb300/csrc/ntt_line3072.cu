@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPt
         me = mul.b3 ? 0 : 1;
         mn = mods.n[j], mi = mods.ninv[j];
     }
-    run_line3072<MODE, FIX>(P, smem, g, mulp, me, mn, mi);
+    run_line3072<MODE, FIX>(fast::CtaTeam{}, P, smem, g, mulp, me, mn, mi);
 }
 
 template <int MODE, bool FIX, int THREADS, int MINB>

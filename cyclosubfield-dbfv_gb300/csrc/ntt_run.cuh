@@ -19,12 +19,12 @@ __device__ __forceinline__ const int64_t* multiplier(const KView& mul, int64_t i
 
 /// One [2, 3, 8, 64] line g of plan P through the CTA's shared-memory line buffer s; FIX: the plan is
 /// fixed.
-template <int MODE, bool FIX>
-__device__ __forceinline__ void run_line3072(const DevPlanHeader* P, int64_t* s, int64_t* g, const int64_t* mulp,
+template <int MODE, bool FIX, class TEAM>
+__device__ __forceinline__ void run_line3072(const TEAM& tm, const DevPlanHeader* P, int64_t* s, int64_t* g, const int64_t* mulp,
                                              int64_t me, int64_t mn, int64_t mi) {
     const auto c = make_ctx<PassCtx<FIX>>(P);
     with_sched<HC_SHAPE_L3072, (MODE & 1) != 0, FIX>(
-        P, [&](const auto& sch) { fast::line3072<MODE>(sch, c, s, g, mulp, me, mn, mi); });
+        P, [&](const auto& sch) { fast::line3072<MODE>(tm, sch, c, s, g, mulp, me, mn, mi); });
 }
 
 /// One specialised column g[0], g[ge], ... of shape SHAPE transformed in registers; it is read
@@ -70,6 +70,43 @@ __device__ __forceinline__ void run_column(const DevPlanHeader* P, int64_t* g, i
             }
         }
     });
+}
+
+/// The lead pass of a field_49152 slab at one position p of its blocks (see crt_slab.cu): the four-point
+/// columns, with DIR 0 their products with the dimension-2 kernel m2 [4], and the radix-3 stage of the
+/// four rows, from gs[k ss2 + 4096 b] to g[k s2 + 4096 b].
+template <int DIR, int LG>
+__device__ __forceinline__ void lead12288(const fast::CtxL& c2, const fast::CtxL& c3, const int64_t* gs, int64_t ss2,
+                                          int64_t* g, int64_t s2, const BarrettLimbs* m2, int64_t n) {
+    constexpr bool inv = DIR == 1;
+    const FixedSched<HC_SHAPE_C4, LG, inv> sch2{};
+    const FixedSched<HC_SHAPE_L12288, LG, inv> sch3{};
+    const fast::SF f2[2] = {fast::sflags(sch2, 0), fast::sflags(sch2, 1)};
+    const fast::SF f3 = fast::sflags(sch3, 0);
+    int64_t x[3][4];
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[b][k] = gs[k * ss2 + 4096 * b];
+#pragma unroll
+    for (int b = 0; b < 3; b++) fast::col4(c2, f2, inv, false, x[b]);
+    const fast::MontC mont{mont_const_mod(n)};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (DIR == 0) {
+            const BarrettLimbs w = load_limbs(m2 + k);
+#pragma unroll
+            for (int b = 0; b < 3; b++) x[b][k] = mont.mul(x[b][k], w);
+        }
+        if (f3.red) {
+#pragma unroll
+            for (int b = 0; b < 3; b++) x[b][k] = fast::red1(c3, x[b][k]);
+        }
+        if (inv) fast::inv3(c3, f3, x[0][k], x[1][k], x[2][k]);
+        else fast::fwd3<true>(c3, f3, false, 0, x[0][k], x[1][k], x[2][k]);
+#pragma unroll
+        for (int b = 0; b < 3; b++) g[k * s2 + 4096 * b] = x[b][k];
+    }
 }
 
 }  // namespace

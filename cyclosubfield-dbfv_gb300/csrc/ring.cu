@@ -1948,6 +1948,19 @@ struct CrtGroup {
 struct hc_crt_batch_s {
     hc_context ctx = nullptr;
     std::vector<CrtGroup> groups;  // by shape class; groups[0] holds the most residues
+    // with several groups: all but the first run on `side`, forked from and joined to the caller's stream
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    void create_side() {
+        CK(cuda_check(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "batch side stream"));
+        CK(cuda_check(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "batch event"));
+        CK(cuda_check(cudaEventCreateWithFlags(&join, cudaEventDisableTiming), "batch event"));
+    }
+    ~hc_crt_batch_s() {
+        if (side) cudaStreamDestroy(side);  // returns at once; its pending work completes
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+    }
 };
 
 namespace {
@@ -2150,6 +2163,7 @@ hc_status hc_crt_batch_create(hc_context ctx, const hc_crt_item* items, size_t n
             g.tw_words = std::max(g.tw_words, tws[i]);
             g.residues += (int64_t)slabs[i].dl * slabs[i].dk;
         }
+        if (b->groups.size() > 1) b->create_side();
         // the group with the most residues first: its launch shape is the batch's reported one
         std::stable_sort(b->groups.begin(), b->groups.end(),
                          [](const CrtGroup& x, const CrtGroup& y) { return x.residues > y.residues; });
@@ -2174,7 +2188,24 @@ hc_status hc_crt_batch_create(hc_context ctx, const hc_crt_item* items, size_t n
 hc_status hc_crt_batch_run(hc_crt_batch b) {
     return guard([&] {
         REQUIRE(b, HC_ERR_ARG, "null batch");
-        for (CrtGroup& g : b->groups) CK(crt_group_run(b->ctx, g));
+        // the classes' persistent launches side by side: each leaves the SMs to the others as its last
+        // slabs run out, and a class of few slabs never has them alone (128 mixed elements 3.62 -> 3.39 ms, 20 1.13 -> 1.01)
+        const cudaStream_t main = stream_of(b->ctx);
+        if (b->groups.size() > 1) {
+            CK(cuda_check(cudaEventRecord(b->fork, main), "batch fork"));
+            CK(cuda_check(cudaStreamWaitEvent(b->side, b->fork, 0), "batch fork"));
+        }
+        hc_status st = HC_OK;
+        for (size_t i = 0; i < b->groups.size() && !st; i++) {
+            if (i == 1) hc_context_set_stream(b->ctx, b->side);
+            st = crt_group_run(b->ctx, b->groups[i]);
+        }
+        hc_context_set_stream(b->ctx, main);
+        if (b->groups.size() > 1) {
+            CK(cuda_check(cudaEventRecord(b->join, b->side), "batch join"));
+            CK(cuda_check(cudaStreamWaitEvent(main, b->join, 0), "batch join"));
+        }
+        CK(st);
     });
 }
 
