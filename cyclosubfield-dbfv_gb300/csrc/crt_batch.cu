@@ -11,12 +11,12 @@ CrtBatchKernel crt_batch_f36864(int ctas_per_sm);
 CrtBatchKernel crt_batch_f49152(int ctas_per_sm);
 CrtBatchKernel crt_batch_mixed(int ctas_per_sm);
 
-/// Shared-memory words a slab of the batched transform needs: two padded 3072-residue lines (one per team of
-/// 128 threads), one padded 4096-residue block of a 12288-residue line, or the generic tile (the whole
+/// Shared-memory words a slab of the batched transform needs: two 3072-residue lines (one per team of
+/// 128 threads), one 4096-residue block of a 12288-residue line, or the generic tile (the whole
 /// line, or deg_L' x 2^logv dimension-2 columns); the specialised column passes use none.
 size_t crt_slab_tile_words(int32_t shapes, int32_t dl, int32_t dk, int logv) {
-    if (crt_slab_12288(shapes)) return 4096 + 4096 / 8;
-    const size_t w3 = crt_slab_limbs(shapes, 3) ? 2 * (size_t)line_tile_words(HC_SHAPE_L3072) : (size_t)dk;
+    if (crt_slab_12288(shapes)) return BLOCK4096_WORDS;
+    const size_t w3 = crt_slab_limbs(shapes, 3) ? 2 * (size_t)LINE3072_WORDS : (size_t)dk;
     const size_t w2 = crt_slab_limbs(shapes, 2) ? 0 : ((size_t)dl << logv);
     const size_t w = std::max(w3, w2);
     return (w + 1) & ~(size_t)1;

@@ -28,12 +28,14 @@ __device__ __forceinline__ void slab12288_half(const CrtSlab& S, const DevPlanHe
     __syncthreads();
     const auto mont = fast::make_mont<fast::CtxL, MODE>(S.n, S.ninv);
     with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, true>(P3, [&](const auto& sch) {
+        int4* tws = reinterpret_cast<int4*>(s + 4096);
+        fast::stage_tail_twiddles<(MODE & 1) != 0>(fast::CtaTeam{}, c3, sch, tws, 1, 63, 7);
         for (int q = 0; q < 12; q++) {
             const int k = q / 3, blk = q - 3 * (q / 3);
             const int64_t* mulp = MODE == 6   ? fast::block_multiplier<MODE>(kk, 1, blk)
                                   : MODE == 3 ? S.op + k * S.op_s2 + 4096 * blk
                                               : nullptr;
-            fast::block4096<MODE>(fast::CtaTeam{}, sch, c3, s, S.data + k * S.s2 + 4096 * blk, mulp, 1, mont);
+            fast::block4096<MODE>(fast::CtaTeam{}, sch, c3, s, tws, S.data + k * S.s2 + 4096 * blk, mulp, 1, mont);
             __syncthreads();  // the tile is refilled by the next block
         }
     });
@@ -45,9 +47,10 @@ template <int MODE>
 __device__ __forceinline__ void slab_lines3072(const CrtSlab& S, const DevPlanHeader* P, int64_t* s, const int64_t* mulrow) {
     const int teams = blockDim.x == 256 ? 2 : 1, t = (int)threadIdx.x / 128 % teams;
     const fast::PartTeam tm{(int)threadIdx.x - 128 * t, (int)blockDim.x / teams, 1 + t};
-    int64_t* tile = s + t * line_tile_words(HC_SHAPE_L3072);
+    int64_t* tile = s + t * LINE3072_WORDS;
     for (int k = t; k < S.dl; k += teams) {
-        run_line3072<MODE, true>(tm, P, tile, S.data + k * S.s2, MODE == 3 ? S.op + k * S.op_s2 : mulrow, 1, S.n, S.ninv);
+        run_line3072<MODE, true>(tm, P, tile, S.data + k * S.s2, MODE == 3 ? S.op + k * S.op_s2 : mulrow, 1, S.n, S.ninv,
+                                 k == t);
         tm.sync();
     }
     __syncthreads();

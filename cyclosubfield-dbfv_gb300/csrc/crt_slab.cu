@@ -27,7 +27,7 @@ int32_t plan_shape(hc_ntt_plan p);
 namespace {
 
 constexpr int LEAD_THREADS = 256;
-constexpr size_t SMEM4096 = 4608 * 8;  // one padded 4096-residue block
+constexpr size_t SMEM4096 = (size_t)BLOCK4096_WORDS * 8;
 
 /// lead: CTAs over (slab, 256 positions). DIR 0: forward, times the dimension-2 kernel m2 [r][4] (limbs),
 /// reading src, writing t; DIR 1: inverse, in place (src = t).
@@ -68,7 +68,9 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS)
         mulp = kat<int64_t>(pm, i, j, k, 0) + me * 4096 * blk;
     }
     with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, true>(P, [&](const auto& sch) {
-        fast::block4096<MODE>(fast::CtaTeam{}, sch, c, smem, g, mulp, me, fast::make_mont<fast::CtxL, MODE>(mods.n[j], mods.ninv[j]));
+        int4* tws = reinterpret_cast<int4*>(smem + 4096);
+        fast::stage_tail_twiddles<(MODE & 1) != 0>(fast::CtaTeam{}, c, sch, tws, 1, 63, 7);
+        fast::block4096<MODE>(fast::CtaTeam{}, sch, c, smem, tws, g, mulp, me, fast::make_mont<fast::CtxL, MODE>(mods.n[j], mods.ninv[j]));
     });
 }
 

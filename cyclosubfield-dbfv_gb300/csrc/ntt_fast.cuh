@@ -8,9 +8,9 @@
 //    immediate offsets;
 //  * lines: the first register pass reads its elements straight from global memory and runs the
 //    leading radix-2/radix-3 factors together; the remaining radix-2 stages run three at a time on
-//    eight elements per thread; the tile lives in shared memory padded by one word per eight
-//    words, which keeps the strided 64-bit accesses of every pass free of bank conflicts while
-//    leaving all offsets inside a group constant;
+//    eight elements per thread; the tile lives in shared memory, its columns swizzled so that
+//    every pass's 64-bit accesses are free of bank conflicts (sw), with the twiddles of the passes
+//    behind the first beside it;
 //  * columns: one thread transforms a whole column (12 or 4 residues) in registers, loading and
 //    storing it coalesced across neighbouring columns - no shared memory at all;
 //  * a twiddle-1 butterfly skips its multiplication only where the skip is uniform across the
@@ -20,11 +20,16 @@
 
 namespace fast {
 
-/// Index of tile element i in the padded shared-memory layout.
-__device__ __forceinline__ int pad8(int i) { return i + (i >> 3); }
-/// Constant offset of group element m (stride `span`) from the padded group base (valid for the
-/// group geometries used here: span a multiple of 8, or span < 8 with the base's low bits < span).
-__host__ __device__ constexpr int goff(int m, int span) { return m * span + ((m * span) >> 3); }
+/// Slot of tile element i: its low four bits XOR-ed with bits 4..6, bit 6 entering twice (bits 2 and 3).
+/// Sixteen 8-byte words span the banks, and every access of a half-warp here is one of: sixteen
+/// neighbours, eight words apart (neighbours' groups), or two runs of eight 64 apart; each of these
+/// falls into sixteen distinct columns. (One word of padding per eight, the layout before, made the
+/// sixteen neighbours collide: a third of the shared-memory cycles.) The map is linear over XOR.
+__host__ __device__ constexpr int sw(int i) { return i ^ ((i >> 4) & 7) ^ ((i >> 3) & 8); }
+/// Element base + part of a tile, for a constant part whose bits are clear in base; swb = sw(base).
+__device__ __forceinline__ int64_t& el(int64_t* s, int swb, int part) {
+    return s[(swb ^ (sw(part) & 127)) + (sw(part) & ~127)];
+}
 
 /// Products of a plan with any schedule and modulus: (z, u) pairs.
 struct Ctx {
@@ -47,6 +52,22 @@ struct CtxL {
     typedef BarrettLimbs Tw;
     __device__ __forceinline__ Tw get(int idx) const {
         const int4 a = __ldg(tw + idx);
+        return BarrettLimbs{a.x, a.y, a.z, a.w};
+    }
+    __device__ __forceinline__ int64_t mul(const Tw& w, int64_t x) const { return barrett_mul(w, x, m); }
+    __device__ __forceinline__ int64_t scale(int64_t x) const { return barrett_mul(il, x, m); }
+    __device__ __forceinline__ int64_t red(int64_t x) const { return barrett_red(x, m); }
+};
+
+/// CtxL with a pass's twiddles in shared memory (stage_tail_twiddles).
+struct CtxS {
+    static constexpr bool LIMBS = true;
+    BarrettMod m;
+    BarrettLimbs il;
+    const int4* tw;
+    typedef BarrettLimbs Tw;
+    __device__ __forceinline__ Tw get(int idx) const {
+        const int4 a = tw[idx];
         return BarrettLimbs{a.x, a.y, a.z, a.w};
     }
     __device__ __forceinline__ int64_t mul(const Tw& w, int64_t x) const { return barrett_mul(w, x, m); }
@@ -109,10 +130,10 @@ struct PartTeam {
 
 // ---------------------------------------------------------------- butterflies
 
-/// Forward radix-2 butterfly of block `tb` (src/hal/ntt.rs:338-349). UNIFORM0: the block is 0
-/// for the whole warp, so a permitted skip avoids the product.
+/// Forward radix-2 butterfly of block `tb` (src/hal/ntt.rs:338-349), whose twiddle is entry `at` of its
+/// stage's. UNIFORM0: the block is 0 for the whole warp, so a permitted skip avoids the product.
 template <bool UNIFORM0, class CTX>
-__device__ __forceinline__ void fwd2(const CTX& c, const SF& f, bool fuse, int tb, int64_t& x, int64_t& y) {
+__device__ __forceinline__ void fwd2(const CTX& c, const SF& f, bool fuse, int tb, int at, int64_t& x, int64_t& y) {
     int64_t t;
     if (UNIFORM0) {
         if (f.skip_ok) {
@@ -121,7 +142,7 @@ __device__ __forceinline__ void fwd2(const CTX& c, const SF& f, bool fuse, int t
             t = c.mul(c.get(f.tw_off), y);
         }
     } else {
-        t = c.mul(c.get(f.tw_off + tb), y);
+        t = c.mul(c.get(f.tw_off + at), y);
         if (f.skip_ok && tb == 0) t = y;
     }
     int64_t o0 = wadd(x, t), o1 = wsub(x, t);
@@ -183,8 +204,9 @@ __device__ __forceinline__ void inv3(const CTX& c, const SF& f, int64_t& a, int6
 // ---------------------------------------------------------------- register groups of radix-2 stages
 
 /// K forward radix-2 stages on the group x[0..2^K) (element m at distance m * span). block0:
-/// the group's twiddle block at the first stage (0 for the whole warp when NB0 == 1).
-template <int K, bool NB1, class CTX>
+/// the group's twiddle block at the first stage (0 for the whole warp when NB0 == 1). BY_PART: the
+/// stages' tables are ordered by the block's compile-time part (stage_tail_twiddles).
+template <int K, bool NB1, bool BY_PART = false, class CTX>
 __device__ __forceinline__ void fwd_group(const CTX& c, const SF* f, const bool* fuse, int block0, int64_t* x) {
     constexpr int M = 1 << K;
 #pragma unroll
@@ -198,15 +220,16 @@ __device__ __forceinline__ void fwd_group(const CTX& c, const SF* f, const bool*
         for (int j = 0; j < M / 2; j++) {
             const int m1 = ((j / half) * 2 * half) + (j % half), m2 = m1 + half;
             const int tbc = m1 >> (K - q);  // compile-time part of the block
-            if (NB1 && tbc == 0) fwd2<true>(c, f[q], fuse[q], 0, x[m1], x[m2]);
-            else fwd2<false>(c, f[q], fuse[q], (block0 << q) + tbc, x[m1], x[m2]);
+            const int tb = (block0 << q) + tbc;
+            if (NB1 && tbc == 0) fwd2<true>(c, f[q], fuse[q], 0, 0, x[m1], x[m2]);
+            else fwd2<false>(c, f[q], fuse[q], tb, BY_PART ? 8 * tbc + block0 : tb, x[m1], x[m2]);
         }
     }
 }
 
 /// K inverse radix-2 stages (distances growing) on the group x[0..2^K); blockK: the group's block
 /// at the pass's last stage (NBK1: 0 for the whole warp).
-template <int K, bool NBK1, class CTX>
+template <int K, bool NBK1, bool BY_PART = false, class CTX>
 __device__ __forceinline__ void inv_group(const CTX& c, const SF* f, int blockK, int64_t* x) {
     constexpr int M = 1 << K;
 #pragma unroll
@@ -230,7 +253,7 @@ __device__ __forceinline__ void inv_group(const CTX& c, const SF* f, int blockK,
                 x[m2] = dif;
             } else {
                 const int tb = (blockK << (K - 1 - q)) + tbc;
-                int64_t t = c.mul(c.get(f[q].tw_off + tb), dif);
+                int64_t t = c.mul(c.get(f[q].tw_off + (BY_PART ? 8 * tbc + blockK : tb)), dif);
                 if (tbc == 0 && tb == 0) t = dif;  // block 0's twiddle is 1, no other block's is
                 x[m1] = sum;
                 x[m2] = t;
@@ -239,7 +262,7 @@ __device__ __forceinline__ void inv_group(const CTX& c, const SF* f, int blockK,
     }
 }
 
-/// One pass of K radix-2 stages of a factor over a padded shared-memory tile: groups of 2^K
+/// One pass of K radix-2 stages of a factor over a shared-memory tile: groups of 2^K
 /// elements at distance SPAN (= 2^LOG_SPAN) inside blocks of 2^LOG_GLEN elements, 2^LOG_NB twiddle
 /// blocks per factor at the pass's reference stage (first stage forward, last stage inverse).
 template <bool INV, int K, int LOG_SPAN, int LOG_GLEN, int LOG_NB, class SCH, class CTX, class TEAM>
@@ -256,15 +279,14 @@ __device__ __forceinline__ void r2_pass(const TEAM& tm, const CTX& c, int64_t* s
     for (int gg = tm.tid(); gg < ngroups; gg += tm.size()) {
         const int g = gg >> LOG_SPAN, o = gg & (SPAN - 1);
         const int blk = g & ((1 << LOG_NB) - 1);
-        const int base = (g << LOG_GLEN) + o;
-        int64_t* p = s + pad8(base);
+        const int swb = sw((g << LOG_GLEN) + o);
         int64_t x[M];
 #pragma unroll
-        for (int m = 0; m < M; m++) x[m] = p[goff(m, SPAN)];
+        for (int m = 0; m < M; m++) x[m] = el(s, swb, m * SPAN);
         if (INV) inv_group<K, LOG_NB == 0>(c, f, blk, x);
         else fwd_group<K, LOG_NB == 0>(c, f, fuse, blk, x);
 #pragma unroll
-        for (int m = 0; m < M; m++) p[goff(m, SPAN)] = x[m];
+        for (int m = 0; m < M; m++) el(s, swb, m * SPAN) = x[m];
     }
 }
 
@@ -306,6 +328,39 @@ __device__ __forceinline__ const int64_t* block_multiplier(const int64_t* mulp, 
     return mulp + me * 4096 * blk * ((MODE & 4) ? 2 : 1);
 }
 
+/// Words of the staged twiddles behind a tile: NA entries of the pass before a tail, 63 of the tail.
+__host__ __device__ constexpr int staged_words(int na) { return 2 * (na + 63); }
+/// Copies the limb twiddles of a line's passes behind its first to shared memory: the `na` entries from
+/// stage sa on (a factor's stages, contiguous), and the 63 of the tail's factor 64 (stages sb ..),
+/// with the three stages whose blocks differ between lanes ordered by the compile-time part of the
+/// block, so that eight lanes' twiddles are neighbours. A 16-byte load through L1 takes the load path
+/// eight cycles however few addresses a warp has, a quarter of the line kernels' load cycles in all.
+/// Visible after the next barrier.
+template <bool INV, class SCH, class TEAM>
+__device__ __forceinline__ void stage_tail_twiddles(const TEAM& tm, const CtxL& c, const SCH& sch, int4* dst, int sa, int na,
+                                                    int sb) {
+    for (int t = tm.tid(); t < na + 63; t += tm.size()) {
+        const int e = t - na;
+        int at = t;
+        if (e >= 0) {
+            // stages of 8 2^k entries, block << k | part
+            const int k = INV ? (e < 32 ? 2 : e < 48 ? 1 : e < 56 ? 0 : -1) : (e >= 31 ? 2 : e >= 15 ? 1 : e >= 7 ? 0 : -1);
+            if (k >= 0) {
+                const int base = INV ? (k == 2 ? 0 : k == 1 ? 32 : 48) : (8 << k) - 1, r = e - base;
+                at = na + base + 8 * (r & ((1 << k) - 1)) + (r >> k);
+            }
+        }
+        dst[at] = __ldg(c.tw + (e < 0 ? sch.tw(sa) + t : sch.tw(sb) + e));
+    }
+}
+/// A pass's context with its staged twiddles (from stage s0 on, at `at`); general plans keep theirs.
+template <class SCH>
+__device__ __forceinline__ CtxS staged_ctx(const CtxL& c, const SCH& sch, const int4* at, int s0) {
+    return CtxS{c.m, c.il, at - sch.tw(s0)};
+}
+template <class SCH>
+__device__ __forceinline__ const Ctx& staged_ctx(const Ctx& c, const SCH&, const int4*, int) { return c; }
+
 /// The last six stages of a line (a factor 64: distances 32 .. 1 forward, 1 .. 32 inverse; first stage s0)
 /// and its way to global memory, multiplying (modes 2 and 3) by mulp[e * me] in Montgomery form.
 /// They act within 64 consecutive elements, so each warp takes 256 of them (32 register groups of
@@ -329,20 +384,18 @@ __device__ __forceinline__ void tail64(const TEAM& tm, const CTX& c, int64_t* s,
     const int lane = tm.tid() & 31;
     for (int e0 = (tm.tid() >> 5) << 8; e0 < len; e0 += tm.size() << 3) {
         // groups of eight at distance 8 (lane = 8 block + offset), and of eight neighbours
-        const int ea = e0 + ((lane >> 3) << 6) + (lane & 7), eb = e0 + (lane << 3);
-        int64_t* pa = s + pad8(ea);
-        int64_t* pb = s + pad8(eb);
+        const int ea = e0 + ((lane >> 3) << 6) + (lane & 7), wa = sw(ea), wb = sw(e0 + (lane << 3));
         int64_t x[8];
         if (!inv) {
 #pragma unroll
-            for (int m = 0; m < 8; m++) x[m] = pa[goff(m, 8)];
+            for (int m = 0; m < 8; m++) x[m] = el(s, wa, 8 * m);
             fwd_group<3, true>(c, f, fuse, 0, x);
 #pragma unroll
-            for (int m = 0; m < 8; m++) pa[goff(m, 8)] = x[m];
+            for (int m = 0; m < 8; m++) el(s, wa, 8 * m) = x[m];
             __syncwarp();
 #pragma unroll
-            for (int m = 0; m < 8; m++) x[m] = pb[m];
-            fwd_group<3, false>(c, f + 3, fuse + 3, lane & 7, x);
+            for (int m = 0; m < 8; m++) x[m] = el(s, wb, m);
+            fwd_group<3, false, CTX::LIMBS>(c, f + 3, fuse + 3, lane & 7, x);
             constexpr int AHEAD = sizeof(typename MONT::W) == 8 ? 8 : 2;  // multipliers in registers
             typename MONT::W w[AHEAD];
             if (mul) {
@@ -350,11 +403,12 @@ __device__ __forceinline__ void tail64(const TEAM& tm, const CTX& c, int64_t* s,
                 for (int m = 0; m < AHEAD; m++) w[m] = mont.load(mulp, (e0 + 32 * m + lane) * me);
             }
 #pragma unroll
-            for (int m = 0; m < 8; m++) pb[m] = x[m];
+            for (int m = 0; m < 8; m++) el(s, wb, m) = x[m];
             __syncwarp();
+            const int wc = sw(e0 + lane);
 #pragma unroll
             for (int m = 0; m < 8; m++) {
-                int64_t v = s[pad8(e0 + 32 * m + lane)];
+                int64_t v = el(s, wc, 32 * m);
                 if (mul) {
                     v = mont.mul(v, w[m % AHEAD]);
                     if (m + AHEAD < 8) w[m % AHEAD] = mont.load(mulp, (e0 + 32 * (m + AHEAD) + lane) * me);
@@ -363,13 +417,13 @@ __device__ __forceinline__ void tail64(const TEAM& tm, const CTX& c, int64_t* s,
             }
         } else {
 #pragma unroll
-            for (int m = 0; m < 8; m++) x[m] = pb[m];
-            inv_group<3, false>(c, f, lane & 7, x);
+            for (int m = 0; m < 8; m++) x[m] = el(s, wb, m);
+            inv_group<3, false, CTX::LIMBS>(c, f, lane & 7, x);
 #pragma unroll
-            for (int m = 0; m < 8; m++) pb[m] = x[m];
+            for (int m = 0; m < 8; m++) el(s, wb, m) = x[m];
             __syncwarp();
 #pragma unroll
-            for (int m = 0; m < 8; m++) x[m] = pa[goff(m, 8)];
+            for (int m = 0; m < 8; m++) x[m] = el(s, wa, 8 * m);
             inv_group<3, true>(c, f + 3, 0, x);
 #pragma unroll
             for (int m = 0; m < 8; m++) {
@@ -390,19 +444,21 @@ __device__ __forceinline__ void red_all(const CTX& c, bool red, int64_t* x) {
     }
 }
 
-/// [2, 3, 8, 64] line (3072 residues): g -> g, via the padded tile s (3456 words). MODE as the
+/// [2, 3, 8, 64] line (3072 residues): g -> g, via the tile s (3072 words); tws: the staged twiddles of
+/// factors 8 and 64 (limb plans; complete at the first barrier here). MODE as the
 /// tile kernel (0 forward, 1 inverse, 2 forward + product, 3 inverse + product); the schedule
 /// SCH is that of the programme of MODE's direction. Stages: 0 = factor 2, 1 = factor 3,
 /// 2..4 = factor 8, 5..10 = factor 64.
 template <int MODE, class SCH, class CTX, class TEAM>
-__device__ __forceinline__ void line3072(const TEAM& tm, const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
-                                         int64_t me, int64_t mn, int64_t mi) {
+__device__ __forceinline__ void line3072(const TEAM& tm, const SCH& sch, const CTX& c, int64_t* s, const int4* tws, int64_t* g,
+                                         const int64_t* mulp, int64_t me, int64_t mn, int64_t mi) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     // pass 1: factors 2 (distance 1536) and 3 (distance 512), straight from global memory
     {
         const SF f0 = sflags(sch, 0), f1 = sflags(sch, 1);
         const bool fz0 = f0.last && reduce_output, fz1 = f1.last && reduce_output;
         for (int o = tm.tid(); o < 512; o += tm.size()) {
+            const int swb = sw(o);
             int64_t x[2][3];
 #pragma unroll
             for (int b = 0; b < 2; b++)
@@ -411,7 +467,7 @@ __device__ __forceinline__ void line3072(const TEAM& tm, const SCH& sch, const C
             red_all<6>(c, f0.red, &x[0][0]);
             if (!inv) {
 #pragma unroll
-                for (int a = 0; a < 3; a++) fwd2<true>(c, f0, fz0, 0, x[0][a], x[1][a]);
+                for (int a = 0; a < 3; a++) fwd2<true>(c, f0, fz0, 0, 0, x[0][a], x[1][a]);
                 red_all<6>(c, f1.red, &x[0][0]);
 #pragma unroll
                 for (int b = 0; b < 2; b++) fwd3<true>(c, f1, fz1, 0, x[b][0], x[b][1], x[b][2]);
@@ -435,17 +491,18 @@ __device__ __forceinline__ void line3072(const TEAM& tm, const SCH& sch, const C
 #pragma unroll
             for (int b = 0; b < 2; b++)
 #pragma unroll
-                for (int a = 0; a < 3; a++) s[pad8(o + 512 * a + 1536 * b)] = x[b][a];
+                for (int a = 0; a < 3; a++) el(s, swb, 512 * a + 1536 * b) = x[b][a];
         }
     }
     tm.sync();
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 0>(tm, c, s, 384, sch, 2, reduce_output);  // factor 8: distances 256, 128, 64
+        r2_pass<false, 3, 6, 9, 0>(tm, staged_ctx(c, sch, tws, 2), s, 384, sch, 2, reduce_output);  // factor 8: distances 256, 128, 64
     } else {
-        r2_pass<true, 3, 6, 9, 0>(tm, c, s, 384, sch, 2, false);  // factor 8: distances 64, 128, 256
+        r2_pass<true, 3, 6, 9, 0>(tm, staged_ctx(c, sch, tws, 2), s, 384, sch, 2, false);  // factor 8: distances 64, 128, 256
     }
     tm.sync();
-    tail64<MODE>(tm, c, s, 3072, sch, 5, reduce_output, g, mulp, me, make_mont<CTX, MODE>(mn, mi));  // factor 64
+    tail64<MODE>(tm, staged_ctx(c, sch, tws + 7, 5), s, 3072, sch, 5, reduce_output, g, mulp, me,
+                 make_mont<CTX, MODE>(mn, mi));  // factor 64
 }
 
 /// One of the three 4096-residue blocks of a [3, 64, 64] line, computed by one CTA of a 3-CTA
@@ -455,7 +512,7 @@ __device__ __forceinline__ void line3072(const TEAM& tm, const SCH& sch, const C
 /// line is transformed in place, so no CTA may store before all three have read their inputs:
 /// `cluster_sync` (a cluster-wide barrier) separates the first pass from the stores.
 template <int MODE, class SCH, class CTX, class SYNC>
-__device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, int64_t* s, int64_t* g, int blk,
+__device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, int64_t* s, const int4* tws, int64_t* g, int blk,
                                                 const int64_t* mulp, int64_t me, int64_t mn, int64_t mi,
                                                 SYNC cluster_sync) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
@@ -514,24 +571,26 @@ __device__ __forceinline__ void line12288_block(const SCH& sch, const CTX& c, in
             if (!inv) fwd_group<3, true>(c, f + 1, fz + 1, 0, x);
             else inv_group<3, false>(c, f + 1, gg >> 6, x);
 #pragma unroll
-            for (int m = 0; m < 8; m++) s[pad8(base + span * m)] = x[m];
+            for (int m = 0; m < 8; m++) el(s, sw(base), span * m) = x[m];
         }
     }
     cluster_sync();  // also a barrier of this CTA
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 3>(CtaTeam{}, c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
+        r2_pass<false, 3, 6, 9, 3>(CtaTeam{}, staged_ctx(c, sch, tws, 1), s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
     } else {
-        r2_pass<true, 3, 9, 12, 0>(CtaTeam{}, c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
+        r2_pass<true, 3, 9, 12, 0>(CtaTeam{}, staged_ctx(c, sch, tws, 1), s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
     }
     __syncthreads();
-    tail64<MODE>(CtaTeam{}, c, s, 4096, sch, 7, reduce_output, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me,
+    tail64<MODE>(CtaTeam{}, staged_ctx(c, sch, tws + 63, 7), s, 4096, sch, 7, reduce_output, g + 4096 * blk, block_multiplier<MODE>(mulp, me, blk), me,
                  make_mont<CTX, MODE>(mn, mi));  // factor 64 (b)
 }
 
 /// Stages 1..12 of one 4096-residue block of a [3, 64, 64] line (the two factors 64, which act within the
-/// block): g -> g via the padded tile s; mulp: the block's multipliers.
+/// block): g -> g via the tile s; tws: the staged twiddles of both (complete at the first barrier here);
+/// mulp: the block's multipliers.
 template <int MODE, class SCH, class CTX, class MONT, class TEAM>
-__device__ __forceinline__ void block4096(const TEAM& tm, const SCH& sch, const CTX& c, int64_t* s, int64_t* g, const int64_t* mulp,
+__device__ __forceinline__ void block4096(const TEAM& tm, const SCH& sch, const CTX& c, int64_t* s, const int4* tws,
+                                          int64_t* g, const int64_t* mulp,
                                           int64_t me, const MONT& mont) {
     constexpr bool inv = MODE & 1, reduce_output = MODE == 0;
     {
@@ -552,17 +611,17 @@ __device__ __forceinline__ void block4096(const TEAM& tm, const SCH& sch, const 
             if (!inv) fwd_group<3, true>(c, f, fz, 0, x);
             else inv_group<3, false>(c, f, gg >> 6, x);
 #pragma unroll
-            for (int m = 0; m < 8; m++) s[pad8(base + span * m)] = x[m];
+            for (int m = 0; m < 8; m++) el(s, sw(base), span * m) = x[m];
         }
     }
     tm.sync();
     if (!inv) {
-        r2_pass<false, 3, 6, 9, 3>(tm, c, s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
+        r2_pass<false, 3, 6, 9, 3>(tm, staged_ctx(c, sch, tws, 1), s, 512, sch, 4, reduce_output);  // factor 64 (a): 256, 128, 64
     } else {
-        r2_pass<true, 3, 9, 12, 0>(tm, c, s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
+        r2_pass<true, 3, 9, 12, 0>(tm, staged_ctx(c, sch, tws, 1), s, 512, sch, 4, false);  // factor 64 (a): 512, 1024, 2048
     }
     tm.sync();
-    tail64<MODE>(tm, c, s, 4096, sch, 7, reduce_output, g, mulp, me, mont);  // factor 64 (b)
+    tail64<MODE>(tm, staged_ctx(c, sch, tws + 63, 7), s, 4096, sch, 7, reduce_output, g, mulp, me, mont);  // factor 64 (b)
 }
 
 // ---------------------------------------------------------------- columns
@@ -582,7 +641,7 @@ __device__ __forceinline__ void col12(const CTX& c, const SF* f, bool inv, bool 
 #pragma unroll
         for (int a = 0; a < 2; a++)
 #pragma unroll
-            for (int b = 0; b < 3; b++) fwd2<true>(c, f[0], z0, 0, x[a][b], x[a + 2][b]);
+            for (int b = 0; b < 3; b++) fwd2<true>(c, f[0], z0, 0, 0, x[a][b], x[a + 2][b]);
         if (f[1].red)
 #pragma unroll
             for (int a = 0; a < 4; a++)
@@ -590,7 +649,7 @@ __device__ __forceinline__ void col12(const CTX& c, const SF* f, bool inv, bool 
                 for (int b = 0; b < 3; b++) x[a][b] = red1(c, x[a][b]);
 #pragma unroll
         for (int b = 0; b < 3; b++) {
-            fwd2<true>(c, f[1], z1, 0, x[0][b], x[1][b]);
+            fwd2<true>(c, f[1], z1, 0, 0, x[0][b], x[1][b]);
             // block 1: an ordinary twiddle (not 1), product always taken
             const int64_t t = c.mul(c.get(f[1].tw_off + 1), x[3][b]);
             int64_t o0 = wadd(x[2][b], t), o1 = wsub(x[2][b], t);
@@ -668,12 +727,12 @@ __device__ __forceinline__ void col4(const CTX& c, const SF* f, bool inv, bool r
 #pragma unroll
             for (int a = 0; a < 4; a++) x[a] = red1(c, x[a]);
         const bool z0 = f[0].last && reduce_output, z1 = f[1].last && reduce_output;
-        fwd2<true>(c, f[0], z0, 0, x[0], x[2]);
-        fwd2<true>(c, f[0], z0, 0, x[1], x[3]);
+        fwd2<true>(c, f[0], z0, 0, 0, x[0], x[2]);
+        fwd2<true>(c, f[0], z0, 0, 0, x[1], x[3]);
         if (f[1].red)
 #pragma unroll
             for (int a = 0; a < 4; a++) x[a] = red1(c, x[a]);
-        fwd2<true>(c, f[1], z1, 0, x[0], x[1]);
+        fwd2<true>(c, f[1], z1, 0, 0, x[0], x[1]);
         const int64_t t = c.mul(c.get(f[1].tw_off + 1), x[3]);
         int64_t o0 = wadd(x[2], t), o1 = wsub(x[2], t);
         if (z1) {

@@ -25,17 +25,18 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(THREADS, 768 / THREA
         mn = mods.n[j], mi = mods.ninv[j];
     }
     auto csync = [] { cooperative_groups::this_cluster().sync(); };
-    // twiddles are read from the plan in global memory (L1-cached): the CTA's shared memory holds
-    // only its 4096-residue block, so that six CTAs fit on an SM
     const auto c = make_ctx<PassCtx<FIX>>(P);
-    with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, FIX>(
-        P, [&](const auto& sch) { fast::line12288_block<MODE>(sch, c, smem, g, blk, mulp, me, mn, mi, csync); });
+    int4* tws = reinterpret_cast<int4*>(smem + 4096);
+    with_sched<HC_SHAPE_L12288, (MODE & 1) != 0, FIX>(P, [&](const auto& sch) {
+        if constexpr (FIX) fast::stage_tail_twiddles<(MODE & 1) != 0>(fast::CtaTeam{}, c, sch, tws, 1, 63, 7);
+        fast::line12288_block<MODE>(sch, c, smem, tws, g, blk, mulp, me, mn, mi, csync);
+    });
 }
 
 template <int MODE, bool FIX, int THREADS>
 hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
-    // one 3-CTA cluster per line: a padded 4096-residue block per CTA
-    constexpr size_t smem = 4608 * 8;
+    // one 3-CTA cluster per line: a 4096-residue block per CTA
+    constexpr size_t smem = (size_t)BLOCK4096_WORDS * 8;
     auto kern = ntt_line3_kernel<MODE, FIX, THREADS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");

@@ -3,10 +3,6 @@
 
 namespace {
 
-#ifndef HC_L3072_MIN_BLOCKS
-#define HC_L3072_MIN_BLOCKS 8  // resident CTAs per SM the 3072-residue line kernel's registers must allow (8 fit its shared memory)
-#endif
-
 /// Specialised dimension-3 NTT: one line (i, j, k) per CTA.
 template <int MODE, bool FIX, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
@@ -28,7 +24,7 @@ __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPt
 
 template <int MODE, bool FIX, int THREADS, int MINB>
 hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
-    constexpr size_t smem = (size_t)line_tile_words(HC_SHAPE_L3072) * 8;
+    constexpr size_t smem = (size_t)LINE3072_WORDS * 8;
     auto kern = ntt_line_kernel<MODE, FIX, THREADS, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
@@ -36,14 +32,15 @@ hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KV
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
 }
-/// 128 threads per line, eight lines per SM: the fewest idle slots in the last wave, and 8 independent
-/// CTAs to cover each other's barriers. Up to two lines per SM (one element of 24 factors is 288
+/// 128 threads per line: the fewest idle slots in the last wave, and seven (forward, 72 registers: ntt_mul
+/// of [24, 20, 12, 3072] 124 us, with eight 130) or eight (inverse: intt 105 us, with seven 107) independent
+/// CTAs per SM to cover each other's barriers. Up to two lines per SM (one element of 24 factors is 288
 /// lines) a line's own latency is the launch's, and 384 threads shorten it: one element at r = 16 41.5
 /// -> 36.7 us per transform; at 384 lines the two are level.
 template <int MODE, bool FIX>
 hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
     if (tiles <= 2 * (int64_t)hc::num_sms(ctx)) return launch_as<MODE, FIX, 384, 2>(ctx, t, pp, mul, mods, tiles);
-    return launch_as<MODE, FIX, 128, HC_L3072_MIN_BLOCKS>(ctx, t, pp, mul, mods, tiles);
+    return launch_as<MODE, FIX, 128, (MODE & 1) ? 8 : 7>(ctx, t, pp, mul, mods, tiles);
 }
 
 template <bool FIX>

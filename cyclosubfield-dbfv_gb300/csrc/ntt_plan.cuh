@@ -88,10 +88,11 @@ namespace {
 #define HC_SHAPE_C12 3     // dimension-2 column [4, 3]
 #define HC_SHAPE_C4 4      // dimension-2 column [4]
 
-__host__ __device__ constexpr int line_len(int shape) { return shape == HC_SHAPE_L3072 ? 3072 : 12288; }
 #define HC_COL_THREADS 256  // of the column kernel
 
-__host__ __device__ constexpr int line_tile_words(int shape) { return line_len(shape) + line_len(shape) / 8; }
+/// Shared-memory words of a 3072-residue line, and of a 4096-residue block of a 12288-residue one: the
+/// tile, then its staged twiddles.
+constexpr int LINE3072_WORDS = 3072 + fast::staged_words(7), BLOCK4096_WORDS = 4096 + fast::staged_words(63);
 
 /// Contexts of a plan: its twiddles are read from global memory (L1-cached).
 template <class CTX>

@@ -17,14 +17,19 @@ __device__ __forceinline__ const int64_t* multiplier(const KView& mul, int64_t i
     else return kat<int64_t>(mul, i, j, k, l);
 }
 
-/// One [2, 3, 8, 64] line g of plan P through the CTA's shared-memory line buffer s; FIX: the plan is
-/// fixed.
+/// One [2, 3, 8, 64] line g of plan P through the team's shared-memory buffer s (LINE3072_WORDS); FIX: the
+/// plan is fixed; stage: its twiddles are not there yet (from the same plan and direction).
 template <int MODE, bool FIX, class TEAM>
 __device__ __forceinline__ void run_line3072(const TEAM& tm, const DevPlanHeader* P, int64_t* s, int64_t* g, const int64_t* mulp,
-                                             int64_t me, int64_t mn, int64_t mi) {
+                                             int64_t me, int64_t mn, int64_t mi, bool stage = true) {
     const auto c = make_ctx<PassCtx<FIX>>(P);
-    with_sched<HC_SHAPE_L3072, (MODE & 1) != 0, FIX>(
-        P, [&](const auto& sch) { fast::line3072<MODE>(tm, sch, c, s, g, mulp, me, mn, mi); });
+    int4* tws = reinterpret_cast<int4*>(s + 3072);
+    with_sched<HC_SHAPE_L3072, (MODE & 1) != 0, FIX>(P, [&](const auto& sch) {
+        if constexpr (FIX) {
+            if (stage) fast::stage_tail_twiddles<(MODE & 1) != 0>(tm, c, sch, tws, 2, 7, 5);
+        }
+        fast::line3072<MODE>(tm, sch, c, s, tws, g, mulp, me, mn, mi);
+    });
 }
 
 /// One specialised column g[0], g[ge], ... of shape SHAPE transformed in registers; it is read

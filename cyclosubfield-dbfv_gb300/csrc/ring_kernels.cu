@@ -610,6 +610,109 @@ __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs
     }
 }
 
+/// giant_kernel where output digits 0 .. NOUT - 1 start at digit 0 and every baby step's coefficient has at
+/// least NOUT digits (any dense transform): input digit i < NOUT then feeds the outputs o >= i with
+/// coefficient digit o - i, so a baby step is straight-line code over its NOUT rows and NOUT
+/// coefficient digits. A thread takes two adjacent positions (16-byte copies and stores) of one of the
+/// two rows; half of the CTA's threads take each row. n0: input digits used (min(d, NOUT)).
+/// What bounds it: memory and the multiply pipe about equally (a step reads every baby row once); the
+/// unit list, masks and single-word copies of giant_kernel kept it issue-bound: 237 us per giant step of
+/// 13 baby steps and three digits at field_49152 r = 23, here @@ us.
+constexpr int TRI_STAGES = 3;
+
+template <int NOUT>
+__global__ void __launch_bounds__(256, NOUT == 4 ? 2 : 3)
+    giant_tri_kernel(GiantArgs a, KMods m, const int64_t* one, int n0, int64_t lines, int chunks) {
+    extern __shared__ __align__(16) int64_t gsm[];  // [TRI_STAGES][NOUT][256] position pairs, then the lcoef limb pairs
+    longlong2* sx = reinterpret_cast<longlong2*>(gsm);
+    int2* slc = reinterpret_cast<int2*>(sx + TRI_STAGES * NOUT * 256);
+    const int64_t tiles = lines * chunks;
+    const int nt = (int)a.lcoef.n0, tid = threadIdx.x;
+    const int row = tid >> 7, lane = tid & 127;  // the ciphertext component, the pair of positions
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t line = tile / chunks;  // (j, k)
+        const int64_t l = (tile - line * chunks) * 256 + 2 * lane;
+        const int64_t k = line % a.dst.n2, j = line / a.dst.n2;
+        __syncthreads();  // the previous tile's readers of slc are done
+        for (int t = tid; t < nt; t += 256) slc[t] = limb_split(*kat<int64_t>(a.lcoef, t, j, k, 0));
+        __syncthreads();
+        if (l >= a.dst.n3) continue;
+        const int64_t rs = a.babies.s0;
+        const int64_t* next = kat<int64_t>(a.babies, row, j, k, l);  // baby step q's rows of this thread, in turn
+        auto issue = [&](int q, int slot) {
+            if (q < a.nbaby) {
+#pragma unroll
+                for (int i = 0; i < NOUT; i++)
+                    if (i < n0) cp_async16(sx + (slot * NOUT + i) * 256 + tid, next + 2 * i * rs);
+                next += 2 * a.d * rs;
+            }
+            cp_async_commit();  // an empty group past the end keeps the count uniform
+        };
+#pragma unroll
+        for (int q = 0; q < TRI_STAGES - 1; q++) issue(q, q);
+        LimbSum s[NOUT][2];
+        uint64_t lo[NOUT][2];
+        int64_t hi[NOUT][2];
+#pragma unroll
+        for (int o = 0; o < NOUT; o++)
+#pragma unroll
+            for (int p = 0; p < 2; p++) s[o][p].zero(), lo[o][p] = 0, hi[o][p] = 0;
+        auto fold = [&] {
+#pragma unroll
+            for (int o = 0; o < NOUT; o++)
+#pragma unroll
+                for (int p = 0; p < 2; p++) s[o][p].fold(lo[o][p], hi[o][p]), s[o][p].zero();
+        };
+        constexpr int FOLD = (LIMB_TERMS2 - 1) / NOUT;  // baby steps whose terms the sums hold
+        int until = FOLD, slot = 0;
+        for (int q = 0; q < a.nbaby; q++) {
+            issue(q + TRI_STAGES - 1, slot == 0 ? TRI_STAGES - 1 : slot - 1);
+            cp_async_wait<TRI_STAGES - 1>();  // baby step q's rows have landed
+            const int2* fc = slc + a.lfirst[q];
+            int2 f[NOUT];
+#pragma unroll
+            for (int o = 0; o < NOUT; o++) f[o] = fc[o];
+#pragma unroll
+            for (int i = 0; i < NOUT; i++) {
+                if (i < n0) {
+                    const longlong2 v = sx[(slot * NOUT + i) * 256 + tid];
+                    const int2 x0 = limb_split(v.x), x1 = limb_split(v.y);
+                    const int xs0 = x0.x + x0.y, xs1 = x1.x + x1.y;
+#pragma unroll
+                    for (int o = i; o < NOUT; o++) {
+                        const int2 w = f[o - i];
+                        s[o][0].mac(x0, xs0, w, w.x + w.y);
+                        s[o][1].mac(x1, xs1, w, w.x + w.y);
+                    }
+                }
+            }
+            if (--until == 0) fold(), until = FOLD;
+            slot = slot == TRI_STAGES - 1 ? 0 : slot + 1;
+        }
+        cp_async_wait<0>();
+        const int2 w = limb_split(one[j]);
+#pragma unroll
+        for (int o = 0; o < NOUT; o++) {
+            if (o < a.nadd) {
+                const longlong2 v = *reinterpret_cast<const longlong2*>(kat<int64_t>(a.add, 2 * o + row, j, k, l));
+                const int2 x0 = limb_split(v.x), x1 = limb_split(v.y);
+                s[o][0].mac(x0, x0.x + x0.y, w, w.x + w.y);
+                s[o][1].mac(x1, x1.x + x1.y, w, w.x + w.y);
+            }
+        }
+        fold();
+        const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
+        const int64_t r2 = m.r2[j];
+#pragma unroll
+        for (int o = 0; o < NOUT; o++) {
+            const bool full = (a.full >> o) & 1;
+            longlong2 r;
+            r.x = finish_wide(lo[o][0], hi[o][0], full, ml, r2), r.y = finish_wide(lo[o][1], hi[o][1], full, ml, r2);
+            *reinterpret_cast<longlong2*>(kat<int64_t>(a.dst, 2 * o + row, j, k, l)) = r;
+        }
+    }
+}
+
 void grid_lines(hc_context ctx, int64_t n3, int64_t lines, int* chunks, unsigned* blocks) {
     *chunks = (int)((n3 + 255) / 256);
     int64_t tiles = lines * *chunks;
@@ -743,6 +846,24 @@ hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, 
     const size_t smem = (size_t)(GIANT_STAGES * 2 * 256 + std::max<int64_t>(lcoef.n0, 1)) * 8;
     if (smem > 49152) return fail(HC_ERR_UNSUPPORTED, "too many coefficient digits");
     if (d >= 64) return fail(HC_ERR_UNSUPPORTED, "too many dBFV digits");
+    // 16-byte accesses of every row, and coefficients with a digit for each output
+    auto pairs = [](const KView& v) {
+        return ((uintptr_t)v.p % 16) == 0 && v.s0 % 2 == 0 && v.s1 % 2 == 0 && v.s2 % 2 == 0 && !v.b3;
+    };
+    bool tri = used <= GIANT_OUT && dst.n3 % 2 == 0 && pairs(babies) && pairs(dst) && (!add || pairs(*add));
+    for (int bj = 0; bj < nbaby; bj++) tri = tri && lcount[bj] >= used;
+    const size_t tri_smem = (size_t)TRI_STAGES * used * 256 * 16 + (size_t)std::max<int64_t>(lcoef.n0, 1) * 8;
+    if (tri && tri_smem <= max_smem_optin(ctx)) {
+        a.out0 = 0, a.nout = used;
+        a.full = 0;
+        for (int o = 0; o < used; o++) a.full |= (unsigned)(full[o] != 0) << o;
+        auto kern = used == 1 ? giant_tri_kernel<1> : used == 2 ? giant_tri_kernel<2> : used == 3 ? giant_tri_kernel<3> : giant_tri_kernel<4>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem);
+        if (e != cudaSuccess) return cuda_check(e, "giant-step smem attribute");
+        kern<<<blocks, 256, tri_smem, stream_of(ctx)>>>(a, m, one_dev, std::min(d, used), lines, chunks);
+        count_launch(ctx);
+        return cuda_check(cudaGetLastError(), "giant-step kernel launch");
+    }
     for (int o0 = 0; o0 < used; o0 += GIANT_OUT) {
         a.out0 = o0;
         a.nout = std::min(GIANT_OUT, used - o0);
