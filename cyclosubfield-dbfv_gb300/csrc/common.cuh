@@ -57,6 +57,19 @@ struct BconvConsts {
     int chunk;             // acc_before_reduce of the reference
 };
 
+/// One digit of the dBFV reduction (launch_dbfv_split): its constants, in device memory.
+struct DbfvSplit {
+    const int64_t* rqinv;    // [r] Montgomery factors of the lifts
+    const int64_t* mat;      // [limbs + 1][r]: the sums' matrix, the correction row last
+    const int64_t* nbd[2];   // [r] mont^2(-b Delta 2^(64 k)) of overflow limb k
+    const int64_t* delta[2]; // [r] mont^2(Delta 2^(64 k)) of carry limb k
+    const int64_t* one;      // [r] mont(1)
+    i128 f0, f1;             // Q and -Q^-1 modulo 2^log2m
+    int limbs, shift, log2m;
+    int corr_limb;           // the correction row's products with 29-bit limbs stay in range
+    int have_carry, full_in, full_out;  // a carry comes in; the two sums need the double reduction
+};
+
 /// Montgomery moduli of one call, by value in the kernel's parameter space.
 struct KMods {
     int64_t n[HC_MAX_MODS];

@@ -26,6 +26,7 @@
 namespace hc {
 hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst, const BconvConsts& c, int r, int rd,
                              int nb, const KMods& sm, const KMods& dm, int64_t ns, const BarrettLimbs* sub_mul);
+hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& carry, const DbfvSplit& d, const KMods& m);
 hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const uint32_t* p2, const uint32_t* p3);
 hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys, int nterms, const KView* add0,
                            const KView* add1, int full0, int full1, const KView& dst, const KMods& m,
@@ -2699,6 +2700,7 @@ struct SplitData {
     size_t log2_r = 0, log2_gamma = 0;
     i128 q_mod_r = 0, neg_q_inv_mod_r = 0;
     Tensor rqinv, matrix;
+    bool corr_limb = false;  // the correction row sums in 29-bit limbs (lifts below 2^57)
     std::vector<Tensor> neg_b_delta_mont2;
     size_t limbs() const { return log2_r <= 62 ? 1 : 2; }
     SplitData(hc_ring R, size_t log2_b, size_t log2_t, const Base& b) {
@@ -2726,6 +2728,9 @@ struct SplitData {
             const i128 p = R->prime(i);
             mat.push_back((int64_t)((gamma + p / 2) / p));
         }
+        int64_t maxmq = 0;
+        for (size_t u = 0; u < b.size(); u++) maxmq = std::max(maxmq, std::abs(mat[L * b.size() + u]));
+        corr_limb = maxmq < ((int64_t)1 << 30) && (i128)maxmq * ((i128)1 << 29) * (i128)b.size() < ((i128)1 << 63);
         matrix = Tensor(R->ctx, 1, (int64_t)L + 1, (int64_t)b.size(), 1);
         CK(hc_import(R->ctx, matrix.view(), mat.data(), mat.size()));
         q_mod_r = (i128)(q_mod_2_128(R, b) & rmask);
@@ -2748,31 +2753,6 @@ struct SplitData {
             }));
     }
 };
-
-/// src/dbfv.rs:891-950: x <- x_lo in place; returns the overflow limbs [count, limbs, ...]
-Tensor split_overflow(hc_ring R, const SplitData& D, const hc_view& x, u128 x_bound, const Base& b) {
-    const int64_t count = x.shape[0], r = (int64_t)b.size(), L = (int64_t)D.limbs();
-    std::vector<hc_modulus> m = R->mods(b);
-    Tensor lifts(R->ctx, count, r, R->dl(), R->dk(), false, false);
-    CK(hc_assign(R->ctx, lifts.view(), x));
-    CK(hc_mul_mont64(R->ctx, lifts.view(), D.rqinv.view(), m.data(), m.size()));
-    Tensor sums(R->ctx, count, L + 1, R->dl(), R->dk(), true, false);
-    CK(hc_matmul_i64(R->ctx, sums.view(), D.matrix.view(), lifts.view()));
-    Tensor overflow(R->ctx, count, L, R->dl(), R->dk(), false, false);
-    if (L == 1) {
-        CK(hc_bconv_correct_pow2(R->ctx, overflow.view(), sums.view(), (int64_t)D.q_mod_r, (int64_t)D.neg_q_inv_mod_r,
-                                 D.log2_gamma, D.log2_r));
-    } else {
-        const int64_t f0[2] = {(int64_t)(uint64_t)D.q_mod_r, (int64_t)(D.q_mod_r >> 64)};
-        const int64_t f1[2] = {(int64_t)(uint64_t)D.neg_q_inv_mod_r, (int64_t)(D.neg_q_inv_mod_r >> 64)};
-        CK(hc_bconv_correct_pow2_wide(R->ctx, overflow.view(), sums.view(), f0, f1, D.log2_gamma, D.log2_r));
-    }
-    Wide acc(R, count, b);
-    for (int64_t k = 0; k < L; k++) acc.fma_unbounded(0, (size_t)count, dim1(overflow.view(), k, k + 1), D.neg_b_delta_mont2[(size_t)k].view());
-    acc.add(0, (size_t)count, x, x_bound);
-    acc.reduce_into(x);
-    return overflow;
-}
 
 /// The reduction's tables of one (log2 b, log2 t, base): SplitOverflowData and the carries'
 /// delta factors, built once per ring (their uploads would otherwise block the host every call).
@@ -2812,20 +2792,32 @@ Tensor dbfv_reduce(hc_ring R, size_t log2_b, size_t log2_t, const hc_view& ct, u
     const std::vector<Tensor>& delta_mont2 = T.delta_mont2;
     Tensor result(R->ctx, 2 * (int64_t)digits, rr, R->dl(), R->dk());
     CK(hc_assign(R->ctx, vrows(result.view(), 0, 2 * (int64_t)d), ct));
-    Tensor carry;
-    bool have = false;
+    // one launch per digit: the incoming carry, the overflow and the digit's remainder
+    const int64_t L = (int64_t)D.limbs();
+    Tensor carry(R->ctx, 2, L, R->dl(), R->dk(), false, false);
+    const int64_t maxp = R->max_p(b), minp = R->min_p(b);
+    auto words = [](const Tensor& t) { return (const int64_t*)t.view().ptr; };
+    DbfvSplit S{};
+    S.rqinv = words(D.rqinv), S.mat = words(D.matrix), S.one = words(R->scalar_tensor(b, 1));
+    for (int64_t k = 0; k < L; k++) S.nbd[k] = words(D.neg_b_delta_mont2[(size_t)k]), S.delta[k] = words(delta_mont2[(size_t)k]);
+    S.f0 = D.q_mod_r, S.f1 = D.neg_q_inv_mod_r;
+    S.limbs = (int)L, S.shift = (int)D.log2_gamma, S.log2m = (int)D.log2_r;
+    S.corr_limb = D.corr_limb;
+    const KMods km = R->kmods(b);
     for (size_t i = 0; i < digits; i++) {
+        // the wide accumulators' bounds: limbs any 64-bit words, the rows their bound (Wide)
+        auto full = [&](u128 row_bound) {
+            u128 bound = 0;
+            for (int64_t k = 0; k < L; k++) bound += (u128)maxp << 63;
+            const u128 nb = bound + row_bound * ((u128)maxp * (u128)maxp);
+            REQUIRE(nb >= bound && nb <= (u128)I128MAX, HC_ERR_ARG, "wide ring element overflow");
+            return nb > ((u128)minp << 63);
+        };
+        S.have_carry = i > 0;
         const u128 in_bound = i < d ? bound : 1;
-        hc_view rows = vrows(result.view(), 2 * (int64_t)i, 2 * (int64_t)i + 2);
-        if (have) {
-            Wide acc(R, 2, b);
-            for (size_t k = 0; k < delta_mont2.size(); k++)
-                acc.fma_unbounded(0, 2, dim1(carry.view(), (int64_t)k, (int64_t)k + 1), delta_mont2[k].view());
-            acc.add(0, 2, rows, in_bound);
-            acc.reduce_into(rows);
-        }
-        carry = split_overflow(R, D, rows, have ? 1 : in_bound, b);
-        have = true;
+        S.full_in = S.have_carry && full(in_bound);
+        S.full_out = full(S.have_carry ? 1 : in_bound);
+        CK(launch_dbfv_split(R->ctx, kv(vrows(result.view(), 2 * (int64_t)i, 2 * (int64_t)i + 2)), kv(carry.view()), S, km));
     }
     *rows_out = 2 * digits;
     return result;

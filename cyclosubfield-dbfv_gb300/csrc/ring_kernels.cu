@@ -214,6 +214,83 @@ __global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs
     if (j < jend) bconv_outputs<ONE_CHUNK, SUB, 1>(a, dm, b, j, u0, u1, xcol, q, dstp);
 }
 
+/// A sum of at most HC_MAX_TERMS + 1 products of words within 2p: reduced once, or twice and back to
+/// Montgomery form.
+__device__ __forceinline__ int64_t finish_wide(uint64_t lo, int64_t hi, bool full, const MontLimbs& m, int64_t r2) {
+    return full ? mont_mul(mont_red_double(lo, hi, m), r2, m) : mont_red(lo, hi, m);
+}
+
+/// One digit of the dBFV reduction at one position per thread (dbfv_reduce, src/dbfv.rs:968-1032, with
+/// split_overflow, :891-950): rows x <- reduce(x mont(1) + sum_k carry_k Delta_k) when a carry comes in,
+/// then the overflow of x modulo Q as limbs (lifts, the matrix sums, the power-of-two correction of
+/// src/hal/cpu.rs:983-1057), then x <- reduce(x mont(1) + sum_k overflow_k (-b Delta)_k). The position's
+/// words stay in shared memory between the three, and the overflow replaces the carry.
+/// What bounds it: the multiply pipe, about 100 wide products per word. As the calls of the tensor HAL a digit took
+/// 10 to 17 launches and wrote its lifts, 128-bit sums and accumulators to memory: a product of two
+/// three-digit ciphertexts at field_49152 r = 16 took 2617 us and takes 2117 (26 to 37 us per digit here).
+/// x [c, r, dl, dk] and carry [c, limbs, dl, dk] in place; CTAs over (128 positions, row).
+__global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KView carry, DbfvSplit d, int r, KMods m,
+                                                                   int64_t npos) {
+    extern __shared__ int64_t sx[];  // [r][BCONV_THREADS]
+    const int64_t pos = (int64_t)blockIdx.x * BCONV_THREADS + threadIdx.x;
+    if (pos >= npos) return;
+    const int64_t i = blockIdx.y, k = pos / x.n3, l = pos - k * x.n3;
+    int64_t* xp = kat<int64_t>(x, i, 0, k, l);
+    int64_t* cp = kat<int64_t>(carry, i, 0, k, l);
+    auto fma = [](i128 acc, int64_t a, int64_t b) { return (i128)((u128)acc + (u128)((i128)a * (i128)b)); };
+    auto finish = [&](i128 acc, int j, bool full) {
+        return finish_wide((uint64_t)acc, (int64_t)(acc >> 64), full, mont_limbs(m.n[j], m.ninv[j]), m.r2[j]);
+    };
+    int64_t c[2] = {0, 0};
+    if (d.have_carry)
+        for (int q = 0; q < d.limbs; q++) c[q] = cp[q * carry.s1];
+    // the sums modulo 2^128; one limb only needs them modulo 2^64 (log2m <= 62)
+    i128 v = 0, corr = 0;
+    uint64_t v64 = 0;
+    int64_t c0 = 0, c1 = 0;
+    const int64_t* mq = d.mat + d.limbs * r;
+    for (int u = 0; u < r; u++) {
+        int64_t w = xp[u * x.s1];
+        if (d.have_carry) {
+            i128 acc = (i128)w * (i128)__ldg(d.one + u);
+            for (int q = 0; q < d.limbs; q++) acc = fma(acc, c[q], __ldg(d.delta[q] + u));
+            w = finish(acc, u, d.full_in);
+        }
+        sx[u * BCONV_THREADS + threadIdx.x] = w;
+        const int64_t lift = mul_mont(w, __ldg(d.rqinv + u), m.n[u], m.ninv[u]);  // w: any word the bound allows
+        if (d.limbs == 1) v64 += (uint64_t)__ldg(d.mat + u) * (uint64_t)lift;
+        else v = (i128)((u128)fma(v, __ldg(d.mat + u), lift) + ((u128)((uint64_t)__ldg(d.mat + r + u) * (uint64_t)lift) << 64));
+        if (d.corr_limb) {
+            const int2 y = limb_split(lift);
+            const int g = (int)__ldg(mq + u);
+            c0 = mad_wide(y.x, g, c0);
+            c1 = mad_wide(y.y, g, c1);
+        } else {
+            corr = fma(corr, __ldg(mq + u), lift);
+        }
+    }
+    if (d.corr_limb) corr = (i128)c0 + (i128)((u128)(i128)c1 << LIMB_BITS);
+    const i128 quot = (i128)((u128)corr + ((u128)1 << (d.shift - 1))) >> d.shift;
+    int64_t o[2] = {0, 0};
+    if (d.limbs == 1) {
+        const uint64_t y = (v64 - (uint64_t)quot * (uint64_t)d.f0) * (uint64_t)d.f1;
+        const int64_t mod = (int64_t)1 << d.log2m, red = (int64_t)(y & (uint64_t)(mod - 1));
+        o[0] = red > mod / 2 ? red - mod : red;
+    } else {
+        const u128 y = ((u128)v - (u128)quot * (u128)d.f0) * (u128)d.f1;
+        const i128 mod = (i128)1 << d.log2m, red = (i128)(y & ((u128)mod - 1));
+        const i128 e = red > mod / 2 ? red - mod : red;
+        o[0] = (int64_t)(uint64_t)e;
+        o[1] = (int64_t)((e - (i128)o[0]) >> 64);
+    }
+    for (int q = 0; q < d.limbs; q++) cp[q * carry.s1] = o[q];
+    for (int u = 0; u < r; u++) {
+        i128 acc = (i128)sx[u * BCONV_THREADS + threadIdx.x] * (i128)__ldg(d.one + u);
+        for (int q = 0; q < d.limbs; q++) acc = fma(acc, o[q], __ldg(d.nbd[q] + u));
+        xp[u * x.s1] = finish(acc, u, d.full_out);
+    }
+}
+
 /// dst[i,j,k,l] = src[i,j,p2[k],p3[l]]
 __global__ void __launch_bounds__(256) galois_kernel(KView d, KView s, const uint32_t* p2, const uint32_t* p3,
                                                      int64_t lines, int chunks) {
@@ -261,12 +338,6 @@ struct KsArgs {
     // on the tiles that launch read last, which are still in L2
     int reverse;
 };
-
-/// A sum of at most HC_MAX_TERMS + 1 products of words within 2p: reduced once, or twice and back to
-/// Montgomery form.
-__device__ __forceinline__ int64_t finish_wide(uint64_t lo, int64_t hi, bool full, const MontLimbs& m, int64_t r2) {
-    return full ? mont_mul(mont_red_double(lo, hi, m), r2, m) : mont_red(lo, hi, m);
-}
 
 /// R accumulators of one position: one digit word times R key words per step.
 template <int R>
@@ -617,7 +688,7 @@ __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs
 /// two rows; half of the CTA's threads take each row. n0: input digits used (min(d, NOUT)).
 /// What bounds it: memory and the multiply pipe about equally (a step reads every baby row once); the
 /// unit list, masks and single-word copies of giant_kernel kept it issue-bound: 237 us per giant step of
-/// 13 baby steps and three digits at field_49152 r = 23, here @@ us.
+/// 13 baby steps and three digits at field_49152 r = 23, here 159 us.
 constexpr int TRI_STAGES = 3;
 
 template <int NOUT>
@@ -761,6 +832,22 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
     kern<<<grid, BCONV_THREADS, smem, stream_of(ctx)>>>(a, sm, dm);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "bconv kernel launch");
+}
+
+hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& carry, const DbfvSplit& d, const KMods& m) {
+    const int r = (int)x.n1;
+    const int64_t npos = x.n2 * x.n3;
+    if (npos == 0 || x.n0 == 0) return HC_OK;
+    const size_t smem = (size_t)r * BCONV_THREADS * 8;
+    if (smem > max_smem_optin(ctx) || x.n0 > 65535) return fail(HC_ERR_UNSUPPORTED, "dBFV reduction: too many rows");
+    if (smem > 49152) {
+        cudaError_t e = cudaFuncSetAttribute(dbfv_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_check(e, "dBFV reduction smem attribute");
+    }
+    dim3 grid((unsigned)((npos + BCONV_THREADS - 1) / BCONV_THREADS), (unsigned)x.n0);
+    dbfv_split_kernel<<<grid, BCONV_THREADS, smem, stream_of(ctx)>>>(x, carry, d, r, m, npos);
+    count_launch(ctx);
+    return cuda_check(cudaGetLastError(), "dBFV reduction launch");
 }
 
 hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const uint32_t* p2, const uint32_t* p3) {

@@ -1,0 +1,171 @@
+"""The fused kernels and size rules of the ring layer and the transforms, bit-exact against the oracle at the sizes
+where they could go wrong: the dBFV reduction's one launch per digit, key switches around the gadget-digit counts at
+which the limb sums fold, giant steps of every output count with dense and missing coefficient digits, the one-launch
+transforms of small rings, and transforms on both sides of the line counts at which the CTA's size changes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+WORD = (1 << 63) - 1
+
+
+@pytest.fixture(scope="module")
+def rings(po, be):
+    import ringcuda
+
+    cache = {}
+
+    def get(*key):
+        if key not in cache:
+            cache[key] = (po.Ring(*key), ringcuda.RingContext(*key, backend=be))
+        return cache[key]
+
+    return get
+
+
+def residues(g, shape, primes, bound=1, edges=False):
+    """[count, r, ...] words within +-bound p; with edges, half of them at the bound, 0 and +-1."""
+    out = np.empty(shape, dtype=np.int64)
+    for j in range(shape[1]):
+        m = min(bound * primes[j], WORD)
+        out[:, j] = g.integers(-m, m, size=out[:, j].shape, endpoint=True)
+        if edges:
+            v = g.choice(np.array([m, -m, m - 1, 1 - m, 0, 1, -1]), size=out[:, j].shape)
+            out[:, j] = np.where(g.integers(0, 2, size=v.shape) == 1, v, out[:, j])
+    return out
+
+
+# one word of overflow (log2 t - log2 b <= 62) and two; fewer digits in than out; up to the whole word in use
+# (63 p for primes just below 2^57)
+@pytest.mark.parametrize("ring", [("field_192", 200, 220, 4), ("field_18", 520, 540, 32), ("field_18", 2300, 2340, 4),
+                                  ("field_2", 200, 220, 4)], ids=lambda v: "%s-%d" % v[:2])
+@pytest.mark.parametrize("log2_b,log2_t,digits", [(8, 70, 9), (7, 70, 4), (4, 68, 17), (16, 100, 7), (32, 126, 4), (1, 2, 1),
+                                                  (63, 126, 2), (64, 126, 1), (125, 126, 2)])
+@pytest.mark.parametrize("bound", [1, 2, 63])
+def test_dbfv_reduction(rings, ring, log2_b, log2_t, digits, bound):
+    import ringcuda
+
+    o, d = rings(*ring)
+    base = o.initial_base()
+    g = np.random.default_rng(log2_b * 1000 + log2_t + bound)
+    ct = residues(g, o.shape(2 * digits, len(base)), [o.primes[i] for i in base], bound, edges=True)
+    exp = o.dbfv_reduce(log2_b, log2_t, ct, base, bound=bound)
+    got = ringcuda.dbfv_reduce(d, log2_b, log2_t, d.tensor(ct), base, bound=bound).to_numpy()
+    assert got.shape == exp.shape and (got == exp).all()
+
+
+@pytest.mark.parametrize("nd", [1, 2, 13, 14, 15, 16, 27, 28, 29, 41])
+def test_key_switch_digit_counts(rings, nd):
+    """The sums of a key switch hold 15 gadget digits' products before they fold (csrc/common.cuh: LIMB_TERMS2)."""
+    import ringcuda
+
+    o, d = rings("field_192", 2300, 2340, 4)
+    base = o.initial_base()
+    assert len(base) == 41
+    digits = [tuple(v) for v in ringcuda.select_digits(nd, len(base))]
+    primes = [o.primes[i] for i in base]
+    g = np.random.default_rng(nd)
+    c0, c1 = (residues(g, o.shape(1, len(base)), primes, edges=True) for _ in range(2))
+    key = residues(g, o.shape(2 * nd, len(base)), primes, edges=True)
+    exp = o.key_switch(c0, c1, base, key.reshape((nd, 2) + key.shape[1:]), digits)
+    got = d.key_switch(d.tensor(c0), d.tensor(c1), base, d.tensor(key), digits)
+    assert (got.to_numpy() == exp).all()
+
+
+@pytest.mark.parametrize("ring,gen", [(("field_18", 300, 320, 4), 932), (("field_49152", 200, 230, 2), 20965738)],
+                         ids=["field_18", "field_49152"])
+@pytest.mark.parametrize("log2_b,log2_t,dct,length", [(4, 4, 1, 3), (4, 8, 2, 3), (4, 12, 2, 5), (4, 16, 4, 6), (3, 15, 2, 6)])
+@pytest.mark.parametrize("dense", [True, False])
+def test_giant_steps(po, rings, ring, gen, log2_b, log2_t, dct, length, dense):
+    """One to five output digits, as many and fewer input digits; dense: every coefficient has all its
+    digits, otherwise some are short and some zero."""
+    import ringcuda
+
+    o, d = rings(*ring)
+    base = o.initial_base()
+    m = o.info["m"]
+    digits = po.select_digits(min(3, len(base)), len(base))
+    baby = min(range(1, length + 1), key=lambda c: (c + 3 * ((length - 1) // c + 1), c))
+    g = np.random.default_rng(log2_t + length)
+    primes = [o.primes[i] for i in base]
+    gks = {}
+    for e in sorted(set(pow(gen, j, m) for j in list(range(1, baby)) + ([baby] if baby < length else []))):
+        gks[e] = residues(g, o.shape(2 * len(digits), len(base)), primes).reshape((len(digits), 2) + o.shape(1, len(base))[1:])
+    ks = ringcuda.Keyset(d, digits, o.initial_len, 1 << 40)
+    for e, k in gks.items():
+        full = np.zeros((2 * len(digits), o.initial_len) + o.shape(1, 1)[2:], dtype=np.int64)
+        full[:, : len(base)] = k.reshape((-1,) + k.shape[2:])
+        gks[e] = full.reshape((len(digits), 2) + full.shape[1:])
+        ks.add(e, d.tensor(full))
+    t = 1 << log2_t
+    if dense:
+        coeffs = [[int(v) for v in g.integers(t // 4, t, size=o.dl)] for _ in range(length)]
+    else:
+        coeffs = [[int(v) for v in g.integers(0, [t, 1, 2][j % 3], size=o.dl)] for j in range(length)]
+    ct = residues(g, o.shape(2 * dct, len(base)), primes, edges=True)
+    exp = o.dbfv_hom_cyclic_transform(log2_b, log2_t, gen, coeffs, ct, base, gks, digits)
+    got = ringcuda.dbfv_hom_cyclic_transform(d, log2_b, log2_t, gen, coeffs, d.tensor(ct), base, ks).to_numpy()
+    assert got.shape == exp.shape and (got == exp).all()
+
+
+@pytest.mark.parametrize("field", ["field_2", "field_18", "field_192"])
+@pytest.mark.parametrize("count,base", [(1, [0]), (5, [1, 0, 3]), (70, [0, 1, 2, 3])])
+def test_small_ring_transforms(be, rings, field, count, base):
+    """One launch per transform against the oracle, in place on views inside a larger tensor (rows and factors around
+    them untouched), operands within 2p."""
+    o, d = rings(field, 200, 220, 4)
+    r = len(base)
+    g = np.random.default_rng(count)
+    whole = residues(g, o.shape(count + 2, r + 2), [o.primes[base[0]]] * (r + 2), 1)
+    whole[1:-1, 1:-1] = residues(g, o.shape(count, r), [o.primes[i] for i in base], 2, edges=True)
+    for op in (d.pb_to_crt, d.crt_to_pb):
+        op(d.allocate(1, r), base)  # builds the tables of this base
+    for op in ("pb_to_crt", "crt_to_pb"):
+        exp = whole.copy()
+        exp[1:-1, 1:-1] = getattr(o, op)(np.ascontiguousarray(whole[1:-1, 1:-1]), base)
+        t = d.tensor(whole)
+        l0 = be.launch_count()
+        getattr(d, op)(t.rows(1, count + 1).base_range(1, r + 1), base)
+        assert be.launch_count() - l0 == 1
+        assert (t.to_numpy() == exp).all(), op
+
+
+# (inner shape, slab, dimension, elements per count): 300 | 312 lines of 3072 (384 or 128 threads on 152 SMs),
+# 152 | 156 of 12288 (256 or 128 threads)
+@pytest.mark.parametrize("inner,shape,dim,count", [([2, 3, 8, 64], (12, 3072), 3, 25), ([2, 3, 8, 64], (12, 3072), 3, 26),
+                                                   ([3, 64, 64], (4, 12288), 3, 38), ([3, 64, 64], (4, 12288), 3, 39)],
+                         ids=lambda v: str(v))
+def test_line_transforms_around_the_cta_rule(be, po, inner, shape, dim, count):
+    o = po.Ring("field_36864" if shape[0] == 12 else "field_49152", 200, 230, 2)
+    p = o.primes[0]
+    g = np.random.default_rng(count)
+    data = residues(g, (count, 1) + shape, [p], 2, edges=True)
+    m = be.hal_create_modulus(p)
+    plan = [be.hal_create_ntt_plan(m, inner)]
+    for mode in ("ntt", "intt"):
+        exp = data.copy()
+        po.ntt_dim(exp, [p], inner, dim, mode)
+        t = be.tensor(data)
+        getattr(be, "hal_%s_mont64_dim" % mode)(t, plan, dim)
+        assert (t.to_numpy() == exp).all(), mode
+
+
+@pytest.mark.parametrize("field,count", [("field_36864", 13), ("field_49152", 12), ("field_49152", 13)])
+def test_batched_and_single_transforms_agree(rings, field, count):
+    """More slabs than the batched kernels' resident teams, and field_49152's blocks around three per SM (38 slabs of
+    twelve blocks): the batched, the single and the oracle's transforms."""
+    import ringcuda
+
+    o, d = rings(field, 200, 230, 2)
+    base = o.initial_base()[:3]
+    primes = [o.primes[i] for i in base]
+    x = residues(np.random.default_rng(count), o.shape(count, len(base)), primes, 2, edges=True)
+    for name, flag in (("pb_to_crt", ringcuda.CRT_FORWARD), ("crt_to_pb", ringcuda.CRT_INVERSE)):
+        exp = getattr(o, name)(x, base)
+        t, u = d.tensor(x), d.tensor(x)
+        getattr(d, name)(t, base)
+        batch = ringcuda.CrtBatch([(d, u, None, base)], flag)
+        batch.run()
+        batch.close()
+        assert (t.to_numpy() == exp).all() and (u.to_numpy() == exp).all(), name
