@@ -62,7 +62,7 @@ hc_status launch_crt_batch(hc_context ctx, const CrtSlab* slabs, int nslabs, int
     if (grid > nslabs) grid = nslabs;
     hc_status st = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), stream_of(ctx)), "batched transform counter");
     if (st) return st;
-    kern<<<(unsigned)grid, (unsigned)L.threads, smem, stream_of(ctx)>>>(slabs, nslabs, counter, L.logv,
+    hc::launch_kernel(kern, (unsigned)grid, (unsigned)L.threads, smem, stream_of(ctx), slabs, nslabs, counter, L.logv,
                                                                       (int)tile_words);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "batched transform launch");

@@ -119,6 +119,7 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
 template <bool GENERIC, int CLS, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
     crt_batch_kernel(const CrtSlab* __restrict__ slabs, int nslabs, int* counter, int logv, int tile_words) {
+    grid_wait();
     extern __shared__ int64_t smem[];
     __shared__ int s_next;
     for (;;) {

@@ -34,6 +34,7 @@ constexpr size_t SMEM4096 = (size_t)BLOCK4096_WORDS * 8;
 template <int DIR>
 __global__ void __launch_bounds__(LEAD_THREADS, 4)
     lead12288_kernel(KView t, KView src, PlanPtrs p2, PlanPtrs p3, const BarrettLimbs* m2, KMods mods) {
+    grid_wait();
     // tiles last to first (as the column kernel's: what the last launch wrote last is still in L2)
     const int64_t tile = gridDim.x - 1 - blockIdx.x;
     const int64_t slab = tile / (4096 / LEAD_THREADS), j = slab % t.n1, i = slab / t.n1;
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(LEAD_THREADS, 4)
 template <int MODE, int THREADS>
 __global__ void __launch_bounds__(THREADS, 768 / THREADS)
     block4096_kernel(KView t, PlanPtrs p3, const BarrettLimbs* m3, KView pm, KMods mods) {
+    grid_wait();
     extern __shared__ int64_t smem[];
     const int64_t tile = blockIdx.x / 3;
     const int blk = (int)(blockIdx.x % 3);
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS)
 template <int MODE, int THREADS>
 hc_status launch_blocks_as(hc_context ctx, int64_t ctas, const KView& t, const PlanPtrs& p3, const BarrettLimbs* m3,
                            const KView& pm, const KMods& mods) {
-    block4096_kernel<MODE, THREADS><<<(unsigned)ctas, THREADS, SMEM4096, hc::stream_of(ctx)>>>(t, p3, m3, pm, mods);
+    hc::launch_kernel(block4096_kernel<MODE, THREADS>, (unsigned)ctas, THREADS, SMEM4096, hc::stream_of(ctx), t, p3, m3, pm, mods);
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "CRT block pass launch");
 }
@@ -131,8 +133,8 @@ hc_status launch_crt_pass(hc_context ctx, int dir, const KView& t, const KView* 
     const int64_t slabs = t.n0 * t.n1;
     if (slabs == 0) return HC_OK;
     const unsigned grid = (unsigned)(slabs * (4096 / LEAD_THREADS));
-    if (dir == 0) lead12288_kernel<0><<<grid, LEAD_THREADS, 0, stream_of(ctx)>>>(t, src ? *src : t, p2, p3, m2, mods);
-    else lead12288_kernel<1><<<grid, LEAD_THREADS, 0, stream_of(ctx)>>>(t, t, p2, p3, nullptr, mods);
+    if (dir == 0) hc::launch_kernel(lead12288_kernel<0>, grid, LEAD_THREADS, 0, stream_of(ctx), t, src ? *src : t, p2, p3, m2, mods);
+    else hc::launch_kernel(lead12288_kernel<1>, grid, LEAD_THREADS, 0, stream_of(ctx), t, t, p2, p3, nullptr, mods);
     count_launch(ctx);
     hc_status st = cuda_check(cudaGetLastError(), "CRT lead pass launch");
     if (st) return st;

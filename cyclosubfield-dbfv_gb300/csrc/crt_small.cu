@@ -61,6 +61,7 @@ __device__ __forceinline__ Program stage_program(const DevPlanHeader* P, const S
 static_assert(sizeof(DevStage) % 8 == 0 && sizeof(DevPass) % 8 == 0, "staged in 8-byte words");
 
 __global__ void __launch_bounds__(256) crt_small_kernel(SmallArgs a, KMods mods) {
+    grid_wait();
     extern __shared__ int64_t smem[];
     const int dl = (int)a.t.n2, dk = (int)a.t.n3, total = dl * dk;
     const int64_t j = blockIdx.x % a.t.n1, i = blockIdx.x / a.t.n1;
@@ -143,7 +144,7 @@ hc_status launch_crt_small(hc_context ctx, const KView& t, const KView* src, con
     a.div_dl = make_fastdiv((uint32_t)t.n2), a.div_dk = make_fastdiv((uint32_t)t.n3);
     // a butterfly or two per thread; at least two warps, for the staging
     const int threads = (int)std::min<int64_t>(256, std::max<int64_t>(64, (total / 4 + 31) / 32 * 32));
-    crt_small_kernel<<<(unsigned)slabs, threads, smem, stream_of(ctx)>>>(a, mods);
+    hc::launch_kernel(crt_small_kernel, (unsigned)slabs, threads, smem, stream_of(ctx), a, mods);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "small CRT transform launch");
 }

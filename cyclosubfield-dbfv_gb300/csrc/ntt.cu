@@ -95,6 +95,7 @@ namespace {
 /// element (e, v) at k = e, l = cb * V + v.
 __global__ void __launch_bounds__(256, HC_NTT_MIN_BLOCKS) ntt_tile_kernel(KView t, PlanPtrs plans, int dim, int mode, KView mul,
                                                        KMods mods, int logv, int ntile2, int use_smem) {
+    grid_wait();
     extern __shared__ int64_t smem[];
     const int V = 1 << logv;
     const int len = dim == 3 ? (int)t.n3 : (int)t.n2;
@@ -498,7 +499,7 @@ hc_status launch_ntt(hc_context ctx, const KView& t, const hc_ntt_plan* plans, s
     // about 24 elements (three groups of eight) per thread, 64..256 threads
     int64_t threads = ((len * V / 24) + 31) / 32 * 32;
     threads = threads < 64 ? 64 : (threads > 256 ? 256 : threads);
-    ntt_tile_kernel<<<(unsigned)tiles, (unsigned)threads, smem, stream_of(ctx)>>>(t, pp, dim, mode, mul, mods, logv,
+    hc::launch_kernel(ntt_tile_kernel, (unsigned)tiles, (unsigned)threads, smem, stream_of(ctx), t, pp, dim, mode, mul, mods, logv,
                                                                     (int)ntile2, use_smem);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "ntt kernel launch");

@@ -11,6 +11,7 @@ namespace {
 template <int SHAPE, int MODE, bool FIX>
 __global__ void __launch_bounds__(HC_COL_THREADS, SHAPE == HC_SHAPE_C12 ? HC_COL12_MIN_BLOCKS : 4) ntt_col_kernel(KView t, PlanPtrs plans, KView mul, KMods mods,
                                                                     int ncb, KView src) {
+    grid_wait();
     // tiles last to first: a transform's column pass follows a line pass (or the input's producer)
     // that wrote the tensor first to last, so the CTAs scheduled first read what is still in L2,
     // and the next line pass, first to last, starts on what this pass wrote last
@@ -36,8 +37,7 @@ __global__ void __launch_bounds__(HC_COL_THREADS, SHAPE == HC_SHAPE_C12 ? HC_COL
 template <int SHAPE, int MODE, bool FIX>
 hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles, int ncb,
                       const KView& src) {
-    ntt_col_kernel<SHAPE, MODE, FIX>
-        <<<(unsigned)tiles, HC_COL_THREADS, 0, hc::stream_of(ctx)>>>(t, pp, mul, mods, ncb, src);
+    hc::launch_kernel(ntt_col_kernel<SHAPE, MODE, FIX>, (unsigned)tiles, HC_COL_THREADS, 0, hc::stream_of(ctx), t, pp, mul, mods, ncb, src);
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
 }

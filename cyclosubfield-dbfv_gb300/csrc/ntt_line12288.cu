@@ -10,6 +10,7 @@ namespace {
 template <int MODE, bool FIX, int THREADS>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(THREADS, 768 / THREADS)
     ntt_line3_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
+    grid_wait();
     extern __shared__ int64_t smem[];
     const int64_t tile = blockIdx.x / 3;
     const int blk = (int)(blockIdx.x % 3);
@@ -41,7 +42,7 @@ hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KV
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
     if (tiles * 3 > 0x7fffffff) return hc::fail(HC_ERR_UNSUPPORTED, "too many NTT lines in one call");
-    kern<<<(unsigned)(tiles * 3), THREADS, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
+    hc::launch_kernel(kern, (unsigned)(tiles * 3), THREADS, smem, hc::stream_of(ctx), t, pp, mul, mods);
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
 }

@@ -6,6 +6,7 @@ namespace {
 /// Specialised dimension-3 NTT: one line (i, j, k) per CTA.
 template <int MODE, bool FIX, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
+    grid_wait();
     extern __shared__ int64_t smem[];
     const int64_t tile = blockIdx.x;
     const int64_t k = tile % t.n2, r = tile / t.n2;
@@ -28,7 +29,7 @@ hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KV
     auto kern = ntt_line_kernel<MODE, FIX, THREADS, MINB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return hc::cuda_check(e, "ntt smem attribute");
-    kern<<<(unsigned)tiles, THREADS, smem, hc::stream_of(ctx)>>>(t, pp, mul, mods);
+    hc::launch_kernel(kern, (unsigned)tiles, THREADS, smem, hc::stream_of(ctx), t, pp, mul, mods);
     hc::count_launch(ctx);
     return hc::cuda_check(cudaGetLastError(), "ntt kernel launch");
 }

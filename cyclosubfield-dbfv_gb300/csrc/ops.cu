@@ -66,6 +66,7 @@ __device__ __forceinline__ void pw_apply(const KView& d, const KView& a, const K
 
 template <int OP>
 __global__ void __launch_bounds__(256) pw_kernel(KView d, KView a, KView b, KMods m, int64_t lines, int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;
@@ -85,6 +86,7 @@ constexpr int LINE_SPAN = 1024;
 
 template <int OP>
 __global__ void __launch_bounds__(256) pw_line_kernel(KView d, KView a, KView b, KMods m) {
+    grid_wait();
     const int line = (int)blockIdx.y;
     const int k = line % (int)d.n2, r = line / (int)d.n2;
     const int j = r % (int)d.n1, i = r / (int)d.n1;
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(256) pw_line_kernel(KView d, KView a, KView b,
 /// each digit's columns); the sums are the same wrapping sums.
 __global__ void __launch_bounds__(256) matmul_kernel(KView d, KView lhs, KView rhs, int64_t U, int64_t lines,
                                                      int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;  // (i, k)
@@ -140,6 +143,7 @@ struct Terms {
 
 /// dst = sum_t lhs[t] * rhs[t], overwriting (src/hal/cpu.rs:707-788).
 __global__ void __launch_bounds__(256) inner_product_kernel(KView d, Terms terms, int64_t lines, int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;
@@ -158,6 +162,7 @@ __global__ void __launch_bounds__(256) inner_product_kernel(KView d, Terms terms
 
 /// inner_product_kernel over the line grid of pw_line_kernel.
 __global__ void __launch_bounds__(256) inner_product_line_kernel(KView d, Terms terms) {
+    grid_wait();
     const int line = (int)blockIdx.y;
     const int k = line % (int)d.n2, r = line / (int)d.n2;
     const int j = r % (int)d.n1, i = r / (int)d.n1;
@@ -177,6 +182,7 @@ __global__ void __launch_bounds__(256) inner_product_line_kernel(KView d, Terms 
 /// (src/hal/cpu.rs:950-980)
 __global__ void __launch_bounds__(256) bconv_correct_kernel(KView d, KView lhs, KView rhs, KMods m, int shift,
                                                             int64_t lines, int chunks) {
+    grid_wait();
     const i128 half = (i128)1 << (shift - 1);
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -195,6 +201,7 @@ __global__ void __launch_bounds__(256) bconv_correct_kernel(KView d, KView lhs, 
 
 /// bconv_correct_kernel over the line grid of pw_line_kernel.
 __global__ void __launch_bounds__(256) bconv_correct_line_kernel(KView d, KView lhs, KView rhs, KMods m, int shift) {
+    grid_wait();
     const i128 half = (i128)1 << (shift - 1);
     const int line = (int)blockIdx.y;
     const int k = line % (int)d.n2, r = line / (int)d.n2;
@@ -214,6 +221,7 @@ __global__ void __launch_bounds__(256) bconv_correct_line_kernel(KView d, KView 
 /// src/hal/cpu.rs:983-1015 (wide == 0) and :1018-1057 (wide == 1)
 __global__ void __launch_bounds__(256) bconv_pow2_kernel(KView d, KView src, i128 f0, i128 f1, int shift, int log2m,
                                                          int wide, int64_t lines, int chunks) {
+    grid_wait();
     const i128 half = (i128)1 << (shift - 1);
     const u128 mask = ((u128)1 << log2m) - 1;
     const i128 modulus = (i128)1 << log2m;
@@ -251,6 +259,7 @@ __global__ void __launch_bounds__(256) bconv_pow2_kernel(KView d, KView src, i12
 /// dst[e] = src[perm[e]] along dimension 2 or 3 (src/hal/cpu.rs:1086-1122)
 __global__ void __launch_bounds__(256) permute_kernel(KView d, KView s, const uint32_t* perm, int dim, int64_t lines,
                                                       int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;
@@ -292,8 +301,8 @@ hc_status launch_pointwise(hc_context ctx, int op, const KView& d, const KView& 
     const bool by_line = line_grid(d, lines, &lg);
 #define HC_PW(OPV)                                                      \
     case OPV:                                                           \
-        if (by_line) pw_line_kernel<OPV><<<lg, 256, 0, s>>>(d, a, b, m); \
-        else pw_kernel<OPV><<<blocks, 256, 0, s>>>(d, a, b, m, lines, chunks); \
+        if (by_line) hc::launch_kernel(pw_line_kernel<OPV>, lg, 256, 0, s, d, a, b, m); \
+        else hc::launch_kernel(pw_kernel<OPV>, blocks, 256, 0, s, d, a, b, m, lines, chunks); \
         break;
     switch (op) {
         HC_PW(OP_ASSIGN)
@@ -324,7 +333,7 @@ hc_status launch_matmul(hc_context ctx, const KView& d, const KView& lhs, const 
     int chunks;
     unsigned blocks;
     grid_for(ctx, d, lines, &chunks, &blocks);
-    matmul_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(d, lhs, rhs, U, lines, chunks);
+    hc::launch_kernel(matmul_kernel, blocks, 256, 0, stream_of(ctx), d, lhs, rhs, U, lines, chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "matmul kernel launch");
 }
@@ -339,10 +348,10 @@ hc_status launch_inner_product(hc_context ctx, const KView& d, const KView* l, c
     unsigned blocks;
     dim3 lg;
     if (line_grid(d, lines, &lg)) {
-        inner_product_line_kernel<<<lg, 256, 0, stream_of(ctx)>>>(d, t);
+        hc::launch_kernel(inner_product_line_kernel, lg, 256, 0, stream_of(ctx), d, t);
     } else {
         grid_for(ctx, d, lines, &chunks, &blocks);
-        inner_product_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(d, t, lines, chunks);
+        hc::launch_kernel(inner_product_kernel, blocks, 256, 0, stream_of(ctx), d, t, lines, chunks);
     }
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "inner product kernel launch");
@@ -356,10 +365,10 @@ hc_status launch_bconv_correct(hc_context ctx, const KView& d, const KView& lhs,
     unsigned blocks;
     dim3 lg;
     if (line_grid(d, lines, &lg)) {
-        bconv_correct_line_kernel<<<lg, 256, 0, stream_of(ctx)>>>(d, lhs, rhs, m, shift);
+        hc::launch_kernel(bconv_correct_line_kernel, lg, 256, 0, stream_of(ctx), d, lhs, rhs, m, shift);
     } else {
         grid_for(ctx, d, lines, &chunks, &blocks);
-        bconv_correct_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(d, lhs, rhs, m, shift, lines, chunks);
+        hc::launch_kernel(bconv_correct_kernel, blocks, 256, 0, stream_of(ctx), d, lhs, rhs, m, shift, lines, chunks);
     }
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "bconv correction kernel launch");
@@ -372,7 +381,7 @@ hc_status launch_bconv_pow2(hc_context ctx, const KView& d, const KView& src, i1
     int chunks;
     unsigned blocks;
     grid_for(ctx, d, lines, &chunks, &blocks);
-    bconv_pow2_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(d, src, f0, f1, shift, log2m, wide, lines, chunks);
+    hc::launch_kernel(bconv_pow2_kernel, blocks, 256, 0, stream_of(ctx), d, src, f0, f1, shift, log2m, wide, lines, chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "bconv pow2 kernel launch");
 }
@@ -383,7 +392,7 @@ hc_status launch_permute(hc_context ctx, const KView& d, const KView& s, const u
     int chunks;
     unsigned blocks;
     grid_for(ctx, d, lines, &chunks, &blocks);
-    permute_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(d, s, perm, dim, lines, chunks);
+    hc::launch_kernel(permute_kernel, blocks, 256, 0, stream_of(ctx), d, s, perm, dim, lines, chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "permute kernel launch");
 }

@@ -169,6 +169,7 @@ __device__ __forceinline__ void bconv_outputs(const BconvArgs& a, const KMods& d
 /// primes); SUB: rescale's subtract-and-multiply store (BconvArgs::sub_mul).
 template <bool ONE_CHUNK, bool SUB>
 __global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs a, KMods sm, KMods dm) {
+    grid_wait();
     extern __shared__ int2 xs[];  // [r][BCONV_THREADS]
     const int b = (int)(blockIdx.y % (unsigned)a.nb);
     const int64_t i = blockIdx.y / (unsigned)a.nb;
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs
     const int64_t pos = (int64_t)blockIdx.x * BCONV_THREADS + threadIdx.x;
     if (pos >= a.npos) return;
     const int64_t k = pos / a.src.n3, l = pos - k * a.src.n3;
-    const int64_t* __restrict__ srcp = kat<int64_t>(a.src, i, 0, k, l);  // row u at u * src.s1
+    const int64_t* srcp = kat<int64_t>(a.src, i, 0, k, l);  // row u at u * src.s1
     int64_t* dstp = kat<int64_t>(a.dst, i * a.nb + b, 0, k, l);          // row j at j * dst.s1
     // the source is multiplied by (Q/p)^-1 in Montgomery form, giving plain lifts in (-p, p)
     for (int u = u0; u < u1; u++) {
@@ -231,6 +232,7 @@ __device__ __forceinline__ int64_t finish_wide(uint64_t lo, int64_t hi, bool ful
 /// x [c, r, dl, dk] and carry [c, limbs, dl, dk] in place; CTAs over (128 positions, row).
 __global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KView carry, DbfvSplit d, int r, KMods m,
                                                                    int64_t npos) {
+    grid_wait();
     extern __shared__ int64_t sx[];  // [r][BCONV_THREADS]
     const int64_t pos = (int64_t)blockIdx.x * BCONV_THREADS + threadIdx.x;
     if (pos >= npos) return;
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KVie
 /// dst[i,j,k,l] = src[i,j,p2[k],p3[l]]
 __global__ void __launch_bounds__(256) galois_kernel(KView d, KView s, const uint32_t* p2, const uint32_t* p3,
                                                      int64_t lines, int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;
@@ -369,6 +372,7 @@ struct KsAcc {
 
 __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, const int64_t* one, int64_t lines,
                                                         int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;  // (j, k)
@@ -413,6 +417,7 @@ constexpr int KS_STAGES = 3;
 template <bool COMMON, bool FOLD>
 __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods m, const int64_t* one,
                                                                  int64_t lines, int chunks) {
+    grid_wait();
     __shared__ int64_t sx[KS_STAGES][2][256];
     __shared__ longlong2 skey[KS_STAGES][2][256];
     const int tid = threadIdx.x;
@@ -515,6 +520,7 @@ template <int W>
 __global__ void __launch_bounds__(256) tensor_kernel(KView d, KView lhs_lo, KView lhs_hi, KView rhs_lo, KView rhs_hi,
                                                      int rsplit, KMods m, int full0, int full1, int full2,
                                                      int64_t lines, int chunks) {
+    grid_wait();
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         int64_t line = tile / chunks;  // (i, j, k)
@@ -600,6 +606,7 @@ struct GiantUnits {
 template <int NOUT>
 __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs a, GiantUnits un, KMods m, const int64_t* one,
                                                              int64_t lines, int chunks) {
+    grid_wait();
     extern __shared__ int64_t gsm[];  // [GIANT_STAGES][2][256] staging, then the tile's lcoef as limb pairs
     int2* slc = reinterpret_cast<int2*>(gsm + GIANT_STAGES * 2 * 256);
     const int64_t tiles = lines * chunks;
@@ -694,6 +701,7 @@ constexpr int TRI_STAGES = 3;
 template <int NOUT>
 __global__ void __launch_bounds__(256, NOUT == 4 ? 2 : 3)
     giant_tri_kernel(GiantArgs a, KMods m, const int64_t* one, int n0, int64_t lines, int chunks) {
+    grid_wait();
     extern __shared__ __align__(16) int64_t gsm[];  // [TRI_STAGES][NOUT][256] position pairs, then the lcoef limb pairs
     longlong2* sx = reinterpret_cast<longlong2*>(gsm);
     int2* slc = reinterpret_cast<int2*>(sx + TRI_STAGES * NOUT * 256);
@@ -829,7 +837,7 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
         if (best < 0 || cost < best) best = cost, a.ochunk = oc;
     }
     dim3 grid((unsigned)cols, (unsigned)(ns * nb), (unsigned)((rd + a.ochunk - 1) / a.ochunk));
-    kern<<<grid, BCONV_THREADS, smem, stream_of(ctx)>>>(a, sm, dm);
+    hc::launch_kernel(kern, grid, BCONV_THREADS, smem, stream_of(ctx), a, sm, dm);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "bconv kernel launch");
 }
@@ -845,7 +853,7 @@ hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& carry, 
         if (e != cudaSuccess) return cuda_check(e, "dBFV reduction smem attribute");
     }
     dim3 grid((unsigned)((npos + BCONV_THREADS - 1) / BCONV_THREADS), (unsigned)x.n0);
-    dbfv_split_kernel<<<grid, BCONV_THREADS, smem, stream_of(ctx)>>>(x, carry, d, r, m, npos);
+    hc::launch_kernel(dbfv_split_kernel, grid, BCONV_THREADS, smem, stream_of(ctx), x, carry, d, r, m, npos);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "dBFV reduction launch");
 }
@@ -856,7 +864,7 @@ hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const ui
     int chunks;
     unsigned blocks;
     grid_lines(ctx, d.n3, lines, &chunks, &blocks);
-    galois_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(d, s, p2, p3, lines, chunks);
+    hc::launch_kernel(galois_kernel, blocks, 256, 0, stream_of(ctx), d, s, p2, p3, lines, chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "galois kernel launch");
 }
@@ -889,7 +897,7 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
     unsigned blocks;
     if (!pair) {
         grid_lines(ctx, dst.n3, lines, &chunks, &blocks);
-        keyswitch1_kernel<<<blocks, 256, 0, stream_of(ctx)>>>(a, m, one_dev, lines, chunks);
+        hc::launch_kernel(keyswitch1_kernel, blocks, 256, 0, stream_of(ctx), a, m, one_dev, lines, chunks);
         count_launch(ctx);
         return cuda_check(cudaGetLastError(), "keyswitch kernel launch");
     }
@@ -903,7 +911,7 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
     const bool fold = nterms >= LIMB_TERMS2;  // with the summand more than LIMB_TERMS2 terms
     auto kern = common ? (fold ? keyswitch_async_kernel<true, true> : keyswitch_async_kernel<true, false>)
                        : (fold ? keyswitch_async_kernel<false, true> : keyswitch_async_kernel<false, false>);
-    kern<<<blocks, 256, 0, stream_of(ctx)>>>(a, m, one_dev, lines, chunks);
+    hc::launch_kernel(kern, blocks, 256, 0, stream_of(ctx), a, m, one_dev, lines, chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "keyswitch kernel launch");
 }
@@ -947,7 +955,7 @@ hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, 
         auto kern = used == 1 ? giant_tri_kernel<1> : used == 2 ? giant_tri_kernel<2> : used == 3 ? giant_tri_kernel<3> : giant_tri_kernel<4>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem);
         if (e != cudaSuccess) return cuda_check(e, "giant-step smem attribute");
-        kern<<<blocks, 256, tri_smem, stream_of(ctx)>>>(a, m, one_dev, std::min(d, used), lines, chunks);
+        hc::launch_kernel(kern, blocks, 256, tri_smem, stream_of(ctx), a, m, one_dev, std::min(d, used), lines, chunks);
         count_launch(ctx);
         return cuda_check(cudaGetLastError(), "giant-step kernel launch");
     }
@@ -976,7 +984,7 @@ hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, 
                     : a.nout == 2 ? giant_kernel<2>
                     : a.nout == 3 ? giant_kernel<3>
                                   : giant_kernel<4>;
-        kern<<<blocks, 256, smem, stream_of(ctx)>>>(a, un, m, one_dev, lines, chunks);
+        hc::launch_kernel(kern, blocks, 256, smem, stream_of(ctx), a, un, m, one_dev, lines, chunks);
         count_launch(ctx);
         hc_status st = cuda_check(cudaGetLastError(), "giant-step kernel launch");
         if (st) return st;
@@ -998,11 +1006,11 @@ hc_status launch_tensor(hc_context ctx, const KView& d, const KView& lhs_lo, con
     unsigned blocks;
     if (pair) {
         grid_lines(ctx, d.n3 / 2, lines, &chunks, &blocks);
-        tensor_kernel<2><<<blocks, 256, 0, stream_of(ctx)>>>(d, lhs_lo, lhs_hi, rhs_lo, rhs_hi, rsplit, m, f0, f1, f2,
+        hc::launch_kernel(tensor_kernel<2>, blocks, 256, 0, stream_of(ctx), d, lhs_lo, lhs_hi, rhs_lo, rhs_hi, rsplit, m, f0, f1, f2,
                                                               lines, chunks);
     } else {
         grid_lines(ctx, d.n3, lines, &chunks, &blocks);
-        tensor_kernel<1><<<blocks, 256, 0, stream_of(ctx)>>>(d, lhs_lo, lhs_hi, rhs_lo, rhs_hi, rsplit, m, f0, f1, f2,
+        hc::launch_kernel(tensor_kernel<1>, blocks, 256, 0, stream_of(ctx), d, lhs_lo, lhs_hi, rhs_lo, rhs_hi, rsplit, m, f0, f1, f2,
                                                               lines, chunks);
     }
     count_launch(ctx);

@@ -169,3 +169,57 @@ def test_batched_and_single_transforms_agree(rings, field, count):
         batch.run()
         batch.close()
         assert (t.to_numpy() == exp).all() and (u.to_numpy() == exp).all(), name
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (1, 3, 5, 77), (2, 3, 12, 3072), (3, 40, 12, 3072)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("graph", [False, True])
+def test_dependent_launches_keep_their_order(be, shape, graph):
+    """Launches may be placed before their predecessor has finished (csrc/common.cuh: launch_kernel): a chain in which
+    each reads what the one before wrote and overwrites what that one read, with a second stream joining in between."""
+    import halcuda
+
+    g = np.random.default_rng(5)
+    x, y, z = (g.integers(-WORD, WORD, size=shape, dtype=np.int64) for _ in range(3))
+    a, b, c = be.tensor(x), be.tensor(y), be.tensor(z)
+
+    def chain():
+        for _ in range(20):
+            be.hal_add_i64(a, b)
+            be.hal_sub_i64(b, a)
+            be.hal_assign(c, b)
+            be.hal_add_i64(c, a)
+            be.hal_add_i64(b, c)
+
+    def apply(x, y, z):
+        with np.errstate(over="ignore"):
+            for _ in range(20):
+                x = x + y
+                y = y - x
+                z = y + x
+                y = y + z
+        return x, y, z
+
+    runs = 3
+    if graph:
+        be.synchronize()
+        gr = halcuda.Graph(be, chain)
+        for _ in range(runs):
+            gr.launch()
+    else:
+        other = halcuda.Stream()
+        for i in range(runs):
+            ev = halcuda.Event()
+            if i % 2:
+                ev.record(be)
+                with be.on(other):
+                    ev.wait(be)
+                    chain()
+                    ev = halcuda.Event()
+                    ev.record(be)
+                ev.wait(be)
+            else:
+                chain()
+    for _ in range(runs):
+        x, y, z = apply(x, y, z)
+    be.synchronize()
+    assert (a.to_numpy() == x).all() and (b.to_numpy() == y).all() and (c.to_numpy() == z).all()
