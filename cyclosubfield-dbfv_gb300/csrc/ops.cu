@@ -1,7 +1,7 @@
 // Pointwise, contraction, correction and permutation kernels of the Backend trait
 // (cyclosubfield-dbfv/src/hal/cpu.rs:591-1122). Every kernel walks the destination as
 // (line, l) with l the contiguous dimension 3; sources are broadcast through zero strides.
-#include "common.cuh"
+#include "limb_sum.cuh"
 
 namespace {
 
@@ -96,41 +96,93 @@ __global__ void __launch_bounds__(256) pw_line_kernel(KView d, KView a, KView b,
 }
 
 /// dst[i,j,k,l] = sum_u lhs[li,j,u,0] * rhs[ri,u,k,l] (src/hal/cpu.rs:791-818), i128 wrapping.
-/// Four output rows j per pass share each rhs load (the matrix entries are warp-uniform loads),
-/// and columns whose four entries are zero are skipped (a gadget conversion matrix is zero outside
-/// each digit's columns); the sums are the same wrapping sums.
-__global__ void __launch_bounds__(256) matmul_kernel(KView d, KView lhs, KView rhs, int64_t U, int64_t lines,
-                                                     int chunks) {
+/// Four output rows j per pass share each rhs load. The columns u go in chunks of LIMB_TERMS: the first
+/// warp splits the chunk's matrix entries into limbs and lists its columns that are not zero in all four
+/// rows (a gadget conversion matrix is zero outside each digit's columns); the others add nothing.
+/// A chunk whose words are all below 2^57 in absolute value (residues and centred constants are) is summed
+/// in limbs, found out for the matrix by the first warp and for the right-hand side by each warp as it
+/// goes; a warp that meets a larger word sums the chunk again as 128-bit products, so every word is allowed.
+/// What bounds it: the multiply pipe, 13 cycles a term instead of 33; a trait-path ct-mult (five
+/// products at field_36864 r = 16) 921 -> 839 us. Four columns unrolled or four CTAs per SM spill (852, 854).
+constexpr int MATMUL_ROWS = 4, MATMUL_UNROLL = 2;
+__global__ void __launch_bounds__(256, 3) matmul_kernel(KView d, KView lhs, KView rhs, int64_t U, int64_t lines,
+                                                        int chunks) {
     grid_wait();
+    __shared__ __align__(16) int2 sm[LIMB_TERMS][MATMUL_ROWS];
+    __shared__ int sidx[LIMB_TERMS], scount, slarge;
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        int64_t line = tile / chunks;  // (i, k)
-        int64_t l = (tile - line * chunks) * blockDim.x + threadIdx.x;
-        if (l >= d.n3) continue;
-        int64_t k = line % d.n2, i = line / d.n2;
-        int64_t j = 0;
-        for (; j + 4 <= d.n1; j += 4) {
-            i128 acc[4] = {0, 0, 0, 0};
-            for (int64_t u = 0; u < U; u++) {
-                int64_t c[4];
+        const int64_t line = tile / chunks;  // (i, k)
+        const int64_t l = (tile - line * chunks) * blockDim.x + threadIdx.x;
+        const int64_t k = line % d.n2, i = line / d.n2;
+        // a thread past the line's end reads its last position and stores nothing
+        const int64_t* x0 = kat<int64_t>(rhs, i, 0, k, l < d.n3 ? l : d.n3 - 1);
+        for (int64_t j = 0; j < d.n1; j += MATMUL_ROWS) {
+            const int rows = (int)(d.n1 - j < MATMUL_ROWS ? d.n1 - j : MATMUL_ROWS);
+            uint64_t lo[MATMUL_ROWS] = {};
+            int64_t hi[MATMUL_ROWS] = {};
+            for (int64_t u0 = 0; u0 < U; u0 += LIMB_TERMS) {
+                __syncthreads();  // the previous chunk's readers are done
+                if (threadIdx.x < 32) {
+                    const bool in = threadIdx.x < LIMB_TERMS && u0 + threadIdx.x < U;
+                    int64_t c[MATMUL_ROWS];
+                    uint64_t any = 0, large = 0;
 #pragma unroll
-                for (int q = 0; q < 4; q++) c[q] = *kat<int64_t>(lhs, i, j + q, u, 0);
-                if ((c[0] | c[1] | c[2] | c[3]) == 0) continue;  // zero columns (a gadget matrix's) add nothing
-                const int64_t x = *kat<int64_t>(rhs, i, u, k, l);
+                    for (int q = 0; q < MATMUL_ROWS; q++) {
+                        c[q] = in && q < rows ? *kat<int64_t>(lhs, i, j + q, u0 + threadIdx.x, 0) : 0;
+                        any |= (uint64_t)c[q];
+                        large |= ((uint64_t)c[q] + ((uint64_t)1 << 57)) >> 58;
+                    }
+                    const unsigned mask = __ballot_sync(0xffffffffu, any != 0);
+                    const int wide = __any_sync(0xffffffffu, large != 0);
+                    if (any != 0) {
+                        const int at = __popc(mask & ((1u << threadIdx.x) - 1));
+                        sidx[at] = (int)threadIdx.x;
 #pragma unroll
-                for (int q = 0; q < 4; q++) acc[q] = (i128)((u128)acc[q] + (u128)((i128)c[q] * (i128)x));
+                        for (int q = 0; q < MATMUL_ROWS; q++) sm[at][q] = limb_split(c[q]);
+                    }
+                    if (threadIdx.x == 0) scount = __popc(mask), slarge = wide;
+                }
+                __syncthreads();
+                const int n = scount;
+                const int64_t* xu = x0 + u0 * rhs.s1;
+                uint64_t large = slarge;
+                if (!large) {
+                    LimbSum s[MATMUL_ROWS];
+#pragma unroll
+                    for (int q = 0; q < MATMUL_ROWS; q++) s[q].zero();
+#pragma unroll MATMUL_UNROLL
+                    for (int t = 0; t < n; t++) {
+                        const int64_t v = xu[sidx[t] * rhs.s1];
+                        large |= ((uint64_t)v + ((uint64_t)1 << 57)) >> 58;
+                        const int2 x = limb_split(v);
+                        const int xs = x.x + x.y;
+#pragma unroll
+                        for (int q = 0; q < MATMUL_ROWS; q++) {
+                            const int2 w = sm[t][q];
+                            s[q].mac(x, xs, w, w.x + w.y);
+                        }
+                    }
+                    if (!__any_sync(0xffffffffu, large != 0)) {
+#pragma unroll
+                        for (int q = 0; q < MATMUL_ROWS; q++) s[q].fold(lo[q], hi[q]);
+                        continue;
+                    }
+                }
+                for (int t = 0; t < n; t++) {
+                    const int64_t v = xu[sidx[t] * rhs.s1];
+#pragma unroll
+                    for (int q = 0; q < MATMUL_ROWS; q++) {
+                        const int64_t c = q < rows ? *kat<int64_t>(lhs, i, j + q, u0 + sidx[t], 0) : 0;
+                        const u128 s = (((u128)(uint64_t)hi[q] << 64) | lo[q]) + (u128)((i128)c * (i128)v);
+                        lo[q] = (uint64_t)s, hi[q] = (int64_t)(s >> 64);
+                    }
+                }
             }
+            if (l < d.n3)
 #pragma unroll
-            for (int q = 0; q < 4; q++) st128(kat<longlong2>(d, i, j + q, k, l), acc[q]);
-        }
-        for (; j < d.n1; j++) {
-            i128 acc = 0;
-            for (int64_t u = 0; u < U; u++) {
-                int64_t c = *kat<int64_t>(lhs, i, j, u, 0);
-                int64_t x = *kat<int64_t>(rhs, i, u, k, l);
-                acc = (i128)((u128)acc + (u128)((i128)c * (i128)x));
-            }
-            st128(kat<longlong2>(d, i, j, k, l), acc);
+                for (int q = 0; q < MATMUL_ROWS; q++)
+                    if (q < rows) st128(kat<longlong2>(d, i, j + q, k, l), (i128)(((u128)(uint64_t)hi[q] << 64) | lo[q]));
         }
     }
 }

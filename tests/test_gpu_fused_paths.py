@@ -223,3 +223,29 @@ def test_dependent_launches_keep_their_order(be, shape, graph):
         x, y, z = apply(x, y, z)
     be.synchronize()
     assert (a.to_numpy() == x).all() and (b.to_numpy() == y).all() and (c.to_numpy() == z).all()
+
+
+@pytest.mark.parametrize("rows", [1, 4, 5, 7])
+@pytest.mark.parametrize("cols", [1, 27, 28, 29, 57])
+@pytest.mark.parametrize("l", [5, 256, 300])
+def test_matmul_chunks_and_word_sizes(be, po, rows, cols, l):
+    """Chunks of 28 columns (csrc/ops.cu: matmul_kernel) with words of at most 57 bits and larger ones met by the
+    matrix, by one warp of the right-hand side, by one word; zero and partly zero columns."""
+    g = np.random.default_rng(rows * 100 + cols)
+    edge = np.array([(1 << 57) - 1, -(1 << 57), 1 << 57, -(1 << 57) - 1, WORD, -WORD - 1, 0, 1, -1])
+    lhs = g.integers(-(1 << 57), (1 << 57) - 1, size=(2, rows, cols, 1), endpoint=True)
+    rhs = g.integers(-(1 << 57), (1 << 57) - 1, size=(2, cols, 3, l), endpoint=True)
+    lhs[:, :, cols // 2] = 0
+    lhs[:, rows // 2, cols // 3] = 0
+    rhs[0, :, 0] = g.choice(edge[:2], size=rhs[0, :, 0].shape)
+    rhs[0, cols - 1, 1, l - 1] = WORD
+    rhs[1, :, 1, : min(l, 32)] = g.choice(edge, size=rhs[1, :, 1, : min(l, 32)].shape)
+    for big in (False, True):
+        if big:
+            lhs[1, rows - 1, cols - 1] = -WORD - 1
+        d = be.hal_allocate_i128((2, rows, 3, l))
+        be.hal_matmul_i64(d, be.tensor(lhs), be.tensor(rhs))
+        got = d.to_numpy()
+        exp = np.zeros_like(got)
+        po.matmul_i64(exp, lhs, rhs)
+        assert (got == exp).all()
