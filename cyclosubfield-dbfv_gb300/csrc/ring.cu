@@ -26,7 +26,10 @@
 namespace hc {
 hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst, const BconvConsts& c, int r, int rd,
                              int nb, const KMods& sm, const KMods& dm, int64_t ns, const BarrettLimbs* sub_mul);
-hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& carry, const DbfvSplit& d, const KMods& m);
+hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& src, const KView& carry, const DbfvSplit& d,
+                            const KMods& m);
+hc_status launch_dbfv_tensor(hc_context ctx, const KView& d, const KView& lhs, const KView& rhs, int dout, const KMods& m,
+                             int full_above);
 hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const uint32_t* p2, const uint32_t* p3);
 hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys, int nterms, const KView* add0,
                            const KView* add1, int full0, int full1, const KView& dst, const KMods& m,
@@ -1410,8 +1413,8 @@ Tensor lift_to_extended(hc_ring R, const hc_view& pb, const hc_view* crt, const 
         R->transform(hi, ext, false);
         CK(hc_assign(R->ctx, vbase(res.view(), 0, r), *crt));
     } else {
-        CK(hc_assign(R->ctx, vbase(res.view(), 0, r), pb));
-        R->transform(res.view(), lifted, false);
+        R->transform(vbase(res.view(), 0, r), base, false, nullptr, &pb);
+        R->transform(hi, ext, false);
     }
     return res;
 }
@@ -2790,8 +2793,7 @@ Tensor dbfv_reduce(hc_ring R, size_t log2_b, size_t log2_t, const hc_view& ct, u
     const DbfvTables& T = dbfv_tables(R, log2_b, log2_t, b);
     const SplitData& D = T.D;
     const std::vector<Tensor>& delta_mont2 = T.delta_mont2;
-    Tensor result(R->ctx, 2 * (int64_t)digits, rr, R->dl(), R->dk());
-    CK(hc_assign(R->ctx, vrows(result.view(), 0, 2 * (int64_t)d), ct));
+    Tensor result(R->ctx, 2 * (int64_t)digits, rr, R->dl(), R->dk(), false, false);
     // one launch per digit: the incoming carry, the overflow and the digit's remainder
     const int64_t L = (int64_t)D.limbs();
     Tensor carry(R->ctx, 2, L, R->dl(), R->dk(), false, false);
@@ -2817,7 +2819,9 @@ Tensor dbfv_reduce(hc_ring R, size_t log2_b, size_t log2_t, const hc_view& ct, u
         const u128 in_bound = i < d ? bound : 1;
         S.full_in = S.have_carry && full(in_bound);
         S.full_out = full(S.have_carry ? 1 : in_bound);
-        CK(launch_dbfv_split(R->ctx, kv(vrows(result.view(), 2 * (int64_t)i, 2 * (int64_t)i + 2)), kv(carry.view()), S, km));
+        const int64_t row = 2 * (int64_t)i;
+        CK(launch_dbfv_split(R->ctx, kv(vrows(result.view(), row, row + 2)), i < d ? kv(vrows(ct, row, row + 2)) : KView(),
+                             kv(carry.view()), S, km));
     }
     *rows_out = 2 * digits;
     return result;
@@ -2882,55 +2886,59 @@ hc_status hc_dbfv_hom_mul(hc_ring R, size_t log2_b, size_t log2_t, hc_view lhs, 
         check_view(lhs, lhs.shape[0], rr, R->dl(), R->dk(), "lhs");
         check_view(rhs, rhs.shape[0], rr, R->dl(), R->dk(), "rhs");
         size_t r1 = 0, r2 = 0;
-        Tensor l = dbfv_reduce(R, log2_b, log2_t, lhs, 1, b, &r1), rt = dbfv_reduce(R, log2_b, log2_t, rhs, 1, b, &r2);
+        auto lifted_digits = [&](const hc_view& ct, size_t* rows) {
+            Tensor t = dbfv_reduce(R, log2_b, log2_t, ct, 1, b, rows);
+            return *rows ? lift_to_extended(R, vrows(t.view(), 0, (int64_t)*rows), nullptr, b) : Tensor();
+        };
+        // the operands are independent: the second is reduced and lifted on the side stream
+        SideBranch lifts(R);
+        lifts.begin();
+        Tensor rl = lifted_digits(rhs, &r2);
+        lifts.back();
+        Tensor ll = lifted_digits(lhs, &r1);
+        lifts.join();
         *out_rows = 0;
         if (r1 == 0 || r2 == 0) return;
         const size_t d1 = r1 / 2, d2 = r2 / 2, d_out = std::min(mdig, d1 + d2 - 1);
         check_view(out, out.shape[0], rr, R->dl(), R->dk(), "output");
         REQUIRE(out.shape[0] >= 2 * (int64_t)d_out, HC_ERR_SHAPE, "output has too few rows");
-        Tensor ll = lift_to_extended(R, vrows(l.view(), 0, (int64_t)r1), nullptr, b);
-        Tensor rl = lift_to_extended(R, vrows(rt.view(), 0, (int64_t)r2), nullptr, b);
         Base lifted = b;
         for (int64_t i = rr; i < ll.shape[1]; i++) lifted.push_back(R->initial_len + (size_t)(i - rr));
-        // all 3-component digit products, rows 3k .. 3k + 3 for output digit k (src/dbfv.rs:1081-1126)
-        Wide acc(R, 3 * (int64_t)d_out, lifted);
-        auto row = [](const Tensor& t, size_t i) { return vrows(t.view(), (int64_t)i, (int64_t)i + 1); };
-        for (size_t k = 0; k < d_out; k++) {
-            std::vector<hc_view> a0, b0, a1, b1, a2, b2;
-            const size_t jlo = k >= d2 - 1 ? k - (d2 - 1) : 0, jhi = std::min(k, d1 - 1);
-            for (size_t j = jlo; j <= jhi; j++) {
-                a0.push_back(row(ll, 2 * j)), b0.push_back(row(rl, 2 * (k - j)));
-                a1.push_back(row(ll, 2 * j)), b1.push_back(row(rl, 2 * (k - j) + 1));
-                a1.push_back(row(ll, 2 * j + 1)), b1.push_back(row(rl, 2 * (k - j)));
-                a2.push_back(row(ll, 2 * j + 1)), b2.push_back(row(rl, 2 * (k - j) + 1));
-            }
-            acc.inner_product(3 * k, 3 * k + 1, a0, b0);
-            acc.inner_product(3 * k + 1, 3 * k + 2, a1, b1);
-            acc.inner_product(3 * k + 2, 3 * k + 3, a2, b2);
-        }
-        Tensor prod(R->ctx, 3 * (int64_t)d_out, (int64_t)lifted.size(), R->dl(), R->dk(), false, false);
-        acc.reduce_into(prod.view());
-        R->transform(prod.view(), lifted, true);
-        const i128 t = (i128)1 << log2_t;
-        Tensor resc = rescale_to_base(R, prod.view(), lifted, r, t);
-        // relinearisation of every output digit at once (src/bfv.rs:699-741)
+        // all 3-component digit products (src/dbfv.rs:1081-1126): rows 2k, 2k + 1 are (c0, c1) of output digit
+        // k, row 2 d_out + k its c2
         const int64_t D = (int64_t)d_out;
+        const u128 mp = (u128)R->max_p(lifted), pairs = std::min({d1, d2, d_out});
+        REQUIRE(2 * pairs <= HC_MAX_TERMS, HC_ERR_UNSUPPORTED, "too many inner-product terms");
+        REQUIRE(2 * pairs * mp * mp <= (u128)I128MAX, HC_ERR_ARG, "wide ring element overflow");
+        const u128 above = ((u128)R->min_p(lifted) << 63) / (mp * mp);
+        Tensor prod = temp(R->ctx, 3 * D, (int64_t)lifted.size(), R->dl(), R->dk());
+        CK(launch_dbfv_tensor(R->ctx, kv(prod.view()), kv(ll.view()), kv(rl.view()), (int)D, R->kmods(lifted),
+                              (int)std::min<u128>(above, 1 << 30)));
+        const i128 t = (i128)1 << log2_t;
+        const hc_view tsv = R->scalar_tensor(lifted, t).view();
+        // relinearisation of every output digit at once (src/bfv.rs:699-741); c2's transform, rescale and
+        // gadget decomposition run on the side stream beside c0's and c1's
         Digits dg = clip(digits_of(digits, d), r);
         REQUIRE(rk.shape[0] >= 2 * (int64_t)dg.size() && rk.shape[1] >= rr, HC_ERR_SHAPE, "relinearisation key shape");
-        Tensor c2(R->ctx, D, rr, R->dl(), R->dk(), false, false);
-        CK(hc_assign(R->ctx, c2.view(), vstep(resc.view(), 2, 3, D)));
+        const hc_view p01 = vrows(prod.view(), 0, 2 * D), p2 = vrows(prod.view(), 2 * D, 3 * D);
+        SideBranch c2_branch(R);
+        c2_branch.begin();
+        R->transform(p2, lifted, true, &tsv);
+        Tensor c2 = rescale_to_base(R, p2, lifted, r, t, true);
         Tensor parts = gadget_decompose(R, c2.view(), b, dg);
-        hc_view c0 = vstep(resc.view(), 0, 3, D), c1 = vstep(resc.view(), 1, 3, D);
-        hc_view o = vrows(out, 0, 2 * D);
+        c2_branch.back();
+        R->transform(p01, lifted, true, &tsv);
+        Tensor resc = rescale_to_base(R, p01, lifted, r, t, true);
+        const hc_view c01 = resc.view(), o = vrows(out, 0, 2 * D);
+        if (!period_output) R->transform(c01, b, false);
+        c2_branch.join();
         if (!period_output) {
-            R->transform(c0, b, false);
-            R->transform(c1, b, false);
+            hc_view c0 = vstep(c01, 0, 2, D), c1 = vstep(c01, 1, 2, D);
             keyswitch(R, parts.view(), rk, b, dg.size(), &c0, &c1, o);
         } else {
             keyswitch(R, parts.view(), rk, b, dg.size(), nullptr, nullptr, o);
             R->transform(o, b, true);
-            CK(hc_add_i64(R->ctx, vstep(o, 0, 2, D), c0));
-            CK(hc_add_i64(R->ctx, vstep(o, 1, 2, D), c1));
+            CK(hc_add_i64(R->ctx, o, c01));
         }
         *out_rows = 2 * d_out;
     });

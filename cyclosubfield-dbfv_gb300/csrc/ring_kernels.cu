@@ -197,15 +197,16 @@ __device__ __forceinline__ int64_t finish_wide(uint64_t lo, int64_t hi, bool ful
 /// What bounds it: the multiply pipe, about 100 wide products per word. As the calls of the tensor HAL a digit took
 /// 10 to 17 launches and wrote its lifts, 128-bit sums and accumulators to memory: a product of two
 /// three-digit ciphertexts at field_49152 r = 16 took 2617 us and takes 2117 (26 to 37 us per digit here).
-/// x [c, r, dl, dk] and carry [c, limbs, dl, dk] in place; CTAs over (128 positions, row).
-__global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KView carry, DbfvSplit d, int r, KMods m,
-                                                                   int64_t npos) {
+/// src [c, r, dl, dk] (p null: zeros) to x, carry [c, limbs, dl, dk] in place; CTAs over (128 positions, row).
+__global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KView src, KView carry, DbfvSplit d, int r,
+                                                                   KMods m, int64_t npos) {
     grid_wait();
     extern __shared__ int64_t sx[];  // [r][BCONV_THREADS]
     const int64_t pos = (int64_t)blockIdx.x * BCONV_THREADS + threadIdx.x;
     if (pos >= npos) return;
     const int64_t i = blockIdx.y, k = pos / x.n3, l = pos - k * x.n3;
     int64_t* xp = kat<int64_t>(x, i, 0, k, l);
+    const int64_t* sp = src.p ? kat<int64_t>(src, i, 0, k, l) : nullptr;
     int64_t* cp = kat<int64_t>(carry, i, 0, k, l);
     auto fma = [](i128 acc, int64_t a, int64_t b) { return (i128)((u128)acc + (u128)((i128)a * (i128)b)); };
     auto finish = [&](i128 acc, int j, bool full) {
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KVie
     int64_t c0 = 0, c1 = 0;
     const int64_t* mq = d.mat + d.limbs * r;
     for (int u = 0; u < r; u++) {
-        int64_t w = xp[u * x.s1];
+        int64_t w = sp ? sp[u * src.s1] : 0;
         if (d.have_carry) {
             i128 acc = (i128)w * (i128)__ldg(d.one + u);
             for (int q = 0; q < d.limbs; q++) acc = fma(acc, c[q], __ldg(d.delta[q] + u));
@@ -531,6 +532,74 @@ __global__ void __launch_bounds__(256) tensor_kernel(KView d, KView lhs_lo, KVie
     }
 }
 
+/// The three-component products of two dBFV ciphertexts' digits with reduce_wide (dbfv_mul_convolve,
+/// src/dbfv.rs:1081-1126): output digit o (rows 2o, 2o + 1 and, its c2, 2 dout + o of d) sums the products
+/// of lhs digit q and rhs digit o - q, operands within 2p, folded every DBFV_FOLD digit pairs. Sums of more
+/// than full_above terms take the double reduction (the wide accumulator's bound).
+/// What bounds it: memory and the multiply pipe about equally (a position's 2 (d1 + d2) words in, 3 dout out, three
+/// products per pair of digits in four limb sums and 3 dout reductions): 84 us for three digits each at
+/// field_49152 with 34 factors. As nine inner products into a 128-bit tensor, its reduction and rescale's
+/// product by t (now in the inverse transform's last pass) 305 us.
+constexpr int DBFV_FOLD = (LIMB_TERMS2 - 1) / 2;
+template <int W>
+__global__ void __launch_bounds__(256) dbfv_tensor_kernel(KView d, KView lhs, KView rhs, int d1, int d2, int dout, KMods m,
+                                                          int full_above, int64_t lines, int chunks) {
+    grid_wait();
+    const int64_t tiles = lines * chunks;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t line = tile / chunks;  // (j, k)
+        const int64_t l = W * ((tile - line * chunks) * blockDim.x + threadIdx.x);
+        if (l >= d.n3) continue;
+        const int64_t k = line % d.n2, j = line / d.n2;
+        const int64_t* lp = kat<int64_t>(lhs, 0, j, k, l);
+        const int64_t* rp = kat<int64_t>(rhs, 0, j, k, l);
+        const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
+        const int64_t r2 = m.r2[j];
+        for (int o = 0; o < dout; o++) {
+            const int q0 = o >= d2 ? o - (d2 - 1) : 0, q1 = o < d1 ? o : d1 - 1;
+            LimbSum s[3][W];
+            uint64_t lo[3][W];
+            int64_t hi[3][W];
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int w = 0; w < W; w++) s[c][w].zero(), lo[c][w] = 0, hi[c][w] = 0;
+            auto fold = [&] {
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+#pragma unroll
+                    for (int w = 0; w < W; w++) s[c][w].fold(lo[c][w], hi[c][w]), s[c][w].zero();
+            };
+            int until = DBFV_FOLD;
+            for (int q = q0; q <= q1; q++) {
+                int64_t l0[W], l1[W], r0[W], r1[W];
+                load_words<W>(lp + 2 * q * lhs.s0, l0), load_words<W>(lp + (2 * q + 1) * lhs.s0, l1);
+                load_words<W>(rp + 2 * (o - q) * rhs.s0, r0), load_words<W>(rp + (2 * (o - q) + 1) * rhs.s0, r1);
+#pragma unroll
+                for (int w = 0; w < W; w++) {
+                    const int2 x0 = limb_split(l0[w]), x1 = limb_split(l1[w]), y0 = limb_split(r0[w]), y1 = limb_split(r1[w]);
+                    const int xs0 = x0.x + x0.y, xs1 = x1.x + x1.y, ys0 = y0.x + y0.y, ys1 = y1.x + y1.y;
+                    s[0][w].mac(x0, xs0, y0, ys0);
+                    s[1][w].mac(x0, xs0, y1, ys1), s[1][w].mac(x1, xs1, y0, ys0);
+                    s[2][w].mac(x1, xs1, y1, ys1);
+                }
+                if (--until == 0) fold(), until = DBFV_FOLD;
+            }
+            fold();
+            const int n = q1 - q0 + 1;
+            int64_t v[3][W];
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int w = 0; w < W; w++)
+                    v[c][w] = finish_wide(lo[c][w], hi[c][w], (c == 1 ? 2 * n : n) > full_above, ml, r2);
+            store_words<W>(kat<int64_t>(d, 2 * o, j, k, l), v[0]);
+            store_words<W>(kat<int64_t>(d, 2 * o + 1, j, k, l), v[1]);
+            store_words<W>(kat<int64_t>(d, 2 * dout + o, j, k, l), v[2]);
+        }
+    }
+}
+
 /// One giant step of the homomorphic CRT transform: output digit o (rows 2o, 2o + 1 of dst) is
 /// sum over the baby steps j and input digits i of baby(j, i) * L(coef_j, o - i), plus the carried
 /// digit o through mont(1), reduced. Each thread holds the accumulators of up to GIANT_OUT output
@@ -810,7 +879,8 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
     return cuda_check(cudaGetLastError(), "bconv kernel launch");
 }
 
-hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& carry, const DbfvSplit& d, const KMods& m) {
+hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& src, const KView& carry, const DbfvSplit& d,
+                            const KMods& m) {
     const int r = (int)x.n1;
     const int64_t npos = x.n2 * x.n3;
     if (npos == 0 || x.n0 == 0) return HC_OK;
@@ -821,7 +891,7 @@ hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& carry, 
         if (e != cudaSuccess) return cuda_check(e, "dBFV reduction smem attribute");
     }
     dim3 grid((unsigned)((npos + BCONV_THREADS - 1) / BCONV_THREADS), (unsigned)x.n0);
-    hc::launch_kernel(dbfv_split_kernel, grid, BCONV_THREADS, smem, stream_of(ctx), x, carry, d, r, m, npos);
+    hc::launch_kernel(dbfv_split_kernel, grid, BCONV_THREADS, smem, stream_of(ctx), x, src, carry, d, r, m, npos);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "dBFV reduction launch");
 }
@@ -958,6 +1028,21 @@ hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, 
         if (st) return st;
     }
     return HC_OK;
+}
+
+hc_status launch_dbfv_tensor(hc_context ctx, const KView& d, const KView& lhs, const KView& rhs, int dout, const KMods& m,
+                             int full_above) {
+    const int64_t lines = d.n1 * d.n2;
+    if (lines == 0 || d.n3 == 0) return HC_OK;
+    auto aligned = [](const KView& v) { return ((uintptr_t)v.p % 16) == 0 && v.s0 % 2 == 0 && v.s1 % 2 == 0 && v.s2 % 2 == 0; };
+    const bool pair = d.n3 % 2 == 0 && aligned(d) && aligned(lhs) && aligned(rhs);
+    int chunks;
+    unsigned blocks;
+    grid_lines(ctx, pair ? d.n3 / 2 : d.n3, lines, &chunks, &blocks);
+    hc::launch_kernel(pair ? dbfv_tensor_kernel<2> : dbfv_tensor_kernel<1>, blocks, 256, 0, stream_of(ctx), d, lhs, rhs,
+                      (int)(lhs.n0 / 2), (int)(rhs.n0 / 2), dout, m, full_above, lines, chunks);
+    count_launch(ctx);
+    return cuda_check(cudaGetLastError(), "dBFV tensor kernel launch");
 }
 
 hc_status launch_tensor(hc_context ctx, const KView& d, const KView& lhs_lo, const KView& lhs_hi, const KView& rhs_lo,

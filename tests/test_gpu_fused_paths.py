@@ -55,6 +55,40 @@ def test_dbfv_reduction(rings, ring, log2_b, log2_t, digits, bound):
     assert got.shape == exp.shape and (got == exp).all()
 
 
+# digit pairs per output digit around the fold at seven; unequal digit counts; positions of odd length (field_2)
+@pytest.mark.parametrize("ring", [("field_192", 200, 220, 64), ("field_18", 500, 520, 64), ("field_2", 200, 220, 64)],
+                         ids=lambda v: v[0])
+@pytest.mark.parametrize("log2_b,log2_t,d1,d2", [(8, 8, 1, 1), (8, 24, 3, 3), (8, 24, 1, 3), (4, 24, 6, 6), (4, 28, 7, 2), (4, 32, 8, 8),
+                                                 (4, 60, 15, 15), (2, 64, 32, 32)])
+@pytest.mark.parametrize("period", [False, True])
+def test_dbfv_product(rings, ring, log2_b, log2_t, d1, d2, period):
+    import ringcuda
+
+    o, d = rings(*ring)
+    base = o.initial_base()
+    primes = [o.primes[i] for i in base]
+    g = np.random.default_rng(log2_t + d1)
+    lhs, rhs = (residues(g, o.shape(2 * n, len(base)), primes, edges=True) for n in (d1, d2))
+    digits = [tuple(v) for v in ringcuda.select_digits(min(3, len(base)), len(base))]
+    rk = residues(g, o.shape(2 * len(digits), len(base)), primes)
+    exp = o.dbfv_hom_mul(log2_b, log2_t, lhs, rhs, base, rk.reshape((len(digits), 2) + rk.shape[1:]), digits, period_output=period)
+    got = ringcuda.dbfv_hom_mul(d, log2_b, log2_t, d.tensor(lhs), d.tensor(rhs), base, d.tensor(rk), digits,
+                                period_output=period).to_numpy()
+    assert got.shape == exp.shape and (got == exp).all()
+
+
+def test_dbfv_product_of_too_many_digits_is_refused(rings):
+    import halcuda
+    import ringcuda
+
+    o, d = rings("field_192", 200, 220, 64)
+    base = o.initial_base()
+    z = np.zeros(o.shape(66, len(base)), dtype=np.int64)
+    digits = [tuple(v) for v in ringcuda.select_digits(1, len(base))]
+    with pytest.raises(halcuda.HalError, match="too many"):
+        ringcuda.dbfv_hom_mul(d, 2, 66, d.tensor(z), d.tensor(z), base, d.allocate(2, len(base)), digits)
+
+
 @pytest.mark.parametrize("nd", [1, 2, 13, 14, 15, 16, 27, 28, 29, 41])
 def test_key_switch_digit_counts(rings, nd):
     """The sums of a key switch hold 15 gadget digits' products before they fold (csrc/common.cuh: LIMB_TERMS2)."""
