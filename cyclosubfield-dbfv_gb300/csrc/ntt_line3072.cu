@@ -35,12 +35,13 @@ hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KV
 }
 /// 128 threads per line: the fewest idle slots in the last wave, and seven (forward, 72 registers: ntt_mul
 /// of [24, 20, 12, 3072] 124 us, with eight 130) or eight (inverse: intt 105 us, with seven 107) independent
-/// CTAs per SM to cover each other's barriers. Up to two lines per SM (one element of 24 factors is 288
-/// lines) a line's own latency is the launch's, and 384 threads shorten it: one element at r = 16 41.5
-/// -> 36.7 us per transform; at 384 lines the two are level.
+/// CTAs per SM to cover each other's barriers. Up to three lines per SM (one
+/// element of 38 factors) a line's own latency is the launch's, and 384 threads shorten it: one element at
+/// r = 16 41.5 -> 36.7 us per transform; with the line at two per SM instead a ct-mult at r = 16 (384 lines beside
+/// another stream's launches) 407 us, at three 400, at six 404, and one per SM costs the one element 5 us.
 template <int MODE, bool FIX>
 hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
-    if (tiles <= 2 * (int64_t)hc::num_sms(ctx)) return launch_as<MODE, FIX, 384, 2>(ctx, t, pp, mul, mods, tiles);
+    if (tiles <= 3 * (int64_t)hc::num_sms(ctx)) return launch_as<MODE, FIX, 384, 2>(ctx, t, pp, mul, mods, tiles);
     return launch_as<MODE, FIX, 128, (MODE & 1) ? 8 : 7>(ctx, t, pp, mul, mods, tiles);
 }
 
