@@ -55,6 +55,8 @@ struct BconvConsts {
     int corr_limb;         // the correction row fits the limb products
     int shift;             // log2 of the correction's fixed-point scale
     int chunk;             // acc_before_reduce of the reference
+    const int2* hmat;      // host: each block's own columns of mat2, [nb][rd][columns], hwords entries (0: none)
+    int hwords;
 };
 
 /// First statement of every kernel: its launch may begin before the stream's previous kernel has finished

@@ -482,6 +482,7 @@ int64_t mul_mont_host(int64_t a, int64_t b, int64_t n, int64_t ninv) {
 ///    products too.
 struct BconvTables {
     DBuf qinv, mat, mat2, qmodp, qtab, r2, ucol;
+    std::vector<int2> hmat;
     BconvConsts c{};
 };
 
@@ -525,7 +526,18 @@ void build_bconv_tables(hc_context ctx, BconvTables& t, const std::vector<int64_
     t.qtab = DBuf(ctx, qtab.data(), qtab.size() * 8);
     t.r2 = DBuf(ctx, r2l.data(), rd * sizeof(BarrettLimbs));
     t.ucol = DBuf(ctx, uc.data(), uc.size() * 4);
+    // each block's own columns, where the blocks' ranges follow one another from column 0
+    bool in_order = true;
+    for (size_t b = 0; b < nb; b++) in_order = in_order && uc[2 * b] == (b ? uc[2 * b - 1] : 0);
+    if (in_order)
+        for (size_t b = 0; b < nb; b++)
+            for (size_t j = 0; j < rd; j++)
+                for (int32_t u = uc[2 * b]; u < uc[2 * b + 1]; u++) {
+                    const size_t o = ((b * rd + j) * r + (size_t)u) * 2;
+                    t.hmat.push_back(make_int2(m2[o], m2[o + 1]));
+                }
     BconvConsts& c = t.c;
+    c.hmat = t.hmat.data(), c.hwords = (int)std::min<size_t>(t.hmat.size(), 1 << 30);
     c.qinv = t.qinv.as<BarrettLimbs>(), c.mat = t.mat.as<int64_t>();
     c.mat2 = t.mat2.as<int2>(), c.qmodp = t.qmodp.as<int64_t>(), c.qtab = t.qtab.as<int64_t>();
     c.r2 = t.r2.as<BarrettLimbs>(), c.ucol = t.ucol.as<int32_t>();

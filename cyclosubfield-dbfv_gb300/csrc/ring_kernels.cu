@@ -15,6 +15,7 @@
 //    src/dbfv.rs:291-399), the addition of the carried result (dbfv_acc_add, :153-163) and the
 //    reduction (dbfv_finish_accumulator, :401-404), without the wide accumulator in HBM.
 #include <algorithm>
+#include <cstring>
 
 #include "limb_sum.cuh"
 
@@ -32,12 +33,23 @@ struct BconvArgs {
     const BarrettLimbs* sub_mul;  // optional [rd]: store mul_mont(dst - v, b_j) instead of v
 };
 
+/// The conversion matrix as a kernel parameter (BconvConsts::hmat), read as uniform constants that never
+/// pass the load path: up to 1152 entries (9 KB: bases of 33 factors; field_49152 r = 23 has 552); one
+/// entry: the matrix is read from memory (mat2).
+template <int N>
+struct BconvMatrix {
+    static constexpr int ENTRIES = N;
+    int2 m[N];
+};
+typedef BconvMatrix<1152> BconvParam;
+typedef BconvMatrix<1> BconvMemory;
+
 constexpr int LIMB_UNROLL = 16;  // terms unrolled together
 
 /// Multiply-accumulate of O output rows (r limb pairs each, consecutive from m) over the lifts u in
 /// [lo, hi): the exact sums sum_u m_u x_u (|x| < 2^57, |m| < 2^56) as 128-bit words h:l.
 /// N terms (n of them valid) into the column sums.
-template <int O, int N>
+template <int O, int N, bool PARAM>
 __device__ __forceinline__ void limb_terms(const int2* __restrict__ xp, const int2* __restrict__ m, int r, int n,
                                            LimbSum (&s)[O]) {
 #pragma unroll
@@ -47,13 +59,13 @@ __device__ __forceinline__ void limb_terms(const int2* __restrict__ xp, const in
             const int xs = x.x + x.y;
 #pragma unroll
             for (int o = 0; o < O; o++) {
-                const int2 w = __ldg(m + o * r + t);
+                const int2 w = PARAM ? m[o * r + t] : __ldg(m + o * r + t);
                 s[o].mac(x, xs, w, w.x + w.y);
             }
         }
     }
 }
-template <int O>
+template <int O, bool PARAM>
 __device__ __forceinline__ void limb_mac(const int2* __restrict__ xcol, const int2* __restrict__ m, int r, int lo, int hi,
                                          uint64_t (&l)[O], int64_t (&h)[O]) {
 #pragma unroll
@@ -66,8 +78,8 @@ __device__ __forceinline__ void limb_mac(const int2* __restrict__ xcol, const in
         const int2* xp = xcol + g0 * BCONV_THREADS;
         // sixteen terms fully unrolled (every address an immediate offset), the rest in steps of four
         int t = 0;
-        if (n >= LIMB_UNROLL) limb_terms<O, LIMB_UNROLL>(xp, m + g0, r, n, s), t = LIMB_UNROLL;
-        for (; t < n; t += 4) limb_terms<O, 4>(xp + t * BCONV_THREADS, m + g0 + t, r, n - t, s);
+        if (n >= LIMB_UNROLL) limb_terms<O, LIMB_UNROLL, PARAM>(xp, m + g0, r, n, s), t = LIMB_UNROLL;
+        for (; t < n; t += 4) limb_terms<O, 4, PARAM>(xp + t * BCONV_THREADS, m + g0 + t, r, n - t, s);
 #pragma unroll
         for (int o = 0; o < O; o++) s[o].fold(l[o], h[o]);
     }
@@ -91,10 +103,12 @@ __device__ __forceinline__ void bconv_store(const BconvArgs& a, const KMods& dm,
 }
 
 /// Outputs j .. j + O - 1 of the conversion (dst row j at d + j * s1).
-template <bool ONE_CHUNK, bool SUB, int O>
+template <bool ONE_CHUNK, bool SUB, int O, class MAT>
 __device__ __forceinline__ void bconv_outputs(const BconvArgs& a, const KMods& dm, int b, int j, int u0, int u1,
-                                              const int2* xcol, int64_t q, int64_t* d) {
-    const int2* m = a.c.mat2 + ((int64_t)b * a.rd + j) * a.r;
+                                              const int2* xcol, int64_t q, int64_t* d, const MAT& mx) {
+    constexpr bool PARAM = MAT::ENTRIES > 1;
+    const int stride = PARAM ? u1 - u0 : a.r;
+    const int2* m = PARAM ? mx.m + u0 * a.rd + j * stride - u0 : a.c.mat2 + ((int64_t)b * a.rd + j) * a.r;
     // the subtract-and-multiply store's operands, loaded before the sums so that their latency hides
     // behind the multiply-accumulate
     int64_t old[O] = {}, v[O] = {};
@@ -110,7 +124,7 @@ __device__ __forceinline__ void bconv_outputs(const BconvArgs& a, const KMods& d
     bool first = true;
     for (int c0 = 0; ONE_CHUNK ? first : c0 < a.r; c0 += a.c.chunk) {
         const int lo = ONE_CHUNK ? u0 : max(c0, u0), hi = ONE_CHUNK ? u1 : min(min(c0 + a.c.chunk, a.r), u1);
-        limb_mac<O>(xcol, m, a.r, lo, hi, l, h);
+        limb_mac<O, PARAM>(xcol, m, stride, lo, hi, l, h);
 #pragma unroll
         for (int o = 0; o < O; o++) {
             const int64_t r = mont_red_double(l[o], h[o], mont_limbs(dm.n[j + o], dm.ninv[j + o]));
@@ -127,16 +141,18 @@ __device__ __forceinline__ void bconv_outputs(const BconvArgs& a, const KMods& d
 /// (a gadget digit), outputs [z ochunk, (z + 1) ochunk) of the block; only the block's own source
 /// columns are lifted. The products with the conversion matrix use its limb form: the shared array
 /// holds each lift as its limb pair (x mod 2^29, x >> 29).
-/// What bounds it: the multiply pipe, 70 % busy; each lane's copy of a matrix entry takes the load path
-/// as long as a lift does, so a thread holds four output rows (one lift and four 8-byte entries for
-/// twelve wide products, the entries' limb sums formed, not read). With two rows and 16-byte entries
-/// the load path was 75 % busy beside 67 % of the multiply pipe: [2, 16 -> 18] of field_36864 32 -> 24
-/// us, [6, 23 -> 24] of field_49152 160 -> 130 us, [24, 16 -> 18] 209 -> 202 us. Two positions per
-/// thread on top take 128 registers and gain nothing.
+/// What bounds it: the multiply pipe, near 0.9 of its products' time ([24, 16 -> 18] of field_36864 134 us, 119 for
+/// 441 cycles of lifts and 18 times 277 of sums and reductions per warp). Each lane's copy of a matrix
+/// entry from memory takes the load path as long as a lift does, so a thread holds four output rows (one
+/// lift and four 8-byte entries for twelve wide products, the entries' limb sums formed, not read), and
+/// matrices that fit come as kernel parameters (BconvMatrix). Two rows and 16-byte entries: 75 % of the load path
+/// busy beside 67 % of the multiply pipe, [2, 16 -> 18] 32 us against 24, [6, 23 -> 24] of field_49152 160 against
+/// 130; the parameters on top: a field_49152 r = 23 ct-mult 813 -> 788 us, batched r = 16 of field_36864 2769 -> 2744. Two
+/// positions per thread take 128 registers and gain nothing.
 /// ONE_CHUNK: the block's columns form one chunk of the reference's chunked matmul (always for 57-bit
 /// primes); SUB: rescale's subtract-and-multiply store (BconvArgs::sub_mul).
-template <bool ONE_CHUNK, bool SUB>
-__global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs a, KMods sm, KMods dm) {
+template <bool ONE_CHUNK, bool SUB, class MAT>
+__global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs a, KMods sm, KMods dm, const __grid_constant__ MAT mx) {
     grid_wait();
     extern __shared__ int2 xs[];  // [r][BCONV_THREADS]
     const int b = (int)(blockIdx.y % (unsigned)a.nb);
@@ -178,9 +194,9 @@ __global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs
     }
     const int64_t q = (int64_t)((i128)((u128)corr + (u128)half) >> a.c.shift);
     int j = jbeg;
-    for (; j + 4 <= jend; j += 4) bconv_outputs<ONE_CHUNK, SUB, 4>(a, dm, b, j, u0, u1, xcol, q, dstp);
-    if (j + 2 <= jend) bconv_outputs<ONE_CHUNK, SUB, 2>(a, dm, b, j, u0, u1, xcol, q, dstp), j += 2;
-    if (j < jend) bconv_outputs<ONE_CHUNK, SUB, 1>(a, dm, b, j, u0, u1, xcol, q, dstp);
+    for (; j + 4 <= jend; j += 4) bconv_outputs<ONE_CHUNK, SUB, 4>(a, dm, b, j, u0, u1, xcol, q, dstp, mx);
+    if (j + 2 <= jend) bconv_outputs<ONE_CHUNK, SUB, 2>(a, dm, b, j, u0, u1, xcol, q, dstp, mx), j += 2;
+    if (j < jend) bconv_outputs<ONE_CHUNK, SUB, 1>(a, dm, b, j, u0, u1, xcol, q, dstp, mx);
 }
 
 /// A sum of at most HC_MAX_TERMS + 1 products of words within 2p: reduced once, or twice and back to
@@ -854,12 +870,6 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
     const size_t smem = (size_t)r * BCONV_THREADS * 8;
     if (smem > max_smem_optin(ctx)) return fail(HC_ERR_UNSUPPORTED, "base conversion: too many source rows");
     const bool one_chunk = c.chunk >= r, sub = sub_mul != nullptr;
-    auto kern = one_chunk ? (sub ? bconv_fused_kernel<true, true> : bconv_fused_kernel<true, false>)
-                          : (sub ? bconv_fused_kernel<false, true> : bconv_fused_kernel<false, false>);
-    if (smem > 49152) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return cuda_check(e, "bconv smem attribute");
-    }
     // the outputs of a position are split over CTAs while the grid leaves SMs short of work; each
     // split lifts the block's columns again. An SM is busy with four CTAs, so chunks of `oc` outputs
     // take about max(CTAs per SM, 4) times a CTA's cost, in wide products: 8 per lifted column, and per
@@ -874,9 +884,26 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
         if (best < 0 || cost < best) best = cost, a.ochunk = oc;
     }
     dim3 grid((unsigned)cols, (unsigned)(ns * nb), (unsigned)((rd + a.ochunk - 1) / a.ochunk));
-    hc::launch_kernel(kern, grid, BCONV_THREADS, smem, stream_of(ctx), a, sm, dm);
-    count_launch(ctx);
-    return cuda_check(cudaGetLastError(), "bconv kernel launch");
+    auto run = [&](auto kern, const auto& mx) {
+        if (smem > 49152) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return cuda_check(e, "bconv smem attribute");
+        }
+        hc::launch_kernel(kern, grid, BCONV_THREADS, smem, stream_of(ctx), a, sm, dm, mx);
+        count_launch(ctx);
+        return cuda_check(cudaGetLastError(), "bconv kernel launch");
+    };
+    if (one_chunk && c.hwords > 0 && c.hwords <= BconvParam::ENTRIES) {
+        BconvParam mx;
+        std::memcpy(mx.m, c.hmat, (size_t)c.hwords * sizeof(int2));
+        return sub ? run(bconv_fused_kernel<true, true, BconvParam>, mx) : run(bconv_fused_kernel<true, false, BconvParam>, mx);
+    }
+    const BconvMemory none{};
+    if (one_chunk)
+        return sub ? run(bconv_fused_kernel<true, true, BconvMemory>, none)
+                   : run(bconv_fused_kernel<true, false, BconvMemory>, none);
+    return sub ? run(bconv_fused_kernel<false, true, BconvMemory>, none)
+               : run(bconv_fused_kernel<false, false, BconvMemory>, none);
 }
 
 hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& src, const KView& carry, const DbfvSplit& d,

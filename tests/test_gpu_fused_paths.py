@@ -283,3 +283,29 @@ def test_matmul_chunks_and_word_sizes(be, po, rows, cols, l):
         exp = np.zeros_like(got)
         po.matmul_i64(exp, lhs, rhs)
         assert (got == exp).all()
+
+
+@pytest.mark.parametrize("r,rd", [(32, 36), (33, 34), (33, 35), (1, 42), (41, 28), (41, 29), (41, 43)])
+def test_base_conversion_matrix_as_parameter(rings, r, rd):
+    """Conversion matrices of up to 1152 entries are kernel parameters, larger ones are read from memory."""
+    o, d = rings("field_192", 2300, 2340, 4)
+    src, dst = list(range(r)), list(range(r, r + rd))
+    x = residues(np.random.default_rng(r), o.shape(2, r), [o.primes[i] for i in src], edges=True)
+    out = d.allocate(2, rd)
+    d.bconv(out, dst, d.tensor(x), src)
+    assert (out.to_numpy() == o.bconv(x, src, dst)).all()
+
+
+@pytest.mark.parametrize("r", [16, 33, 34, 41])
+@pytest.mark.parametrize("nd", [1, 3, 5])
+def test_gadget_matrix_as_parameter(rings, r, nd):
+    import ringcuda
+
+    o, d = rings("field_192", 2300, 2340, 4)
+    base = o.initial_base()[:r]
+    digits = [tuple(v) for v in ringcuda.select_digits(nd, r)]
+    x = residues(np.random.default_rng(r), o.shape(2, r), [o.primes[i] for i in base], edges=True)
+    got = d.allocate(2 * nd, r)
+    d.bconv_gadget(got, d.tensor(x), base, digits)
+    exp = np.concatenate([o.bconv_gadget(x[i:i + 1], base, digits) for i in range(2)])  # the oracle takes one element
+    assert got.shape == exp.shape and (got.to_numpy() == exp).all()
