@@ -23,44 +23,59 @@ enum PwOp {
     OP_I64_TO_MONT,
 };
 
+/// What operation OP reads at one position: the destination's old value (p, wp) and its operands, 8-byte
+/// words or 16-byte ones (w*).
+struct PwIn {
+    int64_t p, a, b;
+    i128 wp, wa;
+};
+
+constexpr bool pw_wide_dst(int op) { return op == OP_ASSIGN_I128 || op == OP_ADD_I128 || op == OP_FMA_I64 || op == OP_MUL_I64; }
+constexpr bool pw_wide_src(int op) {
+    return op == OP_ASSIGN_NARROW || op == OP_ASSIGN_I128 || op == OP_ADD_I128 || op == OP_ADD_RED_DOUBLE ||
+           op == OP_RED_DOUBLE || op == OP_ADD_RED || op == OP_RED || op == OP_I128_TO_MONT;
+}
+constexpr bool pw_reads_dst(int op) {
+    return op == OP_ADD_I64 || op == OP_SUB_I64 || op == OP_ADD_I128 || op == OP_FMA_I64 || op == OP_MUL_MONT ||
+           op == OP_ADD_RED_DOUBLE || op == OP_ADD_RED || op == OP_I64_TO_MONT;
+}
+
 template <int OP>
-__device__ __forceinline__ void pw_apply(const KView& d, const KView& a, const KView& b, const KMods& m, int64_t i,
-                                         int64_t j, int64_t k, int64_t l) {
-    if (OP == OP_ASSIGN) {
-        *kat<int64_t>(d, i, j, k, l) = *kat<int64_t>(a, i, j, k, l);
-    } else if (OP == OP_ASSIGN_NARROW) {
-        *kat<int64_t>(d, i, j, k, l) = kat<longlong2>(a, i, j, k, l)->x;  // low word of the i128
-    } else if (OP == OP_ASSIGN_I128) {
-        *kat<longlong2>(d, i, j, k, l) = *kat<longlong2>(a, i, j, k, l);
-    } else if (OP == OP_ADD_I64) {
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        *p = wadd(*p, *kat<int64_t>(a, i, j, k, l));
-    } else if (OP == OP_SUB_I64) {
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        *p = wsub(*p, *kat<int64_t>(a, i, j, k, l));
-    } else if (OP == OP_ADD_I128) {
-        longlong2* p = kat<longlong2>(d, i, j, k, l);
-        st128(p, (i128)((u128)ld128(p) + (u128)ld128(kat<longlong2>(a, i, j, k, l))));
-    } else if (OP == OP_FMA_I64 || OP == OP_MUL_I64) {
-        longlong2* p = kat<longlong2>(d, i, j, k, l);
-        i128 prod = (i128)*kat<int64_t>(a, i, j, k, l) * (i128)*kat<int64_t>(b, i, j, k, l);
-        st128(p, OP == OP_FMA_I64 ? (i128)((u128)ld128(p) + (u128)prod) : prod);
-    } else if (OP == OP_MUL_MONT) {
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        *p = mul_mont(*p, *kat<int64_t>(a, i, j, k, l), m.n[j], m.ninv[j]);
-    } else if (OP == OP_ADD_RED_DOUBLE || OP == OP_RED_DOUBLE) {
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        int64_t r = double_red128(ld128(kat<longlong2>(a, i, j, k, l)), m.n[j], m.ninv[j]);
-        *p = OP == OP_RED_DOUBLE ? r : wadd(*p, r);
-    } else if (OP == OP_ADD_RED || OP == OP_RED) {
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        int64_t r = red128(ld128(kat<longlong2>(a, i, j, k, l)), m.n[j], m.ninv[j]);
-        *p = OP == OP_RED ? r : wadd(*p, r);
-    } else if (OP == OP_I128_TO_MONT) {
-        *kat<int64_t>(d, i, j, k, l) = to_mont128(ld128(kat<longlong2>(a, i, j, k, l)), m.n[j], m.ninv[j], m.r3[j]);
-    } else if (OP == OP_I64_TO_MONT) {
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        *p = to_mont64(*p, m.n[j], m.ninv[j], m.r2[j]);
+__device__ __forceinline__ void pw_load(PwIn& v, const KView& d, const KView& a, const KView& b, int64_t i, int64_t j,
+                                        int64_t k, int64_t l) {
+    if constexpr (pw_reads_dst(OP)) {
+        if constexpr (pw_wide_dst(OP)) v.wp = ld128(kat<longlong2>(d, i, j, k, l));
+        else v.p = *kat<int64_t>(d, i, j, k, l);
+    }
+    if constexpr (pw_wide_src(OP)) v.wa = ld128(kat<longlong2>(a, i, j, k, l));
+    else if constexpr (OP != OP_I64_TO_MONT) v.a = *kat<int64_t>(a, i, j, k, l);
+    if constexpr (OP == OP_FMA_I64 || OP == OP_MUL_I64) v.b = *kat<int64_t>(b, i, j, k, l);
+}
+
+template <int OP>
+__device__ __forceinline__ void pw_store(const PwIn& v, const KView& d, const KMods& m, int64_t i, int64_t j, int64_t k,
+                                         int64_t l) {
+    if constexpr (pw_wide_dst(OP)) {
+        i128 r;
+        if constexpr (OP == OP_ASSIGN_I128) r = v.wa;
+        else if constexpr (OP == OP_ADD_I128) r = (i128)((u128)v.wp + (u128)v.wa);
+        else if constexpr (OP == OP_FMA_I64) r = (i128)((u128)v.wp + (u128)((i128)v.a * (i128)v.b));
+        else r = (i128)v.a * (i128)v.b;
+        st128(kat<longlong2>(d, i, j, k, l), r);
+    } else {
+        int64_t r;
+        if constexpr (OP == OP_ASSIGN) r = v.a;
+        else if constexpr (OP == OP_ASSIGN_NARROW) r = (int64_t)(uint64_t)v.wa;  // low word of the i128
+        else if constexpr (OP == OP_ADD_I64) r = wadd(v.p, v.a);
+        else if constexpr (OP == OP_SUB_I64) r = wsub(v.p, v.a);
+        else if constexpr (OP == OP_MUL_MONT) r = mul_mont(v.p, v.a, m.n[j], m.ninv[j]);
+        else if constexpr (OP == OP_RED_DOUBLE) r = double_red128(v.wa, m.n[j], m.ninv[j]);
+        else if constexpr (OP == OP_ADD_RED_DOUBLE) r = wadd(v.p, double_red128(v.wa, m.n[j], m.ninv[j]));
+        else if constexpr (OP == OP_RED) r = red128(v.wa, m.n[j], m.ninv[j]);
+        else if constexpr (OP == OP_ADD_RED) r = wadd(v.p, red128(v.wa, m.n[j], m.ninv[j]));
+        else if constexpr (OP == OP_I128_TO_MONT) r = to_mont128(v.wa, m.n[j], m.ninv[j], m.r3[j]);
+        else r = to_mont64(v.p, m.n[j], m.ninv[j], m.r2[j]);
+        *kat<int64_t>(d, i, j, k, l) = r;
     }
 }
 
@@ -74,15 +89,19 @@ __global__ void __launch_bounds__(256) pw_kernel(KView d, KView a, KView b, KMod
         if (l >= d.n3) continue;
         int64_t k = line % d.n2, r = line / d.n2;
         int64_t j = r % d.n1, i = r / d.n1;
-        pw_apply<OP>(d, a, b, m, i, j, k, l);
+        PwIn v;
+        pw_load<OP>(v, d, a, b, i, j, k, l);
+        pw_store<OP>(v, d, m, i, j, k, l);
     }
 }
 
 /// pw_kernel over a 2-D grid: blockIdx.y is the destination line (i, j, k), decomposed once per
-/// thread with 32-bit arithmetic, and each thread walks LINE_SPAN / 256 positions of it, so that
+/// thread with 32-bit arithmetic, and each thread takes LINE_SPAN / 256 positions of it, so that
 /// the per-element work is the operation itself (the tile form pays several 64-bit divisions per
-/// element). Used while the line count fits the grid's y dimension.
-constexpr int LINE_SPAN = 1024;
+/// element). Used while the line count fits the grid's y dimension. What bounds the short launches of
+/// one ciphertext is the latency of the reads, so all of a thread's are in flight before its first store: a
+/// trait-path ct-mult at field_36864 r = 16 (42 of its 77 launches are of this file) 842 -> 819 us.
+constexpr int LINE_SPAN = 1024, LINE_STEPS = LINE_SPAN / 256;
 
 template <int OP>
 __global__ void __launch_bounds__(256) pw_line_kernel(KView d, KView a, KView b, KMods m) {
@@ -91,8 +110,13 @@ __global__ void __launch_bounds__(256) pw_line_kernel(KView d, KView a, KView b,
     const int k = line % (int)d.n2, r = line / (int)d.n2;
     const int j = r % (int)d.n1, i = r / (int)d.n1;
     const int64_t l0 = (int64_t)blockIdx.x * LINE_SPAN;
-    const int64_t l1 = l0 + LINE_SPAN < d.n3 ? l0 + LINE_SPAN : d.n3;
-    for (int64_t l = l0 + threadIdx.x; l < l1; l += 256) pw_apply<OP>(d, a, b, m, i, j, k, l);
+    PwIn v[LINE_STEPS];
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++)
+        if (l0 + 256 * s + threadIdx.x < d.n3) pw_load<OP>(v[s], d, a, b, i, j, k, l0 + 256 * s + threadIdx.x);
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++)
+        if (l0 + 256 * s + threadIdx.x < d.n3) pw_store<OP>(v[s], d, m, i, j, k, l0 + 256 * s + threadIdx.x);
 }
 
 /// dst[i,j,k,l] = sum_u lhs[li,j,u,0] * rhs[ri,u,k,l] (src/hal/cpu.rs:791-818), i128 wrapping.
@@ -219,15 +243,23 @@ __global__ void __launch_bounds__(256) inner_product_line_kernel(KView d, Terms 
     const int k = line % (int)d.n2, r = line / (int)d.n2;
     const int j = r % (int)d.n1, i = r / (int)d.n1;
     const int64_t l0 = (int64_t)blockIdx.x * LINE_SPAN;
-    const int64_t l1 = l0 + LINE_SPAN < d.n3 ? l0 + LINE_SPAN : d.n3;
-    for (int64_t l = l0 + threadIdx.x; l < l1; l += 256) {
-        i128 acc = 0;
-        for (int t = 0; t < terms.n; t++) {
-            i128 prod = (i128)*kat<int64_t>(terms.l[t], i, j, k, l) * (i128)*kat<int64_t>(terms.r[t], i, j, k, l);
-            acc = (i128)((u128)acc + (u128)prod);
+    i128 acc[LINE_STEPS];
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++) acc[s] = 0;
+    for (int t = 0; t < terms.n; t++) {
+        int64_t x[LINE_STEPS], y[LINE_STEPS];
+#pragma unroll
+        for (int s = 0; s < LINE_STEPS; s++) {
+            // positions past the line's end repeat its last one
+            const int64_t l = min(l0 + 256 * s + threadIdx.x, d.n3 - 1);
+            x[s] = *kat<int64_t>(terms.l[t], i, j, k, l), y[s] = *kat<int64_t>(terms.r[t], i, j, k, l);
         }
-        st128(kat<longlong2>(d, i, j, k, l), acc);
+#pragma unroll
+        for (int s = 0; s < LINE_STEPS; s++) acc[s] = (i128)((u128)acc[s] + (u128)((i128)x[s] * (i128)y[s]));
     }
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++)
+        if (l0 + 256 * s + threadIdx.x < d.n3) st128(kat<longlong2>(d, i, j, k, l0 + 256 * s + threadIdx.x), acc[s]);
 }
 
 /// dst[i,j,k,l] += red(((lhs[i,0,k,l] + 2^(shift-1)) >> shift) * rhs[ri,j,0,0])
@@ -261,12 +293,17 @@ __global__ void __launch_bounds__(256) bconv_correct_line_kernel(KView d, KView 
     const int64_t c = *kat<int64_t>(rhs, i, j, 0, 0);
     const int64_t n = m.n[j], ninv = m.ninv[j];
     const int64_t l0 = (int64_t)blockIdx.x * LINE_SPAN;
-    const int64_t l1 = l0 + LINE_SPAN < d.n3 ? l0 + LINE_SPAN : d.n3;
-    for (int64_t l = l0 + threadIdx.x; l < l1; l += 256) {
-        i128 x = ld128(kat<longlong2>(lhs, i, 0, k, l));
-        int64_t q = (int64_t)((i128)((u128)x + (u128)half) >> shift);
-        int64_t* p = kat<int64_t>(d, i, j, k, l);
-        *p = wadd(*p, mul_mont(q, c, n, ninv));
+    i128 x[LINE_STEPS];
+    int64_t v[LINE_STEPS];
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++) {
+        const int64_t l = min(l0 + 256 * s + threadIdx.x, d.n3 - 1);  // past the end: the last position again
+        x[s] = ld128(kat<longlong2>(lhs, i, 0, k, l)), v[s] = *kat<int64_t>(d, i, j, k, l);
+    }
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++) {
+        const int64_t q = (int64_t)((i128)((u128)x[s] + (u128)half) >> shift);
+        if (l0 + 256 * s + threadIdx.x < d.n3) *kat<int64_t>(d, i, j, k, l0 + 256 * s + threadIdx.x) = wadd(v[s], mul_mont(q, c, n, ninv));
     }
 }
 
