@@ -846,8 +846,8 @@ def transform_roofline(be, R, field, rows, reps, bpeak, peaks):
     """CRT transforms as the ring runs them: pb_to_crt of a [rows, r + e, deg_L', deg_K] tensor of
     lifted residues (larger than L2), timed with CUDA events on the library's stream, beside the
     same transform as the reference's four HAL calls (one launch per dimension and direction).
-    field_49152 runs as two fused cluster launches (csrc/crt_fused.cu), field_36864 as the four
-    column / line launches. Algorithmic bytes: one read and one write of every residue per
+    field_49152 runs as four launches split where its data's coupling splits (csrc/crt_slab.cu),
+    field_36864 as the four column / line launches. Algorithmic bytes: one read and one write of every residue per
     launch; algorithmic products: TRANSFORM_PRODUCTS per residue."""
     import numpy as np
 

@@ -1,7 +1,7 @@
-// Integer-pipe peak of the NTT's Barrett product (bmul, common.cuh): a register-only kernel whose
-// rate is the denominator of the compute-bound transforms' integer roofline. No memory traffic
-// but one word per thread at the end; every chain stays within |x| <= 3n/4 (bmul's bound), so the
-// work is exactly the transforms' product on in-range operands.
+// Integer-pipe peak of the NTT's Barrett product in limbs (barrett_mul, common.cuh): a register-only kernel
+// whose rate is the denominator of the compute-bound transforms' integer roofline. No memory traffic
+// but one word per thread at the end; every chain stays within |x| <= 3n/4 (the product's bound), so
+// the work is exactly the transforms' product on in-range operands.
 #include "common.cuh"
 
 namespace {
@@ -9,7 +9,7 @@ namespace {
 constexpr int PEAK_THREADS = 256;
 constexpr int PEAK_CHAINS = 8;  // independent products in flight per thread
 
-__global__ void __launch_bounds__(PEAK_THREADS) barrett_peak_kernel(int64_t z, int64_t u, int64_t n, int iters,
+__global__ void __launch_bounds__(PEAK_THREADS) barrett_peak_kernel(BarrettLimbs w, BarrettMod m, int64_t n, int iters,
                                                                     int64_t* out) {
     const int64_t tid = (int64_t)blockIdx.x * PEAK_THREADS + threadIdx.x;
     int64_t x[PEAK_CHAINS];
@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(PEAK_THREADS) barrett_peak_kernel(int64_t z, i
     for (int c = 0; c < PEAK_CHAINS; c++) x[c] = (tid * 7919 + c * 104729) % n;
     for (int it = 0; it < iters; it++) {
 #pragma unroll
-        for (int c = 0; c < PEAK_CHAINS; c++) x[c] = bmul(z, u, x[c], n);
+        for (int c = 0; c < PEAK_CHAINS; c++) x[c] = barrett_mul(w, x[c], m);
     }
     int64_t acc = 0;
 #pragma unroll
@@ -107,6 +107,9 @@ hc_status hc_barrett_peak(hc_context ctx, double* products_per_s) {
     const int64_t n = ((int64_t)1 << 57) - 13, z = 0x123456789abcdLL % n;
     const i128 num = -((i128)z << 64);
     const int64_t u = (int64_t)((num >= 0 ? num + n / 2 : num - n / 2) / n);
+    const BarrettLimbs w = barrett_limbs(z, u, n);
+    BarrettMod m{};
+    m.n0 = (int32_t)lo32(n), m.nn0 = (int32_t)(0u - lo32(n)), m.nn1 = -bal_hi(n);
     const int blocks = num_sms(ctx) * 8, iters = 4096;
     const size_t words = (size_t)blocks * PEAK_THREADS;
     cudaStream_t s = stream_of(ctx);
@@ -119,9 +122,9 @@ hc_status hc_barrett_peak(hc_context ctx, double* products_per_s) {
     if (!st) st = cuda_check(cudaEventCreate(&e1), "peak event");
     float ms = 0.f;
     if (!st) {
-        barrett_peak_kernel<<<blocks, PEAK_THREADS, 0, s>>>(z, u, n, iters / 8, out);  // warm-up
+        barrett_peak_kernel<<<blocks, PEAK_THREADS, 0, s>>>(w, m, n, iters / 8, out);  // warm-up
         cudaEventRecord(e0, s);
-        barrett_peak_kernel<<<blocks, PEAK_THREADS, 0, s>>>(z, u, n, iters, out);
+        barrett_peak_kernel<<<blocks, PEAK_THREADS, 0, s>>>(w, m, n, iters, out);
         cudaEventRecord(e1, s);
         count_launch(ctx, 2);
         st = cuda_check(cudaGetLastError(), "peak kernel launch");

@@ -20,7 +20,7 @@
  * Threads and streams: a ring (its table caches and its side streams) is used from one host thread
  * at a time; calls are asynchronous on the context's current stream (hc_context_set_stream), and
  * calls issued on different streams of one context may run concurrently on the GPU. Some calls
- * (hc_bfv_hom_mul) run independent parts on the ring's side stream, forked from and joined back
+ * (hc_bfv_hom_mul, hc_dbfv_hom_mul) run independent parts on the ring's side stream, forked from and joined back
  * into the current stream, which a CUDA-graph capture of the call records as parallel paths.
  */
 #ifndef RINGCUDA_H
@@ -122,8 +122,9 @@ hc_status hc_bfv_hom_gal_batch(hc_ring ring, hc_view ct, const size_t* base, siz
  * crt_to_pb (:1140-1161), in place and bit-identical to those calls made one by one. The batch
  * keeps device pointers to the items' tensors and to the rings' tables: both must outlive it.
  * Running it issues, per shape class of its slabs (each field's specialised line and column
- * shapes; one class for the rest), a counter reset and one persistent kernel on the context's
- * stream (graph-capturable). */
+ * shapes; one class for the rest), a counter reset and one persistent kernel: the first class on the
+ * context's stream, the others beside it on a side stream forked from and joined back into it
+ * (graph-capturable). */
 #define HC_CRT_FORWARD 1 /* period basis -> CRT basis (input bound 2) */
 #define HC_CRT_MUL 2     /* Montgomery product with `op` (CRT basis) */
 #define HC_CRT_INVERSE 4 /* CRT basis -> period basis */
