@@ -65,6 +65,17 @@ struct BconvConsts {
 /// kernel launched by launch_kernel waits, so that a finished kernel implies all before it.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+/// Keys of one launch of the key switch over the same gadget digits and summands (launch_keyswitch): each
+/// with its automorphism and its output.
+constexpr int KS_GROUP = 16;
+struct KsGroup {
+    int n;
+    int64_t off[KS_GROUP];        // words from the first key's tensor to this key's (equal strides)
+    int64_t* dst[KS_GROUP];       // [2B, r, dl, dk], equal strides
+    const uint32_t* p2[KS_GROUP]; // optional Galois permutation applied to the digits and summands (apply_galois
+    const uint32_t* p3[KS_GROUP]; // fused into the read, src/bfv.rs:819-820); null means identity
+};
+
 /// One digit of the dBFV reduction (launch_dbfv_split): its constants, in device memory.
 struct DbfvSplit {
     const int64_t* rqinv;    // [r] Montgomery factors of the lifts

@@ -33,7 +33,7 @@ hc_status launch_dbfv_tensor(hc_context ctx, const KView& d, const KView& lhs, c
 hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const uint32_t* p2, const uint32_t* p3);
 hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys, int nterms, const KView* add0,
                            const KView* add1, int full0, int full1, const KView& dst, const KMods& m,
-                           const int64_t* one_dev, const uint32_t* p2, const uint32_t* p3, bool reverse = false);
+                           const int64_t* one_dev, const KsGroup& group, bool reverse = false);
 hc_status launch_tensor(hc_context ctx, const KView& d, const KView& lhs_lo, const KView& lhs_hi, const KView& rhs_lo,
                         const KView& rhs_hi, int rsplit, const KMods& m, int f0,
                         int f1, int f2);
@@ -1321,10 +1321,16 @@ void check_keys(hc_ring R, const hc_view& keys, int64_t r, size_t nd) {
 
 /// acc[0..2] = sum_t parts[t] * key_t (+ summands through mont(1)), reduced (fused), for B
 /// ciphertexts at once: parts [B d, r] (row i d + t), summand views with one row per ciphertext,
-/// out [2B, r] (rows 2i, 2i + 1).
+/// out [2B, r] (rows 2i, 2i + 1). With `more` the same digits and summands under more keys in the launch (key
+/// and output of equal strides, their own permutation).
+struct MoreKeys {
+    hc_view key, out;
+    const uint32_t *p2, *p3;
+};
 void keyswitch(hc_ring R, const hc_view& parts, const hc_view& keys, const Base& base, size_t nd,
                const hc_view* add0, const hc_view* add1, const hc_view& out, const uint32_t* p2 = nullptr,
-               const uint32_t* p3 = nullptr, bool reverse = false) {
+               const uint32_t* p3 = nullptr, bool reverse = false,
+               const std::vector<MoreKeys>& more = {}) {
     const int64_t r = (int64_t)base.size(), B = out.shape[0] / 2;
     check_keys(R, keys, r, nd);
     REQUIRE(parts.shape[0] == B * (int64_t)nd, HC_ERR_SHAPE, "gadget digits per ciphertext");
@@ -1339,10 +1345,18 @@ void keyswitch(hc_ring R, const hc_view& parts, const hc_view& keys, const Base&
         step += mp * mp;
     }
     u128 b0 = step + (add0 ? mp * mp : 0), b1 = step + (add1 ? mp * mp : 0);
+    KsGroup group{};
+    auto member = [&](const hc_view& key, const hc_view& o, const uint32_t* q2, const uint32_t* q3) {
+        group.off[group.n] = (const int64_t*)key.ptr - (const int64_t*)keys.ptr;
+        group.dst[group.n] = (int64_t*)o.ptr;
+        group.p2[group.n] = q2, group.p3[group.n++] = q3;
+    };
+    member(keys, out, p2, p3);
+    for (auto& k : more) check_keys(R, k.key, r, nd), member(k.key, k.out, k.p2, k.p3);
     KView a0 = add0 ? kv(*add0) : KView(), a1 = add1 ? kv(*add1) : KView();
     int64_t minp = R->min_p(base);
     CK(launch_keyswitch(R->ctx, pv.data(), kvv.data(), (int)nd, add0 ? &a0 : nullptr, add1 ? &a1 : nullptr,
-                        needs_full(b0, minp), needs_full(b1, minp), kv(out), R->kmods(base), R->one_dev(base), p2, p3,
+                        needs_full(b0, minp), needs_full(b1, minp), kv(out), R->kmods(base), R->one_dev(base), group,
                         reverse));
 }
 
@@ -2318,8 +2332,8 @@ struct hc_keyset_s {
     }
     /// Runs fn(i, key view) for the keys of gs in order on the context stream; resident keys are
     /// used in place, streamed keys are staged one ahead.
-    template <typename F>
-    void each(const std::vector<uint64_t>& gs, F fn) {
+    template <typename F, typename B>
+    void each(const std::vector<uint64_t>& gs, F fn, B before_streamed) {
         cudaStream_t st = stream_of(R->ctx);
         std::vector<const Entry*> es;
         for (uint64_t g : gs) {
@@ -2342,14 +2356,15 @@ struct hc_keyset_s {
             hc_view kv;
             if (es[i]->host) {
                 const int s = slot_of[i];
+                before_streamed();
                 CK(cuda_check(cudaStreamWaitEvent(st, ready[s], 0), "keyset ready wait"));
                 issue_next(i + 1);  // overlaps the key switch of key i
                 kv = view_of(slot[s].p);
-                fn(i, kv);
+                fn(i, kv, false);
                 CK(cuda_check(cudaEventRecord(freed[s], st), "keyset slot event"));
             } else {
                 kv = view_of(es[i]->dev.p);
-                fn(i, kv);
+                fn(i, kv, true);
             }
         }
     }
@@ -2360,7 +2375,8 @@ namespace {
 /// bfv_hom_gal (src/bfv.rs:783-841) with the keys of a keyset and one output view per automorphism.
 /// bfv_hom_gal (src/bfv.rs:783-841) of B ciphertexts at once (ct [2B, r], rows 2i, 2i + 1; each
 /// out [2B, r]) under the automorphisms gs with keys from a keyset: one gadget decomposition of all
-/// B ciphertexts, hoisted over gs, and one key-switch launch per automorphism for the whole batch.
+/// B ciphertexts, hoisted over gs, and one key-switch launch per KS_GROUP resident keys (or one streamed
+/// key) for the whole batch.
 void hom_gal_keyset(hc_ring R, const hc_view& ct, const Base& b, const std::vector<uint64_t>& gs, hc_keyset ks,
                     const std::vector<hc_view>& outs) {
     if (gs.empty()) return;
@@ -2376,13 +2392,29 @@ void hom_gal_keyset(hc_ring R, const hc_view& ct, const Base& b, const std::vect
     R->transform(c1.view(), b, true, nullptr, &c1_crt);
     Tensor parts = gadget_decompose(R, c1.view(), b, dg);
     hc_view c0 = vstep(ct, 0, 2, B);
-    // consecutive key switches over the same digits alternate their tile order (KsArgs::reverse)
+    // keys resident in HBM go KS_GROUP to a launch, factor by factor, so that a factor's digits stay in L2
+    // for all of them; a streamed key goes alone, as its slot is given back. Consecutive launches over
+    // the same digits alternate their tile order (KsArgs::reverse).
     size_t launched = 0;
-    ks->each(gs, [&](size_t gi, const hc_view& key) {
+    std::vector<MoreKeys> group;
+    auto flush = [&] {
+        if (group.empty()) return;
+        const MoreKeys first = group.front();
+        group.erase(group.begin());
+        keyswitch(R, parts.view(), first.key, b, dg.size(), &c0, nullptr, first.out, first.p2, first.p3,
+                  (launched++ & 1) != 0, group);
+        group.clear();
+    };
+    auto same_strides = [](const hc_view& x, const hc_view& y) { return std::equal(x.strides, x.strides + 4, y.strides); };
+    ks->each(gs, [&](size_t gi, const hc_view& key, bool resident) {
         PermCache& pc = R->perms(gs[gi]);
-        keyswitch(R, parts.view(), key, b, dg.size(), &c0, nullptr, outs[gi], pc.p2.as<uint32_t>(), pc.p3.as<uint32_t>(),
-                  (launched++ & 1) != 0);
-    });
+        if (group.size() == KS_GROUP ||
+            (!group.empty() && !(same_strides(group[0].key, key) && same_strides(group[0].out, outs[gi]))))
+            flush();
+        group.push_back({key, outs[gi], pc.p2.as<uint32_t>(), pc.p3.as<uint32_t>()});
+        if (!resident) flush();
+    }, flush);  // what is waiting runs beside the streamed key's copy
+    flush();
 }
 
 /// src/dbfv.rs:97-121

@@ -317,11 +317,8 @@ struct KsArgs {
     KView add0, add1;  // optional (has_add*) CRT-basis summands of rows 0 / 1, multiplied by mont(1)
     int has_add0, has_add1;
     int full0, full1;  // rows needing the full double reduction
-    KView dst;         // [2B, r, dl, dk]
-    // optional Galois permutation applied to parts and summands (apply_galois fused into the
-    // read, src/bfv.rs:819-820); null means identity
-    const uint32_t* p2;
-    const uint32_t* p3;
+    KView dst;         // [2B, r, dl, dk], its pointer group.dst
+    KsGroup group;
     // tiles in reverse order: a launch that follows one over the same parts and summands starts
     // on the tiles that launch read last, which are still in L2
     int reverse;
@@ -365,7 +362,7 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
         if (l >= a.dst.n3) continue;
         int64_t k = line % a.dst.n2, r = line / a.dst.n2;
         int64_t j = r % a.dst.n1, i = r / a.dst.n1;
-        const int64_t sk = a.p2 ? (int64_t)a.p2[k] : k, sl = a.p3 ? (int64_t)a.p3[l] : l;
+        const int64_t sk = a.group.p2[0] ? (int64_t)a.group.p2[0][k] : k, sl = a.group.p3[0] ? (int64_t)a.group.p3[0][l] : l;
         KsAcc<2> acc;
         acc.start();
         for (int t = 0; t < a.nterms; t++) {
@@ -393,6 +390,9 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
 /// (no barrier). Tiles run as ((j, k), chunk, i) with the ciphertext index innermost: the B tiles
 /// that read one block of the key are adjacent, so the key comes from DRAM once and B - 1 reads
 /// hit L2.
+/// A launch takes up to KS_GROUP keys over the same digits (a keyset's automorphisms), factor by factor, so
+/// that a factor's digits (7 MB for three field_49152 ciphertexts of six) come from DRAM once for all of them: the
+/// homomorphic CRT step at r = 23 (12 keys) 4979 -> 4892 us, at r = 12 with 40 coefficients 636 -> 604.
 /// COMMON: every term's digit view shares the strides of parts[0] and every key view those of
 /// keys[0] (the layouts the ring layer passes), so each thread forms its offsets once and a term's
 /// addresses are one addition each.
@@ -406,21 +406,25 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
     __shared__ int64_t sx[KS_STAGES][2][256];
     __shared__ longlong2 skey[KS_STAGES][2][256];
     const int tid = threadIdx.x;
-    const int64_t tiles = lines * chunks;
-    for (int64_t t0 = blockIdx.x; t0 < tiles; t0 += gridDim.x) {
-        const int64_t tile = a.reverse ? tiles - 1 - t0 : t0;
-        const int64_t i = tile % a.batch, u = tile / a.batch;
-        const int64_t line = u / chunks;  // (j, k)
-        const int64_t l = 2 * ((u - line * chunks) * blockDim.x + tid);
+    const uint32_t tiles = (uint32_t)lines * (uint32_t)chunks * (uint32_t)a.group.n;
+    const uint32_t per = (uint32_t)a.batch * (uint32_t)a.dst.n2 * (uint32_t)chunks;  // tiles of one factor under one key
+    for (uint32_t t0 = blockIdx.x; t0 < tiles; t0 += gridDim.x) {
+        const uint32_t tile = a.reverse ? tiles - 1 - t0 : t0;
+        const uint32_t j = tile / (per * (uint32_t)a.group.n), e = tile - j * per * (uint32_t)a.group.n;
+        const uint32_t key = e / per, w = e - key * per;
+        const uint32_t u = w / (uint32_t)a.batch, i = w - u * (uint32_t)a.batch;
+        const uint32_t k = u / (uint32_t)chunks;
+        const int64_t l = 2 * (int64_t)((u - k * (uint32_t)chunks) * blockDim.x + tid);
         if (l >= a.dst.n3) continue;
-        const int64_t k = line % a.dst.n2, j = line / a.dst.n2;
-        const int64_t sk = a.p2 ? (int64_t)a.p2[k] : k;
-        const int64_t sl0 = a.p3 ? (int64_t)a.p3[l] : l, sl1 = a.p3 ? (int64_t)a.p3[l + 1] : l + 1;
+        const uint32_t* p2 = a.group.p2[key];
+        const uint32_t* p3 = a.group.p3[key];
+        const int64_t sk = p2 ? (int64_t)p2[k] : k;
+        const int64_t sl0 = p3 ? (int64_t)p3[l] : l, sl1 = p3 ? (int64_t)p3[l + 1] : l + 1;
         // COMMON offsets (in words) of this thread's digit words and key pairs within every term
         const KView& P = a.parts[0];
         const KView& K = a.keys[0];
         const int64_t po = i * P.s0 + j * P.s1 + sk * P.s2, po0 = po + (P.b3 ? 0 : sl0), po1 = po + (P.b3 ? 0 : sl1);
-        const int64_t ko0 = j * K.s1 + k * K.s2 + l, ko1 = ko0 + K.s0;
+        const int64_t ko0 = j * K.s1 + k * K.s2 + l + a.group.off[key], ko1 = ko0 + K.s0;
         auto issue = [&](int t) {
             if (t < a.nterms) {
                 const int s = t % KS_STAGES;
@@ -434,8 +438,8 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
                 } else {
                     cp_async8(&sx[s][0][tid], kat<int64_t>(a.parts[t], i, j, sk, sl0));
                     cp_async8(&sx[s][1][tid], kat<int64_t>(a.parts[t], i, j, sk, sl1));
-                    cp_async16(&skey[s][0][tid], kat<int64_t>(a.keys[t], 0, j, k, l));
-                    cp_async16(&skey[s][1][tid], kat<int64_t>(a.keys[t], 1, j, k, l));
+                    cp_async16(&skey[s][0][tid], kat<int64_t>(a.keys[t], 0, j, k, l) + a.group.off[key]);
+                    cp_async16(&skey[s][1][tid], kat<int64_t>(a.keys[t], 1, j, k, l) + a.group.off[key]);
                 }
             }
             cp_async_commit();  // an empty group past the end keeps the count uniform
@@ -455,14 +459,14 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
             if (FOLD && (t + 1) % (LIMB_TERMS2 - 1) == 0) acc0.fold(), acc1.fold();
         }
         cp_async_wait<0>();
-        const int64_t o = one[j];
+        const int64_t mone = one[j];
         if (a.has_add0) {
-            acc0.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl0), o);
-            acc1.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl1), o);
+            acc0.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl0), mone);
+            acc1.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl1), mone);
         }
         if (a.has_add1) {
-            acc0.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl0), o);
-            acc1.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl1), o);
+            acc0.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl0), mone);
+            acc1.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl1), mone);
         }
         acc0.fold(), acc1.fold();
         const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
@@ -470,8 +474,9 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
         longlong2 w0, w1;
         w0.x = finish_wide(acc0.lo[0], acc0.hi[0], a.full0, ml, r2), w0.y = finish_wide(acc1.lo[0], acc1.hi[0], a.full0, ml, r2);
         w1.x = finish_wide(acc0.lo[1], acc0.hi[1], a.full1, ml, r2), w1.y = finish_wide(acc1.lo[1], acc1.hi[1], a.full1, ml, r2);
-        *reinterpret_cast<longlong2*>(kat<int64_t>(a.dst, 2 * i, j, k, l)) = w0;
-        *reinterpret_cast<longlong2*>(kat<int64_t>(a.dst, 2 * i + 1, j, k, l)) = w1;
+        int64_t* o = a.group.dst[key] + 2 * i * a.dst.s0 + j * a.dst.s1 + k * a.dst.s2 + l;
+        *reinterpret_cast<longlong2*>(o) = w0;
+        *reinterpret_cast<longlong2*>(o + a.dst.s0) = w1;
     }
 }
 
@@ -936,7 +941,7 @@ hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const ui
 
 hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys, int nterms, const KView* add0,
                            const KView* add1, int full0, int full1, const KView& dst, const KMods& m,
-                           const int64_t* one_dev, const uint32_t* p2, const uint32_t* p3, bool reverse) {
+                           const int64_t* one_dev, const KsGroup& group, bool reverse) {
     if (nterms > HC_MAX_TERMS) return fail(HC_ERR_UNSUPPORTED, "too many gadget digits");
     KsArgs a;
     a.reverse = reverse;
@@ -948,7 +953,7 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
     if (add1) a.add1 = *add1;
     a.full0 = full0, a.full1 = full1;
     a.dst = dst;
-    a.p2 = p2, a.p3 = p3;
+    a.group = group;
     a.batch = dst.n0 / 2;
     int64_t lines = a.batch * dst.n1 * dst.n2;
     if (lines == 0 || dst.n3 == 0) return HC_OK;
@@ -957,16 +962,25 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
         return ((uintptr_t)v.p % 16) == 0 && v.s0 % 2 == 0 && v.s1 % 2 == 0 && v.s2 % 2 == 0 && !v.b3;
     };
     bool pair = dst.n3 % 2 == 0 && aligned(dst);
+    for (int g = 0; g < group.n; g++) pair = pair && ((uintptr_t)group.dst[g] % 16) == 0 && group.off[g] % 2 == 0;
     for (int t = 0; t < nterms; t++) pair = pair && aligned(keys[t]);
     int chunks;
     unsigned blocks;
     if (!pair) {
         grid_lines(ctx, dst.n3, lines, &chunks, &blocks);
-        hc::launch_kernel(keyswitch1_kernel, blocks, 256, 0, stream_of(ctx), a, m, one_dev, lines, chunks);
-        count_launch(ctx);
-        return cuda_check(cudaGetLastError(), "keyswitch kernel launch");
+        for (int g = 0; g < group.n; g++) {
+            a.dst.p = (char*)group.dst[g];
+            a.group.p2[0] = group.p2[g], a.group.p3[0] = group.p3[g];
+            for (int t = 0; t < nterms; t++) a.keys[t].p = keys[t].p + 8 * group.off[g];
+            hc::launch_kernel(keyswitch1_kernel, blocks, 256, 0, stream_of(ctx), a, m, one_dev, lines, chunks);
+            count_launch(ctx);
+            hc_status st = cuda_check(cudaGetLastError(), "keyswitch kernel launch");
+            if (st) return st;
+        }
+        return HC_OK;
     }
-    grid_lines(ctx, dst.n3 / 2, lines, &chunks, &blocks);
+    grid_lines(ctx, dst.n3 / 2, lines * group.n, &chunks, &blocks);
+    if (lines * chunks * group.n > INT32_MAX) return fail(HC_ERR_UNSUPPORTED, "key switch: too many positions");
     bool common = true;
     for (int t = 1; t < nterms; t++) {
         const KView &p = parts[t], &p0 = parts[0], &k = keys[t], &k0 = keys[0];

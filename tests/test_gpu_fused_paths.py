@@ -309,3 +309,30 @@ def test_gadget_matrix_as_parameter(rings, r, nd):
     d.bconv_gadget(got, d.tensor(x), base, digits)
     exp = np.concatenate([o.bconv_gadget(x[i:i + 1], base, digits) for i in range(2)])  # the oracle takes one element
     assert got.shape == exp.shape and (got.to_numpy() == exp).all()
+
+
+@pytest.mark.parametrize("ring", [("field_18", 300, 320, 4), ("field_2", 300, 320, 4), ("field_36864", 200, 230, 2)], ids=lambda v: v[0])
+@pytest.mark.parametrize("n,budget", [(1, 100), (15, 100), (16, 100), (17, 100), (33, 100), (18, 0), (18, 3)])
+def test_key_switches_of_a_keyset(po, rings, ring, n, budget):
+    """Resident keys go 16 to a launch, streamed ones alone, in the automorphisms' order."""
+    import ringcuda
+
+    o, d = rings(*ring)
+    if n > 18 and o.n > 1000:
+        n = 18
+    base = o.initial_base()
+    m = o.info["m"]
+    gen = list(o.info["gens"])[0]
+    gs = [pow(gen, 1 + j % 5, m) for j in range(n)]
+    digits = [tuple(v) for v in ringcuda.select_digits(min(2, len(base)), len(base))]
+    primes = [o.primes[i] for i in base]
+    g = np.random.default_rng(n)
+    keys = {e: residues(g, o.shape(2 * len(digits), o.initial_len), o.primes[: o.initial_len]) for e in set(gs)}
+    ks = ringcuda.Keyset(d, digits, o.initial_len, budget * next(iter(keys.values())).nbytes)
+    for e in sorted(keys):
+        ks.add(e, d.tensor(keys[e]))
+    ct = residues(g, o.shape(2, len(base)), primes, edges=True)
+    got = ringcuda.hom_gal_keyset(d, d.tensor(ct), base, gs, ks).to_numpy()
+    stacked = np.stack([keys[e].reshape((len(digits), 2) + keys[e].shape[1:]) for e in gs])
+    exp = o.hom_gal(ct, base, gs, stacked, digits)
+    assert (got == exp.reshape(got.shape)).all()
