@@ -754,10 +754,13 @@ __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs
 /// What bounds it: memory and the multiply pipe about equally (a step reads every baby row once); the
 /// unit list, masks and single-word copies of giant_kernel kept it issue-bound: 237 us per giant step of
 /// 13 baby steps and three digits at field_49152 r = 23, here 159 us.
-constexpr int TRI_STAGES = 3;
+/// One output digit has few sums, so four CTAs per SM and four stages keep more reads in flight: a step at r = 12
+/// with 40 one-digit coefficients 601 -> 580 us; with more digits four CTAs spill (5138 us against 4896 at three digits)
+/// and two are 1 % slower.
+constexpr int TRI_STAGES = 4;
 
 template <int NOUT>
-__global__ void __launch_bounds__(256, NOUT == 4 ? 2 : 3)
+__global__ void __launch_bounds__(256, NOUT == 4 ? 2 : NOUT >= 2 ? 3 : 4)
     giant_tri_kernel(GiantArgs a, KMods m, const int64_t* one, int n0, int64_t lines, int chunks) {
     grid_wait();
     extern __shared__ __align__(16) int64_t gsm[];  // [TRI_STAGES][NOUT][256] position pairs, then the lcoef limb pairs
