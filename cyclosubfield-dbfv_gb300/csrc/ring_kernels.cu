@@ -342,9 +342,11 @@ struct KsAcc {
             s[q].mac(v, v.x + v.y, w, w.x + w.y);
         }
     }
-    __device__ __forceinline__ void add1(int q, int64_t x, int64_t y) {
-        const int2 v = limb_split(x), w = limb_split(y);
-        s[q].mac(v, v.x + v.y, w, w.x + w.y);
+    /// A summand's product, after the fold: in 128 bits, as c0 and c1 are the caller's and may be lazy sums of any
+    /// size, while the limbs hold words up to 2^60 only. Once per output word; it costs what the limb product did.
+    __device__ __forceinline__ void add_wide(int q, int64_t x, int64_t y) {
+        const u128 v = (((u128)(uint64_t)hi[q] << 64) | lo[q]) + (u128)((i128)x * (i128)y);
+        lo[q] = (uint64_t)v, hi[q] = (int64_t)(v >> 64);
     }
     __device__ __forceinline__ void fold() {
 #pragma unroll
@@ -371,10 +373,10 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
             acc.add(x, y);
             if ((t + 1) % (LIMB_TERMS2 - 1) == 0) acc.fold();
         }
-        const int64_t o = one[j];
-        if (a.has_add0) acc.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl), o);
-        if (a.has_add1) acc.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl), o);
         acc.fold();
+        const int64_t o = one[j];
+        if (a.has_add0) acc.add_wide(0, *kat<int64_t>(a.add0, i, j, sk, sl), o);
+        if (a.has_add1) acc.add_wide(1, *kat<int64_t>(a.add1, i, j, sk, sl), o);
         const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
         *kat<int64_t>(a.dst, 2 * i, j, k, l) = finish_wide(acc.lo[0], acc.hi[0], a.full0, ml, m.r2[j]);
         *kat<int64_t>(a.dst, 2 * i + 1, j, k, l) = finish_wide(acc.lo[1], acc.hi[1], a.full1, ml, m.r2[j]);
@@ -460,15 +462,12 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
         }
         cp_async_wait<0>();
         const int64_t mone = one[j];
-        if (a.has_add0) {
-            acc0.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl0), mone);
-            acc1.add1(0, *kat<int64_t>(a.add0, i, j, sk, sl1), mone);
-        }
-        if (a.has_add1) {
-            acc0.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl0), mone);
-            acc1.add1(1, *kat<int64_t>(a.add1, i, j, sk, sl1), mone);
-        }
+        int64_t c0[2] = {0, 0}, c1[2] = {0, 0};  // the summands of the two positions, in flight during the fold
+        if (a.has_add0) c0[0] = *kat<int64_t>(a.add0, i, j, sk, sl0), c0[1] = *kat<int64_t>(a.add0, i, j, sk, sl1);
+        if (a.has_add1) c1[0] = *kat<int64_t>(a.add1, i, j, sk, sl0), c1[1] = *kat<int64_t>(a.add1, i, j, sk, sl1);
         acc0.fold(), acc1.fold();
+        if (a.has_add0) acc0.add_wide(0, c0[0], mone), acc1.add_wide(0, c0[1], mone);
+        if (a.has_add1) acc0.add_wide(1, c1[0], mone), acc1.add_wide(1, c1[1], mone);
         const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);
         const int64_t r2 = m.r2[j];
         longlong2 w0, w1;
@@ -990,7 +989,7 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
         common = common && p.s0 == p0.s0 && p.s1 == p0.s1 && p.s2 == p0.s2 && p.b3 == p0.b3 && k.s0 == k0.s0 &&
                  k.s1 == k0.s1 && k.s2 == k0.s2;
     }
-    const bool fold = nterms >= LIMB_TERMS2;  // with the summand more than LIMB_TERMS2 terms
+    const bool fold = nterms >= LIMB_TERMS2;  // the sums fold every LIMB_TERMS2 - 1 digits
     auto kern = common ? (fold ? keyswitch_async_kernel<true, true> : keyswitch_async_kernel<true, false>)
                        : (fold ? keyswitch_async_kernel<false, true> : keyswitch_async_kernel<false, false>);
     hc::launch_kernel(kern, blocks, 256, 0, stream_of(ctx), a, m, one_dev, lines, chunks);

@@ -17,6 +17,10 @@
  * (low, high) int64 words. Random numbers come from the reference's splitmix64 generator
  * (src/bfv.rs:880-886) whose 64-bit state the caller owns and which the call advances.
  *
+ * Words: the result of every call is almost reduced (|x| <= p). Transforms and what runs them on its
+ * inputs take |x| <= 2p. The summand c0 of the key switches and rotations may be any word, a lazy sum of
+ * many elements included.
+ *
  * Threads and streams: a ring (its table caches and its side streams) is used from one host thread
  * at a time; calls are asynchronous on the context's current stream (hc_context_set_stream), and
  * calls issued on different streams of one context may run concurrently on the GPU. Some calls

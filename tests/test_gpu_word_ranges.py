@@ -1,0 +1,79 @@
+"""Words beyond the bounds that almost reduced elements have, where a call forms one exact product or conversion of
+each: lazily summed key-switch summands, unreduced keys, base-conversion sources up to the whole word, operands of the
+batched product and multipliers of the HAL transforms. Bit-exact against the oracle, which forms every product in 128
+bits; the sums themselves stay exact integers, so every tolerance is zero."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+WORD = (1 << 63) - 1
+# rings of primes just below 2^57: an element's bound of 64 p is the whole word
+RINGS = [("field_192", 2300, 2340, 4), ("field_18", 560, 572, 4), ("field_2", 220, 229, 4), ("field_36864", 200, 230, 2)]
+
+
+@pytest.fixture(scope="module")
+def rings(po, be):
+    import ringcuda
+
+    cache = {}
+
+    def get(*key):
+        if key not in cache:
+            cache[key] = (po.Ring(*key), ringcuda.RingContext(*key, backend=be))
+        return cache[key]
+
+    return get
+
+
+def words(g, shape, primes, bound):
+    """[count, r, ...] words within +-bound p, half of them at the bound or next to it."""
+    out = np.empty(shape, dtype=np.int64)
+    for j in range(shape[1]):
+        m = min(bound * primes[j], WORD)
+        out[:, j] = g.integers(-m, m, size=out[:, j].shape, endpoint=True)
+        v = g.choice(np.array([m, -m, m - 1, 1 - m]), size=out[:, j].shape)
+        out[:, j] = np.where(g.integers(0, 2, size=v.shape) == 1, v, out[:, j])
+    return out
+
+
+def key_switch_forms(rings, ring, seed, c0_bound, key_bound):
+    """Every form of the key switch: single, several automorphisms, a batch, a keyset, and a batch into rows of odd
+    stride (the kernel without 16-byte accesses)."""
+    import ringcuda
+
+    o, d = rings(*ring)
+    base = o.initial_base()
+    primes = [o.primes[i] for i in base]
+    digits = [tuple(v) for v in ringcuda.select_digits(min(3, len(base)), len(base))]
+    nd = len(digits)
+    g = np.random.default_rng(seed)
+    gen, m = list(o.info["gens"])[0], o.info["m"]
+    gs = [gen, pow(gen, 2, m)]
+    keys = [words(g, o.shape(2 * nd, len(base)), primes, key_bound) for _ in gs]
+    split = [k.reshape((nd, 2) + k.shape[1:]) for k in keys]
+    cts = words(g, o.shape(6, len(base)), primes, 1)
+    cts[0::2] = words(g, o.shape(3, len(base)), primes, c0_bound)
+    ct = np.ascontiguousarray(cts[:2])
+    dk = [d.tensor(k) for k in keys]
+    got = d.key_switch(d.tensor(ct[:1]), d.tensor(ct[1:]), base, dk[0], digits)
+    assert (got.to_numpy() == o.key_switch(ct[:1], ct[1:], base, split[0], digits)).all()
+    exp = o.hom_gal(ct, base, gs, np.stack(split), digits).reshape(o.shape(4, len(base)))
+    got = d.hom_gal(d.tensor(ct), base, gs, d.tensor(np.concatenate(keys)), digits)
+    assert (got.to_numpy() == exp).all()
+    ks = ringcuda.Keyset(d, digits, len(base), 1 << 40)
+    for e, k in zip(gs, dk):
+        ks.add(e, k)
+    assert (ringcuda.hom_gal_keyset(d, d.tensor(ct), base, gs, ks).to_numpy() == exp).all()
+    exp = np.concatenate([o.hom_gal(cts[2 * i:2 * i + 2], base, gs[:1], split[0][None], digits)[0] for i in range(3)])
+    assert (d.hom_gal_batch(d.tensor(cts), base, gs[0], dk[0], digits).to_numpy() == exp).all()
+    wide = d.backend.hal_allocate_i64(exp.shape[:3] + (exp.shape[3] + 1,))
+    out = wide.slice(None, None, None, (1, exp.shape[3] + 1))
+    assert (d.hom_gal_batch(d.tensor(cts), base, gs[0], dk[0], digits, out=out).to_numpy() == exp).all()
+
+
+@pytest.mark.parametrize("ring", RINGS, ids=lambda v: v[0])
+@pytest.mark.parametrize("bound", [6, 7, 63, 64])
+def test_key_switch_of_a_lazy_sum(rings, ring, bound):
+    """c0 as a lazy sum of up to 64 elements (csrc/ring_kernels.cu: KsAcc::add_wide)."""
+    key_switch_forms(rings, ring, bound, bound, 1)
