@@ -324,6 +324,17 @@ struct KsArgs {
     int reverse;
 };
 
+/// Whether keys' words went beyond the range of the limb sums, |y| <= 2^58 (LIMB_TERMS2): the caller's keys may be
+/// unreduced. Three instructions for two words beside the 36 multiply-adds and splits of a digit; a thread
+/// that met such a word sums its positions again in 128 bits.
+struct KeyRange {
+    uint32_t seen = 0;
+    __device__ __forceinline__ void see(int64_t y0, int64_t y1) {
+        seen |= (hi32(y0) + (1u << 26)) | (hi32(y1) + (1u << 26));
+    }
+    __device__ __forceinline__ bool beyond() const { return (seen >> 27) != 0; }
+};
+
 /// R accumulators of one position: one digit word times R key words per step.
 template <int R>
 struct KsAcc {
@@ -366,14 +377,23 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
         int64_t j = r % a.dst.n1, i = r / a.dst.n1;
         const int64_t sk = a.group.p2[0] ? (int64_t)a.group.p2[0][k] : k, sl = a.group.p3[0] ? (int64_t)a.group.p3[0][l] : l;
         KsAcc<2> acc;
+        KeyRange range;
         acc.start();
         for (int t = 0; t < a.nterms; t++) {
             const int64_t x = *kat<int64_t>(a.parts[t], i, j, sk, sl);
             const int64_t y[2] = {*kat<int64_t>(a.keys[t], 0, j, k, l), *kat<int64_t>(a.keys[t], 1, j, k, l)};
+            range.see(y[0], y[1]);
             acc.add(x, y);
             if ((t + 1) % (LIMB_TERMS2 - 1) == 0) acc.fold();
         }
         acc.fold();
+        if (range.beyond()) {
+            acc.start();
+            for (int t = 0; t < a.nterms; t++) {
+                const int64_t x = *kat<int64_t>(a.parts[t], i, j, sk, sl);
+                for (int q = 0; q < 2; q++) acc.add_wide(q, x, *kat<int64_t>(a.keys[t], q, j, k, l));
+            }
+        }
         const int64_t o = one[j];
         if (a.has_add0) acc.add_wide(0, *kat<int64_t>(a.add0, i, j, sk, sl), o);
         if (a.has_add1) acc.add_wide(1, *kat<int64_t>(a.add1, i, j, sk, sl), o);
@@ -449,6 +469,7 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
 #pragma unroll
         for (int t = 0; t < KS_STAGES - 1; t++) issue(t);
         KsAcc<2> acc0, acc1;  // rows 0, 1 of the two positions
+        KeyRange range;
         acc0.start(), acc1.start();
         for (int t = 0; t < a.nterms; t++) {
             issue(t + KS_STAGES - 1);
@@ -456,6 +477,7 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
             const int s = t % KS_STAGES;
             const longlong2 k0 = skey[s][0][tid], k1 = skey[s][1][tid];
             const int64_t y0[2] = {k0.x, k1.x}, y1[2] = {k0.y, k1.y};
+            range.see(k0.x, k0.y), range.see(k1.x, k1.y);
             acc0.add(sx[s][0][tid], y0);
             acc1.add(sx[s][1][tid], y1);
             if (FOLD && (t + 1) % (LIMB_TERMS2 - 1) == 0) acc0.fold(), acc1.fold();
@@ -466,6 +488,16 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
         if (a.has_add0) c0[0] = *kat<int64_t>(a.add0, i, j, sk, sl0), c0[1] = *kat<int64_t>(a.add0, i, j, sk, sl1);
         if (a.has_add1) c1[0] = *kat<int64_t>(a.add1, i, j, sk, sl0), c1[1] = *kat<int64_t>(a.add1, i, j, sk, sl1);
         acc0.fold(), acc1.fold();
+        if (range.beyond()) {
+            acc0.start(), acc1.start();
+            for (int t = 0; t < a.nterms; t++) {
+                const int64_t x0 = *kat<int64_t>(a.parts[t], i, j, sk, sl0), x1 = *kat<int64_t>(a.parts[t], i, j, sk, sl1);
+                for (int q = 0; q < 2; q++) {
+                    const int64_t* y = kat<int64_t>(a.keys[t], q, j, k, l) + a.group.off[key];
+                    acc0.add_wide(q, x0, y[0]), acc1.add_wide(q, x1, y[1]);
+                }
+            }
+        }
         if (a.has_add0) acc0.add_wide(0, c0[0], mone), acc1.add_wide(0, c0[1], mone);
         if (a.has_add1) acc0.add_wide(1, c1[0], mone), acc1.add_wide(1, c1[1], mone);
         const MontLimbs ml = mont_limbs(m.n[j], m.ninv[j]);

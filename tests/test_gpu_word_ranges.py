@@ -77,3 +77,10 @@ def key_switch_forms(rings, ring, seed, c0_bound, key_bound):
 def test_key_switch_of_a_lazy_sum(rings, ring, bound):
     """c0 as a lazy sum of up to 64 elements (csrc/ring_kernels.cu: KsAcc::add_wide)."""
     key_switch_forms(rings, ring, bound, bound, 1)
+
+
+@pytest.mark.parametrize("ring", RINGS, ids=lambda v: v[0])
+@pytest.mark.parametrize("bound", [2, 3, 7, 63, 64])
+def test_key_switch_with_unreduced_keys(rings, ring, bound):
+    """Keys beyond the range of the limb sums (|word| <= 2^58, twice a factor)."""
+    key_switch_forms(rings, ring, bound, 2, bound)
