@@ -366,6 +366,12 @@ inline BarrettLimbs mont_const_limbs(int64_t b, int64_t n, int64_t ninv) {
     w.e1 = bal_hi(b);
     return w;
 }
+/// Whether |x| stays within the range of the limb products' variable operand, 0.9 x 2^63.
+__device__ __forceinline__ bool limb_range(int64_t x) { return hi32(x) + 0x73000000u < 0xe6000000u; }
+/// The constant b of mont_const_limbs: u = b ninv and n ninv = -1, both modulo 2^64.
+__device__ __forceinline__ int64_t mont_const_value(const BarrettLimbs& w, int64_t n) {
+    return (int64_t)(0 - (((uint64_t)(uint32_t)w.u1 << 32) + (uint64_t)(int64_t)w.u0) * (uint64_t)n);
+}
 __device__ __forceinline__ BarrettLimbs load_limbs(const BarrettLimbs* p) {
     const int4 a = __ldg(reinterpret_cast<const int4*>(p));
     return BarrettLimbs{a.x, a.y, a.z, a.w};

@@ -164,11 +164,21 @@ __global__ void __launch_bounds__(BCONV_THREADS, 5) bconv_fused_kernel(BconvArgs
     const int64_t k = pos / a.src.n3, l = pos - k * a.src.n3;
     const int64_t* srcp = kat<int64_t>(a.src, i, 0, k, l);  // row u at u * src.s1
     int64_t* dstp = kat<int64_t>(a.dst, i * a.nb + b, 0, k, l);          // row j at j * dst.s1
-    // the source is multiplied by (Q/p)^-1 in Montgomery form, giving plain lifts in (-p, p)
+    // the source is multiplied by (Q/p)^-1 in Montgomery form, giving plain lifts in (-p, p); the source's words are
+    // the caller's, and those beyond the limb product's range (64 p of a prime just below 2^57 is the whole
+    // word) are lifted by the general product, in a second pass over the columns of a thread that met one
+    bool beyond = false;
     for (int u = u0; u < u1; u++) {
-        const int64_t x = barrett_mul(load_limbs(a.c.qinv + u), srcp[u * a.src.s1], mont_const_mod(sm.n[u]));
-        xs[u * BCONV_THREADS + threadIdx.x] = limb_split(x);
+        const int64_t w = srcp[u * a.src.s1];
+        beyond = beyond || !limb_range(w);
+        xs[u * BCONV_THREADS + threadIdx.x] = limb_split(barrett_mul(load_limbs(a.c.qinv + u), w, mont_const_mod(sm.n[u])));
     }
+    if (beyond)
+        for (int u = u0; u < u1; u++) {
+            const int64_t w = srcp[u * a.src.s1], n = sm.n[u];
+            if (!limb_range(w))
+                xs[u * BCONV_THREADS + threadIdx.x] = limb_split(mul_mont(w, mont_const_value(load_limbs(a.c.qinv + u), n), n, sm.ninv[u]));
+        }
     const i128 half = (i128)1 << (a.c.shift - 1);
     const int2* xcol = xs + threadIdx.x;  // this thread's lifts, stride BCONV_THREADS
     const int64_t* __restrict__ mq = a.c.mat + ((int64_t)b * (a.rd + 1) + a.rd) * a.r;

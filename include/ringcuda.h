@@ -19,7 +19,7 @@
  *
  * Words: the result of every call is almost reduced (|x| <= p). Transforms and what runs them on its
  * inputs take |x| <= 2p. The summand c0 of the key switches and rotations may be any word, a lazy sum of
- * many elements included, and so may the keys' words.
+ * many elements included, and so may the keys' words and the sources of base conversions and mod_switch_down.
  *
  * Threads and streams: a ring (its table caches and its side streams) is used from one host thread
  * at a time; calls are asynchronous on the context's current stream (hc_context_set_stream), and

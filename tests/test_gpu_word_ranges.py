@@ -84,3 +84,34 @@ def test_key_switch_of_a_lazy_sum(rings, ring, bound):
 def test_key_switch_with_unreduced_keys(rings, ring, bound):
     """Keys beyond the range of the limb sums (|word| <= 2^58, twice a factor)."""
     key_switch_forms(rings, ring, bound, 2, bound)
+
+
+@pytest.mark.parametrize("ring", RINGS, ids=lambda v: v[0])
+def test_base_conversions_of_any_word(rings, ring):
+    """Source words up to the whole word, where the limb product of the lift has no room left: from 0.9 x 2^63 on the
+    general product is taken."""
+    import ringcuda
+
+    o, d = rings(*ring)
+    base = o.initial_base()
+    primes = [o.primes[i] for i in base]
+    r, cut = len(base), (len(base) + 1) // 2
+    g = np.random.default_rng(64)
+    edge = [WORD, -WORD, -WORD - 1, WORD - 1, (1 << 63) - (1 << 31), (1 << 63) - (1 << 31) - 1, (1 << 63) - (1 << 31) + 1]
+    for hi in (0x73000000, 0x72ffffff, 0x73333333, 0x7fffffff):
+        edge += [s * ((hi << 32) + lo) for s in (1, -1) for lo in (-1, 0, 1, 1 << 31, (1 << 32) - 1)]
+    edge = np.array([v for v in edge if -WORD - 1 <= v <= WORD], dtype=np.int64)
+    x = words(g, o.shape(3, r), primes, 64)
+    x[1] = g.choice(edge, size=x[1].shape)
+    x[2, :, :, ::2] = g.choice(edge, size=x[2, :, :, ::2].shape)
+    for src, dst in ((base[:cut], base[cut:] + o.extension_base(base)[:1]), (base[cut:], base[:cut])):
+        y = np.ascontiguousarray(x[:, : len(src)])
+        out = d.allocate(3, len(dst))
+        d.bconv(out, dst, d.tensor(y), src)
+        assert (out.to_numpy() == o.bconv(y, src, dst)).all()
+    digits = [tuple(v) for v in ringcuda.select_digits(min(3, r), r)]
+    out = d.allocate(3 * len(digits), r)
+    d.bconv_gadget(out, d.tensor(x), base, digits)
+    exp = np.concatenate([o.bconv_gadget(x[i:i + 1], base, digits) for i in range(3)])
+    assert (out.to_numpy() == exp).all()
+    assert (d.mod_switch_down(d.tensor(x), base, cut).to_numpy() == o.mod_switch_down(x, base, cut)).all()
