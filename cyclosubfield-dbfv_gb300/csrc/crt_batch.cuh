@@ -12,7 +12,7 @@ __host__ __device__ inline bool crt_slab_12288(int32_t shapes) {
 
 /// Half a transform of a field_49152 slab, as crt_slab.cu's two kernels run it: the lead pass over its
 /// positions, then its twelve blocks one after the other. MODE 6: forward, times the kernels kl [4] and
-/// kk [12288] (limbs); 1: inverse; 3: inverse, times the operand.
+/// kk [12288] (limbs); 1: inverse; 11: inverse, times the operand.
 template <int MODE>
 __device__ __forceinline__ void slab12288_half(const CrtSlab& S, const DevPlanHeader* P2, const DevPlanHeader* P3, int64_t* s,
                                                const int64_t* kl, const int64_t* kk) {
@@ -32,9 +32,9 @@ __device__ __forceinline__ void slab12288_half(const CrtSlab& S, const DevPlanHe
         fast::stage_tail_twiddles<(MODE & 1) != 0>(fast::CtaTeam{}, c3, sch, tws, 1, 63, 7);
         for (int q = 0; q < 12; q++) {
             const int k = q / 3, blk = q - 3 * (q / 3);
-            const int64_t* mulp = MODE == 6   ? fast::block_multiplier<MODE>(kk, 1, blk)
-                                  : MODE == 3 ? S.op + k * S.op_s2 + 4096 * blk
-                                              : nullptr;
+            const int64_t* mulp = MODE == 6    ? fast::block_multiplier<MODE>(kk, 1, blk)
+                                  : MODE == 11 ? S.op + k * S.op_s2 + 4096 * blk
+                                               : nullptr;
             fast::block4096<MODE>(fast::CtaTeam{}, sch, c3, s, tws, S.data + k * S.s2 + 4096 * blk, mulp, 1, mont);
             __syncthreads();  // the tile is refilled by the next block
         }
@@ -49,8 +49,8 @@ __device__ __forceinline__ void slab_lines3072(const CrtSlab& S, const DevPlanHe
     const fast::PartTeam tm{(int)threadIdx.x - 128 * t, (int)blockDim.x / teams, 1 + t};
     int64_t* tile = s + t * LINE3072_WORDS;
     for (int k = t; k < S.dl; k += teams) {
-        run_line3072<MODE, true>(tm, P, tile, S.data + k * S.s2, MODE == 3 ? S.op + k * S.op_s2 : mulrow, 1, S.n, S.ninv,
-                                 k == t);
+        run_line3072<MODE, true>(tm, P, tile, S.data + k * S.s2, MODE == 11 ? S.op + k * S.op_s2 : mulrow, 1, S.n,
+                                 S.ninv, k == t);
         tm.sync();
     }
     __syncthreads();
@@ -69,7 +69,7 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
     const bool fix = (S.shapes >> (dim == 3 ? 16 : 17)) & 1;
     if (fix && dim == 3 && shape == HC_SHAPE_L3072) {
         if (mode == 2) slab_lines3072<6>(S, P, s, mulrow);
-        else if (mode == 3) slab_lines3072<3>(S, P, s, mulrow);
+        else if (mode == 3) slab_lines3072<11>(S, P, s, mulrow);
         else slab_lines3072<1>(S, P, s, mulrow);
         return;
     }
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         auto half = [&](auto mode3, int mode2, const int64_t* kl, const int64_t* kk) {
             constexpr int M = decltype(mode3)::value;
             if (CLS != 1 && slab12288) {
-                slab12288_half<M == 2 ? 6 : M>(S, P2, P3, smem, kl, kk);
+                slab12288_half<M == 2 ? 6 : M == 3 ? 11 : M>(S, P2, P3, smem, kl, kk);
             } else if constexpr (CLS != 2) {
                 slab_pass<GENERIC>(S, P2, tw2, smem, 2, mode2, kl, logv);
                 slab_pass<GENERIC>(S, P3, tw3, smem, 3, M, kk, logv);

@@ -458,6 +458,14 @@ hc_status launch_ntt(hc_context ctx, const KView& t, const hc_ntt_plan* plans, s
         if (plans[j]->shape != shape) shape = HC_SHAPE_GENERIC;
     bool fix = true;
     for (size_t j = 0; j < nplans; j++) fix = fix && plans[j]->fixed;
+    if (mode == 2) {
+        // the limb product of the caller's multipliers wants their moduli below 2^57 (they need not be the plans') and
+        // reads some of them again after its first stores, so they may not lie in t (MontAny)
+        for (size_t j = 0; j < nplans; j++) fix = fix && mods.n[j] < LIMB_MOD_MAX;
+        const int64_t lt = (t.n0 - 1) * t.s0 + (t.n1 - 1) * t.s1 + (t.n2 - 1) * t.s2 + t.n3 - 1;
+        const int64_t lm = (t.n0 - 1) * mul.s0 + (t.n1 - 1) * mul.s1 + (t.n2 - 1) * mul.s2 + (mul.b3 ? 0 : t.n3 - 1);
+        fix = fix && (mul.p > t.p + 8 * lt || t.p > mul.p + 8 * lm);
+    }
     if (dim == 3 && (shape == HC_SHAPE_L3072 || shape == HC_SHAPE_L12288)) {
         const int64_t tiles = t.n0 * t.n1 * t.n2;
         if (tiles <= 0x7fffffff)

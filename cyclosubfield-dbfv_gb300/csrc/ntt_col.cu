@@ -9,7 +9,7 @@ namespace {
 
 /// Specialised dimension-2 NTT: one thread per column (i, j, l), CTAs over (i, j, column block).
 template <int SHAPE, int MODE, bool FIX>
-__global__ void __launch_bounds__(HC_COL_THREADS, SHAPE == HC_SHAPE_C12 ? HC_COL12_MIN_BLOCKS : 4) ntt_col_kernel(KView t, PlanPtrs plans, KView mul, KMods mods,
+__global__ void __launch_bounds__(HC_COL_THREADS, SHAPE == HC_SHAPE_C12 ? HC_COL12_MIN_BLOCKS : MODE == 2 && FIX ? 6 : 4) ntt_col_kernel(KView t, PlanPtrs plans, KView mul, KMods mods,
                                                                     int ncb, KView src) {
     grid_wait();
     // tiles last to first: a transform's column pass follows a line pass (or the input's producer)

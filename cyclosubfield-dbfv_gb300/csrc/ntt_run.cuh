@@ -42,6 +42,32 @@ __device__ __forceinline__ void run_column(const DevPlanHeader* P, int64_t* g, i
     typedef PassCtx<FIX> CTX;
     const CTX c = make_ctx<CTX>(P);
     const auto mont = fast::make_mont<CTX, MODE>(mn, mi);
+    auto store = [&](auto& x) {
+        constexpr int A = sizeof(x) / sizeof(x[0]), B = sizeof(x[0]) / 8;
+        uint32_t seen = 0;
+#pragma unroll
+        for (int a = 0; a < A; a++)
+#pragma unroll
+            for (int b = 0; b < B; b++) {
+                int64_t v = x[a][b];
+                if constexpr ((MODE & 2) != 0) {
+                    const auto w = mont.load(mulp, (B * a + b) * mstride);
+                    if constexpr (MODE == 2 && FIX) mont.see(seen, w);
+                    v = mont.mul(v, w);
+                }
+                g[(B * a + b) * ge] = v;
+            }
+        if constexpr (MODE == 2 && FIX) {
+            if (mont.out(seen)) {
+                int64_t u[A * B];  // in memory, unlike x
+#pragma unroll
+                for (int a = 0; a < A; a++)
+#pragma unroll
+                    for (int b = 0; b < B; b++) u[B * a + b] = x[a][b];
+                fast::mul_mont_column<A * B>(u, g, ge, mulp, mstride, mont.n(), mont.ninv());
+            }
+        }
+    };
     constexpr int NST = SHAPE == HC_SHAPE_C12 ? 3 : 2;
     with_sched<SHAPE, inv, FIX>(P, [&](const auto& sch) {
         fast::SF f[NST];
@@ -54,25 +80,13 @@ __device__ __forceinline__ void run_column(const DevPlanHeader* P, int64_t* g, i
 #pragma unroll
                 for (int b = 0; b < 3; b++) x[a][b] = gs[(3 * a + b) * gse];
             fast::col12(c, f, inv, MODE == 0, x);
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    int64_t v = x[a][b];
-                    if (MODE & 2) v = mont.mul(v, mont.load(mulp, (3 * a + b) * mstride));
-                    g[(3 * a + b) * ge] = v;
-                }
+            store(x);
         } else {
-            int64_t x[4];
+            int64_t x[1][4];
 #pragma unroll
-            for (int a = 0; a < 4; a++) x[a] = gs[a * gse];
-            fast::col4(c, f, inv, MODE == 0, x);
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                int64_t v = x[a];
-                if (MODE & 2) v = mont.mul(v, mont.load(mulp, a * mstride));
-                g[a * ge] = v;
-            }
+            for (int a = 0; a < 4; a++) x[0][a] = gs[a * gse];
+            fast::col4(c, f, inv, MODE == 0, x[0]);
+            store(x);
         }
     });
 }

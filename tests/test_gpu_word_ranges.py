@@ -115,3 +115,60 @@ def test_base_conversions_of_any_word(rings, ring):
     exp = np.concatenate([o.bconv_gadget(x[i:i + 1], base, digits) for i in range(3)])
     assert (out.to_numpy() == exp).all()
     assert (d.mod_switch_down(d.tensor(x), base, cut).to_numpy() == o.mod_switch_down(x, base, cut)).all()
+
+
+@pytest.mark.parametrize("field", ["field_18", "field_36864", "field_49152"])
+@pytest.mark.parametrize("ops", [2, 3, 7])
+def test_batched_product_with_any_operand(po, rings, field, ops):
+    """The batch's operand: any word, with and without a transform before the product."""
+    import ringcuda
+
+    o, d = rings(field, 200, 230, 2)
+    base = o.initial_base()[:3]
+    primes = [o.primes[i] for i in base]
+    g = np.random.default_rng(ops)
+    x = words(g, o.shape(2, len(base)), primes, 1)
+    op = words(g, o.shape(2, len(base)), primes, 64)
+    edge = np.array([WORD, -WORD, -WORD - 1, (1 << 63) - (1 << 31), (1 << 63) - (1 << 31) - 1, (0x73 << 56) - 1, 0x73 << 56])
+    op[1] = g.choice(edge, size=op[1].shape)
+    exp = o.pb_to_crt(x, base) if ops & 1 else x.copy()
+    po.mul_mont64(exp, op, primes)
+    if ops & 4:
+        exp = o.crt_to_pb(exp, base)
+    t = d.tensor(x)
+    batch = ringcuda.CrtBatch([(d, t, d.tensor(op), base)], ops)
+    batch.run()
+    batch.close()
+    assert (t.to_numpy() == exp).all()
+
+
+@pytest.mark.parametrize("inner,shape,dim", [([2, 3, 8, 64], (12, 3072), 3), ([4, 3], (12, 3072), 2), ([3, 64, 64], (4, 12288), 3),
+                                             ([4], (4, 12288), 2)], ids=lambda v: str(v))
+def test_transform_times_any_multiplier(be, po, inner, shape, dim):
+    """hal_ntt_mul_mont64_dim: the lazily bounded transform times any word, around the 2^58 up to which its limb product
+    is exact, and times words of a Montgomery modulus of more than 57 bits (the multiplication's moduli are the call's
+    own, not the plan's)."""
+    o = po.Ring("field_36864" if shape[0] == 12 else "field_49152", 200, 230, 2)
+    p = o.primes[0]
+    g = np.random.default_rng(dim)
+    x = np.stack([words(g, (1, 1) + shape, [p], 2)[0] for _ in range(3)])
+    mul = words(g, (3, 1) + shape, [p], 64)
+    edge = [s * (1 << b) + e for b in (57, 58, 59, 62) for s in (1, -1) for e in (-1, 0, 1)]
+    mul[1] = g.choice(np.array(edge + [WORD, -WORD, -WORD - 1, (1 << 63) - (1 << 31)], dtype=np.int64), size=mul[1].shape)
+    mul[2] = g.integers(-2 * p, 2 * p, size=mul[2].shape)
+    m = be.hal_create_modulus(p)
+    plan = be.hal_create_ntt_plan(m, inner)
+    lazy = x.copy()
+    for i in range(3):
+        # the transform along `dim`, unreduced: elements shape[1] apart along dimension 2, vectors of one line along 3
+        if dim == 2:
+            po.plan_apply(p, inner, lazy[i, 0], shape[1], shape[1], False, False)
+        else:
+            for k in range(shape[0]):
+                po.plan_apply(p, inner, lazy[i, 0, k], 1, 1, False, False)
+    for q in (p, (1 << 61) - 1):
+        exp = lazy.copy()
+        po.mul_mont64(exp, mul, [q])
+        t = be.tensor(x)
+        be.hal_ntt_mul_mont64_dim(t, [plan], dim, be.tensor(mul), [be.hal_create_modulus(q)])
+        assert (t.to_numpy() == exp).all()
