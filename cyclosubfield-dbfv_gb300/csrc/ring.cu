@@ -46,7 +46,8 @@ hc_status launch_crt_pass(hc_context ctx, int dir, const KView& t, const KView* 
                           const KView& pm, bool post, const KMods& mods);
 hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, int nbaby, int d, const int* lfirst,
                        const int* lcount, const KView* add, int nadd, const unsigned char* full, int used,
-                       const KView& dst, const KMods& m, const int64_t* one_dev);
+                       const KView& dst, const KMods& m, const int64_t* one_dev, const int* beyond);
+hc_status launch_copy_range(hc_context ctx, const KView& d, const KView& s, int* beyond);
 size_t crt_slab_tile_words(int32_t shapes, int32_t dl, int32_t dk, int logv);
 bool crt_slab_limbs(int32_t shapes, int dim);
 }  // namespace hc
@@ -2628,9 +2629,10 @@ hc_status hc_dbfv_hom_cyclic_transform(hc_ring R, size_t log2_b, size_t log2_t, 
             for (size_t j = 1; j < baby; j++) baby_exps.push_back(pow_mod_m(g, j, m));
             // babys: block j (rows j 2d .. (j + 1) 2d) = sigma^j(ct)
             Tensor B(R->ctx, (int64_t)(baby * 2 * d), rr, dl, dk, false, false);
+            Tensor beyond(R->ctx, 1, 1, 1, 1);  // set by the copy: the ciphertext has words beyond the limb sums
             if (d > 0) {
                 // all d digits in one hoisted batch: block j holds sigma^j of every digit
-                CK(hc_assign(R->ctx, vrows(B.view(), 0, 2 * (int64_t)d), ct));
+                CK(launch_copy_range(R->ctx, kv(vrows(B.view(), 0, 2 * (int64_t)d)), kv(ct), beyond.buf.as<int>()));
                 std::vector<hc_view> outs;
                 for (size_t j = 1; j < baby; j++)
                     outs.push_back(vrows(B.view(), (int64_t)(j * 2 * d), (int64_t)((j + 1) * 2 * d)));
@@ -2674,7 +2676,7 @@ hc_status hc_dbfv_hom_cyclic_transform(hc_ring R, size_t log2_b, size_t log2_t, 
                 KView addv = od > 0 ? kv(O.view()) : KView();
                 CK(launch_giant(R->ctx, kv(B.view()), nt > 0 ? kv(L.view()) : KView(), d > 0 ? (int)nterm : 0, (int)d,
                                 lf.data(), lc.data(), od > 0 ? &addv : nullptr, (int)od, fullv.data(), (int)used,
-                                kv(n.view()), km, one));
+                                kv(n.view()), km, one, beyond.buf.as<int>()));
                 O = std::move(n);
                 od = used;
             }

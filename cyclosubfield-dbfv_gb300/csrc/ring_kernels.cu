@@ -215,6 +215,23 @@ __device__ __forceinline__ int64_t finish_wide(uint64_t lo, int64_t hi, bool ful
     return full ? mont_mul(mont_red_double(lo, hi, m), r2, m) : mont_red(lo, hi, m);
 }
 
+/// Whether words went beyond the range of the limb sums, |y| <= 2^58 (LIMB_TERMS2): the caller's keys and
+/// ciphertexts may be unreduced. Three instructions for two words; a thread that met such a word forms its
+/// sums again in 128 bits.
+struct WordRange {
+    uint32_t seen = 0;
+    __device__ __forceinline__ void see(int64_t y0, int64_t y1) {
+        seen |= (hi32(y0) + (1u << 26)) | (hi32(y1) + (1u << 26));
+    }
+    __device__ __forceinline__ bool beyond() const { return (seen >> 27) != 0; }
+};
+
+/// finish_wide of any sum, also where lo and hi wrapped.
+__device__ __noinline__ int64_t finish_any(uint64_t lo, int64_t hi, bool full, int64_t n, int64_t ninv, int64_t r2) {
+    const i128 v = (i128)(((u128)(uint64_t)hi << 64) | lo);
+    return full ? to_mont64(double_red128(v, n, ninv), n, ninv, r2) : red128(v, n, ninv);
+}
+
 /// One digit of the dBFV reduction at one position per thread (dbfv_reduce, src/dbfv.rs:968-1032, with
 /// split_overflow, :891-950): rows x <- reduce(x mont(1) + sum_k carry_k Delta_k) when a carry comes in,
 /// then the overflow of x modulo Q as limbs (lifts, the matrix sums, the power-of-two correction of
@@ -334,17 +351,6 @@ struct KsArgs {
     int reverse;
 };
 
-/// Whether keys' words went beyond the range of the limb sums, |y| <= 2^58 (LIMB_TERMS2): the caller's keys may be
-/// unreduced. Three instructions for two words beside the 36 multiply-adds and splits of a digit; a thread
-/// that met such a word sums its positions again in 128 bits.
-struct KeyRange {
-    uint32_t seen = 0;
-    __device__ __forceinline__ void see(int64_t y0, int64_t y1) {
-        seen |= (hi32(y0) + (1u << 26)) | (hi32(y1) + (1u << 26));
-    }
-    __device__ __forceinline__ bool beyond() const { return (seen >> 27) != 0; }
-};
-
 /// R accumulators of one position: one digit word times R key words per step.
 template <int R>
 struct KsAcc {
@@ -387,7 +393,7 @@ __global__ void __launch_bounds__(256) keyswitch1_kernel(KsArgs a, KMods m, cons
         int64_t j = r % a.dst.n1, i = r / a.dst.n1;
         const int64_t sk = a.group.p2[0] ? (int64_t)a.group.p2[0][k] : k, sl = a.group.p3[0] ? (int64_t)a.group.p3[0][l] : l;
         KsAcc<2> acc;
-        KeyRange range;
+        WordRange range;
         acc.start();
         for (int t = 0; t < a.nterms; t++) {
             const int64_t x = *kat<int64_t>(a.parts[t], i, j, sk, sl);
@@ -479,7 +485,7 @@ __global__ void __launch_bounds__(256, 4) keyswitch_async_kernel(KsArgs a, KMods
 #pragma unroll
         for (int t = 0; t < KS_STAGES - 1; t++) issue(t);
         KsAcc<2> acc0, acc1;  // rows 0, 1 of the two positions
-        KeyRange range;
+        WordRange range;
         acc0.start(), acc1.start();
         for (int t = 0; t < a.nterms; t++) {
             issue(t + KS_STAGES - 1);
@@ -542,6 +548,21 @@ __device__ __forceinline__ void store_words(int64_t* p, const int64_t (&v)[W]) {
     }
 }
 
+/// tensor_kernel's three products of `count` positions in 128 bits, for ciphertexts (the caller's) with words beyond the
+/// limb sums; the rows' reductions as bits of `full`.
+__device__ __noinline__ void tensor_any(const int64_t* lp, int64_t ls, const int64_t* rp, int64_t rs, int64_t* d01, int64_t ds,
+                                        int64_t* d2, int count, int64_t n, int64_t ninv, int64_t r2, int full) {
+    auto finish = [&](u128 v, int q) { return finish_any((uint64_t)v, (int64_t)(v >> 64), (full >> q) & 1, n, ninv, r2); };
+    auto prod = [](int64_t x, int64_t y) { return (u128)((i128)x * (i128)y); };
+#pragma unroll 1
+    for (int w = 0; w < count; w++) {
+        const int64_t l0 = lp[w], l1 = lp[w + ls], r0 = rp[w], r1 = rp[w + rs];
+        d01[w] = finish(prod(l0, r0), 0);
+        d01[w + ds] = finish(prod(l0, r1) + prod(l1, r0), 1);
+        d2[w] = finish(prod(l1, r1), 2);
+    }
+}
+
 /// (l0 r0, l0 r1 + l1 r0, l1 r1) of B pairs of 2-row ciphertext tensors ([2B, ...] each),
 /// reduced per row into [3B, ...]: rows 2i and 2i + 1 receive the first two components of pair i,
 /// row 2B + i the third. Each operand comes in two parts along the RNS dimension: rows j < rsplit
@@ -569,8 +590,10 @@ __global__ void __launch_bounds__(256) tensor_kernel(KView d, KView lhs_lo, KVie
         int64_t l0[W], l1[W], r0[W], r1[W], o0[W], o1[W], o2[W];
         load_words<W>(lp, l0), load_words<W>(lp + ls, l1);
         load_words<W>(rp, r0), load_words<W>(rp + rs, r1);
+        WordRange range;
 #pragma unroll
         for (int w = 0; w < W; w++) {
+            range.see(l0[w], l1[w]), range.see(r0[w], r1[w]);
             const int2 x0 = limb_split(l0[w]), x1 = limb_split(l1[w]), y0 = limb_split(r0[w]), y1 = limb_split(r1[w]);
             const int xs0 = x0.x + x0.y, xs1 = x1.x + x1.y, ys0 = y0.x + y0.y, ys1 = y1.x + y1.y;
             LimbSum s[3];
@@ -591,6 +614,9 @@ __global__ void __launch_bounds__(256) tensor_kernel(KView d, KView lhs_lo, KVie
         store_words<W>(kat<int64_t>(d, 2 * i, j, k, l), o0);
         store_words<W>(kat<int64_t>(d, 2 * i + 1, j, k, l), o1);
         store_words<W>(kat<int64_t>(d, 2 * B + i, j, k, l), o2);
+        if (range.beyond())
+            tensor_any(lp, ls, rp, rs, kat<int64_t>(d, 2 * i, j, k, l), d.s0, kat<int64_t>(d, 2 * B + i, j, k, l), W, m.n[j],
+                       m.ninv[j], r2, full0 | full1 << 1 | full2 << 2);
     }
 }
 
@@ -680,6 +706,7 @@ struct GiantArgs {
     int nadd;
     unsigned full;                 // bit o - out0: output digit o needs the full double reduction
     KView dst;                     // [2 used, ...]
+    const int* beyond;             // not 0: block 0, the caller's ciphertext, has words beyond the limb sums
 };
 
 /// The lcoef values of a tile's line (j, k) are the same for all its positions: the CTA stages
@@ -702,8 +729,41 @@ struct GiantUnits {
     int n;
 };
 
+/// A copy of a ciphertext that notes in `beyond` whether a word lies beyond the limb sums. The giant steps read it
+/// once per CTA: seeing the words on the way, in their loop, cost them 5 % (the step at r = 23 4765 -> 4879 us).
+__global__ void __launch_bounds__(256) copy_range_kernel(KView d, KView s, int* beyond, int64_t lines, int chunks) {
+    grid_wait();
+    const int64_t tiles = lines * chunks;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t line = tile / chunks, l = (tile - line * chunks) * blockDim.x + threadIdx.x;
+        if (l >= d.n3) continue;
+        const int64_t k = line % d.n2, r = line / d.n2, j = r % d.n1, i = r / d.n1;
+        const int64_t v = *kat<int64_t>(s, i, j, k, l);
+        WordRange range;
+        range.see(v, v);
+        if (range.beyond()) *beyond = 1;
+        *kat<int64_t>(d, i, j, k, l) = v;
+    }
+}
+
+/// Component `row` of the launch's output digits at one position in 128-bit sums: for ciphertexts (block 0 of the
+/// baby steps, the caller's) with words beyond the limb sums. The other blocks are key switches' results.
+__device__ __noinline__ void giant_any(const GiantArgs& a, int64_t n, int64_t ninv, int64_t r2, int64_t one, int64_t j, int64_t k,
+                                       int64_t l, int row) {
+    for (int o = a.out0; o < a.out0 + a.nout; o++) {
+        u128 v = o < a.nadd ? (u128)((i128)*kat<int64_t>(a.add, 2 * o + row, j, k, l) * (i128)one) : 0;
+        for (int q = 0; q < a.nbaby; q++)
+            for (int i = 0; i < a.d && i <= o; i++)
+                if (o - i < a.lcount[q])
+                    v += (u128)((i128)*kat<int64_t>(a.babies, 2 * (a.d * q + i) + row, j, k, l) *
+                                (i128)*kat<int64_t>(a.lcoef, a.lfirst[q] + o - i, j, k, 0));
+        *kat<int64_t>(a.dst, 2 * o + row, j, k, l) =
+            finish_any((uint64_t)v, (int64_t)(v >> 64), (a.full >> (o - a.out0)) & 1, n, ninv, r2);
+    }
+}
+
 template <int NOUT>
-__global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs a, GiantUnits un, KMods m, const int64_t* one,
+__global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(const __grid_constant__ GiantArgs a, GiantUnits un, KMods m, const int64_t* one,
                                                              int64_t lines, int chunks) {
     grid_wait();
     extern __shared__ int64_t gsm[];  // [GIANT_STAGES][2][256] staging, then the tile's lcoef as limb pairs
@@ -711,6 +771,7 @@ __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs
     const int64_t tiles = lines * chunks;
     const int nt = (int)a.lcoef.n0;
     const int tid = threadIdx.x;
+    const bool beyond = *a.beyond != 0;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t line = tile / chunks;  // (j, k)
         const int64_t l = (tile - line * chunks) * blockDim.x + tid;
@@ -719,6 +780,10 @@ __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(GiantArgs
         for (int t = tid; t < nt; t += blockDim.x) slc[t] = limb_split(*kat<int64_t>(a.lcoef, t, j, k, 0));
         __syncthreads();
         if (l >= a.dst.n3) continue;
+        if (beyond) {
+            for (int row = 0; row < 2; row++) giant_any(a, m.n[j], m.ninv[j], m.r2[j], one[j], j, k, l, row);
+            continue;
+        }
         const int64_t rs = a.babies.s0;  // row stride of the baby-step tensor
         const int64_t* xb = kat<int64_t>(a.babies, 0, j, k, l);
         auto issue = [&](int u) {
@@ -802,13 +867,14 @@ constexpr int TRI_STAGES = 4;
 
 template <int NOUT>
 __global__ void __launch_bounds__(256, NOUT == 4 ? 2 : NOUT >= 2 ? 3 : 4)
-    giant_tri_kernel(GiantArgs a, KMods m, const int64_t* one, int n0, int64_t lines, int chunks) {
+    giant_tri_kernel(const __grid_constant__ GiantArgs a, KMods m, const int64_t* one, int n0, int64_t lines, int chunks) {
     grid_wait();
     extern __shared__ __align__(16) int64_t gsm[];  // [TRI_STAGES][NOUT][256] position pairs, then the lcoef limb pairs
     longlong2* sx = reinterpret_cast<longlong2*>(gsm);
     int2* slc = reinterpret_cast<int2*>(sx + TRI_STAGES * NOUT * 256);
     const int64_t tiles = lines * chunks;
     const int nt = (int)a.lcoef.n0, tid = threadIdx.x;
+    const bool beyond = *a.beyond != 0;
     const int row = tid >> 7, lane = tid & 127;  // the ciphertext component, the pair of positions
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t line = tile / chunks;  // (j, k)
@@ -818,6 +884,10 @@ __global__ void __launch_bounds__(256, NOUT == 4 ? 2 : NOUT >= 2 ? 3 : 4)
         for (int t = tid; t < nt; t += 256) slc[t] = limb_split(*kat<int64_t>(a.lcoef, t, j, k, 0));
         __syncthreads();
         if (l >= a.dst.n3) continue;
+        if (beyond) {
+            for (int p = 0; p < 2; p++) giant_any(a, m.n[j], m.ninv[j], m.r2[j], one[j], j, k, l + p, row);
+            continue;
+        }
         const int64_t rs = a.babies.s0;
         const int64_t* next = kat<int64_t>(a.babies, row, j, k, l);  // baby step q's rows of this thread, in turn
         auto issue = [&](int q, int slot) {
@@ -972,6 +1042,17 @@ hc_status launch_dbfv_split(hc_context ctx, const KView& x, const KView& src, co
     return cuda_check(cudaGetLastError(), "dBFV reduction launch");
 }
 
+hc_status launch_copy_range(hc_context ctx, const KView& d, const KView& s, int* beyond) {
+    const int64_t lines = d.n0 * d.n1 * d.n2;
+    if (lines == 0 || d.n3 == 0) return HC_OK;
+    int chunks;
+    unsigned blocks;
+    grid_lines(ctx, d.n3, lines, &chunks, &blocks);
+    hc::launch_kernel(copy_range_kernel, blocks, 256, 0, stream_of(ctx), d, s, beyond, lines, chunks);
+    count_launch(ctx);
+    return cuda_check(cudaGetLastError(), "ciphertext copy launch");
+}
+
 hc_status launch_galois(hc_context ctx, const KView& d, const KView& s, const uint32_t* p2, const uint32_t* p3) {
     int64_t lines = d.n0 * d.n1 * d.n2;
     if (lines == 0 || d.n3 == 0) return HC_OK;
@@ -1041,7 +1122,7 @@ hc_status launch_keyswitch(hc_context ctx, const KView* parts, const KView* keys
 
 hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, int nbaby, int d, const int* lfirst,
                        const int* lcount, const KView* add, int nadd, const unsigned char* full, int used,
-                       const KView& dst, const KMods& m, const int64_t* one_dev) {
+                       const KView& dst, const KMods& m, const int64_t* one_dev, const int* beyond) {
     if (nbaby > GIANT_MAX_BABY) return fail(HC_ERR_UNSUPPORTED, "too many baby steps");
     int64_t lines = dst.n1 * dst.n2;
     if (lines == 0 || dst.n3 == 0 || used == 0) return HC_OK;
@@ -1050,6 +1131,7 @@ hc_status launch_giant(hc_context ctx, const KView& babies, const KView& lcoef, 
     a.lcoef = lcoef;
     a.lcoef.b3 = 1;  // broadcast along dimension 3
     a.nbaby = nbaby, a.d = d;
+    a.beyond = beyond;
     for (int j = 0; j < nbaby; j++) {
         if (lfirst[j] > 32767 || lcount[j] > 32767) return fail(HC_ERR_UNSUPPORTED, "too many coefficient digits");
         a.lfirst[j] = (short)lfirst[j], a.lcount[j] = (short)lcount[j];

@@ -17,9 +17,10 @@
  * (low, high) int64 words. Random numbers come from the reference's splitmix64 generator
  * (src/bfv.rs:880-886) whose 64-bit state the caller owns and which the call advances.
  *
- * Words: the result of every call is almost reduced (|x| <= p). Transforms and what runs them on its
- * inputs take |x| <= 2p. The summand c0 of the key switches and rotations may be any word, a lazy sum of
- * many elements included, and so may the keys' words and the sources of base conversions and mod_switch_down.
+ * Words: the results of calls are almost reduced (|x| <= p) unless a call says otherwise. Transforms, and
+ * the calls that transform their inputs, are exact for |x| <= 2p; in between no call forms a sum or product
+ * of its inputs in less than their full words: the summand c0 of key switches and rotations may be a lazy sum
+ * of any size, and keys, products' operands and the sources of base conversions and mod_switch_down any words.
  *
  * Threads and streams: a ring (its table caches and its side streams) is used from one host thread
  * at a time; calls are asynchronous on the context's current stream (hc_context_set_stream), and

@@ -172,3 +172,38 @@ def test_transform_times_any_multiplier(be, po, inner, shape, dim):
         t = be.tensor(x)
         be.hal_ntt_mul_mont64_dim(t, [plan], dim, be.tensor(mul), [be.hal_create_modulus(q)])
         assert (t.to_numpy() == exp).all()
+
+
+@pytest.mark.parametrize("ring", [("field_192", 2300, 2340, 32), ("field_18", 560, 572, 4), ("field_36864", 200, 230, 24),
+                                  ("field_49152", 200, 230, 24)], ids=lambda v: v[0])
+@pytest.mark.parametrize("bound", [3, 7, 64])
+def test_products_and_transforms_of_lazy_sums(rings, ring, bound):
+    """Ciphertexts beyond 2p in the tensor product and the giant steps (csrc/ring_kernels.cu: tensor_any, giant_any), one
+    to five output digits: the limb sums hold about 6 p. The transforms' wrapping agrees with the oracle's as well."""
+    import ringcuda
+
+    o, d = rings(*ring)
+    base = o.initial_base()[:5]
+    primes = [o.primes[i] for i in base]
+    digits = [tuple(v) for v in ringcuda.select_digits(min(3, len(base)), len(base))]
+    nd, full = len(digits), o.initial_len
+    g = np.random.default_rng(bound)
+    rk = words(g, o.shape(2 * nd, len(base)), primes, 1)
+    ct = [words(g, o.shape(2, len(base)), primes, b) for b in (bound, bound, 1)]
+    for a, b in ((ct[0], ct[1]), (ct[0], ct[2]), (ct[2], ct[1])):
+        exp = o.hom_mul(256, a, b, base, rk.reshape((nd, 2) + rk.shape[1:]), digits)
+        assert (d.hom_mul(256, d.tensor(a), d.tensor(b), base, d.tensor(rk), digits).to_numpy() == exp).all()
+    gen, m, length = list(o.info["gens"])[0], o.info["m"], 6
+    baby = min(range(1, length + 1), key=lambda c: (c + 3 * ((length - 1) // c + 1), c))
+    gks, ks = {}, ringcuda.Keyset(d, digits, full, 1 << 40)
+    for e in sorted({pow(gen, j, m) for j in range(1, baby + 1)}):
+        k = words(g, o.shape(2 * nd, full), o.primes[:full], 1)
+        gks[e] = k.reshape((nd, 2) + k.shape[1:])
+        ks.add(e, d.tensor(k))
+    for log2_t, dct, dense in ((4, 1, True), (12, 2, True), (16, 4, False), (20, 3, True)):
+        t = 1 << log2_t
+        coeffs = [[int(v) for v in g.integers(t // 4 if dense else 0, t if dense else [t, 1, 2][j % 3], size=o.dl)] for j in range(length)]
+        x = words(g, o.shape(2 * dct, len(base)), primes, bound)
+        exp = o.dbfv_hom_cyclic_transform(4, log2_t, gen, coeffs, x, base, gks, digits)
+        got = ringcuda.dbfv_hom_cyclic_transform(d, 4, log2_t, gen, coeffs, d.tensor(x), base, ks).to_numpy()
+        assert got.shape == exp.shape and (got == exp).all()
