@@ -120,20 +120,27 @@ __global__ void __launch_bounds__(256) pw_line_kernel(KView d, KView a, KView b,
 }
 
 /// dst[i,j,k,l] = sum_u lhs[li,j,u,0] * rhs[ri,u,k,l] (src/hal/cpu.rs:791-818), i128 wrapping.
-/// Four output rows j per pass share each rhs load. The columns u go in chunks of LIMB_TERMS: the first
-/// warp splits the chunk's matrix entries into limbs and lists its columns that are not zero in all four
-/// rows (a gadget conversion matrix is zero outside each digit's columns); the others add nothing.
+/// Four output rows j per pass share each rhs load. The columns u go in chunks of LIMB_TERMS: a warp
+/// splits a chunk's matrix entries into limbs and lists its columns that are not zero in all four
+/// rows (a gadget conversion matrix is zero outside each digit's columns; the others add nothing), four warps
+/// four chunks at a time, so that a short line waits for the matrix once.
 /// A chunk whose words are all below 2^57 in absolute value (residues and centred constants are) is summed
-/// in limbs, found out for the matrix by the first warp and for the right-hand side by each warp as it
-/// goes; a warp that meets a larger word sums the chunk again as 128-bit products, so every word is allowed.
+/// in limbs, found out for the matrix by the staging warp and for the right-hand side by each warp as it
+/// goes; a warp that meets a larger word sums the chunk and the rest of the tile as 128-bit products, so every
+/// word is allowed.
 /// What bounds it: the multiply pipe, 13 cycles a term instead of 33; a trait-path ct-mult (five
-/// products at field_36864 r = 16) 921 -> 839 us. Four columns unrolled or four CTAs per SM spill (852, 854).
+/// products at field_36864 r = 16) 921 -> 839 us. Four columns unrolled in the limb sums or four CTAs per SM spill
+/// (852, 854). [2, 18 x 16, 12, 3072] of small words 20.5 us, 33 with larger ones on the right and 30 in the matrix
+/// (as 128-bit products alone, two at a time, 37).
 constexpr int MATMUL_ROWS = 4, MATMUL_UNROLL = 2;
+/// MATMUL_STAGED: 1 for matrices of one chunk, whose staging indexes then fold away, else 4.
+template <int MATMUL_STAGED>
 __global__ void __launch_bounds__(256, 3) matmul_kernel(KView d, KView lhs, KView rhs, int64_t U, int64_t lines,
                                                         int chunks) {
     grid_wait();
-    __shared__ __align__(16) int2 sm[LIMB_TERMS][MATMUL_ROWS];
-    __shared__ int sidx[LIMB_TERMS], scount, slarge;
+    __shared__ __align__(16) int2 sm[MATMUL_STAGED][LIMB_TERMS][MATMUL_ROWS];
+    __shared__ __align__(16) int64_t sw[MATMUL_STAGED][LIMB_TERMS][MATMUL_ROWS];  // the entries whole
+    __shared__ int sidx[MATMUL_STAGED][LIMB_TERMS], scount[MATMUL_STAGED], slarge[MATMUL_STAGED];
     const int64_t tiles = lines * chunks;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t line = tile / chunks;  // (i, k)
@@ -141,64 +148,71 @@ __global__ void __launch_bounds__(256, 3) matmul_kernel(KView d, KView lhs, KVie
         const int64_t k = line % d.n2, i = line / d.n2;
         // a thread past the line's end reads its last position and stores nothing
         const int64_t* x0 = kat<int64_t>(rhs, i, 0, k, l < d.n3 ? l : d.n3 - 1);
+        bool beyond = false;  // the warp has met a larger word of this tile
         for (int64_t j = 0; j < d.n1; j += MATMUL_ROWS) {
             const int rows = (int)(d.n1 - j < MATMUL_ROWS ? d.n1 - j : MATMUL_ROWS);
             uint64_t lo[MATMUL_ROWS] = {};
             int64_t hi[MATMUL_ROWS] = {};
             for (int64_t u0 = 0; u0 < U; u0 += LIMB_TERMS) {
-                __syncthreads();  // the previous chunk's readers are done
-                if (threadIdx.x < 32) {
-                    const bool in = threadIdx.x < LIMB_TERMS && u0 + threadIdx.x < U;
-                    int64_t c[MATMUL_ROWS];
-                    uint64_t any = 0, large = 0;
+                const int g = (int)(u0 / LIMB_TERMS) % MATMUL_STAGED;
+                if (g == 0) {
+                    __syncthreads();  // the previous chunks' readers are done
+                    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+                    const int64_t u = u0 + LIMB_TERMS * warp + lane;
+                    if (warp < MATMUL_STAGED && u0 + LIMB_TERMS * warp < U) {
+                        const bool in = lane < LIMB_TERMS && u < U;
+                        int64_t c[MATMUL_ROWS];
+                        uint64_t any = 0, large = 0;
 #pragma unroll
-                    for (int q = 0; q < MATMUL_ROWS; q++) {
-                        c[q] = in && q < rows ? *kat<int64_t>(lhs, i, j + q, u0 + threadIdx.x, 0) : 0;
-                        any |= (uint64_t)c[q];
-                        large |= ((uint64_t)c[q] + ((uint64_t)1 << 57)) >> 58;
-                    }
-                    const unsigned mask = __ballot_sync(0xffffffffu, any != 0);
-                    const int wide = __any_sync(0xffffffffu, large != 0);
-                    if (any != 0) {
-                        const int at = __popc(mask & ((1u << threadIdx.x) - 1));
-                        sidx[at] = (int)threadIdx.x;
+                        for (int q = 0; q < MATMUL_ROWS; q++) {
+                            c[q] = in && q < rows ? *kat<int64_t>(lhs, i, j + q, u, 0) : 0;
+                            any |= (uint64_t)c[q];
+                            large |= ((uint64_t)c[q] + ((uint64_t)1 << 57)) >> 58;
+                        }
+                        const unsigned mask = __ballot_sync(0xffffffffu, any != 0);
+                        const int wide = __any_sync(0xffffffffu, large != 0);
+                        if (any != 0) {
+                            const int at = __popc(mask & ((1u << lane) - 1));
+                            sidx[warp][at] = lane;
 #pragma unroll
-                        for (int q = 0; q < MATMUL_ROWS; q++) sm[at][q] = limb_split(c[q]);
+                            for (int q = 0; q < MATMUL_ROWS; q++) sm[warp][at][q] = limb_split(c[q]), sw[warp][at][q] = c[q];
+                        }
+                        if (lane == 0) scount[warp] = __popc(mask), slarge[warp] = wide;
                     }
-                    if (threadIdx.x == 0) scount = __popc(mask), slarge = wide;
+                    __syncthreads();
                 }
-                __syncthreads();
-                const int n = scount;
+                const int n = scount[g];
                 const int64_t* xu = x0 + u0 * rhs.s1;
-                uint64_t large = slarge;
-                if (!large) {
+                if (!beyond && !slarge[g]) {
+                    uint64_t large = 0;
                     LimbSum s[MATMUL_ROWS];
 #pragma unroll
                     for (int q = 0; q < MATMUL_ROWS; q++) s[q].zero();
 #pragma unroll MATMUL_UNROLL
                     for (int t = 0; t < n; t++) {
-                        const int64_t v = xu[sidx[t] * rhs.s1];
+                        const int64_t v = xu[sidx[g][t] * rhs.s1];
                         large |= ((uint64_t)v + ((uint64_t)1 << 57)) >> 58;
                         const int2 x = limb_split(v);
                         const int xs = x.x + x.y;
 #pragma unroll
                         for (int q = 0; q < MATMUL_ROWS; q++) {
-                            const int2 w = sm[t][q];
+                            const int2 w = sm[g][t][q];
                             s[q].mac(x, xs, w, w.x + w.y);
                         }
                     }
-                    if (!__any_sync(0xffffffffu, large != 0)) {
+                    beyond = __any_sync(0xffffffffu, large != 0);
+                    if (!beyond) {
 #pragma unroll
                         for (int q = 0; q < MATMUL_ROWS; q++) s[q].fold(lo[q], hi[q]);
                         continue;
                     }
                 }
+#pragma unroll 4
                 for (int t = 0; t < n; t++) {
-                    const int64_t v = xu[sidx[t] * rhs.s1];
+                    const int64_t v = xu[sidx[g][t] * rhs.s1];
 #pragma unroll
                     for (int q = 0; q < MATMUL_ROWS; q++) {
-                        const int64_t c = q < rows ? *kat<int64_t>(lhs, i, j + q, u0 + sidx[t], 0) : 0;
-                        const u128 s = (((u128)(uint64_t)hi[q] << 64) | lo[q]) + (u128)((i128)c * (i128)v);
+                        const u128 s = (((u128)(uint64_t)hi[q] << 64) | lo[q]) + (u128)((i128)sw[g][t][q] * (i128)v);
                         lo[q] = (uint64_t)s, hi[q] = (int64_t)(s >> 64);
                     }
                 }
@@ -422,7 +436,8 @@ hc_status launch_matmul(hc_context ctx, const KView& d, const KView& lhs, const 
     int chunks;
     unsigned blocks;
     grid_for(ctx, d, lines, &chunks, &blocks);
-    hc::launch_kernel(matmul_kernel, blocks, 256, 0, stream_of(ctx), d, lhs, rhs, U, lines, chunks);
+    hc::launch_kernel(U <= LIMB_TERMS ? matmul_kernel<1> : matmul_kernel<4>, blocks, 256, 0, stream_of(ctx), d, lhs, rhs, U, lines,
+                      chunks);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "matmul kernel launch");
 }

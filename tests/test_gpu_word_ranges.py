@@ -207,3 +207,24 @@ def test_products_and_transforms_of_lazy_sums(rings, ring, bound):
         exp = o.dbfv_hom_cyclic_transform(4, log2_t, gen, coeffs, x, base, gks, digits)
         got = ringcuda.dbfv_hom_cyclic_transform(d, 4, log2_t, gen, coeffs, d.tensor(x), base, ks).to_numpy()
         assert got.shape == exp.shape and (got == exp).all()
+
+
+@pytest.mark.parametrize("cols", [27, 28, 29, 57, 112, 113, 141, 225])
+@pytest.mark.parametrize("rows,l", [(1, 7), (6, 300)])
+def test_matmul_of_one_sign_and_mixed_chunks(be, po, cols, rows, l):
+    """Column sums at their largest (every word the same extreme of 57 bits: 33 unfolded terms overflow), and larger words met
+    late in a tile, over the chunks of 28 columns that are staged four at a time (csrc/ops.cu: matmul_kernel)."""
+    g = np.random.default_rng(cols)
+    top, low = (1 << 57) - 1, -(1 << 57)
+    mixed = g.integers(low, top, size=(2, cols, 2, l), endpoint=True)
+    mixed[1, cols - 1, 1, l // 2] = WORD
+    mixed[0, cols // 2, 0, 0] = -WORD - 1
+    for a, b in ((top, top), (low, low), (top, low), (low, top), (None, None), (WORD, top)):
+        lhs = np.full((1, rows, cols, 1), a) if a is not None else g.integers(low, top, size=(1, rows, cols, 1), endpoint=True)
+        rhs = np.full(mixed.shape, b) if b is not None else mixed
+        d = be.hal_allocate_i128((2, rows, 2, l))
+        be.hal_matmul_i64(d, be.tensor(lhs), be.tensor(rhs))
+        got = d.to_numpy()
+        exp = np.zeros_like(got)
+        po.matmul_i64(exp, np.ascontiguousarray(lhs), np.ascontiguousarray(rhs))
+        assert (got == exp).all()
