@@ -321,19 +321,20 @@ __global__ void __launch_bounds__(256) galois_kernel(KView d, KView s, const uin
 }
 
 // Asynchronous global -> shared copies (cp.async): a thread's copies complete in the order of its
-// commit groups, and wait_group N returns once at most N of its groups are still in flight.
+// commit groups, and wait_group N returns once at most N of its groups are still in flight. All clobber memory: a
+// slot's reads stay behind its wait and in front of the next copy into it.
 __device__ __forceinline__ void cp_async8(int64_t* smem, const int64_t* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 struct KsArgs {

@@ -1,0 +1,23 @@
+"""Properties of the kernels' sources that no run shows until a compiler makes use of their absence."""
+import glob
+import os
+import re
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = sorted(glob.glob(os.path.join(ROOT, "cyclosubfield-dbfv_gb300", "csrc", "*.cu*")))
+
+
+def source(path):
+    with open(path) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+@pytest.mark.parametrize("path", CSRC, ids=os.path.basename)
+def test_copies_and_waits_order_memory(path):
+    """Asynchronous copies, waits and barriers written as inline assembly clobber memory: otherwise the compiler may move
+    a thread's reads of a staged slot across the wait in front of them or the next copy into the slot."""
+    for stmt in re.findall(r"asm\s+volatile\s*\((.*?)\);", source(path), re.S):
+        if re.search(r"cp\.async|bar\.sync|barrier|mbarrier|griddepcontrol", stmt):
+            assert '"memory"' in stmt, stmt
