@@ -1366,7 +1366,8 @@ void keyswitch(hc_ring R, const hc_view& parts, const hc_view& keys, const Base&
 /// current again while the branch keeps running, join() makes the original stream wait for the
 /// branch (device-side; the host does not block). Inside a graph capture the branch becomes a
 /// parallel path of the graph. The destructor restores the original stream and joins on every
-/// exit path.
+/// exit path; tensors that outlive the branch's own calls are declared before it, so that an
+/// exception frees them behind the join.
 struct SideBranch {
     hc_ring R;
     void* main;
@@ -1767,11 +1768,12 @@ hc_status hc_bfv_hom_mul(hc_ring R, const int64_t t[2], hc_view ct1, hc_view ct2
             return lift_extension_rows(R, pb.view(), b, ext);
         };
         // the two lifts are independent: the second runs on the side stream beside the first
+        Tensor rh, lh;
         SideBranch lifts(R);
         lifts.begin();
-        Tensor rh = lift(ct2);
+        rh = lift(ct2);
         lifts.back();
-        Tensor lh = lift(ct1);
+        lh = lift(ct1);
         lifts.join();
         Base lifted = b;
         lifted.insert(lifted.end(), ext.begin(), ext.end());
@@ -1793,14 +1795,15 @@ hc_status hc_bfv_hom_mul(hc_ring R, const int64_t t[2], hc_view ct1, hc_view ct2
         // transform, rescale and gadget decomposition run on the side stream beside c0, c1's
         // transform, rescale and (CRT output) forward transform
         const hc_view p01 = vrows(prod.view(), 0, 2 * B), p2 = vrows(prod.view(), 2 * B, 3 * B);
+        Tensor resc2, parts, resc01;
         SideBranch c2_branch(R);
         c2_branch.begin();
         R->transform(p2, lifted, true, &tsv);
-        Tensor resc2 = rescale_to_base(R, p2, lifted, r, words(t), true);
-        Tensor parts = gadget_decompose(R, resc2.view(), b, dg);
+        resc2 = rescale_to_base(R, p2, lifted, r, words(t), true);
+        parts = gadget_decompose(R, resc2.view(), b, dg);
         c2_branch.back();
         R->transform(p01, lifted, true, &tsv);
-        Tensor resc01 = rescale_to_base(R, p01, lifted, r, words(t), true);
+        resc01 = rescale_to_base(R, p01, lifted, r, words(t), true);
         const hc_view c01 = resc01.view();
         if (!period_output) R->transform(c01, b, false);
         c2_branch.join();
@@ -2937,11 +2940,12 @@ hc_status hc_dbfv_hom_mul(hc_ring R, size_t log2_b, size_t log2_t, hc_view lhs, 
             return *rows ? lift_to_extended(R, vrows(t.view(), 0, (int64_t)*rows), nullptr, b) : Tensor();
         };
         // the operands are independent: the second is reduced and lifted on the side stream
+        Tensor rl, ll;
         SideBranch lifts(R);
         lifts.begin();
-        Tensor rl = lifted_digits(rhs, &r2);
+        rl = lifted_digits(rhs, &r2);
         lifts.back();
-        Tensor ll = lifted_digits(lhs, &r1);
+        ll = lifted_digits(lhs, &r1);
         lifts.join();
         *out_rows = 0;
         if (r1 == 0 || r2 == 0) return;
@@ -2967,14 +2971,15 @@ hc_status hc_dbfv_hom_mul(hc_ring R, size_t log2_b, size_t log2_t, hc_view lhs, 
         Digits dg = clip(digits_of(digits, d), r);
         REQUIRE(rk.shape[0] >= 2 * (int64_t)dg.size() && rk.shape[1] >= rr, HC_ERR_SHAPE, "relinearisation key shape");
         const hc_view p01 = vrows(prod.view(), 0, 2 * D), p2 = vrows(prod.view(), 2 * D, 3 * D);
+        Tensor c2, parts, resc;
         SideBranch c2_branch(R);
         c2_branch.begin();
         R->transform(p2, lifted, true, &tsv);
-        Tensor c2 = rescale_to_base(R, p2, lifted, r, t, true);
-        Tensor parts = gadget_decompose(R, c2.view(), b, dg);
+        c2 = rescale_to_base(R, p2, lifted, r, t, true);
+        parts = gadget_decompose(R, c2.view(), b, dg);
         c2_branch.back();
         R->transform(p01, lifted, true, &tsv);
-        Tensor resc = rescale_to_base(R, p01, lifted, r, t, true);
+        resc = rescale_to_base(R, p01, lifted, r, t, true);
         const hc_view c01 = resc.view(), o = vrows(out, 0, 2 * D);
         if (!period_output) R->transform(c01, b, false);
         c2_branch.join();

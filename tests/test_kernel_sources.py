@@ -21,3 +21,13 @@ def test_copies_and_waits_order_memory(path):
     for stmt in re.findall(r"asm\s+volatile\s*\((.*?)\);", source(path), re.S):
         if re.search(r"cp\.async|bar\.sync|barrier|mbarrier|griddepcontrol", stmt):
             assert '"memory"' in stmt, stmt
+
+
+def test_side_branches_join_before_their_tensors_go():
+    """A function's tensors filled on a side stream are declared before its SideBranch: when an exception leaves the
+    function, the branch's destructor joins the streams first and the tensors are freed on the caller's stream behind it."""
+    text = source(os.path.join(ROOT, "cyclosubfield-dbfv_gb300", "csrc", "ring.cu"))
+    bodies = re.findall(r"\bSideBranch (\w+)\(R\);(.*?)\b\1\.join\(\);", text, re.S)
+    assert len(bodies) >= 4
+    for name, body in bodies:
+        assert not re.search(r"\n        Tensor \w+ *=", body), (name, body)
