@@ -40,7 +40,7 @@ int crt_slab_kernel_class(int32_t shapes) { return (shapes & 0xff) == HC_SHAPE_L
 /// Launches the persistent batched-transform kernel over `nslabs` device slab descriptors.
 /// `tile_words`: largest tile (deg_K, or deg_L' x 2^logv); `tw_words`: largest pair of twiddle
 /// tables (dimension-2 + dimension-3 plan) of a slab. `counter` is reset on the stream first.
-hc_status launch_crt_batch(hc_context ctx, const CrtSlab* slabs, int nslabs, int* counter, size_t tile_words,
+hc_status launch_crt_batch(hc_context ctx, cudaStream_t stream, const CrtSlab* slabs, int nslabs, int* counter, size_t tile_words,
                            size_t tw_words, const CrtLaunch& L, bool generic, int cls) {
     if (nslabs <= 0) return HC_OK;
     CrtBatchKernel kern = generic    ? crt_batch_kernel<true, 0, 256, 2>
@@ -60,10 +60,9 @@ hc_status launch_crt_batch(hc_context ctx, const CrtSlab* slabs, int nslabs, int
     int per = L.ctas_per_sm < 1 ? 1 : (L.ctas_per_sm < occ ? L.ctas_per_sm : occ);
     int64_t grid = (int64_t)num_sms(ctx) * per;
     if (grid > nslabs) grid = nslabs;
-    hc_status st = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), stream_of(ctx)), "batched transform counter");
+    hc_status st = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), stream), "batched transform counter");
     if (st) return st;
-    hc::launch_kernel(kern, (unsigned)grid, (unsigned)L.threads, smem, stream_of(ctx), slabs, nslabs, counter, L.logv,
-                                                                      (int)tile_words);
+    hc::launch_kernel(kern, (unsigned)grid, (unsigned)L.threads, smem, stream, slabs, nslabs, counter, L.logv, (int)tile_words);
     count_launch(ctx);
     return cuda_check(cudaGetLastError(), "batched transform launch");
 }

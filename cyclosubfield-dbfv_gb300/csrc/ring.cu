@@ -1959,7 +1959,7 @@ extern "C" hc_status hc_bfv_key_switch_noalloc(hc_ring R, hc_view c0, hc_view c1
 // ------------------------------------------------------------------------- batched CRT transforms
 
 namespace hc {
-hc_status launch_crt_batch(hc_context ctx, const CrtSlab* slabs, int nslabs, int* counter, size_t tile_words,
+hc_status launch_crt_batch(hc_context ctx, cudaStream_t stream, const CrtSlab* slabs, int nslabs, int* counter, size_t tile_words,
                            size_t tw_words, const CrtLaunch& L, bool generic, int cls);
 int crt_slab_kernel_class(int32_t shapes);
 bool crt_slab_specialised(int32_t shapes);
@@ -2044,11 +2044,11 @@ int crt_group_kernel_class(const CrtGroup& g) {
     return c;
 }
 
-hc_status crt_group_run(hc_context ctx, CrtGroup& g) {
+hc_status crt_group_run(hc_context ctx, cudaStream_t stream, CrtGroup& g) {
     size_t tile = 0;
     for (const CrtSlab& s : g.host) tile = std::max(tile, crt_tile_words(s, g.launch.logv));
     const bool generic = crt_generic(g.host);
-    return launch_crt_batch(ctx, g.dev.as<CrtSlab>(), (int)g.host.size(), g.counter.as<int>(), tile, g.tw_words,
+    return launch_crt_batch(ctx, stream, g.dev.as<CrtSlab>(), (int)g.host.size(), g.counter.as<int>(), tile, g.tw_words,
                             g.launch, generic, generic ? 0 : crt_group_kernel_class(g));
 }
 
@@ -2093,7 +2093,7 @@ hc_status crt_group_tune(hc_context ctx, CrtGroup& g, int reps) {
             CrtLaunch L{sh.threads, sh.ctas_per_sm, lv};
             size_t tile = 0;
             for (const CrtSlab& s : sample) tile = std::max(tile, crt_tile_words(s, lv));
-            rc = launch_crt_batch(ctx, sdev.as<CrtSlab>(), (int)sample.size(), cnt.as<int>(), tile, g.tw_words, L,
+            rc = launch_crt_batch(ctx, st, sdev.as<CrtSlab>(), (int)sample.size(), cnt.as<int>(), tile, g.tw_words, L,
                                   generic, cls);
             if (rc == HC_ERR_UNSUPPORTED) {  // shape does not fit an SM
                 rc = HC_OK;
@@ -2102,7 +2102,7 @@ hc_status crt_group_tune(hc_context ctx, CrtGroup& g, int reps) {
             if (rc) break;
             cudaEventRecord(e0, st);
             for (int r = 0; r < reps && !rc; r++)
-                rc = launch_crt_batch(ctx, sdev.as<CrtSlab>(), (int)sample.size(), cnt.as<int>(), tile, g.tw_words,
+                rc = launch_crt_batch(ctx, st, sdev.as<CrtSlab>(), (int)sample.size(), cnt.as<int>(), tile, g.tw_words,
                                       L, generic, cls);
             if (rc) break;
             cudaEventRecord(e1, st);
@@ -2222,20 +2222,18 @@ hc_status hc_crt_batch_create(hc_context ctx, const hc_crt_item* items, size_t n
 hc_status hc_crt_batch_run(hc_crt_batch b) {
     return guard([&] {
         REQUIRE(b, HC_ERR_ARG, "null batch");
-        // the classes' persistent launches side by side: each leaves the SMs to the others as its last
-        // slabs run out, and a class of few slabs never has them alone (128 mixed elements 3.62 -> 3.39 ms, 20 1.13 -> 1.01)
+        // the classes' persistent launches side by side: each leaves the SMs to the others as its last slabs run out,
+        // and a class of few slabs never has them alone (when it came, 128 mixed elements 3.62 -> 3.39 ms, 20 1.13 ->
+        // 1.01; the 128 take 3.19 now). The context's stream is only read: other threads may issue on it meanwhile
         const cudaStream_t main = stream_of(b->ctx);
-        if (b->groups.size() > 1) {
+        const bool fork = b->groups.size() > 1;
+        if (fork) {
             CK(cuda_check(cudaEventRecord(b->fork, main), "batch fork"));
             CK(cuda_check(cudaStreamWaitEvent(b->side, b->fork, 0), "batch fork"));
         }
         hc_status st = HC_OK;
-        for (size_t i = 0; i < b->groups.size() && !st; i++) {
-            if (i == 1) hc_context_set_stream(b->ctx, b->side);
-            st = crt_group_run(b->ctx, b->groups[i]);
-        }
-        hc_context_set_stream(b->ctx, main);
-        if (b->groups.size() > 1) {
+        for (size_t i = 0; i < b->groups.size() && !st; i++) st = crt_group_run(b->ctx, i ? b->side : main, b->groups[i]);
+        if (fork) {
             CK(cuda_check(cudaEventRecord(b->join, b->side), "batch join"));
             CK(cuda_check(cudaStreamWaitEvent(main, b->join, 0), "batch join"));
         }

@@ -26,7 +26,9 @@
  * at a time; calls are asynchronous on the context's current stream (hc_context_set_stream), and
  * calls issued on different streams of one context may run concurrently on the GPU. Some calls
  * (hc_bfv_hom_mul, hc_dbfv_hom_mul) run independent parts on the ring's side stream, forked from and joined back
- * into the current stream, which a CUDA-graph capture of the call records as parallel paths.
+ * into the current stream, which a CUDA-graph capture of the call records as parallel paths. Other threads
+ * issue on the context meanwhile only between such calls, as these make the side stream current for a while;
+ * running a batch (hc_crt_batch_run, one thread at a time per batch) leaves the context's stream alone.
  */
 #ifndef RINGCUDA_H
 #define RINGCUDA_H
