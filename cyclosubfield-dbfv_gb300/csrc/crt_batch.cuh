@@ -120,7 +120,7 @@ template <bool GENERIC, int CLS, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
     crt_batch_kernel(const CrtSlab* __restrict__ slabs, int nslabs, int* counter, int logv, int tile_words) {
     grid_wait();
-    extern __shared__ int64_t smem[];
+    extern __shared__ __align__(16) int64_t smem[];
     __shared__ int s_next;
     for (;;) {
         __syncthreads();  // every thread has read s_next and left the previous slab's tiles

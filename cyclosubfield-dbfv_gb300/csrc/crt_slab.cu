@@ -53,7 +53,7 @@ template <int MODE, int THREADS>
 __global__ void __launch_bounds__(THREADS, 768 / THREADS)
     block4096_kernel(KView t, PlanPtrs p3, const BarrettLimbs* m3, KView pm, KMods mods) {
     grid_wait();
-    extern __shared__ int64_t smem[];
+    extern __shared__ __align__(16) int64_t smem[];
     const int64_t tile = blockIdx.x / 3;
     const int blk = (int)(blockIdx.x % 3);
     const int64_t k = tile % t.n2, r = tile / t.n2;

@@ -62,7 +62,7 @@ static_assert(sizeof(DevStage) % 8 == 0 && sizeof(DevPass) % 8 == 0, "staged in 
 
 __global__ void __launch_bounds__(256) crt_small_kernel(SmallArgs a, KMods mods) {
     grid_wait();
-    extern __shared__ int64_t smem[];
+    extern __shared__ __align__(16) int64_t smem[];
     const int dl = (int)a.t.n2, dk = (int)a.t.n3, total = dl * dk;
     const int64_t j = blockIdx.x % a.t.n1, i = blockIdx.x / a.t.n1;
     int64_t* s = smem;

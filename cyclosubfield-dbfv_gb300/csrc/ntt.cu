@@ -96,7 +96,7 @@ namespace {
 __global__ void __launch_bounds__(256, HC_NTT_MIN_BLOCKS) ntt_tile_kernel(KView t, PlanPtrs plans, int dim, int mode, KView mul,
                                                        KMods mods, int logv, int ntile2, int use_smem) {
     grid_wait();
-    extern __shared__ int64_t smem[];
+    extern __shared__ __align__(16) int64_t smem[];
     const int V = 1 << logv;
     const int len = dim == 3 ? (int)t.n3 : (int)t.n2;
     int64_t tile = blockIdx.x;

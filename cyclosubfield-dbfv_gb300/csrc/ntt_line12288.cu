@@ -11,7 +11,7 @@ template <int MODE, bool FIX, int THREADS>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(THREADS, 768 / THREADS)
     ntt_line3_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
     grid_wait();
-    extern __shared__ int64_t smem[];
+    extern __shared__ __align__(16) int64_t smem[];
     const int64_t tile = blockIdx.x / 3;
     const int blk = (int)(blockIdx.x % 3);
     const int64_t k = tile % t.n2, r = tile / t.n2;

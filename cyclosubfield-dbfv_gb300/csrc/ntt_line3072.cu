@@ -7,7 +7,7 @@ namespace {
 template <int MODE, bool FIX, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) ntt_line_kernel(KView t, PlanPtrs plans, KView mul, KMods mods) {
     grid_wait();
-    extern __shared__ int64_t smem[];
+    extern __shared__ __align__(16) int64_t smem[];
     const int64_t tile = blockIdx.x;
     const int64_t k = tile % t.n2, r = tile / t.n2;
     const int64_t j = r % t.n1, i = r / t.n1;

@@ -93,6 +93,7 @@ namespace {
 /// Shared-memory words of a 3072-residue line, and of a 4096-residue block of a 12288-residue one: the
 /// tile, then its staged twiddles.
 constexpr int LINE3072_WORDS = 3072 + fast::staged_words(7), BLOCK4096_WORDS = 4096 + fast::staged_words(63);
+static_assert(LINE3072_WORDS % 2 == 0 && BLOCK4096_WORDS % 2 == 0, "staged twiddles are read 16 bytes at a time");
 
 /// Contexts of a plan: its twiddles are read from global memory (L1-cached).
 template <class CTX>

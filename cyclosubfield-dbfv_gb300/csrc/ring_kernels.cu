@@ -244,7 +244,7 @@ __device__ __noinline__ int64_t finish_any(uint64_t lo, int64_t hi, bool full, i
 __global__ void __launch_bounds__(BCONV_THREADS) dbfv_split_kernel(KView x, KView src, KView carry, DbfvSplit d, int r,
                                                                    KMods m, int64_t npos) {
     grid_wait();
-    extern __shared__ int64_t sx[];  // [r][BCONV_THREADS]
+    extern __shared__ __align__(16) int64_t sx[];  // [r][BCONV_THREADS]
     const int64_t pos = (int64_t)blockIdx.x * BCONV_THREADS + threadIdx.x;
     if (pos >= npos) return;
     const int64_t i = blockIdx.y, k = pos / x.n3, l = pos - k * x.n3;
@@ -767,7 +767,7 @@ template <int NOUT>
 __global__ void __launch_bounds__(256, NOUT <= 2 ? 4 : 3) giant_kernel(const __grid_constant__ GiantArgs a, GiantUnits un, KMods m, const int64_t* one,
                                                              int64_t lines, int chunks) {
     grid_wait();
-    extern __shared__ int64_t gsm[];  // [GIANT_STAGES][2][256] staging, then the tile's lcoef as limb pairs
+    extern __shared__ __align__(16) int64_t gsm[];  // [GIANT_STAGES][2][256] staging, then the tile's lcoef as limb pairs
     int2* slc = reinterpret_cast<int2*>(gsm + GIANT_STAGES * 2 * 256);
     const int64_t tiles = lines * chunks;
     const int nt = (int)a.lcoef.n0;

@@ -31,3 +31,10 @@ def test_side_branches_join_before_their_tensors_go():
     assert len(bodies) >= 4
     for name, body in bodies:
         assert not re.search(r"\n        Tensor \w+ *=", body), (name, body)
+
+
+@pytest.mark.parametrize("path", CSRC, ids=os.path.basename)
+def test_dynamic_shared_memory_is_aligned_for_its_widest_access(path):
+    """Tiles of words hold twiddles and position pairs that are read 16 bytes at a time; a static variable may lie in front."""
+    for decl in re.findall(r"extern __shared__ ([^;]*);", source(path)):
+        assert "int64_t" not in decl or "__align__(16)" in decl, decl
