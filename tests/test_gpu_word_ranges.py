@@ -228,3 +228,60 @@ def test_matmul_of_one_sign_and_mixed_chunks(be, po, cols, rows, l):
         exp = np.zeros_like(got)
         po.matmul_i64(exp, np.ascontiguousarray(lhs), np.ascontiguousarray(rhs))
         assert (got == exp).all()
+
+
+@pytest.mark.parametrize("nd", [14, 15, 16, 28, 29, 41])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_key_switch_sums_of_one_sign(po, rings, nd, sign):
+    """Every digit word at factor j the same, near p / 2 with its low limb full, times keys at the limb sums' edge: unfolded,
+    the middle column overflows from 26 digits. The integer 1 has the period-basis coefficients -1, so the element with
+    coefficients -v is v at every position, and v's lift, small beside every digit, is each digit's value."""
+    import ringcuda
+
+    o, d = rings("field_192", 2300, 2340, 4)
+    base = o.initial_base()
+    primes = [o.primes[i] for i in base]
+    j = min(range(len(base)), key=lambda i: primes[i])
+    p = primes[j]
+    x = sign * ((((p // 2) >> 29) << 29) - 1)
+    v = x * pow(2, -64, p) % p
+    v -= p if 2 * v > p else 0
+    c1 = np.empty(o.shape(1, len(base)), dtype=np.int64)
+    for i, q in enumerate(primes):
+        w = -v * (1 << 64) % q
+        c1[:, i] = w - q if 2 * w > q else w
+    digits = [tuple(s) for s in ringcuda.select_digits(nd, len(base))]
+    parts = o.pb_to_crt(o.bconv_gadget(c1, base, digits), base)
+    assert (parts[:, j] == x).all()
+    g = np.random.default_rng(nd)
+    c0 = words(g, o.shape(1, len(base)), primes, 1)
+    for key in ((1 << 58) - 1, -(1 << 58), 1 << 58):
+        k = np.full(o.shape(2 * nd, len(base)), key, dtype=np.int64)
+        exp = o.key_switch(c0, c1, base, k.reshape((nd, 2) + k.shape[1:]), digits)
+        assert (d.key_switch(d.tensor(c0), d.tensor(c1), base, d.tensor(k), digits).to_numpy() == exp).all()
+
+
+@pytest.mark.parametrize("log2_t,dct", [(4, 1), (8, 2), (12, 3), (16, 4), (20, 5)])
+def test_giant_steps_of_many_baby_steps(rings, log2_t, dct):
+    """17 baby steps, more than the sums of any number of output digits hold before they fold (14, 7, 4, 3 steps)."""
+    import ringcuda
+
+    o, d = rings("field_18", 560, 572, 4)
+    base = o.initial_base()[:4]
+    primes = [o.primes[i] for i in base]
+    digits = [tuple(v) for v in ringcuda.select_digits(2, len(base))]
+    nd, full, length = len(digits), o.initial_len, 100
+    gen, m = list(o.info["gens"])[0], o.info["m"]
+    baby = min(range(1, length + 1), key=lambda c: (c + 3 * ((length - 1) // c + 1), c))
+    assert baby == 17
+    g = np.random.default_rng(log2_t)
+    gks, ks = {}, ringcuda.Keyset(d, digits, full, 1 << 40)
+    for e in sorted({pow(gen, j, m) for j in range(1, baby + 1)}):
+        k = words(g, o.shape(2 * nd, full), o.primes[:full], 1)
+        gks[e] = k.reshape((nd, 2) + k.shape[1:])
+        ks.add(e, d.tensor(k))
+    coeffs = [[int(v) for v in g.integers((1 << log2_t) // 4, 1 << log2_t, size=o.dl)] for _ in range(length)]
+    ct = words(g, o.shape(2 * dct, len(base)), primes, 1)
+    exp = o.dbfv_hom_cyclic_transform(4, log2_t, gen, coeffs, ct, base, gks, digits)
+    got = ringcuda.dbfv_hom_cyclic_transform(d, 4, log2_t, gen, coeffs, d.tensor(ct), base, ks).to_numpy()
+    assert got.shape == exp.shape and (got == exp).all()
