@@ -1129,21 +1129,7 @@ struct Wide {
         accumulate(rs, re, src, R->scalar_tensor(base, 1).view());
         step(rs, re, sb * mp2());
     }
-    /// lhs any i64 tensor, rhs bounded by max_p (src/ring.rs:488-493)
-    void fma_unbounded(size_t rs, size_t re, const hc_view& l, const hc_view& r) {
-        accumulate(rs, re, l, r);
-        step(rs, re, (u128)maxp << 63);
-    }
     bool full(size_t row) const { return bound[row] > ((u128)minp << 63); }
-    /// wide[rs..re) = sum_t lhs_t * rhs_t (fresh rows only; src/ring.rs:460-485), all operands
-    /// almost reduced (bound 1)
-    void inner_product(size_t rs, size_t re, const std::vector<hc_view>& lhs, const std::vector<hc_view>& rhs) {
-        for (size_t i = rs; i < re; i++) REQUIRE(bound[i] == 0, HC_ERR_ARG, "inner product into a used row");
-        REQUIRE(!lhs.empty() && lhs.size() == rhs.size(), HC_ERR_ARG, "inner product terms");
-        CK(hc_inner_product_i64(R->ctx, vrows(data.view(), (int64_t)rs, (int64_t)re, true), lhs.data(), rhs.data(),
-                                lhs.size()));
-        step(rs, re, (u128)lhs.size() * mp2());
-    }
     void reduce_into(const hc_view& dst) { reduce_rows_into(dst, bound.size()); }
     /// reduces rows [0, rows) into dst (src/ring.rs:846-865)
     void reduce_rows_into(const hc_view& dst, size_t rows) {
@@ -2736,13 +2722,6 @@ Tensor scalar_tensor_big_mont2(hc_ring R, const Base& b, const std::function<int
     Tensor t(R->ctx, 1, (int64_t)b.size(), 1, 1);
     CK(hc_import(R->ctx, t.view(), v.data(), v.size()));
     return t;
-}
-
-/// rows [s, e) of dimension 1
-hc_view dim1(hc_view v, int64_t s, int64_t e) {
-    v.ptr = (char*)v.ptr + s * v.strides[1] * 8;
-    v.shape[1] = e - s;
-    return v;
 }
 
 /// SplitOverflowData (src/dbfv.rs:735-849)
