@@ -240,8 +240,9 @@ struct __align__(16) BarrettMod {
 /// signed fraction that the rounding cut off, and x1 e1 - F n1 (F: the leading 32 bits of f) misses
 /// that by less than 2^31 - at most 2^30 for n0, 0.9 x 2^30 for e0, 2^25 for F's cut-off and 2^23 for
 /// e x0 - so that it and the low word name one integer.
-/// Five wide products and three low ones, 27.6 cycles of the multiply pipe against 34 of bmul, and 14
-/// instructions against 31: register-only butterflies run at 1209 G/s against 765 G/s.
+/// Five wide products and three low ones, 27.6 cycles of the multiply pipe by count against 34 of bmul, and 14
+/// instructions against 31: register-only chains run at 1367 G/s against 861 G/s (29.5 and 46.8 cycles per product),
+/// butterflies at 1209 against 765.
 __device__ __forceinline__ int64_t barrett_mul(const BarrettLimbs& w, int64_t x, const BarrettMod& m) {
     const int32_t x0 = (int32_t)lo32(x), x1 = bal_hi(x);
     const int64_t a = wadd(mad_wide(w.u1, x0, (int64_t)w.u0 * x1), __mulhi(w.u0, x0));
@@ -443,7 +444,7 @@ hc_status ntt_kernel_dim(hc_context ctx, hc_view dst, const hc_view* src, const 
 /// kernel<<<grid, block, smem, stream>>>(args...), placed on the SMs as soon as the CTAs of the stream's previous
 /// kernel have exited instead of after that kernel's completion has come back through the queue: the calls
 /// here are chains of 3 to 80 short dependent launches (two transforms and a product of one field_36864 element at r = 16 72 ->
-/// 52 us, a ct-mult at r = 5 215 -> 173, the homomorphic CRT step 5.25 -> 5.05 ms). No kernel lets its
+/// 52 us, a ct-mult at r = 5 215 -> 171, the homomorphic CRT step 5.25 -> 4.91 ms). No kernel lets its
 /// successor start earlier (griddepcontrol.launch_dependents): waiting CTAs then hold slots that the rest
 /// of the kernel and the ring's other stream use (64 us, 191 us, 5.13 ms; for grids of up to 608 or 2000 CTAs only 64, 195, 5.25).
 template <class... P, class... A>

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         const DevPlanHeader* P3 = reinterpret_cast<const DevPlanHeader*>(S.plan3);
         int64_t* tw2 = smem + tile_words;
         int64_t* tw3 = tw2 + 2 * P2->ntw;
-        if constexpr (GENERIC) {  // the specialised passes read theirs from the plan (L1-cached)
+        if constexpr (GENERIC) {  // the specialised passes stage theirs with each tile
             stage_twiddles(P2, tw2);
             stage_twiddles(P3, tw3);
             __syncthreads();
