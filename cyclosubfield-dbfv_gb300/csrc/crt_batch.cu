@@ -43,7 +43,7 @@ int crt_slab_kernel_class(int32_t shapes) { return (shapes & 0xff) == HC_SHAPE_L
 hc_status launch_crt_batch(hc_context ctx, cudaStream_t stream, const CrtSlab* slabs, int nslabs, int* counter, size_t tile_words,
                            size_t tw_words, const CrtLaunch& L, bool generic, int cls) {
     if (nslabs <= 0) return HC_OK;
-    CrtBatchKernel kern = generic    ? crt_batch_kernel<true, 0, 256, 2>
+    CrtBatchKernel kern = generic    ? (cls == 3 ? crt_batch_kernel<true, 3, 256, 2> : crt_batch_kernel<true, 0, 256, 2>)
                           : cls == 1 ? crt_batch_f36864(L.ctas_per_sm)
                           : cls == 2 ? crt_batch_f49152(L.ctas_per_sm)
                                      : crt_batch_mixed(L.ctas_per_sm);

@@ -60,13 +60,13 @@ __device__ __forceinline__ void slab_lines3072(const CrtSlab& S, const DevPlanHe
 /// column blocks of 2^logv columns (dimension 2). Modes as tile_run; `mulrow` is the CRT kernel
 /// row of the pass (modes 2 and 3 along dimension 2, mode 2 along dimension 3), while mode 3
 /// along dimension 3 multiplies by the slab's operand.
-template <bool GENERIC>
+template <bool GENERIC, int CLS>
 __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader* P, const int64_t* tw, int64_t* s,
                                           int dim, int mode, const int64_t* mulrow, int logv) {
     // specialised kernels for slabs whose plans are fixed (bit 16: dimension-3 plan, bit 17: dimension-2
     // plan), the generic tile programme otherwise
     const int shape = dim == 3 ? (S.shapes & 0xff) : ((S.shapes >> 8) & 0xff);
-    const bool fix = (S.shapes >> (dim == 3 ? 16 : 17)) & 1;
+    const bool fix = CLS != 3 && ((S.shapes >> (dim == 3 ? 16 : 17)) & 1);
     if (fix && dim == 3 && shape == HC_SHAPE_L3072) {
         if (mode == 2) slab_lines3072<6>(S, P, s, mulrow);
         else if (mode == 3) slab_lines3072<11>(S, P, s, mulrow);
@@ -114,8 +114,9 @@ __device__ __forceinline__ void slab_pass(const CrtSlab& S, const DevPlanHeader*
 /// schedules (both large fields' rings), so the generic tile programme is left out; MINB: the CTAs
 /// of MAXT threads per SM the register allocation must allow (256 threads: 2 -> 128 registers,
 /// 3 -> 80, 4 -> 64 with some spilling), chosen through the autotuned launch shape. GENERIC = true serves other slabs. CLS: the slabs' shape class - 1 every slab has
-/// field_36864's [4, 3] x [2, 3, 8, 64] shapes, 2 field_49152's [4] x [3, 64, 64], 0 any - so that
-/// a launch carries only its class's code.
+/// field_36864's [4, 3] x [2, 3, 8, 64] shapes, 2 field_49152's [4] x [3, 64, 64], 3 none with a specialised
+/// dimension, 0 any - so that a launch carries only its class's code (pb_to_crt of four field_18 elements 22.7 us
+/// with all of it, 18.5 as class 3).
 template <bool GENERIC, int CLS, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
     crt_batch_kernel(const CrtSlab* __restrict__ slabs, int nslabs, int* counter, int logv, int tile_words) {
@@ -142,11 +143,12 @@ __global__ void __launch_bounds__(MAXT, MINB)
         const bool slab12288 = CLS == 2 || (CLS == 0 && crt_slab_12288(S.shapes));
         auto half = [&](auto mode3, int mode2, const int64_t* kl, const int64_t* kk) {
             constexpr int M = decltype(mode3)::value;
-            if (CLS != 1 && slab12288) {
-                slab12288_half<M == 2 ? 6 : M == 3 ? 11 : M>(S, P2, P3, smem, kl, kk);
-            } else if constexpr (CLS != 2) {
-                slab_pass<GENERIC>(S, P2, tw2, smem, 2, mode2, kl, logv);
-                slab_pass<GENERIC>(S, P3, tw3, smem, 3, M, kk, logv);
+            if constexpr (CLS == 0 || CLS == 2) {
+                if (slab12288) return slab12288_half<M == 2 ? 6 : M == 3 ? 11 : M>(S, P2, P3, smem, kl, kk);
+            }
+            if constexpr (CLS != 2) {
+                slab_pass<GENERIC, CLS>(S, P2, tw2, smem, 2, mode2, kl, logv);
+                slab_pass<GENERIC, CLS>(S, P3, tw3, smem, 3, M, kk, logv);
             }
         };
         if (S.ops & HC_CRT_FORWARD) {

@@ -2020,10 +2020,15 @@ bool crt_generic(const std::vector<CrtSlab>& slabs) {
     return false;
 }
 
-/// The kernel class of a group's specialised slabs: their shape class when they all share one,
-/// else 0 (the kernel that carries both classes' code).
+/// The kernel class of a group's slabs: the specialised ones' shape class when they all share one, 3 where no slab
+/// has a specialised dimension, else 0 (the kernel that carries all classes' code).
 int crt_group_kernel_class(const CrtGroup& g) {
     if (g.host.empty()) return 0;
+    if (crt_generic(g.host)) {
+        for (const CrtSlab& s : g.host)
+            if (crt_slab_limbs(s.shapes, 2) || crt_slab_limbs(s.shapes, 3)) return 0;
+        return 3;
+    }
     const int c = crt_slab_kernel_class(g.host[0].shapes);
     for (const CrtSlab& s : g.host)
         if (crt_slab_kernel_class(s.shapes) != c) return 0;
@@ -2035,7 +2040,7 @@ hc_status crt_group_run(hc_context ctx, cudaStream_t stream, CrtGroup& g) {
     for (const CrtSlab& s : g.host) tile = std::max(tile, crt_tile_words(s, g.launch.logv));
     const bool generic = crt_generic(g.host);
     return launch_crt_batch(ctx, stream, g.dev.as<CrtSlab>(), (int)g.host.size(), g.counter.as<int>(), tile, g.tw_words,
-                            g.launch, generic, generic ? 0 : crt_group_kernel_class(g));
+                            g.launch, generic, crt_group_kernel_class(g));
 }
 
 /// Times every launch shape of the candidate set on a scratch copy of a sample of the group's
@@ -2068,7 +2073,7 @@ hc_status crt_group_tune(hc_context ctx, CrtGroup& g, int reps) {
     CrtLaunch best = g.launch;
     float best_ms = -1;
     const bool generic = crt_generic(g.host);
-    const int cls = generic ? 0 : crt_group_kernel_class(g);
+    const int cls = crt_group_kernel_class(g);
     // 128 or 256 threads at 1..4 CTAs per SM
     const CrtLaunch shapes[] = {{128, 1, 0}, {128, 2, 0}, {128, 3, 0}, {128, 4, 0},
                                 {256, 1, 0}, {256, 2, 0}, {256, 3, 0}, {256, 4, 0}};
