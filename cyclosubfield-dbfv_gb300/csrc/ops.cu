@@ -250,30 +250,38 @@ __global__ void __launch_bounds__(256) inner_product_kernel(KView d, Terms terms
     }
 }
 
-/// inner_product_kernel over the line grid of pw_line_kernel.
+/// inner_product_kernel over the line grid of pw_line_kernel. FULL: the CTA's span lies within the line; a
+/// shorter line's threads read only what they store (repeating its last position instead, 100 x 8 x 2 lines of 96
+/// positions took 36.0 us for twelve terms, 31.5 this way), at the price of reads that wait for their own test.
+template <bool FULL>
+__device__ __forceinline__ void inner_product_span(const KView& d, const Terms& terms, int i, int j, int k, int64_t l0) {
+    auto in = [&](int s) { return FULL || l0 + 256 * s + threadIdx.x < d.n3; };
+    i128 acc[LINE_STEPS];
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++) acc[s] = 0;
+    for (int t = 0; t < terms.n; t++) {
+        int64_t x[LINE_STEPS] = {}, y[LINE_STEPS] = {};
+#pragma unroll
+        for (int s = 0; s < LINE_STEPS; s++)
+            if (in(s)) {
+                x[s] = *kat<int64_t>(terms.l[t], i, j, k, l0 + 256 * s + threadIdx.x);
+                y[s] = *kat<int64_t>(terms.r[t], i, j, k, l0 + 256 * s + threadIdx.x);
+            }
+#pragma unroll
+        for (int s = 0; s < LINE_STEPS; s++) acc[s] = (i128)((u128)acc[s] + (u128)((i128)x[s] * (i128)y[s]));
+    }
+#pragma unroll
+    for (int s = 0; s < LINE_STEPS; s++)
+        if (in(s)) st128(kat<longlong2>(d, i, j, k, l0 + 256 * s + threadIdx.x), acc[s]);
+}
 __global__ void __launch_bounds__(256) inner_product_line_kernel(KView d, Terms terms) {
     grid_wait();
     const int line = (int)blockIdx.y;
     const int k = line % (int)d.n2, r = line / (int)d.n2;
     const int j = r % (int)d.n1, i = r / (int)d.n1;
     const int64_t l0 = (int64_t)blockIdx.x * LINE_SPAN;
-    i128 acc[LINE_STEPS];
-#pragma unroll
-    for (int s = 0; s < LINE_STEPS; s++) acc[s] = 0;
-    for (int t = 0; t < terms.n; t++) {
-        int64_t x[LINE_STEPS], y[LINE_STEPS];
-#pragma unroll
-        for (int s = 0; s < LINE_STEPS; s++) {
-            // positions past the line's end repeat its last one
-            const int64_t l = min(l0 + 256 * s + threadIdx.x, d.n3 - 1);
-            x[s] = *kat<int64_t>(terms.l[t], i, j, k, l), y[s] = *kat<int64_t>(terms.r[t], i, j, k, l);
-        }
-#pragma unroll
-        for (int s = 0; s < LINE_STEPS; s++) acc[s] = (i128)((u128)acc[s] + (u128)((i128)x[s] * (i128)y[s]));
-    }
-#pragma unroll
-    for (int s = 0; s < LINE_STEPS; s++)
-        if (l0 + 256 * s + threadIdx.x < d.n3) st128(kat<longlong2>(d, i, j, k, l0 + 256 * s + threadIdx.x), acc[s]);
+    if (l0 + LINE_SPAN <= d.n3) inner_product_span<true>(d, terms, i, j, k, l0);
+    else inner_product_span<false>(d, terms, i, j, k, l0);
 }
 
 /// dst[i,j,k,l] += red(((lhs[i,0,k,l] + 2^(shift-1)) >> shift) * rhs[ri,j,0,0])
