@@ -42,6 +42,7 @@ struct BconvMatrix {
     int2 m[N];
 };
 typedef BconvMatrix<1152> BconvParam;
+typedef BconvMatrix<96> BconvSmall;  // a launch copies its parameters: two field_18 rows 7.9 us with these, 8.2 with all
 typedef BconvMatrix<1> BconvMemory;
 
 constexpr int LIMB_UNROLL = 16;  // terms unrolled together
@@ -1021,11 +1022,13 @@ hc_status launch_bconv_fused(hc_context ctx, const KView& src, const KView& dst,
         count_launch(ctx);
         return cuda_check(cudaGetLastError(), "bconv kernel launch");
     };
-    if (one_chunk && c.hwords > 0 && c.hwords <= BconvParam::ENTRIES) {
-        BconvParam mx;
+    auto param = [&](auto mx) {
+        typedef decltype(mx) MAT;
         std::memcpy(mx.m, c.hmat, (size_t)c.hwords * sizeof(int2));
-        return sub ? run(bconv_fused_kernel<true, true, BconvParam>, mx) : run(bconv_fused_kernel<true, false, BconvParam>, mx);
-    }
+        return sub ? run(bconv_fused_kernel<true, true, MAT>, mx) : run(bconv_fused_kernel<true, false, MAT>, mx);
+    };
+    if (one_chunk && c.hwords > 0 && c.hwords <= BconvSmall::ENTRIES) return param(BconvSmall());
+    if (one_chunk && c.hwords > 0 && c.hwords <= BconvParam::ENTRIES) return param(BconvParam());
     const BconvMemory none{};
     if (one_chunk)
         return sub ? run(bconv_fused_kernel<true, true, BconvMemory>, none)
