@@ -50,7 +50,7 @@ hc_status launch_as(hc_context ctx, const KView& t, const PlanPtrs& pp, const KV
 /// per SM), where a line's own latency is the launch's.
 template <int MODE, bool FIX>
 hc_status launch(hc_context ctx, const KView& t, const PlanPtrs& pp, const KView& mul, const KMods& mods, int64_t tiles) {
-    if (tiles <= hc::num_sms(ctx)) return launch_as<MODE, FIX, 256>(ctx, t, pp, mul, mods, tiles);
+    if (!FIX || tiles <= hc::num_sms(ctx)) return launch_as<MODE, FIX, 256>(ctx, t, pp, mul, mods, tiles);
     return launch_as<MODE, FIX, 128>(ctx, t, pp, mul, mods, tiles);
 }
 
